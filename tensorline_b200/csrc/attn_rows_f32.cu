@@ -1,0 +1,457 @@
+// Exact-order paged attention of the 32-bit engine, the same floats as attn_tokenwise.cu gives: per (token, query head) tiles of
+// 32 keys aligned to absolute position 0 in ascending order, every dot product one chain of fmaf over the head's dimensions, the
+// softmax's sums over the 32 keys of a tile in the order of a warp's shuffles, every output element one chain of fmaf over the
+// keys.  What the token-wise kernel spends its time on is fetching every key anew for every token and head, one row a lane; here
+// the rows (token, head) that read the same keys share them through shared memory, and a step of few tokens has its dot products
+// taken by as many blocks as there are tiles.
+//
+//   attn_rows       a block has up to 64 rows: neighbouring tokens of one request times the query heads of one KV head.  128
+//                   threads; a warp owns 16 rows from the dot products (4 x 4 outputs a lane) over the softmax (half a row a
+//                   lane) to the values (8 rows x 4 NC columns a lane), so between tiles only the tiles themselves are waited
+//                   for: K of the next tile arrives while the values are summed, V of it while the dot products are taken.
+//                   A tile costs 2 x 64 x 32 x d multiply-adds; FMA-bound.
+//   attn_dots, attn_chain   steps of few tokens: the chains over the keys are all that is left in order.  attn_dots: a thread
+//                   a key, all tiles at once, scores to memory; attn_chain: a warp a head and 32 output columns, the softmax of
+//                   128 keys at a time and then their chain.
+// Measured with 28 query heads of 128 on 4 KV heads: 333 tokens on 700 cached 350 us (the token-wise kernel 5,076), 2,048 tokens
+// 1.32 ms (33.4); single tokens at position 1,800: 4 of them 56 us (1,842; attn_rows 478), 64 of them 265 us (3,577; 611).
+// Masks, sinks, gates, caps and slopes: as described in attn_tokenwise.cu.  A sink's term joins the sum with a rounding of its own,
+// the same in both kernels here.
+#include "common.cuh"
+
+struct RowsArgs {
+    const float* q; int q_stride; float* out;
+    const float* k_pages; const float* v_pages;
+    const int* table; int max_pages; int page_size;
+    const int* pos; const int* req_slot;
+    int T, nq, nkv, d, window; float scale;
+    const float* sink; int keep_first; const float* gate;
+    int chunk; const float* slopes; float cap;
+    float* scores; int keys;               // attn_dots / attn_chain: [T, nq, keys]
+    int tq;                                // attn_rows: tokens a block
+    TlLimits L;
+};
+
+__device__ __forceinline__ void rows_copy16(float* dst, const float* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+#define ROWS_COMMIT() asm volatile("cp.async.commit_group;" ::: "memory")
+#define ROWS_WAIT(n) asm volatile("cp.async.wait_group %0;" ::"n"(n) : "memory")
+
+__device__ __forceinline__ void rows_fma2(float& d0, float& d1, float a, float b0, float b1) {       // (d0, d1) += a (b0, b1)
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%0, %1};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(d0), "+f"(d1) : "f"(a), "f"(b0), "f"(b1));
+}
+
+__device__ __forceinline__ int rows_low(const RowsArgs& A, int p) {
+    return A.chunk > 0 ? (p / A.chunk) * A.chunk : (A.window > 0 && p - A.window + 1 > 0) ? p - A.window + 1 : 0;
+}
+__device__ __forceinline__ const float* rows_at(const RowsArgs& A, const float* pages, const int* tab, int j, int kh) {
+    const int page = tl_checked(tab[tl_checked(j / A.page_size, A.max_pages, A.L, TL_K_TOKENWISE)], A.L.total_pages, A.L, TL_K_TOKENWISE);
+    return pages + (((size_t)page * A.nkv + kh) * A.page_size + (j % A.page_size)) * A.d;
+}
+__device__ __forceinline__ float rows_score(const RowsArgs& A, float dot, float slope, int p, int j) {
+    float s = __fmul_rn(dot, A.scale);                   // spelt out: the same roundings in every kernel
+    if (A.cap > 0.f) s = __fmul_rn(A.cap, tanhf(s / A.cap));
+    if (A.slopes) s = fmaf(-slope, (float)(p - j), s);
+    return s;
+}
+// The sink joins a finished row: (its sum with the sink, what the row's values are multiplied by).  One copy for both kernels.
+__device__ __noinline__ float2 rows_sink(float m, float l, float sink) {
+    const float m_new = fmaxf(m, sink);
+    const float alpha = expf(m - m_new);
+    return make_float2(l * alpha + expf(sink - m_new), alpha);
+}
+
+constexpr int ROWS_MAX = 64, ROWS_PS = ROWS_MAX + 4;     // rows a block, and the stride of a key's scores in shared memory
+
+// NC: groups of 64 output columns (d <= 64 NC)
+template <int NC>
+__global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
+    extern __shared__ __align__(16) float sm[];
+    const int d = A.d, g = A.nq / A.nkv, ld = d + 4;
+    float* Qs = sm;                                      // [64][ld], rows beyond the block's last are zeros
+    float* Ks = Qs + ROWS_MAX * ld;                      // [32][ld]
+    float* Vs = Ks + 32 * ld;                            // [32][ld]
+    float* Ps = Vs + 32 * ld;                            // [32 keys][ROWS_PS rows]: dot products, then weights
+    float* al = Ps + 32 * ROWS_PS;                       // [64]
+    const int kh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    // the block's run: the blockIdx.z-th maximal range of tokens of one request among its tq tokens (tq <= 32)
+    const int tb = blockIdx.x * A.tq, te = min(A.T, tb + A.tq);
+    unsigned starts;
+    {
+        const int t = tb + lane;
+        starts = __ballot_sync(0xffffffffu, t < te && (lane == 0 || A.req_slot[t] != A.req_slot[t - 1]));
+    }
+    if ((int)blockIdx.z >= __popc(starts)) return;
+    for (unsigned i = 0; i < blockIdx.z; ++i) starts &= starts - 1;
+    const int first = __ffs(starts) - 1;
+    starts &= starts - 1;
+    const int n = (starts ? __ffs(starts) - 1 : te - tb) - first, t0 = tb + first, rows = n * g;
+    const int* tab = A.table + (size_t)tl_checked(A.req_slot[t0], A.L.table_rows, A.L, TL_K_TOKENWISE) * A.max_pages;
+    for (int i = tid; i < ROWS_MAX * d; i += 128) {
+        const int r = i / d, e = i - r * d;
+        Qs[r * ld + e] = r < rows ? A.q[(size_t)(t0 + r / g) * A.q_stride + (size_t)(kh * g + r % g) * d + e] : 0.f;
+    }
+    // the softmax's row of this lane: 16 rows a warp, a lane and its neighbour 16 further on share a row, 16 keys each
+    const int row = wid * 16 + (lane & 15), kb = lane & 16;
+    const bool live = row < rows;
+    const int p = live ? A.pos[t0 + row / g] : -1, head = kh * g + row % g;
+    const int lo = live ? rows_low(A, p) : 0, kept = min(A.keep_first, lo);
+    const float slope = A.slopes && live ? A.slopes[head] : 0.f;
+    float m = -INFINITY, l = 0.f;
+    int last = -1, low = 0x7fffffff, keep = 0;           // of all the run's tokens
+    for (int i = 0; i < n; ++i) {
+        const int pi = A.pos[t0 + i], li = rows_low(A, pi);
+        last = max(last, pi); low = min(low, li); keep = max(keep, min(A.keep_first, li));
+    }
+    auto next = [&](int j0) { return (j0 >= keep && j0 + 32 <= low) ? (low / 32) * 32 : j0; };
+    auto fetch = [&](float* dst, const float* pages, int j0) {       // four threads a key; keys that no row sees are not read
+        const int j = j0 + (tid >> 2);
+        if (j <= last && (j >= low || j < keep)) {
+            const float* src = rows_at(A, pages, tab, j, kh);
+            for (int e = (tid & 3) * 4; e < d; e += 16) rows_copy16(dst + (tid >> 2) * ld + e, src + e);
+        }
+        ROWS_COMMIT();
+    };
+    float acc[8][4 * NC];
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < 4 * NC; ++c) acc[r][c] = 0.f;
+    const int kl = lane & 7, rl = lane >> 3;             // dot products: keys kl + 8 j, rows 16 wid + 4 i + rl
+    const int dg = (lane & 15) * 4, rg = wid * 16 + (lane >> 4) * 8;      // values: columns dg + 64 c, rows rg ..
+    int j0 = next(0);
+    fetch(Ks, A.k_pages, j0);
+    fetch(Vs, A.v_pages, j0);
+    while (j0 <= last) {
+        const int j1 = next(j0 + 32);
+        ROWS_WAIT(1);
+        __syncthreads();
+        {
+            float s[4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+            const float* qp = Qs + (wid * 16 + rl) * ld;
+            const float* kp = Ks + kl * ld;
+#pragma unroll 2
+            for (int e = 0; e < d; e += 4) {
+                float4 q4[4], k4[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + 4 * i * ld + e);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(kp + 8 * j * ld + e);
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        s[i][j] = fmaf(q4[i].x, k4[j].x, s[i][j]);
+                        s[i][j] = fmaf(q4[i].y, k4[j].y, s[i][j]);
+                        s[i][j] = fmaf(q4[i].z, k4[j].z, s[i][j]);
+                        s[i][j] = fmaf(q4[i].w, k4[j].w, s[i][j]);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) Ps[(kl + 8 * j) * ROWS_PS + wid * 16 + 4 * i + rl] = s[i][j];
+        }
+        __syncthreads();                                 // K is read; a warp's scores are its own
+        if (j1 <= last) fetch(Ks, A.k_pages, j1); else ROWS_COMMIT();
+        bool full;
+        {
+            float s[16];
+            float top = -INFINITY;
+            int valid = 0;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int j = j0 + kb + i;
+                s[i] = -INFINITY;
+                if ((j >= lo || j < kept) && j <= p) {
+                    s[i] = rows_score(A, Ps[(kb + i) * ROWS_PS + row], slope, p, j);
+                    ++valid;
+                }
+                top = fmaxf(top, s[i]);
+            }
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
+            const int any = valid + __shfl_xor_sync(0xffffffffu, valid, 16);
+            const float m_new = fmaxf(m, top);
+            const float alpha = any ? expf(m - m_new) : 1.0f;        // a row without keys in this tile stays as it is
+            bool nonzero = true;
+            float sum[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int j = j0 + kb + i;
+                const float pj = ((j >= lo || j < kept) && j <= p) ? expf(s[i] - m_new) : 0.f;
+                Ps[(kb + i) * ROWS_PS + row] = pj;
+                nonzero = nonzero && pj != 0.f;
+                sum[i] = pj + __shfl_xor_sync(0xffffffffu, pj, 16);  // the order of a warp's sum: keys 16 apart, then 8, 4, 2, 1
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int i = 0; i < o; ++i) sum[i] += sum[i + o];
+            if (any) { l = fmaf(l, alpha, sum[0]); m = m_new; }
+            if (kb == 0) al[row] = alpha;
+            full = __all_sync(0xffffffffu, nonzero || !live);        // no weight of the warp's rows is zero
+        }
+        ROWS_WAIT(1);
+        __syncthreads();                                 // V has landed
+        {
+            const float4 a0 = *reinterpret_cast<const float4*>(al + rg), a1 = *reinterpret_cast<const float4*>(al + rg + 4);
+            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+#pragma unroll
+                for (int c = 0; c < 4 * NC; ++c) acc[r][c] *= av[r];
+            const int keys = min(32, last - j0 + 1);
+            auto key = [&](int k, bool all) {
+                const float4 p0 = *reinterpret_cast<const float4*>(Ps + k * ROWS_PS + rg), p1 = *reinterpret_cast<const float4*>(Ps + k * ROWS_PS + rg + 4);
+                const float pv[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const int e = dg + 64 * c;
+                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (e < d) v = *reinterpret_cast<const float4*>(Vs + k * ld + e);
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) {
+                        if (all || pv[r] != 0.f) {       // a weight of zero (no key, or one far below the maximum) adds nothing,
+                            rows_fma2(acc[r][4 * c], acc[r][4 * c + 1], pv[r], v.x, v.y);      // whatever its value holds
+                            rows_fma2(acc[r][4 * c + 2], acc[r][4 * c + 3], pv[r], v.z, v.w);
+                        }
+                    }
+                }
+            };
+            if (full && keys == 32) {
+#pragma unroll 2
+                for (int k = 0; k < 32; ++k) key(k, true);
+            } else {
+                for (int k = 0; k < keys; ++k) key(k, false);
+            }
+        }
+        __syncthreads();                                 // V and the weights are read
+        if (j1 <= last) fetch(Vs, A.v_pages, j1); else ROWS_COMMIT();
+        j0 = j1;
+    }
+    ROWS_WAIT(0);
+    {
+        float alpha = 1.0f;
+        if (A.sink && live) {
+            const float2 r = rows_sink(m, l, A.sink[head]);
+            l = r.x; alpha = r.y;
+        }
+        float inv = 1.0f / l;
+        if (A.gate && live) inv *= 1.0f / (1.0f + expf(-A.gate[(size_t)(t0 + row / g) * A.nq + head]));
+        if (kb == 0) { al[row] = alpha; Ps[row] = inv; }
+    }
+    __syncwarp();                                        // rows rg .. of this lane are its own warp's
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (rg + r >= rows) continue;
+        const float alpha = al[rg + r], inv = Ps[rg + r];
+        float* o = A.out + ((size_t)(t0 + (rg + r) / g) * A.nq + kh * g + (rg + r) % g) * d;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            const int e = dg + 64 * c;
+            if (e >= d) continue;
+            float4 v = make_float4(acc[r][4 * c], acc[r][4 * c + 1], acc[r][4 * c + 2], acc[r][4 * c + 3]);
+            if (A.sink) { v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha; }
+            v.x *= inv; v.y *= inv; v.z *= inv; v.w *= inv;
+            *reinterpret_cast<float4*>(o + e) = v;
+        }
+    }
+}
+
+// ------------------------------------------------------------------ few tokens
+constexpr int DOTS_KEYS = 128, DOTS_HEADS = 8;
+
+// scores[t, h, j] for every key j that token t's heads see: grid (keys / 128, KV heads, T), a thread a key
+__global__ void __launch_bounds__(DOTS_KEYS) attn_dots_kernel(const RowsArgs A) {
+    extern __shared__ __align__(16) float qs[];          // [heads of the group][d]
+    const int t = blockIdx.z, kh = blockIdx.y, g = A.nq / A.nkv, d = A.d;
+    const int p = min(A.pos[t], A.keys - 1), lo = rows_low(A, p), kept = min(A.keep_first, lo);
+    const int c0 = blockIdx.x * DOTS_KEYS;
+    if (c0 > p || (c0 >= kept && c0 + DOTS_KEYS <= lo)) return;
+    for (int i = threadIdx.x; i < g * d; i += DOTS_KEYS) qs[i] = A.q[(size_t)t * A.q_stride + (size_t)kh * g * d + i];
+    __syncthreads();
+    const int j = c0 + threadIdx.x;
+    if (!((j >= lo || j < kept) && j <= p)) return;
+    const int* tab = A.table + (size_t)tl_checked(A.req_slot[t], A.L.table_rows, A.L, TL_K_TOKENWISE) * A.max_pages;
+    const float* kr = rows_at(A, A.k_pages, tab, j, kh);
+    for (int h0 = 0; h0 < g; h0 += DOTS_HEADS) {
+        float dot[DOTS_HEADS];
+#pragma unroll
+        for (int h = 0; h < DOTS_HEADS; ++h) dot[h] = 0.f;
+#pragma unroll 4
+        for (int e = 0; e < d; e += 4) {
+            const float4 k4 = *reinterpret_cast<const float4*>(kr + e);
+#pragma unroll
+            for (int h = 0; h < DOTS_HEADS; ++h) {
+                const float4 q4 = *reinterpret_cast<const float4*>(qs + min(h0 + h, g - 1) * d + e);
+                dot[h] = fmaf(q4.x, k4.x, dot[h]);
+                dot[h] = fmaf(q4.y, k4.y, dot[h]);
+                dot[h] = fmaf(q4.z, k4.z, dot[h]);
+                dot[h] = fmaf(q4.w, k4.w, dot[h]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < DOTS_HEADS; ++h) {
+            if (h0 + h >= g) break;
+            const int head = kh * g + h0 + h;
+            A.scores[((size_t)t * A.nq + head) * A.keys + j] = rows_score(A, dot[h], A.slopes ? A.slopes[head] : 0.f, p, j);
+        }
+    }
+}
+
+// grid (slices of 32 columns, KV heads * groups of up to 8 of their query heads, T), a warp a head
+constexpr int CHAIN_KEYS = 128, CHAIN_STAGES = 4;
+constexpr int CHAIN_SMEM = (CHAIN_STAGES * CHAIN_KEYS * 32 + DOTS_HEADS * CHAIN_KEYS) * (int)sizeof(float);
+
+__global__ void __launch_bounds__(32 * DOTS_HEADS) attn_chain_kernel(const RowsArgs A) {
+    extern __shared__ __align__(16) float sm[];
+    float (*vs)[CHAIN_KEYS][32] = reinterpret_cast<float (*)[CHAIN_KEYS][32]>(sm);
+    float (*ws)[CHAIN_KEYS] = reinterpret_cast<float (*)[CHAIN_KEYS]>(sm + CHAIN_STAGES * CHAIN_KEYS * 32);
+    const int t = blockIdx.z, g = A.nq / A.nkv, d = A.d, groups = (g + DOTS_HEADS - 1) / DOTS_HEADS;
+    const int kh = blockIdx.y / groups, h0 = (blockIdx.y % groups) * DOTS_HEADS;
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
+    const int p = min(A.pos[t], A.keys - 1), lo = rows_low(A, p), kept = min(A.keep_first, lo);
+    const int e0 = blockIdx.x * 32, e = e0 + lane;
+    const bool live = h0 + wid < g;
+    const int head = kh * g + min(h0 + wid, g - 1);
+    const int* tab = A.table + (size_t)tl_checked(A.req_slot[t], A.L.table_rows, A.L, TL_K_TOKENWISE) * A.max_pages;
+    const float* sr = A.scores + ((size_t)t * A.nq + head) * A.keys;
+    // groups of 128 keys; those wholly between the kept first keys and the window are left out
+    auto next = [&](int c) { return (c >= kept && c + CHAIN_KEYS <= lo) ? (lo / CHAIN_KEYS) * CHAIN_KEYS : c; };
+    auto valid = [&](int j) { return (j >= lo || j < kept) && j <= p; };
+    auto fetch = [&](int c, int stage) {
+        if (c <= p) {
+            for (int i = tid; i < CHAIN_KEYS * 8; i += nt) {
+                const int j = c + (i >> 3), x = (i & 7) * 4;
+                if (valid(j) && e0 + x < d) rows_copy16(&vs[stage][i >> 3][x], rows_at(A, A.v_pages, tab, j, kh) + e0 + x);
+            }
+        }
+        ROWS_COMMIT();
+    };
+    auto load = [&](int c, float (&s)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int j = c + 32 * i + lane;
+            s[i] = valid(j) ? sr[j] : -INFINITY;
+        }
+    };
+    float m = -INFINITY, l = 0.f, acc = 0.f;
+    int c = next(0), ahead = c;
+    for (int i = 0; i < CHAIN_STAGES - 1; ++i) { fetch(ahead, i); ahead = next(ahead + CHAIN_KEYS); }
+    float s[4];
+    load(c, s);
+    for (int step = 0; c <= p; ++step) {
+        const int after = next(c + CHAIN_KEYS);
+        fetch(ahead, (step + CHAIN_STAGES - 1) % CHAIN_STAGES);
+        ahead = next(ahead + CHAIN_KEYS);
+        float top[4], w[4], sum[4], alpha[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) top[i] = warp_max(s[i]);
+        unsigned any = 0;                                // tiles with a key; the others leave everything as it is
+        bool full = true;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const bool here = __any_sync(0xffffffffu, valid(c + 32 * i + lane));
+            if (here) any |= 1u << i;
+            const float m_new = here ? fmaxf(m, top[i]) : m;
+            alpha[i] = here ? expf(m - m_new) : 1.0f;
+            w[i] = valid(c + 32 * i + lane) ? expf(s[i] - m_new) : 0.f;
+            m = m_new;
+            full = full && w[i] != 0.f;
+        }
+        full = __all_sync(0xffffffffu, full);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { sum[i] = warp_sum(w[i]); ws[wid][32 * i + lane] = w[i]; }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) if ((any >> i) & 1u) l = fmaf(l, alpha[i], sum[i]);
+        if (after <= p) load(after, s);
+        ROWS_WAIT(CHAIN_STAGES - 1);
+        __syncthreads();                                 // the step's values have landed
+        const float (*vt)[32] = vs[step % CHAIN_STAGES];
+        if (full) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc *= alpha[i];
+#pragma unroll
+                for (int k = 32 * i; k < 32 * i + 32; k += 4) {
+                    const float4 w4 = *reinterpret_cast<const float4*>(&ws[wid][k]);
+                    acc = fmaf(w4.x, vt[k][lane], acc);
+                    acc = fmaf(w4.y, vt[k + 1][lane], acc);
+                    acc = fmaf(w4.z, vt[k + 2][lane], acc);
+                    acc = fmaf(w4.w, vt[k + 3][lane], acc);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                acc *= alpha[i];
+                for (int k = 32 * i; k < 32 * i + 32; ++k) {
+                    const float wk = ws[wid][k];
+                    if (wk != 0.f) acc = fmaf(wk, vt[k][lane], acc);
+                }
+            }
+        }
+        __syncthreads();                                 // the stage and the weights are read
+        c = after;
+    }
+    ROWS_WAIT(0);
+    if (A.sink) {
+        const float2 r = rows_sink(m, l, A.sink[head]);
+        l = r.x;
+        acc *= r.y;
+    }
+    float inv = 1.0f / l;
+    if (A.gate) inv *= 1.0f / (1.0f + expf(-A.gate[(size_t)t * A.nq + head]));
+    if (live && e < d) A.out[((size_t)t * A.nq + head) * d + e] = acc * inv;
+}
+
+// `scores` (float [T, nq, keys], keys >= every position of the step + 1, or null): scratch of the two kernels of few tokens.
+// Returns 1 where these kernels do not take the shape (the caller then runs the token-wise kernel).
+TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int* table,
+                           int max_pages, int page_size, const int* pos, const int* req_slot, int T, int nq, int nkv, int d, int window,
+                           float scale, const float* sink, int keep_first, const float* gate, int chunk, const float* slopes, float cap,
+                           float* scores, int keys, int table_rows, int total_pages, int* fault, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (nq % nkv || (chunk > 0 && window > 0) || chunk < 0 || d < 4 || d % 4 || d > 256 ||
+        ((((uintptr_t)k_pages) | ((uintptr_t)v_pages) | ((uintptr_t)out)) & 15)) return 1;
+    const int g = nq / nkv;
+    static bool raised[TL_MAX_DEVICES] = {};
+    const int dev = tl_device_index();
+    if (dev < 0) return 1;
+    if (!raised[dev]) {
+        const int most = ((ROWS_MAX + 64) * (256 + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
+        cudaError_t e = cudaFuncSetAttribute(attn_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_rows_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_rows_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SMEM);
+        if (e != cudaSuccess) return (int)e;
+        raised[dev] = true;
+    }
+    RowsArgs A{q, q_stride, out, k_pages, v_pages, table, max_pages, page_size, pos, req_slot, T, nq, nkv, d, window, scale,
+               sink, window > 0 ? keep_first : 0, gate, chunk, slopes, cap, scores, keys, 0, TlLimits{table_rows, total_pages, fault}};
+    if (scores) {
+        const int groups = (g + DOTS_HEADS - 1) / DOTS_HEADS;
+        const size_t smem = (size_t)g * d * sizeof(float);
+        if (smem > 48 * 1024 || nkv > 65535 || T > 65535 || nkv * groups > 65535) return 1;
+        attn_dots_kernel<<<dim3((keys + DOTS_KEYS - 1) / DOTS_KEYS, nkv, T), DOTS_KEYS, smem, stream>>>(A);
+        const int e = tl_launch_status();
+        if (e) return e;
+        attn_chain_kernel<<<dim3((d + 31) / 32, nkv * groups, T), 32 * (g < DOTS_HEADS ? g : DOTS_HEADS), CHAIN_SMEM, stream>>>(A);
+        return tl_launch_status();
+    }
+    if (g > ROWS_MAX || nkv > 65535) return 1;
+    A.tq = ROWS_MAX / g < 32 ? ROWS_MAX / g : 32;
+    const int smem = ((ROWS_MAX + 64) * (d + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
+    const dim3 grid((T + A.tq - 1) / A.tq, nkv, A.tq < T ? A.tq : T);
+    if (d <= 64) attn_rows_kernel<1><<<grid, 128, smem, stream>>>(A);
+    else if (d <= 128) attn_rows_kernel<2><<<grid, 128, smem, stream>>>(A);
+    else attn_rows_kernel<4><<<grid, 128, smem, stream>>>(A);
+    return tl_launch_status();
+}

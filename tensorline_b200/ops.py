@@ -16,7 +16,7 @@ from .csrc.build import CHECK_BUILD, load_library
 
 CORE_SOURCES = ["elementwise.cu", "rope_kv.cu", "attn_tokenwise.cu", "gemm_f32.cu", "sampling.cu", "recurrent.cu", "moe.cu",
                 "delta.cu", "latent.cu", "rglru.cu", "streams.cu", "stream_norm.cu", "attn_mixed_tokenwise.cu",
-                "channel_scan.cu", "differential.cu"]
+                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu"]
 
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -30,6 +30,7 @@ _SIGNATURES = {
     "tl_rope_kv_write": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, ctypes.c_longlong,
                          _I, _P, _P, _F, _I, _I, _I, _I, _P, _P],
     "tl_attn_tokenwise": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _P, _F, _I, _I, _P, _P],
+    "tl_attn_rows": [_P, _I, _P, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _P, _F, _P, _I, _I, _I, _P, _P],
     "tl_gemm_f32": [_P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _P],
     "tl_argmax": [_P, _I, _I, _I, _P, _P, _P],
     "tl_sample": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
@@ -601,6 +602,13 @@ def rope_kv_write(qkv: torch.Tensor, bias: torch.Tensor | None, pos: torch.Tenso
         int(norm_dim), int(norm_cast), table.shape[0], k_pages.shape[0] if write_kv else 0, fault_words(qkv.device), _stream()), "rope_kv_write")
 
 
+# 32-bit steps of up to this many tokens take the attention whose dot products are spread over all tiles of keys (their scores
+# pass through memory, at most this many of them); longer ones the kernel whose rows share the tiles (28 heads on 4, a portion on
+# 700 cached tokens: 64 tokens 124 us against 222, 128 tokens 242 against 239).
+FEW_ROWS_MAX_TOKENS = 64
+FEW_ROWS_MAX_SCORES = 1 << 24
+
+
 def attn_tokenwise(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                    table: torch.Tensor, page_size: int, pos: torch.Tensor, req_slot: torch.Tensor,
                    nq: int, nkv: int, d: int, window: int | None, scale: float, sink: torch.Tensor | None = None,
@@ -627,6 +635,17 @@ def attn_tokenwise(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_pages: t
     if chunk and window:
         raise KernelError("attn_tokenwise: a window or chunks, not both")
     _sink(slopes, nq, "attn_tokenwise (slopes)")
+    if q.dtype == torch.float32 and T and d % 4 == 0 and d <= 256 and nq // nkv <= 64 and nq // nkv * d <= 12288 and \
+            not (out.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) & 15:
+        keys = table.shape[1] * page_size
+        few = T <= FEW_ROWS_MAX_TOKENS and T * nq * keys <= FEW_ROWS_MAX_SCORES
+        scores = torch.empty(T * nq * keys, dtype=torch.float32, device=out.device) if few else None
+        _check(core().tl_attn_rows(_ptr(q), q_stride, _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(table), table.shape[1], page_size,
+                                   _ptr(pos), _ptr(req_slot), T, nq, nkv, d, int(window or 0), float(scale), _ptr(sink), int(keep_first),
+                                   _ptr(gate), int(chunk or 0), _ptr(slopes), float(cap or 0.0), _ptr(scores), keys, table.shape[0],
+                                   k_pages.shape[0], fault_words(out.device), _stream()),
+               "attn_chain" if few else "attn_rows", launches=2 if few else 1)
+        return
     _check(core().tl_attn_tokenwise(_ptr(q), q_stride, _ptr(out), dtype_code(q.dtype), _ptr(k_pages), _ptr(v_pages),
                                     _ptr(table), table.shape[1], page_size, _ptr(pos), _ptr(req_slot), T, nq, nkv, d,
                                     int(window or 0), float(scale), _ptr(sink), int(keep_first), _ptr(gate), int(chunk or 0),
