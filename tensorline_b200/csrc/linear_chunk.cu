@@ -1,0 +1,519 @@
+// The recurrences of recurrent.cu with one decay a head (fixed, or gated with a normaliser) for steps of many tokens: chunks of a
+// request's tokens side by side, their sums as matrix products.
+//
+//   S_t = a_t S_(t-1) + b_t k_t v_t^T,  o_t = S_t^T q_t  (gated: divided by max(|n_t . q_t|, exp(-m_t)) + den_eps)
+//
+// With F_t the sum of the log decays of a chunk up to t and i_s the log input gate (0 for a fixed decay), a token's weight in the
+// state after t is exp(F_t - F_s + i_s - m_t), and of the chunk's start state S exp(F_t + m_start - m_t): nothing but the
+// running maximum m (0 for a fixed decay) passes from token to token.
+//   rotate   retention: q and k rotated and scaled, once for all that read them
+//   local    every chunk: its end state from zero, K^T (w V) [d, dv], against a maximum of its own
+//   carry    per state element, chunk after chunk: the chunk's start state takes the place of its end state; the slot's new state
+//   outputs  every chunk: P = (Q K^T) * weights, then [P | w Q] [V ; S] in one product
+// F and the maxima are sums and maxima in double (64 tokens a chunk and head: a warp's work), every weight the float exponential
+// of one difference of doubles; the products are float multiply-adds.  The state in the slots has the layout of the scan
+// kernel, so the two may take turns on one request.  A position's sums depend on where its step began, to rounding.
+//
+// What the scan kernel is bound by is the chain over the tokens at one block a head and 16 columns (128 blocks, 0.36 us a token);
+// here 12 multiply-adds of matrix products a state element and chunk token pair up in tiles of 4 x 8 and 8 x 8 a thread.
+// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; local 45, carry 25, outputs 81 us.
+// 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
+// L2 once each way, weigh half as much again at 32.
+#include "common.cuh"
+
+constexpr int LC_C = 64;                 // tokens a chunk
+constexpr int LC_COLS = 16;              // columns a slice of the state's layout (the scan kernel's)
+constexpr int LC_AT = LC_C + 4;          // stride of the transposed operands: 16-byte reads, neighbouring rows on other banks
+
+struct LinearChunkArgs {
+    const float* q; const float* k; int qk_stride;           // element (t, h, e) at t * stride + h * d + e
+    const float* v; int v_stride;
+    const float* gates; float cap; const float* decay;       // gated: [T, 2H] pre-activations; else decay [H]
+    float q_scale, k_scale;
+    float* state; long long slot_stride;
+    const int* q_start; const int* slots;
+    const int4* chunks;                  // (request, number of the chunk, the request's chunks, first chunk of the request in the list)
+    const int* firsts;                   // the requests' first chunks
+    float* ends;                         // [chunks][H][d dv (+ d)]: end states from zero, then start states
+    double* marks;                       // [chunks][H][3]: the chunk's F, its maximum, the running maximum in front of it
+    float* out;
+    int H, d, dv, nz; float den_eps;
+};
+
+__device__ __forceinline__ float lc_log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
+__device__ __forceinline__ void lc_fma2(float& d0, float& d1, float a, float b0, float b1) {       // (d0, d1) += a (b0, b1)
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%0, %1};\n\t"
+        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "+f"(d0), "+f"(d1) : "f"(a), "f"(b0), "f"(b1));
+}
+
+// Warp 0: for the n tokens of a chunk that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the running
+// maximum top[t] of u (gated).
+template <bool GATED>
+__device__ __forceinline__ void lc_weights(const LinearChunkArgs& A, int t0, int n, int h, int lane, double* F, double* u, double* top) {
+    if constexpr (!GATED) {
+        const double la = log((double)A.decay[h]);
+        for (int t = lane; t < LC_C; t += 32) { F[t] = (t + 1) * la; u[t] = -F[t]; }
+    } else {
+    double f[2], in[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const int t = 2 * lane + e;
+        f[e] = 0.0; in[e] = -INFINITY;
+        if (t < n) {
+            const float* g = A.gates + (size_t)(t0 + t) * 2 * A.H;
+            in[e] = A.cap * tanhf(g[h] / A.cap);
+            f[e] = lc_log_sigmoid(A.cap * tanhf(g[A.H + h] / A.cap));
+        }
+    }
+    double sum = f[0] + f[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += x;
+    }
+    const double F1 = sum, F0 = sum - f[1], u0 = in[0] - F0, u1 = in[1] - F1;
+    double best = fmax(u0, u1);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, best, o);
+        if (lane >= o) best = fmax(best, x);
+    }
+    double before = __shfl_up_sync(0xffffffffu, best, 1);
+    if (lane == 0) before = -INFINITY;
+    F[2 * lane] = F0; F[2 * lane + 1] = F1;
+    u[2 * lane] = u0; u[2 * lane + 1] = u1;
+    top[2 * lane] = fmax(before, u0); top[2 * lane + 1] = best;
+    }
+}
+
+// ------------------------------------------------------------------ rotation
+// rows [T][2 H d]: q rotated and scaled, k rotated and scaled; a block a token
+__global__ void __launch_bounds__(256) lc_rotate_kernel(const float* __restrict__ proj, int stride, int q_off, int k_off, const float* __restrict__ inv_freq,
+                                                        int rot, int interleaved, const int* __restrict__ pos, float q_scale, float k_scale,
+                                                        float* __restrict__ rows, int H, int d) {
+    extern __shared__ float cs[];                        // cos [rot / 2], sin [rot / 2]
+    const int t = blockIdx.x, half = rot >> 1;
+    for (int i = threadIdx.x; i < half; i += 256) sincosf(__fmul_rn((float)pos[t], inv_freq[i]), &cs[half + i], &cs[i]);
+    __syncthreads();
+    const float* row = proj + (size_t)t * stride;
+    float* to = rows + (size_t)t * 2 * H * d;
+    const int pairs = H * half, rest = d - rot;
+    for (int i = threadIdx.x; i < 2 * pairs; i += 256) {
+        const bool isk = i >= pairs;
+        const int j = isk ? i - pairs : i, h = j / half, p = j - h * half;
+        const int e1 = h * d + (interleaved ? 2 * p : p), e2 = h * d + (interleaved ? 2 * p + 1 : p + half);
+        const float* x = row + (isk ? k_off : q_off);
+        float* y = to + (isk ? H * d : 0);
+        const float sc = isk ? k_scale : q_scale, x1 = x[e1], x2 = x[e2], c = cs[p], s = cs[half + p];
+        y[e1] = (__fmul_rn(x1, c) - __fmul_rn(x2, s)) * sc;
+        y[e2] = (__fmul_rn(x2, c) + __fmul_rn(x1, s)) * sc;
+    }
+    for (int i = threadIdx.x; i < 2 * H * rest; i += 256) {
+        const bool isk = i >= H * rest;
+        const int j = isk ? i - H * rest : i, e = (j / rest) * d + rot + j % rest;
+        to[(isk ? H * d : 0) + e] = row[(isk ? k_off : q_off) + e] * (isk ? k_scale : q_scale);
+    }
+}
+
+// ------------------------------------------------------------------ end states from zero
+// grid (chunks, H, tiles of RB rows and CB columns); 256 threads, 8 along the columns and 4 along the rows a warp
+template <int RB, int CB, bool GATED>
+__global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) {
+    constexpr int TR = RB / 16, TC = CB / 16;
+    extern __shared__ __align__(16) float sm[];
+    float* Ks = sm;                                      // [64][RB], weighted
+    float* Vs = Ks + LC_C * RB;                          // [64][CB]
+    __shared__ double F[LC_C], u[LC_C], top[LC_C];
+    __shared__ float w[LC_C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, col_tiles = (A.dv + CB - 1) / CB, row0 = (blockIdx.z / col_tiles) * RB, col0 = (blockIdx.z % col_tiles) * CB;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    for (int i = tid; i < LC_C * CB / 4; i += 256) {
+        const int t = i / (CB / 4), c = (i % (CB / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n && col0 + c < A.dv) x = *reinterpret_cast<const float4*>(A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c);
+        *reinterpret_cast<float4*>(Vs + t * CB + c) = x;
+    }
+    if (wid == 0) {
+        lc_weights<GATED>(A, t0, n, h, lane, F, u, top);
+        __syncwarp();
+        const double end = F[n - 1], m = GATED ? (double)(float)(end + top[n - 1]) : 0.0;
+        for (int t = lane; t < LC_C; t += 32) w[t] = t < n ? expf((float)(end + u[t] - m)) * A.k_scale : 0.f;
+        if (lane == 0 && blockIdx.z == 0) {
+            double* mk = A.marks + ((size_t)blockIdx.x * A.H + h) * 3;
+            mk[0] = end; mk[1] = m;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < LC_C * RB / 4; i += 256) {
+        const int t = i / (RB / 4), e = (i % (RB / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n && row0 + e < A.d) {
+            x = *reinterpret_cast<const float4*>(A.k + (size_t)(t0 + t) * A.qk_stride + h * A.d + row0 + e);
+            x.x *= w[t]; x.y *= w[t]; x.z *= w[t]; x.w *= w[t];
+        }
+        *reinterpret_cast<float4*>(Ks + t * RB + e) = x;
+    }
+    __syncthreads();
+    const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
+    float acc[TR][TC];
+#pragma unroll
+    for (int i = 0; i < TR; ++i)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
+    const int kn = (n + 3) & ~3;
+#pragma unroll 4
+    for (int t = 0; t < kn; ++t) {
+        float a[TR], b[TC];
+        if constexpr (TR >= 4) {
+#pragma unroll
+            for (int i = 0; i < TR / 4; ++i) *reinterpret_cast<float4*>(a + 4 * i) = *reinterpret_cast<const float4*>(Ks + t * RB + 64 * i + ty * 4);
+        } else *reinterpret_cast<float2*>(a) = *reinterpret_cast<const float2*>(Ks + t * RB + ty * 2);
+#pragma unroll
+        for (int j = 0; j < TC / 4; ++j) *reinterpret_cast<float4*>(b + 4 * j) = *reinterpret_cast<const float4*>(Vs + t * CB + 64 * j + tx * 4);
+#pragma unroll
+        for (int i = 0; i < TR; ++i)
+#pragma unroll
+            for (int j = 0; j < TC; j += 2) lc_fma2(acc[i][j], acc[i][j + 1], a[i], b[j], b[j + 1]);
+    }
+    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
+    float* to = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
+#pragma unroll
+    for (int i = 0; i < TR; ++i) {
+        const int row = row0 + (TR >= 4 ? 64 * (i / 4) + ty * 4 + i % 4 : ty * 2 + i);
+        if (row >= A.d) continue;
+#pragma unroll
+        for (int j = 0; j < TC; j += 4) {
+            const int col = col0 + 16 * j + tx * 4;
+            if (col < A.dv) *reinterpret_cast<float4*>(to + (size_t)row * A.dv + col) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+        }
+    }
+    if (GATED && col0 == 0 && tid < RB && row0 + tid < A.d) {        // the normaliser: the same with v = 1
+        float s = 0.f;
+#pragma unroll 8
+        for (int t = 0; t < LC_C; ++t) s += Ks[t * RB + tid];
+        to[(size_t)A.d * A.dv + row0 + tid] = s;
+    }
+}
+
+// ------------------------------------------------------------------ carry
+// grid (groups of 4 state elements / 256, H, requests)
+constexpr int LC_CARRY = 64;             // chunks whose factors a block holds at a time
+
+template <int R, int IS, bool GATED>
+__global__ void __launch_bounds__(256) lc_carry_kernel(const LinearChunkArgs A) {
+    constexpr int NT = (IS * (LC_COLS + (GATED ? 1 : 0)) + 31) / 32 * 32, PB = R * NT + (GATED ? 4 : 0);
+    __shared__ double mk[LC_CARRY][2];
+    __shared__ double ms[LC_CARRY + 1];
+    __shared__ float keep[LC_CARRY], gain[LC_CARRY];
+    const int first = A.firsts[blockIdx.z], h = blockIdx.y, tid = threadIdx.x;
+    const int4 ck = A.chunks[first];
+    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
+    const size_t i4 = ((size_t)blockIdx.x * 256 + tid) * 4;
+    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + (size_t)h * A.nz * PB;
+    const bool mine = i4 < per, norm = GATED && i4 >= (size_t)A.d * A.dv;
+    const int row = norm ? (int)(i4 - (size_t)A.d * A.dv) : (int)(i4 / A.dv), col = norm ? 0 : (int)(i4 % A.dv);
+    // element c of the four: four columns of a row, or four rows of the normaliser (which every slice of the slot holds)
+    auto at = [&](int c, int z) {
+        const int r = norm ? row + c : row, j = norm ? LC_COLS : (col + c) % LC_COLS, zz = norm ? z : (col + c) / LC_COLS;
+        return (size_t)zz * PB + (size_t)(r % R) * NT + j * IS + r / R;
+    };
+    float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine) S = make_float4(slot[at(0, 0)], slot[at(1, 0)], slot[at(2, 0)], slot[at(3, 0)]);
+    double m = GATED ? (double)slot[R * NT] : 0.0;
+    float* e = A.ends + ((size_t)first * A.H + h) * per + i4;
+    const size_t step = (size_t)A.H * per;
+    for (int c0 = 0; c0 < ck.z; c0 += LC_CARRY) {
+        const int nc = min(LC_CARRY, ck.z - c0);
+        __syncthreads();
+        for (int c = tid; c < nc; c += 256) {
+            const double* g = A.marks + ((size_t)(first + c0 + c) * A.H + h) * 3;
+            mk[c][0] = g[0]; mk[c][1] = g[1];
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double x = m;
+            for (int c = 0; c < nc; ++c) {
+                ms[c] = x;
+                if (GATED) x = (double)(float)fmax(mk[c][0] + x, mk[c][1]);      // a maximum that a float holds: the slot keeps it
+            }
+            ms[nc] = x;
+        }
+        __syncthreads();
+        for (int c = tid; c < nc; c += 256) {
+            keep[c] = expf((float)(mk[c][0] + ms[c] - ms[c + 1]));
+            gain[c] = expf((float)(mk[c][1] - ms[c + 1]));
+            if (blockIdx.x == 0) A.marks[((size_t)(first + c0 + c) * A.H + h) * 3 + 2] = ms[c];
+        }
+        __syncthreads();
+        m = ms[nc];
+        if (mine) {
+            float4 next[4];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) if (x < nc) next[x] = *reinterpret_cast<const float4*>(e + (size_t)x * step);
+            for (int c = 0; c < nc; c += 4) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    if (c + x < nc) {
+                        const float4 E = next[x];
+                        if (c + x + 4 < nc) next[x] = *reinterpret_cast<const float4*>(e + (size_t)(c + x + 4) * step);
+                        *reinterpret_cast<float4*>(e + (size_t)(c + x) * step) = S;
+                        const float a = keep[c + x], b = gain[c + x];
+                        S.x = fmaf(a, S.x, b * E.x); S.y = fmaf(a, S.y, b * E.y); S.z = fmaf(a, S.z, b * E.z); S.w = fmaf(a, S.w, b * E.w);
+                    }
+                }
+            }
+        }
+        e += (size_t)nc * step;
+    }
+    if (mine) {
+        for (int z = 0; z < (norm ? A.nz : 1); ++z) { slot[at(0, z)] = S.x; slot[at(1, z)] = S.y; slot[at(2, z)] = S.z; slot[at(3, z)] = S.w; }
+    }
+}
+// The running maximum into every slice of the slot, after all blocks of the carry have read it.
+__global__ void lc_maximum_kernel(const LinearChunkArgs A, int pb, int at) {
+    const int first = A.firsts[blockIdx.y], h = blockIdx.x;
+    const int4 ck = A.chunks[first];
+    const double* g = A.marks + ((size_t)(first + ck.z - 1) * A.H + h) * 3;
+    const float m = (float)fmax(g[0] + g[2], g[1]);
+    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + (size_t)h * A.nz * pb;
+    for (int z = threadIdx.x; z < A.nz; z += blockDim.x) slot[(size_t)z * pb + at] = m;
+}
+
+// ------------------------------------------------------------------ outputs
+// grid (chunks, H, slices of CB columns); DP: rows a head, padded
+template <int DP, int CB> struct OutShape {
+    static constexpr int LQ = DP + 4;
+    static constexpr int QT = DP * LC_AT > LC_C * LQ ? DP * LC_AT : LC_C * LQ;       // K first, then Q transposed
+    static constexpr int ROWS = 16, STAGES = 3;                                      // rows of [V ; S] a stage
+    static constexpr int FLOATS = LC_C * LQ + LC_C * LC_AT + QT + STAGES * ROWS * CB;
+};
+
+template <int DP, int CB, bool GATED>
+__global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
+    using Sh = OutShape<DP, CB>;
+    constexpr int LQ = Sh::LQ, TC = CB / 16, ROWS = Sh::ROWS, S = Sh::STAGES;
+    extern __shared__ __align__(16) float sm[];
+    float* Qs = sm;                                      // [64][LQ]
+    float* Pt = Qs + LC_C * LQ;                          // [64 s][LC_AT]: P transposed; behind it ...
+    float* Qt = Pt + LC_C * LC_AT;                       // ... K [64][LQ], later the weighted Q transposed [DP][LC_AT]
+    float* Bs = Qt + Sh::QT;                             // [S][ROWS][CB]
+    __shared__ double F[LC_C], u[LC_C], top[LC_C];
+    __shared__ float coef[LC_C], den[LC_C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
+    const float* start = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
+    const double m0 = GATED ? A.marks[((size_t)blockIdx.x * A.H + h) * 3 + 2] : 0.0;
+    const int vr = (n + ROWS - 1) / ROWS * ROWS, sr = (d + ROWS - 1) / ROWS * ROWS, steps = (vr + sr) / ROWS;    // rows of V, of S
+    auto fetch = [&](int step) {                         // rows of [V ; S]: zeros where there are none
+        float* st = Bs + (step % S) * ROWS * CB;
+#pragma unroll
+        for (int i = tid; i < ROWS * CB / 4; i += 256) {
+            const int r = step * ROWS + i / (CB / 4), c = (i % (CB / 4)) * 4, sr0 = r - vr;
+            const bool in = col0 + c < A.dv && (r < vr ? r < n : sr0 < d);
+            const float* src = !in ? A.v : r < vr ? A.v + (size_t)(t0 + r) * A.v_stride + h * A.dv + col0 + c : start + (size_t)sr0 * A.dv + col0 + c;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(st + i * 4)), "l"(src), "r"(in ? 16 : 0)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    fetch(1);                                            // d >= 1: at least two steps
+    for (int i = tid; i < LC_C * DP / 4; i += 256) {
+        const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+        if (t < n && e < d) {
+            const size_t at = (size_t)(t0 + t) * A.qk_stride + h * d + e;
+            q = *reinterpret_cast<const float4*>(A.q + at);
+            k = *reinterpret_cast<const float4*>(A.k + at);
+            q.x *= A.q_scale; q.y *= A.q_scale; q.z *= A.q_scale; q.w *= A.q_scale;
+            k.x *= A.k_scale; k.y *= A.k_scale; k.z *= A.k_scale; k.w *= A.k_scale;
+        }
+        *reinterpret_cast<float4*>(Qs + t * LQ + e) = q;
+        *reinterpret_cast<float4*>(Qt + t * LQ + e) = k;
+    }
+    if (wid == 0) {
+        lc_weights<GATED>(A, t0, n, h, lane, F, u, top);
+        __syncwarp();
+        for (int t = lane; t < LC_C; t += 32) {          // top: the running maximum less F; F: what is added to u for a weight
+            if (GATED) {
+                const double mm = fmax(m0, top[t]);
+                coef[t] = expf((float)(m0 - mm));
+                den[t] = expf((float)(-(F[t] + mm)));
+                top[t] = -mm;
+            } else {
+                coef[t] = expf((float)F[t]);
+                top[t] = F[t];
+            }
+        }
+    }
+    __syncthreads();
+    const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
+    {                                                    // P: tokens ty + 16 i against tx + 16 j, j <= i
+        float s[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+        const float* qp = Qs + ty * LQ;
+        const float* kp = Qt + tx * LQ;
+#pragma unroll 2
+        for (int e = 0; e < DP; e += 4) {
+            float4 q4[4], k4[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + 16 * i * LQ + e);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(kp + 16 * j * LQ + e);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j <= i; ++j) {
+                    s[i][j] = fmaf(q4[i].x, k4[j].x, s[i][j]);
+                    s[i][j] = fmaf(q4[i].y, k4[j].y, s[i][j]);
+                    s[i][j] = fmaf(q4[i].z, k4[j].z, s[i][j]);
+                    s[i][j] = fmaf(q4[i].w, k4[j].w, s[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int t = ty + 16 * i, x = tx + 16 * j;
+                float p = 0.f;
+                if (j <= i && x <= t && t < n) p = s[i][j] * expf((float)(top[t] + u[x]));
+                Pt[x * LC_AT + t] = p;
+            }
+    }
+    __syncthreads();                                     // K is read, P is written
+    for (int i = tid; i < LC_C * DP / 4; i += 256) {     // Q transposed, weighted: neighbouring lanes take neighbouring tokens
+        const int t = i % LC_C, e = (i / LC_C) * 4;
+        const float4 q = *reinterpret_cast<const float4*>(Qs + t * LQ + e);
+        const float c = coef[t];
+        Qt[e * LC_AT + t] = q.x * c; Qt[(e + 1) * LC_AT + t] = q.y * c; Qt[(e + 2) * LC_AT + t] = q.z * c; Qt[(e + 3) * LC_AT + t] = q.w * c;
+    }
+    if (GATED) {                                         // n_t . q_t, four lanes a token
+        const int t = tid >> 2, part = tid & 3;
+        float s = 0.f, r = 0.f;
+#pragma unroll 4
+        for (int x = part; x < LC_C; x += 4) s += Pt[x * LC_AT + t];
+        for (int e = part; e < d; e += 4) r = fmaf(Qs[t * LQ + e], start[(size_t)d * A.dv + e], r);
+        s = fmaf(coef[t], r, s);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        if (part == 0) den[t] = fmaxf(fabsf(s), den[t]) + A.den_eps;
+    }
+    float acc[4][TC];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();                                 // the step's rows have landed, the step before is read; before the first: Qt, den
+        if (step + 2 < steps) fetch(step + 2);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        const int r0 = step * ROWS;
+        const float* at = r0 < vr ? Pt + r0 * LC_AT : Qt + (r0 - vr) * LC_AT;
+        const float* b = Bs + (step % S) * ROWS * CB;
+#pragma unroll 4
+        for (int r = 0; r < ROWS; ++r) {
+            const float4 a4 = *reinterpret_cast<const float4*>(at + r * LC_AT + ty * 4);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+            float bv[TC];
+#pragma unroll
+            for (int j = 0; j < TC / 4; ++j) *reinterpret_cast<float4*>(bv + 4 * j) = *reinterpret_cast<const float4*>(b + r * CB + 64 * j + tx * 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < TC; j += 2) lc_fma2(acc[i][j], acc[i][j + 1], a[i], bv[j], bv[j + 1]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int t = ty * 4 + i;
+        if (t >= n) continue;
+        float* to = A.out + (size_t)(t0 + t) * A.H * A.dv + (size_t)h * A.dv;
+#pragma unroll
+        for (int j = 0; j < TC; j += 4) {
+            const int col = col0 + 16 * j + tx * 4;
+            float4 o = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+            if (GATED) { o.x /= den[t]; o.y /= den[t]; o.z /= den[t]; o.w /= den[t]; }
+            if (col < A.dv) *reinterpret_cast<float4*>(to + col) = o;
+        }
+    }
+}
+
+template <typename F>
+static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
+    const int dev = tl_device_index();
+    if (dev < 0) return 1;
+    if (!raised[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+        raised[dev] = true;
+    }
+    return 0;
+}
+
+template <int DP, int CB, bool GATED>
+static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
+    constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
+    constexpr int NT = (IS * (LC_COLS + (GATED ? 1 : 0)) + 31) / 32 * 32, PB = R * NT + (GATED ? 4 : 0);
+    constexpr int local_smem = LC_C * (RB + CB) * 4, out_smem = OutShape<DP, CB>::FLOATS * 4;
+    static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
+    int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
+    if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
+    if (e) return e;
+    const int col_tiles = (A.dv + CB - 1) / CB, row_tiles = (A.d + RB - 1) / RB;
+    lc_local_kernel<RB, CB, GATED><<<dim3(n_chunks, A.H, row_tiles * col_tiles), 256, local_smem, stream>>>(A);
+    if ((e = tl_launch_status())) return e;
+    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
+    lc_carry_kernel<R, IS, GATED><<<dim3((unsigned)((per / 4 + 255) / 256), A.H, requests), 256, 0, stream>>>(A);
+    if ((e = tl_launch_status())) return e;
+    if (GATED) {
+        lc_maximum_kernel<<<dim3(A.H, requests), 32, 0, stream>>>(A, PB, R * NT);
+        if ((e = tl_launch_status())) return e;
+    }
+    lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
+    return tl_launch_status();
+}
+
+template <int DP>
+static int lc_pick(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
+    if (A.gates) return A.dv <= 64 ? lc_launch<DP, 64, true>(A, n_chunks, requests, stream) : lc_launch<DP, 128, true>(A, n_chunks, requests, stream);
+    return A.dv <= 64 ? lc_launch<DP, 64, false>(A, n_chunks, requests, stream) : lc_launch<DP, 128, false>(A, n_chunks, requests, stream);
+}
+
+TL_EXPORT int tl_linear_chunk() { return LC_C; }
+
+// `rows` (float [T, 2 H d], with a rotation): where q and k go.  ends: float [n_chunks, H, d dv (+ d with gates)], marks: double
+// [n_chunks, H, 3].  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
+TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, int k_off, int v_off, const float* gates, float cap,
+                               const float* decay, const float* inv_freq, int rot, int interleaved, const int* pos, float q_scale,
+                               float k_scale, float* rows, float* state, long long slot_stride, const int* q_start, const int* slots,
+                               const int* chunks, int n_chunks, const int* firsts, int requests, float* ends, double* marks, float* out,
+                               int H, int d, int dv, float den_eps, cudaStream_t stream) {
+    if (n_chunks <= 0 || H <= 0) return 0;
+    if (H > 65535 || requests > 65535 || d < 4 || d > 256 || ((d | dv | stride | q_off | k_off | v_off) & 3) || (rot & 1) || rot > d ||
+        (rot && !rows) || (gates != nullptr) == (decay != nullptr) ||
+        ((((uintptr_t)proj) | ((uintptr_t)rows) | ((uintptr_t)ends) | ((uintptr_t)out)) & 15)) return 1;
+    LinearChunkArgs A{proj + q_off, proj + k_off, stride, proj + v_off, stride, gates, cap, decay, q_scale, k_scale, state, slot_stride,
+                      q_start, slots, (const int4*)chunks, firsts, ends, marks, out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
+    if (rot) {
+        lc_rotate_kernel<<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
+        const int e = tl_launch_status();
+        if (e) return e;
+        A.q = rows; A.k = rows + (size_t)H * d; A.qk_stride = 2 * H * d;
+        A.q_scale = A.k_scale = 1.0f;
+    }
+    if (d <= 32) return lc_pick<32>(A, n_chunks, requests, stream);
+    if (d <= 64) return lc_pick<64>(A, n_chunks, requests, stream);
+    if (d <= 128) return lc_pick<128>(A, n_chunks, requests, stream);
+    return lc_pick<256>(A, n_chunks, requests, stream);
+}

@@ -16,7 +16,7 @@ from .csrc.build import CHECK_BUILD, load_library
 
 CORE_SOURCES = ["elementwise.cu", "rope_kv.cu", "attn_tokenwise.cu", "gemm_f32.cu", "sampling.cu", "recurrent.cu", "moe.cu",
                 "delta.cu", "latent.cu", "rglru.cu", "streams.cu", "stream_norm.cu", "attn_mixed_tokenwise.cu",
-                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu"]
+                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu"]
 
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -38,6 +38,9 @@ _SIGNATURES = {
                        _I, _I, _F, _I, _P, _P, _P],
     "tl_channel_scan": [_P, _I, _I, _I, _I, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
     "tl_channel_chunk": [],
+    "tl_linear_chunks": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P,
+                         _P, _I, _I, _I, _F, _P],
+    "tl_linear_chunk": [],
     "tl_scan_state_floats": [_I, _I],
     "tl_scan_columns": [],
     "tl_head_norm_gate": [_P, _P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _F, _I, _P],
@@ -788,6 +791,63 @@ def linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, 
                                  float(q_scale), float(k_scale), _ptr(state), per_slot, _ptr(q_start), _ptr(slots), _ptr(out),
                                  int(B), H, d, dv, float(den_eps), int(single_tokens), _ptr(lower), _ptr(bias), _stream()),
            "linear_step" if single_tokens else "linear_scan")
+
+
+# From this many tokens of one request a bfloat16 step's matrix memories run as chunks side by side instead of token by token (8 heads of
+# 128 x 256, one request: gated 64 tokens 28 us token by token against 55 in chunks, most of it the host's five launches; 128
+# tokens 51 against 56, 256 tokens 95 against 57, 2,048 tokens 720 against 140).
+LINEAR_CHUNKS_MIN_TOKENS = 128
+
+
+def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int) -> bool:
+    """Whether `linear_chunks` takes these sizes (q, k, v one behind the other in a projection's row) and is the faster way."""
+    return proj.dtype == torch.float32 and max_q_len >= LINEAR_CHUNKS_MIN_TOKENS and d % 4 == 0 and dv % 4 == 0 and d <= 256 and \
+        proj.shape[1] % 4 == 0 and proj.data_ptr() % 16 == 0
+
+
+def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, d: int, dv: int, state: torch.Tensor, ctx, out: torch.Tensor,
+                  *, decay: torch.Tensor | None = None, gates: torch.Tensor | None = None, cap: float = 1.0, inv_freq: torch.Tensor | None = None,
+                  rot: int = 0, pairing: str = "half", q_scale: float = 1.0, k_scale: float = 1.0, den_eps: float = 0.0) -> None:
+    """`linear_scan` with one decay a head (`decay` or `gates`) for steps of several tokens a request: chunks of a request's tokens
+    side by side, as matrix products of floats.  proj float32 with 16-byte rows; the state as `linear_scan` keeps it, so the two may
+    take turns.  A position's sums depend on where its step began, to rounding."""
+    T = proj.shape[0]
+    _contig(proj, "proj"); _contig(state, "state"); _contig(out, "out")
+    if (decay is None) == (gates is None):
+        raise KernelError("linear_chunks: a fixed decay per head or gate pre-activations")
+    if proj.dtype != torch.float32 or out.dtype != torch.float32 or out.shape != (T, H * dv) or state.dtype != torch.float32:
+        raise KernelError("linear_chunks: proj, the state and out [T, H * dv] are float32")
+    per_slot = H * -(-dv // scan_columns()) * scan_state_floats(d, gates is not None)
+    if state[0].numel() != per_slot:
+        raise KernelError(f"linear_chunks: a slot holds {state[0].numel()} floats, these sizes need {per_slot}")
+    for name, off, width in (("q", q_off, H * d), ("k", k_off, H * d), ("v", v_off, H * dv)):
+        if off < 0 or off + width > proj.shape[1]:
+            raise KernelError(f"linear_chunks: {name} does not lie inside a projection row")
+    if (d | dv | q_off | k_off | v_off | proj.shape[1]) & 3 or d > 256 or proj.data_ptr() & 15:
+        raise KernelError("linear_chunks: heads of up to 256, sizes and offsets in multiples of 4, 16-byte rows")
+    if decay is not None and (decay.dtype != torch.float32 or decay.numel() != H):
+        raise KernelError("linear_chunks: decay must be float32 [H]")
+    if gates is not None and (gates.dtype != torch.float32 or gates.shape != (T, 2 * H) or not gates.is_contiguous()):
+        raise KernelError("linear_chunks: gates must be float32 [T, 2H]")
+    if rot and (inv_freq is None or inv_freq.dtype != torch.float32 or inv_freq.numel() != rot // 2):
+        raise KernelError("linear_chunks: inv_freq must be float32 [rot/2]")
+    interleaved = _pairing(pairing, "linear_chunks")
+    key = "linear_chunks"
+    if key not in ctx.scratch:                           # one description a step, for every layer
+        rows, _ = channel_chunks(ctx.h_q_start, core().tl_linear_chunk())
+        firsts = np.nonzero(rows[:, 1] == 0)[0].astype(np.int32)
+        both = torch.from_numpy(np.concatenate([rows.reshape(-1), firsts])).to(proj.device, non_blocking=True)
+        ctx.scratch[key] = (both, len(rows), len(firsts))
+    both, n, requests = ctx.scratch[key]
+    dev = proj.device
+    turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
+    ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
+    marks = torch.empty((n, H, 3), dtype=torch.float64, device=dev)
+    _check(core().tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, _ptr(gates), float(cap), _ptr(decay),
+                                   _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale), float(k_scale),
+                                   _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n,
+                                   requests, _ptr(ends), _ptr(marks), _ptr(out), H, d, dv, float(den_eps), _stream()), "linear_chunks",
+           launches=3 + bool(rot) + (gates is not None))
 
 
 def channel_chunks(h_q_start, chunk: int) -> tuple:

@@ -88,6 +88,10 @@ class _MatrixState(Part):
     def _scan(self, h, proj, ctx, state, o):
         raise NotImplementedError
 
+    def _in_chunks(self, h, proj, ctx) -> bool:
+        """Chunks of a portion side by side; the 32-bit engine walks every step in order: the same floats however cut."""
+        return h.dtype == torch.bfloat16 and not ctx.decode_only and ops.takes_linear_chunks(proj, self.d, self.dv, ctx.max_q_len)
+
     def _head_weight(self):
         return None
 
@@ -120,6 +124,10 @@ class Retention(_MatrixState):
         rotary = self.position.rotary()
         if not isinstance(rotary, Rotary):
             rotary = Rotary(*rotary)
+        if self._in_chunks(h, proj, ctx):
+            ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, o, decay=self.decay, inv_freq=rotary.inv_freq,
+                              rot=rotary.rot, pairing=rotary.pairing, k_scale=d ** -0.5)
+            return
         ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, o, B=ctx.B,
                         decay=self.decay, inv_freq=rotary.inv_freq, rot=rotary.rot, pairing=rotary.pairing,
                         k_scale=d ** -0.5, single_tokens=ctx.decode_only)
@@ -161,6 +169,10 @@ class MLSTM(_MatrixState):
         H, d, dv = self.H, self.d, self.dv
         gates = torch.empty((h.shape[0], 2 * H), dtype=torch.float32, device=h.device)
         ops.small_proj(h, self.w_gates, self.b_gates, gates)
+        if self._in_chunks(h, proj, ctx):
+            ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, o, gates=gates, cap=self.cap, q_scale=d ** -0.5,
+                              den_eps=self.den_eps)
+            return
         ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, o, B=ctx.B,
                         gates=gates, cap=self.cap, q_scale=d ** -0.5, den_eps=self.den_eps, single_tokens=ctx.decode_only)
 

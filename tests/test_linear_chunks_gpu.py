@@ -1,0 +1,109 @@
+"""Matrix memories in chunks (`ops.linear_chunks`): against the recurrence in float64 over the forms it accepts, and against the
+token-by-token kernel, whose state it shares.  Bound: sums of up to a few hundred float products of order one, 2e-5 of the largest."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def slot_rows(S, n, m):
+    """S [H, d, dv] (n [H, d], m [H]) in the scan kernel's slot layout."""
+    H, d, dv = S.shape
+    R, IS = (4, 8) if d <= 32 else (8, 8) if d <= 64 else (8, 16) if d <= 128 else (8, 32)
+    nz, cols = -(-dv // 16), 16 if n is None else 17
+    NT = -(-IS * cols // 32) * 32
+    out = torch.zeros(H, nz, R * NT + (4 if n is not None else 0), dtype=S.dtype)
+    i, j = torch.meshgrid(torch.arange(d), torch.arange(dv), indexing="ij")
+    out[:, j // 16, (i % R) * NT + (j % 16) * IS + i // R] = S
+    if n is not None:
+        i = torch.arange(d)
+        out[:, :, (i % R) * NT + 16 * IS + i // R] = n[:, None, :]
+        out[:, :, R * NT] = m[:, None]
+    return out.reshape(-1)
+
+
+def recurrence(x, gates, decay, H, d, dv, S, n, m, pos, inv_freq, rot, interleaved, cap, q_scale, k_scale, den_eps):
+    T = x.shape[0]
+    q, k, v = x[:, :H * d].view(T, H, d), x[:, H * d:2 * H * d].view(T, H, d), x[:, 2 * H * d:2 * H * d + H * dv].view(T, H, dv)
+    if rot:
+        a = pos.double()[:, None] * inv_freq.double()
+        c, s = torch.cos(a)[:, None], torch.sin(a)[:, None]
+
+        def turn(y):
+            y = y.clone()
+            e1, e2 = (slice(0, rot, 2), slice(1, rot, 2)) if interleaved else (slice(0, rot // 2), slice(rot // 2, rot))
+            y1, y2 = y[..., e1].clone(), y[..., e2].clone()
+            y[..., e1], y[..., e2] = y1 * c - y2 * s, y2 * c + y1 * s
+            return y
+        q, k = turn(q), turn(k)
+    q, k = q * q_scale, k * k_scale
+    o = torch.empty(T, H, dv, dtype=torch.float64)
+    for t in range(T):
+        if decay is not None:
+            S = decay.double()[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
+            o[t] = torch.einsum("hd,hde->he", q[t], S)
+            continue
+        li = cap * torch.tanh(gates[t, :H] / cap)
+        lf = torch.nn.functional.logsigmoid(cap * torch.tanh(gates[t, H:] / cap))
+        new = torch.maximum(lf + m, li)
+        a, b = torch.exp(lf + m - new), torch.exp(li - new)
+        m = new
+        S = a[:, None, None] * S + b[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+        n = a[:, None] * n + b[:, None] * k[t]
+        den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + den_eps
+        o[t] = torch.einsum("hd,hde->he", q[t], S) / den[:, None]
+    return o.reshape(T, H * dv), S, n, m
+
+
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("H,d,dv,lens,rot,interleaved", [
+    (3, 128, 256, [64, 65, 1], 64, False), (2, 64, 64, [200], 64, True), (1, 32, 128, [127, 63, 128], 0, False), (2, 256, 128, [130], 256, False),
+    (2, 20, 36, [70, 3], 8, True), (1, 96, 20, [300, 64], 96, False), (2, 200, 132, [100], 0, False), (1, 4, 4, [193], 0, False)])
+def test_chunks_against_the_recurrence_in_float64_and_the_scan_kernel(gated, H, d, dv, lens, rot, interleaved):
+    from tensorline_b200 import ops
+    g = torch.Generator().manual_seed(d * dv + sum(lens))
+    T, B = sum(lens), len(lens)
+    width = 2 * H * d + H * dv + 12
+    proj = torch.randn(T, width, generator=g)
+    rot = 0 if gated else rot
+    gates = torch.cat([torch.randn(T, H, generator=g) * 2 - 1, torch.randn(T, H, generator=g) * 2 + 3], dim=1) if gated else None
+    if gated:
+        gates[T // 2] = torch.tensor([30.0] * H + [-40.0] * H)      # everything before is forgotten here
+    decay = None if gated else 1.0 - 2.0 ** (-1 - 5.0 * torch.arange(H))
+    inv = 10000.0 ** (-torch.arange(0, rot, 2).float() / max(rot, 1)) if rot else None
+    kw = dict(cap=15.0, q_scale=d ** -0.5, k_scale=1.0, den_eps=1e-6) if gated else dict(k_scale=d ** -0.5, q_scale=1.0)
+    q_start = [0]
+    for n in lens:
+        q_start.append(q_start[-1] + n)
+    starts = [17 * b for b in range(B)]
+    pos = torch.cat([torch.arange(s, s + n) for s, n in zip(starts, lens)]).to(torch.int32)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32)
+    S0 = torch.randn(B, H, d, dv, generator=g) * 0.3
+    n0 = torch.randn(B, H, d, generator=g) * 0.3 if gated else [None] * B
+    m0 = torch.randn(B, H, generator=g) if gated else [None] * B
+    first = torch.stack([torch.zeros_like(slot_rows(S0[0], n0[0], m0[0]))] + [slot_rows(S0[b], n0[b], m0[b]) for b in range(B)][::-1])
+    dev = {k: v.cuda() for k, v in dict(proj=proj, pos=pos, slots=slots, q=torch.tensor(q_start, dtype=torch.int32)).items()}
+    if decay is not None:
+        kw.update(decay=decay.cuda())
+    if gates is not None:
+        kw.update(gates=gates.cuda())
+    if rot:
+        kw.update(inv_freq=inv.cuda(), rot=rot, pairing="interleaved" if interleaved else "half")
+    ctx = SimpleNamespace(h_q_start=q_start, scratch={}, pos=dev["pos"], q_start=dev["q"], slots=dev["slots"])
+    state, out = first.cuda(), torch.full((T, H * dv), 7.0, device="cuda")
+    ops.linear_chunks(dev["proj"], 0, H * d, 2 * H * d, H, d, dv, state, ctx, out, **kw)
+    scan_state, scan_out = first.cuda(), torch.empty_like(out)
+    ops.linear_scan(dev["proj"], 0, H * d, 2 * H * d, H, d, dv, scan_state, dev["q"], dev["slots"], dev["pos"], scan_out, B=B, **kw)
+    for b in range(B):
+        rows = slice(q_start[b], q_start[b + 1])
+        o, S, n, m = recurrence(proj[rows].double(), gates[rows].double() if gated else None, decay, H, d, dv, S0[b].double(),
+                                n0[b].double() if gated else None, m0[b].double() if gated else None, pos[rows], inv, rot, interleaved,
+                                kw.get("cap"), kw["q_scale"], kw["k_scale"], kw.get("den_eps", 0.0))
+        want = slot_rows(S, n, m)
+        for got, scan, x in ((out[rows], scan_out[rows], o), (state[int(slots[b])], scan_state[int(slots[b])], want)):
+            err, base = (float((y.double().cpu() - x).norm()) / float(x.norm()) for y in (got, scan))
+            assert err <= max(2e-6, 1.5 * base), (err, base)
+            assert float((got.double().cpu() - x).abs().max()) <= max(2e-5 * float(x.abs().max()), 4 * float((scan.double().cpu() - x).abs().max()))
+    assert torch.equal(state[0].cpu(), first[0])
