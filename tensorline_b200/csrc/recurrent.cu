@@ -454,10 +454,71 @@ __global__ void head_norm_gate_kernel(const float* __restrict__ o, const TG* __r
     }
 }
 
+// The bfloat16 engine's, rows in 16-byte pieces: a warp a (token, head), NP pieces of four values a lane (dv <= 128 NP), read once
+// and kept in registers until their square is known.  2,048 tokens, 8 heads of 256 with a float gate: 42 MB, 11.9 us (one value at a time,
+// the row read twice: 15.8).
+template <typename TW, typename TG, int NP>
+__global__ void __launch_bounds__(128) head_norm_gate_vec_kernel(const float* __restrict__ o, const TG* __restrict__ g, int g_stride,
+                                                                 const TW* __restrict__ w, bf16* __restrict__ out, int H, int dv, float eps, int act) {
+    const int t = blockIdx.x, h = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    grid_dependency_wait();                              // launched as a dependent: nothing of another kernel is touched before this
+    grid_dependency_trigger();
+    if (h >= H) return;
+    const float* row = o + ((size_t)t * H + h) * dv;
+    const TG* gate = g + (size_t)t * g_stride + h * dv;
+    float4 v[NP], x[NP], c[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int j = (lane + 32 * i) * 4;
+        v[i] = x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        c[i] = make_float4(1.f, 1.f, 1.f, 1.f);
+        if (j < dv) {
+            if (w) c[i] = make_float4(to_f<TW>(w[h * dv + j]), to_f<TW>(w[h * dv + j + 1]), to_f<TW>(w[h * dv + j + 2]), to_f<TW>(w[h * dv + j + 3]));
+            v[i] = *reinterpret_cast<const float4*>(row + j);
+            if (act) {
+                if constexpr (sizeof(TG) == 4) x[i] = *reinterpret_cast<const float4*>(gate + j);
+                else x[i] = make_float4(to_f<TG>(gate[j]), to_f<TG>(gate[j + 1]), to_f<TG>(gate[j + 2]), to_f<TG>(gate[j + 3]));
+            }
+        }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NP; ++i) ss = fmaf(v[i].x, v[i].x, fmaf(v[i].y, v[i].y, fmaf(v[i].z, v[i].z, fmaf(v[i].w, v[i].w, ss))));
+    ss = warp_sum(ss);
+    const float rstd = 1.0f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const int j = (lane + 32 * i) * 4;
+        if (j >= dv) continue;
+        float y[4] = {v[i].x * rstd * c[i].x, v[i].y * rstd * c[i].y, v[i].z * rstd * c[i].z, v[i].w * rstd * c[i].w};
+        const float z[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (act) {
+                const float s = 1.0f / (1.0f + expf(-z[e]));
+                y[e] *= act == 1 ? s : z[e] * s;
+            }
+        }
+        uint2 u;
+        *reinterpret_cast<__nv_bfloat162*>(&u.x) = __floats2bfloat162_rn(y[0], y[1]);
+        *reinterpret_cast<__nv_bfloat162*>(&u.y) = __floats2bfloat162_rn(y[2], y[3]);
+        *reinterpret_cast<uint2*>(out + ((size_t)t * H + h) * dv + j) = u;
+    }
+}
+
 TL_EXPORT int tl_head_norm_gate(const float* o, const void* g, int g_dtype, int g_stride, const void* w, int w_dtype, void* out,
                                 int act_dtype, int T, int H, int dv, float eps, int act, cudaStream_t stream) {
     if (T <= 0 || H <= 0) return 0;
     const dim3 grid(T, (H + 3) / 4), block(128);
+    if (act_dtype != TL_F32 && dv % 4 == 0 && dv <= 512 && ((((uintptr_t)o) | ((uintptr_t)out)) & 15) == 0 &&
+        (!act || g_dtype != TL_F32 || (g_stride % 4 == 0 && ((uintptr_t)g & 15) == 0))) {
+#define HNV_N(TW, TG, NP) return launch_after_wait(head_norm_gate_vec_kernel<TW, TG, NP>, grid, block, 0, stream, o, (const TG*)g, g_stride, (const TW*)w, (bf16*)out, H, dv, eps, act)
+#define HNV(TW, TG) { if (dv <= 128) HNV_N(TW, TG, 1); else if (dv <= 256) HNV_N(TW, TG, 2); else HNV_N(TW, TG, 4); }
+        if (w_dtype == TL_F32) { if (g_dtype == TL_F32) HNV(float, float) else HNV(float, bf16) }
+        else { if (g_dtype == TL_F32) HNV(bf16, float) else HNV(bf16, bf16) }
+#undef HNV
+#undef HNV_N
+    }
 #define HNG(TA, TW, TG) launch_after_wait(head_norm_gate_kernel<TA, TW, TG>, grid, block, 0, stream, o, (const TG*)g, g_stride, (const TW*)w, (TA*)out, H, dv, eps, act)
 #define HNG_G(TA, TW) { if (g_dtype == TL_F32) HNG(TA, TW, float); else HNG(TA, TW, bf16); }
     if (act_dtype == TL_F32) { if (w_dtype == TL_F32) HNG_G(float, float) else HNG_G(float, bf16) }
