@@ -1,0 +1,453 @@
+// The gated delta rule of delta.cu for steps of many tokens: chunks of 32 tokens, inside a chunk matrix products, from chunk to chunk
+// the state.
+//
+//   S <- g_t S;   u_t = beta_t (v_t - S^T k_t);   S <- S + k_t u_t^T;   o_t = S^T q_t
+//
+// With F_t the sum of the log decays of a chunk up to t and S0 its start state, the corrections of a chunk solve a triangular system
+//   u_t + sum_{s<t} A_ts u_s = beta_t (v_t - e^F_t S0^T k_t),      A_ts = beta_t e^(F_t - F_s) k_t . k_s
+// so U = U0 - W S0 with U0 = (I + A)^-1 (beta V) and W = (I + A)^-1 (beta e^F K), and
+//   o_t = e^F_t S0^T q_t + sum_{s<=t} e^(F_t - F_s) (q_t . k_s) u_s,      S = e^F_end S0 + sum_t e^(F_end - F_t) k_t u_t^T.
+//   prepare   every chunk of every head at once: A, the weights P of the outputs, U0 and W (a thread a column of the system)
+//   walk      a block a request, head and 16 columns of the state: chunk after chunk U, the outputs and the state
+//
+// Everything is held in float, and the walk's products are float products on the tensor cores: each factor is cut into three
+// bfloat16 parts (24 bits of it), six of the nine products of parts are taken (the other three lie below a float's last
+// bit), the leading one in an accumulator of its own, so that the others' roundings count 2^-8.  F is a sum of doubles, every weight
+// the float exponential of one difference of them.  The state in the slots has the layout of the scan kernel.  A position's
+// sums depend on where its step began, to rounding.
+//
+// The token-by-token kernel is bound by its chain: two column sums with shuffles a token, 0.31 us.  As float multiply-adds the walk
+// is bound by shared memory: a warp gets 32 floats of it a cycle and needs one for two multiply-adds with 16 columns a
+// block (measured 286 us for 2,048 tokens, 8 heads of 128 x 256; token by token 642).  On mma.sync a warp holds 32 rows of the transposed state [16 columns x 128 rows] as
+// accumulators, which are the next product's first operand as they lie; W, K, Q and P come as bfloat16 parts, cut once
+// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 40.
+#include "common.cuh"
+
+constexpr int DC_C = 32;                 // tokens a chunk
+constexpr int DC_COLS = 16;              // columns a block of the walk and a slice of the state's layout
+constexpr int DC_UB = DC_C * 20 * 4;     // bytes of a slice of U0: 32 rows of 16 floats, 20 apart
+constexpr int DC_PROW = DC_C * 2 + 16, DC_PB = 3 * DC_C * DC_PROW;      // a row of a part of P, the three parts
+constexpr int DC_MB = 2 * DC_C * 4;      // e^F_t, then e^(F_end - F_t)
+__host__ __device__ constexpr int dc_row(int dp) { return dp * 2 + 16; }              // bytes of a row of a part of W, K, Q
+__host__ __device__ constexpr int dc_parts(int dp) { return 3 * DC_C * dc_row(dp); }  // bytes of the three parts
+
+struct DeltaChunkArgs {
+    const float* qkv; int stride; int q_off, k_off, v_off;      // as conv_prep left them
+    const float* gates; int gate_stride; const float* A_log; const float* dt_bias;
+    float* state; long long slot_stride;
+    const int* q_start; const int* slots;
+    const int4* chunks;                  // (request, number of the chunk, the request's chunks, first chunk of the request in the list)
+    const int* firsts;                   // the requests' first chunks
+    unsigned char* W;                    // [chunks][H] parts of W
+    unsigned char* P;                    // [chunks][H] parts of P, row t
+    unsigned char* M;                    // [chunks][H] marks
+    unsigned char* U;                    // [chunks][H][nz] slices of U0
+    unsigned char* K;                    // [chunks][nqk] parts of K, then of Q
+    float* out;
+    int H, nqk, d, dv, nz;
+};
+
+__device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
+// The three bfloat16 parts of two floats, packed (the first in the low half).
+__device__ __forceinline__ void dc_cut(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+    auto pack = [](float x, float y) {
+        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+        return *reinterpret_cast<const uint32_t*>(&v);
+    };
+    hi = pack(a, b);
+    a -= __uint_as_float(hi << 16); b -= __uint_as_float(hi & 0xffff0000u);
+    mid = pack(a, b);
+    a -= __uint_as_float(mid << 16); b -= __uint_as_float(mid & 0xffff0000u);
+    lo = pack(a, b);
+}
+
+// ------------------------------------------------------------------ prepare
+// grid (chunks, H), 256 threads; shared memory K, Q [32][DP + 4], V [32][dv]
+template <int DP>
+__global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A) {
+    constexpr int LD = DP + 4, ROW = dc_row(DP);
+    extern __shared__ __align__(16) float sm[];
+    float* Ks = sm;
+    float* Qs = sm + DC_C * LD;
+    float* Vs = Qs + DC_C * LD;
+    __shared__ __align__(16) float As[DC_C][DC_C];       // A, row t: read as broadcasts
+    __shared__ __align__(16) float Ps[DC_C][DC_C + 4];
+    __shared__ double F[DC_C];
+    __shared__ float beta[DC_C], grow[DC_C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, rep = A.H / A.nqk, hq = h / rep, d = A.d, dv = A.dv;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int t0 = A.q_start[ck.x] + ck.y * DC_C, n = min(DC_C, A.q_start[ck.x + 1] - t0);
+    const size_t at = (size_t)blockIdx.x * A.H + h;
+    auto copy16 = [&](float* dst, const float* src, bool ok) {       // zeros where !ok
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(ok ? src : A.qkv), "r"(ok ? 16 : 0)
+                     : "memory");
+    };
+    for (int i = tid; i < DC_C * DP / 4; i += 256) {
+        const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
+        const float* row = A.qkv + (size_t)(t0 + t) * A.stride + hq * d + e;
+        copy16(Qs + t * LD + e, row + A.q_off, t < n && e < d);
+        copy16(Ks + t * LD + e, row + A.k_off, t < n && e < d);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = tid; i < DC_C * dv / 4; i += 256) {
+        const int t = i / (dv / 4), e = (i - t * (dv / 4)) * 4;
+        copy16(Vs + t * dv + e, A.qkv + (size_t)(t0 + t) * A.stride + A.v_off + h * dv + e, t < n);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (wid == 0) {
+        double x = 0.0;
+        float b = 0.f;
+        if (lane < n) {
+            const float* g = A.gates + (size_t)(t0 + lane) * A.gate_stride;
+            b = 1.0f / (1.0f + expf(-g[h]));
+            x = -expf(A.A_log[h]) * dc_softplus(g[A.H + h] + A.dt_bias[h]);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const double end = __shfl_sync(0xffffffffu, x, 31);          // tokens behind the chunk's last add nothing
+        F[lane] = x; beta[lane] = b; grow[lane] = expf((float)x);
+        float* mk = reinterpret_cast<float*>(A.M + at * DC_MB);
+        mk[lane] = expf((float)x);
+        mk[DC_C + lane] = expf((float)(end - x));
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    if (h == hq * rep) {                                 // the parts of K and Q, once for the heads that share them
+        unsigned char* to = A.K + ((size_t)blockIdx.x * A.nqk + hq) * 2 * dc_parts(DP);
+        for (int i = tid; i < 2 * DC_C * DP / 4; i += 256) {
+            const bool isq = i >= DC_C * DP / 4;
+            const int j = isq ? i - DC_C * DP / 4 : i, t = j / (DP / 4), e = (j % (DP / 4)) * 4;
+            const float4 x = *reinterpret_cast<const float4*>((isq ? Qs : Ks) + t * LD + e);
+            uint2 p[3];
+            dc_cut(x.x, x.y, p[0].x, p[1].x, p[2].x);
+            dc_cut(x.z, x.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) *reinterpret_cast<uint2*>(to + (isq ? dc_parts(DP) : 0) + (c * DC_C + t) * ROW + e * 2) = p[c];
+        }
+    }
+    {                                                    // k_t . k_s and q_t . k_s: tokens ty, ty + 16 against tx, tx + 16
+        const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
+        float kk[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qk[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+        for (int e = 0; e < DP; e += 4) {
+            float4 a[2], q[2], b[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                a[i] = *reinterpret_cast<const float4*>(Ks + (ty + 16 * i) * LD + e);
+                q[i] = *reinterpret_cast<const float4*>(Qs + (ty + 16 * i) * LD + e);
+                b[i] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * i) * LD + e);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j <= i; ++j) {
+                    kk[i][j] = fmaf(a[i].x, b[j].x, kk[i][j]); kk[i][j] = fmaf(a[i].y, b[j].y, kk[i][j]);
+                    kk[i][j] = fmaf(a[i].z, b[j].z, kk[i][j]); kk[i][j] = fmaf(a[i].w, b[j].w, kk[i][j]);
+                    qk[i][j] = fmaf(q[i].x, b[j].x, qk[i][j]); qk[i][j] = fmaf(q[i].y, b[j].y, qk[i][j]);
+                    qk[i][j] = fmaf(q[i].z, b[j].z, qk[i][j]); qk[i][j] = fmaf(q[i].w, b[j].w, qk[i][j]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int t = ty + 16 * i, s = tx + 16 * j;
+                const float w = s <= t && t < n ? expf((float)(F[t] - F[s])) : 0.f;
+                As[t][s] = s < t ? beta[t] * (w * kk[i][j]) : 0.f;
+                Ps[t][s] = w * qk[i][j];
+            }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int i = tid; i < DC_C * DC_C / 2; i += 256) {
+        const int t = i / (DC_C / 2), x = (i % (DC_C / 2)) * 2;
+        const float2 v = *reinterpret_cast<const float2*>(&Ps[t][x]);
+        uint32_t p[3];
+        dc_cut(v.x, v.y, p[0], p[1], p[2]);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(A.P + at * DC_PB + (c * DC_C + t) * DC_PROW + x * 2) = p[c];
+    }
+    const int wide = (dv + 15) & ~15;                    // columns behind the last are zeros, like rows behind d
+    for (int c = tid; c < wide + DP; c += 256) {
+        float u[DC_C];
+        const bool isw = c >= wide;
+        const int e = c - wide;
+#pragma unroll
+        for (int t = 0; t < DC_C; ++t) {
+            if (isw) u[t] = beta[t] * (grow[t] * Ks[t * LD + e]);
+            else u[t] = c < dv ? beta[t] * Vs[t * dv + c] : 0.f;
+        }
+#pragma unroll
+        for (int t = 1; t < DC_C; ++t) {
+            float s0 = 0.f, s1 = 0.f;                    // two chains a row
+#pragma unroll
+            for (int s = 0; s < t; s += 4) {
+                const float4 a = *reinterpret_cast<const float4*>(&As[t][s]);
+                s0 = fmaf(a.x, u[s], s0);
+                if (s + 1 < t) s1 = fmaf(a.y, u[s + 1], s1);
+                if (s + 2 < t) s0 = fmaf(a.z, u[s + 2], s0);
+                if (s + 3 < t) s1 = fmaf(a.w, u[s + 3], s1);
+            }
+            u[t] -= s0 + s1;
+        }
+        if (isw) {
+            __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(A.W + at * dc_parts(DP)) + e;
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) {
+                float x = u[t];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const __nv_bfloat16 b = __float2bfloat16_rn(x);
+                    to[(p * DC_C + t) * (ROW / 2)] = b;
+                    x -= __bfloat162float(b);
+                }
+            }
+        } else {
+            float* to = reinterpret_cast<float*>(A.U + (at * A.nz + c / DC_COLS) * DC_UB) + c % DC_COLS;
+#pragma unroll
+            for (int t = 0; t < DC_C; ++t) to[t * 20] = u[t];
+        }
+    }
+}
+
+// ------------------------------------------------------------------ walk
+__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void dc_load4(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+__device__ __forceinline__ void dc_load4_trans(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+// c (leading parts) and s (the rest) += A B over the parts a[3], b of the fragment pair starting at b[.][i]
+__device__ __forceinline__ void dc_mma6(float (&c)[4], float (&s)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int i) {
+    dc_mma(s, a[2], b[0][i], b[0][i + 1]);
+    dc_mma(c, a[0], b[0][i], b[0][i + 1]);
+    dc_mma(s, a[0], b[2][i], b[2][i + 1]);
+    dc_mma(s, a[1], b[1][i], b[1][i + 1]);
+    dc_mma(s, a[1], b[0][i], b[0][i + 1]);
+    dc_mma(s, a[0], b[1][i], b[1][i + 1]);
+}
+
+template <int DP> struct WalkShape {
+    static constexpr int PARTS = dc_parts(DP);
+    static constexpr int W = 0, K = PARTS, Q = 2 * PARTS, P = 3 * PARTS, U = P + DC_PB, M = U + DC_UB, BUF = M + DC_MB;      // bytes of a buffer
+    static constexpr int LP = 40;                        // stride of a column of the partial sums, in tokens: float pairs of 16 lanes meet no bank twice
+    static constexpr int SUMS = 4 * DC_COLS * LP * 4;    // bytes: [warp][column][LP]
+    static constexpr int BYTES = 2 * BUF + 2 * SUMS;
+};
+
+// grid (requests, H, slices of 16 columns), four warps, DP / 4 rows of the state each
+template <int DP>
+__global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
+    using Sh = WalkShape<DP>;
+    constexpr int ROW = dc_row(DP), RW = DP / 4, NT = RW / 8, KT = RW / 16, LP = Sh::LP;
+    constexpr int R = 8, IS = DP / R, LAYOUT = IS * DC_COLS, PB = R * LAYOUT;      // the slot's layout
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+    float* sums_w = reinterpret_cast<float*>(smem + 2 * Sh::BUF);
+    float* sums_q = sums_w + Sh::SUMS / 4;
+    const int first = A.firsts[blockIdx.x], h = blockIdx.y, hq = h / (A.H / A.nqk), z = blockIdx.z, dv = A.dv;
+    const int4 ck = A.chunks[first];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+    const int row0 = A.q_start[ck.x], T = A.q_start[ck.x + 1] - row0;
+    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + ((size_t)h * A.nz + z) * PB;
+    auto place = [&](int row, int c) { return (row % R) * LAYOUT + c * IS + row / R; };
+    // S transposed: element (column g or g + 8, row wid RW + 8 i + q2 or + 1)
+    float S[NT][4];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const int row = wid * RW + 8 * i + q2;
+        S[i][0] = slot[place(row, g)]; S[i][1] = slot[place(row + 1, g)];
+        S[i][2] = slot[place(row, g + 8)]; S[i][3] = slot[place(row + 1, g + 8)];
+    }
+    auto copy = [&](int to, const unsigned char* from, int bytes) {
+        for (int i = tid * 16; i < bytes; i += 128 * 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + to + i), "l"(from + i) : "memory");
+    };
+    auto fetch = [&](int c) {
+        const int b = (c & 1) * Sh::BUF;
+        const size_t at = (size_t)(first + c) * A.H + h;
+        copy(b + Sh::W, A.W + at * Sh::PARTS, Sh::PARTS);
+        copy(b + Sh::K, A.K + ((size_t)(first + c) * A.nqk + hq) * 2 * Sh::PARTS, 2 * Sh::PARTS);      // K, then Q
+        copy(b + Sh::P, A.P + at * DC_PB, DC_PB);
+        copy(b + Sh::U, A.U + (at * A.nz + z) * DC_UB, DC_UB);
+        copy(b + Sh::M, A.M + at * DC_MB, DC_MB);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    // this lane's addresses in fragments of two tiles: rows (tokens) of W, Q, P, and of K as it is transposed
+    const uint32_t x_at = ((lane & 7) + (lane >> 4) * 8) * ROW + ((lane >> 3) & 1) * 16 + wid * RW * 2;
+    const uint32_t k_at = ((lane & 7) + ((lane >> 3) & 1) * 8) * ROW + (lane >> 4) * 16 + wid * RW * 2;
+    const uint32_t p_at = (wid * 8 + (lane & 7)) * DC_PROW + (lane >> 3) * 16;
+    for (int c = 0; c < ck.z; ++c) {
+        const int n = min(DC_C, T - c * DC_C);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();                                 // the chunk's operands have landed, the chunk before is read
+        if (c + 1 < ck.z) fetch(c + 1);
+        const unsigned char* buf = smem + (c & 1) * Sh::BUF;
+        const uint32_t at = base + (c & 1) * Sh::BUF;
+        const float* u0 = reinterpret_cast<const float*>(buf + Sh::U);
+        const float* mk = reinterpret_cast<const float*>(buf + Sh::M);
+        uint32_t sa[KT][3][4];                           // S transposed as a first operand: [columns][rows]
+#pragma unroll
+        for (int k = 0; k < KT; ++k)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const float (&v)[4] = S[2 * k + (x >> 1)];
+                dc_cut(v[(x & 1) * 2], v[(x & 1) * 2 + 1], sa[k][0][x], sa[k][1][x], sa[k][2][x]);
+            }
+        // (W S)^T and (Q S)^T over this warp's rows: [16 columns][32 tokens]
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+            float big[4][4], rest[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) big[j][x] = rest[j][x] = 0.f;
+#pragma unroll
+            for (int k = 0; k < KT; ++k)
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                    uint32_t b[3][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) dc_load4(b[p], at + (which ? Sh::Q : Sh::W) + (p * DC_C + j * 8) * ROW + x_at + k * 32);
+                    dc_mma6(big[j], rest[j], sa[k], b, 0);
+                    dc_mma6(big[j + 1], rest[j + 1], sa[k], b, 2);
+                }
+            float* to = (which ? sums_q : sums_w) + (wid * DC_COLS + g) * LP + q2;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                *reinterpret_cast<float2*>(to + 8 * j) = make_float2(big[j][0] + rest[j][0], big[j][1] + rest[j][1]);
+                *reinterpret_cast<float2*>(to + 8 * LP + 8 * j) = make_float2(big[j][2] + rest[j][2], big[j][3] + rest[j][3]);
+            }
+        }
+        __syncthreads();
+        // u transposed as a first operand [columns][tokens]: as it is, and weighted for the end state
+        uint32_t ua[2][3][4], wa[2][3][4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int col = g + (x & 1) * 8, t = 16 * k + (x >> 1) * 8 + q2;
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const float2 v = *reinterpret_cast<const float2*>(sums_w + (w * DC_COLS + col) * LP + t);
+                    s.x += v.x; s.y += v.y;
+                }
+                const float a = u0[t * 20 + col] - s.x, b = u0[(t + 1) * 20 + col] - s.y;
+                dc_cut(a, b, ua[k][0][x], ua[k][1][x], ua[k][2][x]);
+                dc_cut(a * mk[DC_C + t], b * mk[DC_C + t + 1], wa[k][0][x], wa[k][1][x], wa[k][2][x]);
+            }
+        // the new state
+        {
+            const float end = mk[n - 1];
+#pragma unroll
+            for (int i = 0; i < NT; i += 2) {
+                float big[2][4] = {}, rest[2][4] = {};
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    uint32_t b[3][4];
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) dc_load4_trans(b[p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at + i * 16);
+                    dc_mma6(big[0], rest[0], wa[k], b, 0);
+                    dc_mma6(big[1], rest[1], wa[k], b, 2);
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) S[i + j][x] = fmaf(end, S[i + j][x], big[j][x] + rest[j][x]);
+            }
+        }
+        // outputs of tokens 8 wid ..
+        {
+            float big[4] = {}, rest[4] = {};
+            uint32_t b[3][4];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) dc_load4(b[p], at + Sh::P + p * DC_C * DC_PROW + p_at);
+            dc_mma6(big, rest, ua[0], b, 0);
+            dc_mma6(big, rest, ua[1], b, 2);
+            const int t = 8 * wid + q2;
+            const float2 e = *reinterpret_cast<const float2*>(mk + t);
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const float2 v = *reinterpret_cast<const float2*>(sums_q + (w * DC_COLS + g + 8 * x) * LP + t);
+                    s.x += v.x; s.y += v.y;
+                }
+                const int col = z * DC_COLS + g + 8 * x;
+                if (col < dv) {
+                    float* to = A.out + (size_t)(row0 + c * DC_C + t) * A.H * dv + (size_t)h * dv + col;
+                    if (t < n) to[0] = fmaf(e.x, s.x, big[2 * x] + rest[2 * x]);
+                    if (t + 1 < n) to[(size_t)A.H * dv] = fmaf(e.y, s.y, big[2 * x + 1] + rest[2 * x + 1]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const int row = wid * RW + 8 * i + q2;
+        slot[place(row, g)] = S[i][0]; slot[place(row + 1, g)] = S[i][1];
+        slot[place(row, g + 8)] = S[i][2]; slot[place(row + 1, g + 8)] = S[i][3];
+    }
+}
+
+template <int DP>
+static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int n_chunks, int requests, cudaStream_t stream) {
+    using Sh = WalkShape<DP>;
+    const int prep_smem = (2 * DC_C * (DP + 4) + DC_C * A.dv) * 4;
+    static int raised[TL_MAX_DEVICES] = {};              // what prepare's shared memory was raised to
+    const int dev = tl_device_index();
+    if (dev < 0) return 1;
+    if (raised[dev] < prep_smem) {
+        cudaError_t e = cudaFuncSetAttribute(dc_prepare_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(dc_walk_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::BYTES);
+        if (e != cudaSuccess) return (int)e;
+        raised[dev] = prep_smem;
+    }
+    const size_t ch = (size_t)n_chunks * A.H;
+    A.W = scratch;
+    A.P = A.W + ch * Sh::PARTS;
+    A.M = A.P + ch * DC_PB;
+    A.U = A.M + ch * DC_MB;
+    A.K = A.U + ch * A.nz * DC_UB;
+    dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), 256, prep_smem, stream>>>(A);
+    const int e = tl_launch_status();
+    if (e) return e;
+    dc_walk_kernel<DP><<<dim3(requests, A.H, A.nz), 128, Sh::BYTES, stream>>>(A);
+    return tl_launch_status();
+}
+
+constexpr int DC_DV_MAX = 1024;          // V of a chunk lies in shared memory beside K and Q
+
+TL_EXPORT int tl_delta_chunk() { return DC_C; }
+// Bytes of scratch a chunk; 0: these sizes run token by token (heads of up to 32, whose state has another layout, and wide ones,
+// whose operands fill shared memory once).
+TL_EXPORT int tl_delta_chunk_bytes(int H, int nqk, int d, int dv) {
+    if (d <= 32 || d > 128 || (d & 3) || (dv & 3) || dv > DC_DV_MAX) return 0;
+    const int parts = d <= 64 ? dc_parts(64) : dc_parts(128);
+    return H * (parts + DC_PB + DC_MB + (dv + DC_COLS - 1) / DC_COLS * DC_UB) + nqk * 2 * parts;
+}
+
+// scratch: `tl_delta_chunk_bytes` bytes a chunk.  The offsets and the stride are multiples of 4, the pointers 16-byte aligned.
+TL_EXPORT int tl_delta_chunks(const float* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, int gate_stride,
+                              const float* A_log, const float* dt_bias, float* state, long long slot_stride, const int* q_start,
+                              const int* slots, const int* chunks, int n_chunks, const int* firsts, int requests, void* scratch, float* out,
+                              int H, int nqk, int d, int dv, cudaStream_t stream) {
+    if (n_chunks <= 0 || H <= 0) return 0;
+    if (H > 65535 || nqk < 1 || H % nqk || !tl_delta_chunk_bytes(H, nqk, d, dv) || ((stride | q_off | k_off | v_off) & 3) ||
+        ((((uintptr_t)qkv) | ((uintptr_t)scratch) | ((uintptr_t)out)) & 15)) return 1;
+    const DeltaChunkArgs A{qkv, stride, q_off, k_off, v_off, gates, gate_stride, A_log, dt_bias, state, slot_stride, q_start, slots,
+                           (const int4*)chunks, firsts, nullptr, nullptr, nullptr, nullptr, nullptr, out, H, nqk, d, dv, (dv + DC_COLS - 1) / DC_COLS};
+    if (d <= 64) return dc_launch<64>(A, (unsigned char*)scratch, n_chunks, requests, stream);
+    return dc_launch<128>(A, (unsigned char*)scratch, n_chunks, requests, stream);
+}

@@ -16,7 +16,7 @@ from .csrc.build import CHECK_BUILD, load_library
 
 CORE_SOURCES = ["elementwise.cu", "rope_kv.cu", "attn_tokenwise.cu", "gemm_f32.cu", "sampling.cu", "recurrent.cu", "moe.cu",
                 "delta.cu", "latent.cu", "rglru.cu", "streams.cu", "stream_norm.cu", "attn_mixed_tokenwise.cu",
-                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu"]
+                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu", "delta_chunk.cu"]
 
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -61,6 +61,9 @@ _SIGNATURES = {
     "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
     "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
+    "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "tl_delta_chunk": [],
+    "tl_delta_chunk_bytes": [_I, _I, _I, _I],
     "tl_delta_state_floats": [_I, _I],
     "tl_delta_columns": [],
     "tl_latent_prep": [_P, _I, _I, _I, _I, _P, _P, _I, _F, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P],
@@ -805,6 +808,17 @@ def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int) -> 
         proj.shape[1] % 4 == 0 and proj.data_ptr() % 16 == 0
 
 
+def _chunk_list(ctx, key: str, chunk: int, device) -> tuple:
+    """The step's chunks of `chunk` tokens on the device (`channel_chunks`' rows, then every request's first row), how many there
+    are, and of how many requests: one description a step, for every layer."""
+    if key not in ctx.scratch:
+        rows, _ = channel_chunks(ctx.h_q_start, chunk)
+        firsts = np.nonzero(rows[:, 1] == 0)[0].astype(np.int32)
+        both = torch.from_numpy(np.concatenate([rows.reshape(-1), firsts])).to(device, non_blocking=True)
+        ctx.scratch[key] = (both, len(rows), len(firsts))
+    return ctx.scratch[key]
+
+
 def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, d: int, dv: int, state: torch.Tensor, ctx, out: torch.Tensor,
                   *, decay: torch.Tensor | None = None, gates: torch.Tensor | None = None, cap: float = 1.0, inv_freq: torch.Tensor | None = None,
                   rot: int = 0, pairing: str = "half", q_scale: float = 1.0, k_scale: float = 1.0, den_eps: float = 0.0) -> None:
@@ -832,13 +846,7 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
     if rot and (inv_freq is None or inv_freq.dtype != torch.float32 or inv_freq.numel() != rot // 2):
         raise KernelError("linear_chunks: inv_freq must be float32 [rot/2]")
     interleaved = _pairing(pairing, "linear_chunks")
-    key = "linear_chunks"
-    if key not in ctx.scratch:                           # one description a step, for every layer
-        rows, _ = channel_chunks(ctx.h_q_start, core().tl_linear_chunk())
-        firsts = np.nonzero(rows[:, 1] == 0)[0].astype(np.int32)
-        both = torch.from_numpy(np.concatenate([rows.reshape(-1), firsts])).to(proj.device, non_blocking=True)
-        ctx.scratch[key] = (both, len(rows), len(firsts))
-    both, n, requests = ctx.scratch[key]
+    both, n, requests = _chunk_list(ctx, "linear_chunks", core().tl_linear_chunk(), proj.device)
     dev = proj.device
     turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
     ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
@@ -1159,6 +1167,45 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt_b
 
 # ---------------------------------------------------------------------------------------------
 # Attention through a latent (csrc/latent.cu)
+
+# From this many tokens of one request a bfloat16 step's delta rule runs chunk by chunk instead of token by token (8 heads of 128 x
+# 256: 64 tokens 24 us token by token against 34, the host's two launches and their scratch; 128 tokens 43 against 33; 2,048 tokens
+# 632 against 171).
+DELTA_CHUNKS_MIN_TOKENS = 96
+
+
+def takes_delta_chunks(qkv: torch.Tensor, H: int, nqk: int, d: int, dv: int, max_q_len: int) -> bool:
+    """Whether `delta_chunks` takes these sizes and is the faster way."""
+    return max_q_len >= DELTA_CHUNKS_MIN_TOKENS and core().tl_delta_chunk_bytes(H, nqk, d, dv) > 0 and qkv.shape[1] % 4 == 0 and \
+        qkv.data_ptr() % 16 == 0
+
+
+def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, ctx,
+                 out: torch.Tensor, *, H: int, nqk: int, d: int, dv: int) -> None:
+    """`delta_scan` (not compensated) for steps of several tokens a request: chunks of 32 tokens, inside a chunk matrix products of
+    floats (on the tensor cores as products of their bfloat16 parts).  The state as `delta_scan` keeps it, so the two may take turns.  A position's sums depend on where its step began, to
+    rounding."""
+    T = qkv.shape[0]
+    _contig(qkv, "qkv"); _contig(out, "out"); _contig(state, "state")
+    if qkv.dtype != torch.float32 or qkv.shape[1] != 2 * nqk * d + H * dv or out.dtype != torch.float32 or out.shape != (T, H * dv):
+        raise KernelError("delta_chunks: qkv float32 [T, 2 nqk d + H dv], out float32 [T, H dv]")
+    if gates.dtype != torch.float32 or gates.shape[1] < 2 * H or gates.stride(1) != 1:
+        raise KernelError("delta_chunks: gates must be float32 with at least 2H columns and unit inner stride")
+    per_slot = H * -(-dv // delta_columns()) * delta_state_floats(d)
+    if state.dtype != torch.float32 or state[0].numel() != per_slot:
+        raise KernelError(f"delta_chunks: a slot holds {state[0].numel()} floats, these sizes need {per_slot}")
+    for name, t in (("A_log", A_log), ("dt_bias", dt_bias)):
+        if t.dtype != torch.float32 or t.numel() != H or not t.is_contiguous():
+            raise KernelError(f"delta_chunks: {name} must be float32 [H]")
+    per_chunk = core().tl_delta_chunk_bytes(H, nqk, d, dv)
+    if not per_chunk or qkv.shape[1] & 3 or qkv.data_ptr() & 15:
+        raise KernelError("delta_chunks: q/k heads of 36 to 128, sizes in multiples of 4, 16-byte rows")
+    both, n, requests = _chunk_list(ctx, "delta_chunks", core().tl_delta_chunk(), qkv.device)
+    scratch = torch.empty(n * per_chunk, dtype=torch.uint8, device=qkv.device)
+    _check(core().tl_delta_chunks(_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias),
+                                  _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n, requests,
+                                  _ptr(scratch), _ptr(out), H, nqk, d, dv, _stream()), "delta_chunks", launches=2)
+
 
 def latent_prep(down: torch.Tensor, qr: int, rank: int, dr: int, wq: torch.Tensor, wkv: torch.Tensor, eps: float,
                 inv_freq: torch.Tensor, rot: int, pos: torch.Tensor, req_slot: torch.Tensor, table: torch.Tensor, page_size: int,

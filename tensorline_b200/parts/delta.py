@@ -90,8 +90,11 @@ class GatedDelta(Part):
         ops.conv_prep(proj, self.taps_w, inputs, ctx.q_start, ctx.slots, qkv, B=ctx.B, max_q_len=ctx.max_q_len, nqk=nqk, d=d,
                       nv=H, dv=dv, unit_eps=self.unit_eps, q_scale=d ** -0.5)
         o = torch.empty((T, H * dv), dtype=torch.float32, device=h.device)
-        ops.delta_scan(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx.q_start, ctx.slots, o, B=ctx.B, H=H,
-                       nqk=nqk, d=d, dv=dv, max_q_len=ctx.max_q_len, compensated=self.compensated)
+        if not self.compensated and not ctx.decode_only and ops.takes_delta_chunks(qkv, H, nqk, d, dv, ctx.max_q_len):
+            ops.delta_chunks(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx, o, H=H, nqk=nqk, d=d, dv=dv)
+        else:
+            ops.delta_scan(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx.q_start, ctx.slots, o, B=ctx.B, H=H,
+                           nqk=nqk, d=d, dv=dv, max_q_len=ctx.max_q_len, compensated=self.compensated)
         y = torch.empty((T, H * dv), dtype=h.dtype, device=h.device)
         ops.head_norm_gate(o, y, H, dv, self.eps, weight=self.head_weight, gate=proj, gate_off=C, act="silu")
         return matmul(y, self.w_o)

@@ -1,0 +1,72 @@
+"""The delta rule in chunks (`ops.delta_chunks`): against the recurrence in float64 over the forms it accepts and beside the
+token-by-token kernel, whose state it shares: its error may be no larger than that kernel's (or 2e-6, a few dozen roundings of
+float sums)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def slot_rows(S):
+    H, d, dv = S.shape
+    R, IS = (4, 8) if d <= 32 else (8, 8) if d <= 64 else (8, 16) if d <= 128 else (8, 32)
+    nz = -(-dv // 16)
+    out = torch.zeros(H, nz, R * IS * 16, dtype=S.dtype)
+    i, j = torch.meshgrid(torch.arange(d), torch.arange(dv), indexing="ij")
+    out[:, j // 16, (i % R) * IS * 16 + (j % 16) * IS + i // R] = S
+    return out.reshape(-1)
+
+
+@pytest.mark.parametrize("H,nqk,d,dv,lens,like", [
+    (4, 2, 128, 256, [64, 33, 1], 0.0), (2, 2, 64, 64, [200], 0.0), (3, 1, 36, 132, [31, 32, 97], 0.0), (2, 1, 64, 36, [70], 0.0),
+    (2, 2, 40, 20, [40, 3], 0.0), (2, 1, 96, 128, [160], 0.9), (1, 1, 124, 64, [65], 0.0), (1, 1, 128, 4, [129], 0.5), (2, 2, 128, 64, [96], 0.99)])
+def test_delta_chunks_against_the_recurrence_in_float64(H, nqk, d, dv, lens, like):
+    """`like`: how alike the keys are (the system of a chunk is the further from the identity)."""
+    from tensorline_b200 import ops
+    g = torch.Generator().manual_seed(d * dv + sum(lens))
+    T, B = sum(lens), len(lens)
+    q, k = torch.randn(T, nqk, d, generator=g), torch.randn(T, nqk, d, generator=g) * (1 - like) + like * torch.randn(1, nqk, d, generator=g)
+    q, k = q / q.norm(dim=-1, keepdim=True) * d ** -0.5, k / k.norm(dim=-1, keepdim=True)
+    v = torch.randn(T, H, dv, generator=g)
+    qkv = torch.cat([q.reshape(T, -1), k.reshape(T, -1), v.reshape(T, -1)], dim=1)
+    gates = torch.randn(T, 2 * H + 4, generator=g)
+    gates[T // 2, H:2 * H] = 60.0                        # everything before is forgotten here
+    A_log, dt_bias = torch.randn(H, generator=g) - 2.0, torch.randn(H, generator=g) - 1.0
+    S0 = torch.randn(B, H, d, dv, generator=g) * 0.3
+    q_start = [0]
+    for n in lens:
+        q_start.append(q_start[-1] + n)
+    slots = torch.arange(B, 0, -1, dtype=torch.int32)
+    first = torch.stack([torch.zeros_like(slot_rows(S0[0]))] + [slot_rows(S0[b]) for b in range(B)][::-1])
+    qs, sl = torch.tensor(q_start, dtype=torch.int32).cuda(), slots.cuda()
+    args = (qkv.cuda(), gates.cuda(), A_log.cuda(), dt_bias.cuda())
+    state, out = first.cuda(), torch.full((T, H * dv), 7.0, device="cuda")
+    ops.delta_chunks(*args, state, SimpleNamespace(h_q_start=q_start, scratch={}, q_start=qs, slots=sl), out, H=H, nqk=nqk, d=d, dv=dv)
+    scan_state, scan_out = first.cuda(), torch.empty_like(out)
+    ops.delta_scan(*args, scan_state, qs, sl, scan_out, B=B, H=H, nqk=nqk, d=d, dv=dv, max_q_len=max(lens))
+    rep = H // nqk
+    q64, k64, v64, g64 = (x.double() for x in (q.repeat_interleave(rep, 1), k.repeat_interleave(rep, 1), v, gates))
+    beta = torch.sigmoid(g64[:, :H])
+    decay = torch.exp(-torch.exp(A_log.double()) * torch.nn.functional.softplus(g64[:, H:2 * H] + dt_bias.double()))
+    for b in range(B):
+        S, o = S0[b].double(), []
+        for t in range(q_start[b], q_start[b + 1]):
+            S = decay[t][:, None, None] * S
+            u = beta[t][:, None] * (v64[t] - torch.einsum("hd,hde->he", k64[t], S))
+            S = S + k64[t][:, :, None] * u[:, None, :]
+            o.append(torch.einsum("hd,hde->he", q64[t], S).reshape(-1))
+        rows = slice(q_start[b], q_start[b + 1])
+        for got, scan, want in ((out[rows], scan_out[rows], torch.stack(o)), (state[int(slots[b])], scan_state[int(slots[b])], slot_rows(S))):
+            err, base = (float((y.double().cpu() - want).norm()) / float(want.norm()) for y in (got, scan))
+            assert err <= max(2e-6, 1.5 * base), (err, base)
+    assert torch.equal(state[0].cpu(), first[0])
+
+
+def test_heads_that_run_token_by_token_are_refused():
+    from tensorline_b200 import ops
+    for d, dv in ((32, 64), (132, 64), (64, 30), (62, 64), (64, 1028)):
+        x = torch.zeros(128, 2 * d + dv, device="cuda")
+        assert not ops.takes_delta_chunks(x, 1, 1, d, dv, 128)
+    assert ops.takes_delta_chunks(torch.zeros(128, 192, device="cuda"), 1, 1, 64, 64, 128)
