@@ -144,6 +144,70 @@ __global__ void __launch_bounds__(256) conv_prep_tile_kernel(const TA* __restric
     }
 }
 
+// The same for steps of many tokens and 2 to 4 taps: a warp a (request, run of CONV_RUN tokens, head); a lane has channels lane + 32 m
+// of the head, their weights and the last taps - 1 inputs in registers, and the next token's inputs on their way while one is worked
+// through: a channel and token cost it one load and no index arithmetic.  What is left is the accurate exponential and division
+// of silu, about 35 instructions an output (134 with rows and weights in shared memory): 2,048 tokens, 3,072 channels 25 us against
+// 47.  The arithmetic of an output is conv_prep_kernel's, operation for operation, so all give the same bits.
+constexpr int CONV_RUN = 16;
+template <typename TA, typename TW, int TAPS>
+__global__ void __launch_bounds__(128) conv_prep_run_kernel(const TA* __restrict__ proj, int stride, const TW* __restrict__ taps_w,
+                                                            const float* __restrict__ conv_state, long long slot_stride,
+                                                            const int* __restrict__ q_start, const int* __restrict__ slots,
+                                                            float* __restrict__ out, int C, int nqk, int d, int nv, int dv,
+                                                            float unit_eps, float q_scale) {
+    const int b = blockIdx.x, lane = threadIdx.x & 31, u = blockIdx.z * 4 + (threadIdx.x >> 5);
+    grid_dependency_wait();
+    grid_dependency_trigger();
+    const int t0 = q_start[b], t1 = q_start[b + 1];
+    const int c0 = t0 + blockIdx.y * CONV_RUN, c1 = min(t1, c0 + CONV_RUN);
+    if (c0 >= t1 || u >= 2 * nqk + nv) return;
+    const bool qk = u < 2 * nqk;
+    const int width = qk ? d : dv, base = (qk ? u * d : 2 * nqk * d + (u - 2 * nqk) * dv) + lane;
+    const float* st = conv_state + (size_t)slots[b] * slot_stride + base;
+    const float unit_scale = u < nqk ? q_scale : 1.0f;
+    float w[CONV_KEEP][TAPS], x[CONV_KEEP][TAPS], next[CONV_KEEP];
+#pragma unroll
+    for (int m = 0; m < CONV_KEEP; ++m) {
+        const bool live = lane + 32 * m < width;
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            w[m][j] = live ? to_f<TW>(taps_w[(size_t)(base + 32 * m) * TAPS + j]) : 0.f;
+            const int src = c0 - t0 - (TAPS - 1) + j;    // x[j], j < TAPS - 1: the input TAPS - 1 - j tokens in front of the run
+            if (j < TAPS - 1)
+                x[m][j + 1] = !live ? 0.f : src >= 0 ? to_f<TA>(proj[(size_t)(t0 + src) * stride + base + 32 * m]) : st[(size_t)(TAPS - 1 + src) * C + 32 * m];
+        }
+        next[m] = live ? to_f<TA>(proj[(size_t)c0 * stride + base + 32 * m]) : 0.f;
+    }
+    for (int t = c0; t < c1; ++t) {
+        float y[CONV_KEEP];
+        float ss = 0.f;
+#pragma unroll
+        for (int m = 0; m < CONV_KEEP; ++m) {
+#pragma unroll
+            for (int j = 0; j < TAPS - 1; ++j) x[m][j] = x[m][j + 1];
+            x[m][TAPS - 1] = next[m];
+            if (t + 1 < c1 && lane + 32 * m < width) next[m] = to_f<TA>(proj[(size_t)(t + 1) * stride + base + 32 * m]);
+        }
+#pragma unroll
+        for (int m = 0; m < CONV_KEEP; ++m) {
+            y[m] = 0.f;
+            if (lane + 32 * m < width) {
+                float acc = 0.f;
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) acc = fmaf(w[m][j], x[m][j], acc);
+                y[m] = acc / (1.0f + expf(-acc));
+            }
+            ss = fmaf(y[m], y[m], ss);
+        }
+        float r = 1.0f;
+        if (qk) r = (1.0f / sqrtf(warp_sum(ss) + unit_eps)) * unit_scale;
+#pragma unroll
+        for (int m = 0; m < CONV_KEEP; ++m)
+            if (lane + 32 * m < width) out[(size_t)t * C + base + 32 * m] = qk ? y[m] * r : y[m];
+    }
+}
+
 // The slot's inputs after the step: the last taps - 1 of (what the slot held, then the step's inputs).  A thread a channel;
 // going from the oldest place on, every place reads a place behind it or the step's rows, so nothing is read after it
 // was overwritten.
@@ -174,7 +238,17 @@ TL_EXPORT int tl_conv_prep(const void* proj, int act_dtype, int stride, const vo
     const int widest = d > dv ? d : dv;
     int tt = (int)(40 * 1024 / sizeof(float)) / widest - (taps - 1);
     tt = tt > 32 ? 32 : tt;
-    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && tt >= 8 && 2 * nqk + nv <= 65535) {
+    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && taps >= 2 && taps <= 4) {
+        const dim3 grid(B, (max_q_len + CONV_RUN - 1) / CONV_RUN, (2 * nqk + nv + 3) / 4);
+        if (grid.y > 65535 || grid.z > 65535) return 1;
+#define CR_N(TA, TW, N) launch_after_wait(conv_prep_run_kernel<TA, TW, N>, grid, dim3(128), 0, stream, (const TA*)proj, stride, (const TW*)taps_w, \
+        (const float*)conv_state, slot_stride, q_start, slots, out, C, nqk, d, nv, dv, unit_eps, q_scale)
+#define CR(TA, TW) { if (taps == 2) CR_N(TA, TW, 2); else if (taps == 3) CR_N(TA, TW, 3); else CR_N(TA, TW, 4); }
+        if (act_dtype == TL_F32) { if (w_dtype == TL_F32) CR(float, float) else CR(float, bf16) }
+        else { if (w_dtype == TL_F32) CR(bf16, float) else CR(bf16, bf16) }
+#undef CR
+#undef CR_N
+    } else if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && tt >= 8 && 2 * nqk + nv <= 65535) {
         const dim3 grid(B, (max_q_len + tt - 1) / tt, 2 * nqk + nv);
         if (grid.y > 65535) return 1;
         const size_t smem = ((size_t)(tt + taps - 1) * widest + (size_t)widest * taps) * sizeof(float);
