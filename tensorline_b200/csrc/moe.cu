@@ -528,13 +528,28 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
     const int per = (P + nw - 1) / nw, lo = wid * per, hi = min(P, lo + per);      // a warp's contiguous range of pairs
     for (int p = lo + lane; p < hi; p += 32) atomicAdd(&cnt[idx[p] * nw + wid], 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int e = 0; e < E; ++e) {
-            base[e] = run;
-            for (int w = 0; w < nw; ++w) { const int c = cnt[e * nw + w]; cnt[e * nw + w] = run; run += c; }
+    // where every (expert, warp) starts: a warp an expert adds up the warps' counts, then one warp the experts' sums (one thread going
+    // through all of them: 23 us a launch with 32 experts, so 14)
+    for (int e = wid; e < E; e += nw) {
+        const int c = lane < nw ? cnt[e * nw + lane] : 0;
+        int run = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += x; }
+        if (lane < nw) cnt[e * nw + lane] = run - c;
+        if (lane == 31) base[e] = run;
+    }
+    __syncthreads();
+    if (wid == 0) {
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int c = e0 + lane < E ? base[e0 + lane] : 0;
+            int run = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) { const int x = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += x; }
+            if (e0 + lane < E) base[e0 + lane] = before + run - c;
+            before += __shfl_sync(0xffffffffu, run, 31);
         }
-        base[E] = run;
+        if (lane == 0) base[E] = before;
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = base[e];
@@ -548,7 +563,7 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
         if (e >= 0) start = cnt[e * nw + wid];
         __syncwarp();
         if (e >= 0) {
-            const int place = start + rank;
+            const int place = base[e] + start + rank;
             place_of[p] = place;
             pair_at[place] = p;
             if (rank == __popc(same) - 1) cnt[e * nw + wid] = start + rank + 1;
@@ -695,10 +710,66 @@ __global__ void moe_combine_kernel(const TA* __restrict__ rows, const int* __res
     }
 }
 
+// The same on bfloat16 rows in 16-byte pieces: a thread eight columns, the chosen rows' pieces four at a time in flight.  2,048 tokens
+// of 2,048 columns, 4 rows each and an addend: 50 MB, 13.5 us (a column a thread, a row after the other: 30).
+__global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* __restrict__ rows, const int* __restrict__ place_of, const int* __restrict__ idx,
+                                                              const int* __restrict__ offsets, int cap, const float* __restrict__ wts,
+                                                              bf16* __restrict__ y, int N, int top, const bf16* __restrict__ extra,
+                                                              const float* __restrict__ extra_gate, int ldg) {
+    __shared__ size_t at[32];
+    __shared__ float ws[32];
+    const int t = blockIdx.x;
+    if (threadIdx.x < top) {
+        const size_t pair = (size_t)t * top + threadIdx.x;
+        at[threadIdx.x] = moe_row(place_of[pair], idx[pair], offsets, cap) * N;
+        ws[threadIdx.x] = wts ? wts[pair] : 1.0f;
+    }
+    const float gt = !extra ? 0.f : extra_gate ? 1.0f / (1.0f + expf(-extra_gate[(size_t)t * ldg])) : 1.0f;
+    __syncthreads();
+    for (int n = threadIdx.x * 8; n < N; n += 256 * 8) {
+        float acc[8] = {};
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (extra) x = *reinterpret_cast<const uint4*>(extra + (size_t)t * N + n);
+        for (int j0 = 0; j0 < top; j0 += 4) {
+            uint4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) if (j0 + j < top) v[j] = *reinterpret_cast<const uint4*>(rows + at[j0 + j] + n);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j0 + j >= top) continue;
+                const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[j]);
+                const float w = ws[j0 + j];              // without weights: times one, exactly the plain sum
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    acc[2 * e] = fmaf(w, __low2float(p[e]), acc[2 * e]);
+                    acc[2 * e + 1] = fmaf(w, __high2float(p[e]), acc[2 * e + 1]);
+                }
+            }
+        }
+        if (extra) {
+            const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                acc[2 * e] = fmaf(gt, __low2float(p[e]), acc[2 * e]);
+                acc[2 * e + 1] = fmaf(gt, __high2float(p[e]), acc[2 * e + 1]);
+            }
+        }
+        uint4 o;
+        __nv_bfloat162* p = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[e] = __floats2bfloat162_rn(acc[2 * e], acc[2 * e + 1]);
+        *reinterpret_cast<uint4*>(y + (size_t)t * N + n) = o;
+    }
+}
+
 TL_EXPORT int tl_moe_combine(const void* rows, int act_dtype, const int* place_of, const int* idx, const int* offsets, int cap,
                              const float* wts, void* y, int T, int N, int top, const void* extra, const float* extra_gate, int ldg,
                              cudaStream_t stream) {
     if (T <= 0) return 0;
+    if (act_dtype != TL_F32 && N % 8 == 0 && top <= 32 && ((((uintptr_t)rows) | ((uintptr_t)y) | ((uintptr_t)extra)) & 15) == 0) {
+        moe_combine_vec_kernel<<<T, 256, 0, stream>>>((const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg);
+        return tl_launch_status();
+    }
     if (act_dtype == TL_F32) moe_combine_kernel<float><<<T, 256, 0, stream>>>((const float*)rows, place_of, idx, offsets, cap, wts, (float*)y, N, top, (const float*)extra, extra_gate, ldg);
     else moe_combine_kernel<bf16><<<T, 256, 0, stream>>>((const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg);
     return tl_launch_status();
