@@ -41,3 +41,48 @@ def test_a_tokens_rows_are_summed_in_the_order_chosen(N, top, weighted, shared):
         e = torch.sigmoid(gate.double())[:, None] * extra.double()
         want, size = want + e, size + e.abs()
     assert float(((y.double() - want).abs() - 2.0 ** -8 * want.abs() - 2.0 ** -20 * size).max()) <= 0.0
+
+
+@pytest.mark.parametrize("adt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,top,K,F,gated", [(1, 1, 8, 3, True), (3, 2, 264, 17, True), (5, 4, 2048, 40, False), (8, 4, 1032, 1, False), (2, 8, 520, 10, True),
+                                             (2, 2, 45, 6, True)])
+def test_streamed_experts_against_float64_and_token_by_token(T, top, K, F, gated, adt):
+    """K products of unit normals with weights of 0.05 in float32, rounded to the activation type (2^-8 for bfloat16)."""
+    from tensorline_b200 import ops
+    E, real = 9, 8
+    g = torch.Generator().manual_seed(T * K + F)
+    h = torch.randn(T, K, generator=g).to(adt)
+    up = (torch.randn(real, (2 if gated else 1) * F, K, generator=g) * 0.05).bfloat16()
+    down = (torch.randn(real, K, F, generator=g) * 0.2).bfloat16()
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    wts = torch.rand(T, top, generator=g)
+    act = "silu" if gated else "relu_squared"
+
+    def run(rows):
+        n = len(rows)
+        a = torch.zeros(n * top, F, dtype=adt, device="cuda")
+        y = torch.empty(n, K, dtype=adt, device="cuda")
+        hd, ix = h[rows].contiguous().cuda(), idx[rows].contiguous().cuda()
+        ops.moe_up(hd, up.cuda(), ix, a, act=act, gated=gated)
+        ops.moe_down(a, down.cuda(), ix, wts[rows].contiguous().cuda(), y, same=hd)
+        return a, y
+    a, y = run(list(range(T)))
+    for t in range(T):
+        a1, y1 = run([t])
+        assert torch.equal(a1, a[t * top:(t + 1) * top]) and torch.equal(y1[0], y[t])
+        want, size = torch.zeros(K, dtype=torch.float64), torch.zeros(K, dtype=torch.float64)
+        for j in range(top):
+            e = int(idx[t, j])
+            if e >= real:
+                p = h[t].double()
+            else:
+                u = up[e].double() @ h[t].double()
+                u = u[:F] * torch.sigmoid(u[:F]) * u[F:] if gated else torch.relu(u) ** 2
+                got = a[t * top + j].double().cpu()
+                assert float((got - u).abs().max()) <= (1e-5 if adt == torch.float32 else 2.0 ** -8) * (1 + float(u.abs().max()))
+                p = down[e].double() @ got
+                size += wts[t, j].double() * (down[e].double().abs() @ got.abs())
+            want += wts[t, j].double() * p
+            size += (wts[t, j].double() * p).abs()
+        rounding = 2.0 ** -8 if adt == torch.bfloat16 else 1e-6
+        assert float(((y[t].double().cpu() - want).abs() - rounding * want.abs() - 1e-5 * (1 + size)).max()) <= 0.0
