@@ -16,7 +16,8 @@
 //
 // What the scan kernel is bound by is the chain over the tokens at one block a head and 16 columns (128 blocks, 0.36 us a token);
 // here 12 multiply-adds of matrix products a state element and chunk token pair up in tiles of 4 x 8 and 8 x 8 a thread.
-// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; local 45, carry 25, outputs 81 us.
+// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; local 36 (45 with K and V fetched behind the weights), carry 25, outputs 81 us
+// (93 as tiles of 8 x 8 in half the threads: fewer floats from shared memory, too few warps to hide them).
 // 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
 // L2 once each way, weigh half as much again at 32.
 #include "common.cuh"
@@ -130,12 +131,19 @@ __global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) 
     const int h = blockIdx.y, col_tiles = (A.dv + CB - 1) / CB, row0 = (blockIdx.z / col_tiles) * RB, col0 = (blockIdx.z % col_tiles) * CB;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    auto copy16 = [&](float* dst, const float* src, bool ok) {       // zeros where !ok
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(ok ? src : A.v), "r"(ok ? 16 : 0)
+                     : "memory");
+    };
+    for (int i = tid; i < LC_C * RB / 4; i += 256) {
+        const int t = i / (RB / 4), e = (i % (RB / 4)) * 4;
+        copy16(Ks + t * RB + e, A.k + (size_t)(t0 + t) * A.qk_stride + h * A.d + row0 + e, t < n && row0 + e < A.d);
+    }
     for (int i = tid; i < LC_C * CB / 4; i += 256) {
         const int t = i / (CB / 4), c = (i % (CB / 4)) * 4;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < n && col0 + c < A.dv) x = *reinterpret_cast<const float4*>(A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c);
-        *reinterpret_cast<float4*>(Vs + t * CB + c) = x;
+        copy16(Vs + t * CB + c, A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c, t < n && col0 + c < A.dv);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
     if (wid == 0) {
         lc_weights<GATED>(A, t0, n, h, lane, F, u, top);
         __syncwarp();
@@ -147,14 +155,13 @@ __global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) 
         }
     }
     __syncthreads();
-    for (int i = tid; i < LC_C * RB / 4; i += 256) {
-        const int t = i / (RB / 4), e = (i % (RB / 4)) * 4;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (t < n && row0 + e < A.d) {
-            x = *reinterpret_cast<const float4*>(A.k + (size_t)(t0 + t) * A.qk_stride + h * A.d + row0 + e);
-            x.x *= w[t]; x.y *= w[t]; x.z *= w[t]; x.w *= w[t];
-        }
-        *reinterpret_cast<float4*>(Ks + t * RB + e) = x;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    for (int i = tid; i < LC_C * RB / 4; i += 256) {     // a thread weighs what it has fetched
+        float4* x = reinterpret_cast<float4*>(Ks + i * 4);
+        const float wt = w[i / (RB / 4)];
+        float4 v = *x;
+        v.x *= wt; v.y *= wt; v.z *= wt; v.w *= wt;
+        *x = v;
     }
     __syncthreads();
     const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
@@ -398,14 +405,14 @@ __global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
     }
     if (GATED) {                                         // n_t . q_t, four lanes a token
         const int t = tid >> 2, part = tid & 3;
-        float s = 0.f, r = 0.f;
+        double s = 0.0, r = 0.0;                         // the sum may nearly cancel, and everything is divided by it
 #pragma unroll 4
         for (int x = part; x < LC_C; x += 4) s += Pt[x * LC_AT + t];
-        for (int e = part; e < d; e += 4) r = fmaf(Qs[t * LQ + e], start[(size_t)d * A.dv + e], r);
-        s = fmaf(coef[t], r, s);
+        for (int e = part; e < d; e += 4) r = fma((double)Qs[t * LQ + e], (double)start[(size_t)d * A.dv + e], r);
+        s = fma((double)coef[t], r, s);
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (part == 0) den[t] = fmaxf(fabsf(s), den[t]) + A.den_eps;
+        if (part == 0) den[t] = fmaxf(fabsf((float)s), den[t]) + A.den_eps;
     }
     float acc[4][TC];
 #pragma unroll

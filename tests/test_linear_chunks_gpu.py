@@ -1,5 +1,8 @@
 """Matrix memories in chunks (`ops.linear_chunks`): against the recurrence in float64 over the forms it accepts, and against the
-token-by-token kernel, whose state it shares.  Bound: sums of up to a few hundred float products of order one, 2e-5 of the largest."""
+token-by-token kernel, whose state it shares.  Bounds: sums of up to a few hundred float products of order one, 2e-5 of the largest, and
+in the norm no further off than the token-by-token kernel.  A gated output is divided by n . q, which may nearly cancel: what both
+kernels can be off by is the roundings of its terms over it, 32 of them (2e-6) times sum |terms| / |n . q| of the output and
+of the values it weighs (the norm then says little more than how one token's roundings fell)."""
 from types import SimpleNamespace
 
 import pytest
@@ -40,6 +43,8 @@ def recurrence(x, gates, decay, H, d, dv, S, n, m, pos, inv_freq, rot, interleav
         q, k = turn(q), turn(k)
     q, k = q * q_scale, k * k_scale
     o = torch.empty(T, H, dv, dtype=torch.float64)
+    terms = torch.zeros(T, H, dtype=torch.float64)       # gated: sum |terms of n . q| / |what is divided by|
+    size = n.abs() if n is not None else None
     for t in range(T):
         if decay is not None:
             S = decay.double()[:, None, None] * S + k[t][:, :, None] * v[t][:, None, :]
@@ -52,9 +57,11 @@ def recurrence(x, gates, decay, H, d, dv, S, n, m, pos, inv_freq, rot, interleav
         m = new
         S = a[:, None, None] * S + b[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
         n = a[:, None] * n + b[:, None] * k[t]
+        size = a[:, None] * size + b[:, None] * k[t].abs()
         den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-m)) + den_eps
+        terms[t] = (size * q[t].abs()).sum(-1) / den
         o[t] = torch.einsum("hd,hde->he", q[t], S) / den[:, None]
-    return o.reshape(T, H * dv), S, n, m
+    return o.reshape(T, H * dv), S, n, m, terms
 
 
 @pytest.mark.parametrize("gated", [True, False])
@@ -98,11 +105,15 @@ def test_chunks_against_the_recurrence_in_float64_and_the_scan_kernel(gated, H, 
     ops.linear_scan(dev["proj"], 0, H * d, 2 * H * d, H, d, dv, scan_state, dev["q"], dev["slots"], dev["pos"], scan_out, B=B, **kw)
     for b in range(B):
         rows = slice(q_start[b], q_start[b + 1])
-        o, S, n, m = recurrence(proj[rows].double(), gates[rows].double() if gated else None, decay, H, d, dv, S0[b].double(),
+        o, S, n, m, terms = recurrence(proj[rows].double(), gates[rows].double() if gated else None, decay, H, d, dv, S0[b].double(),
                                 n0[b].double() if gated else None, m0[b].double() if gated else None, pos[rows], inv, rot, interleaved,
                                 kw.get("cap"), kw["q_scale"], kw["k_scale"], kw.get("den_eps", 0.0))
         want = slot_rows(S, n, m)
         for got, scan, x in ((out[rows], scan_out[rows], o), (state[int(slots[b])], scan_state[int(slots[b])], want)):
+            if gated and x is o:
+                far = (got.double().cpu() - o).abs().view(-1, H, dv) - 2e-6 * terms[:, :, None] * (o.abs().view(-1, H, dv) + float(proj.abs().max()))
+                assert float(far.max()) <= 0.0, float(far.max())
+                continue
             err, base = (float((y.double().cpu() - x).norm()) / float(x.norm()) for y in (got, scan))
             assert err <= max(2e-6, 1.5 * base), (err, base)
             assert float((got.double().cpu() - x).abs().max()) <= max(2e-5 * float(x.abs().max()), 4 * float((scan.double().cpu() - x).abs().max()))
