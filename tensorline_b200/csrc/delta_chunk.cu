@@ -20,7 +20,7 @@
 // is bound by shared memory: a warp gets 32 floats of it a cycle and needs one for two multiply-adds with 16 columns a
 // block (measured 286 us for 2,048 tokens, 8 heads of 128 x 256; token by token 642).  On mma.sync a warp holds 32 rows of the transposed state [16 columns x 128 rows] as
 // accumulators, which are the next product's first operand as they lie; W, K, Q and P come as bfloat16 parts, cut once
-// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 40.
+// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 36.
 #include "common.cuh"
 
 constexpr int DC_C = 32;                 // tokens a chunk
@@ -62,9 +62,10 @@ __device__ __forceinline__ void dc_cut(float a, float b, uint32_t& hi, uint32_t&
 }
 
 // ------------------------------------------------------------------ prepare
-// grid (chunks, H), 256 threads; shared memory K, Q [32][DP + 4], V [32][dv]
+// grid (chunks, H); shared memory K, Q [32][DP + 4], V [32][dv].  384 threads: the columns of a head of 128 x 256 at once
+constexpr int DC_PREP = 384;
 template <int DP>
-__global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A) {
+__global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArgs A) {
     constexpr int LD = DP + 4, ROW = dc_row(DP);
     extern __shared__ __align__(16) float sm[];
     float* Ks = sm;
@@ -83,14 +84,14 @@ __global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(ok ? src : A.qkv), "r"(ok ? 16 : 0)
                      : "memory");
     };
-    for (int i = tid; i < DC_C * DP / 4; i += 256) {
+    for (int i = tid; i < DC_C * DP / 4; i += DC_PREP) {
         const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
         const float* row = A.qkv + (size_t)(t0 + t) * A.stride + hq * d + e;
         copy16(Qs + t * LD + e, row + A.q_off, t < n && e < d);
         copy16(Ks + t * LD + e, row + A.k_off, t < n && e < d);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    for (int i = tid; i < DC_C * dv / 4; i += 256) {
+    for (int i = tid; i < DC_C * dv / 4; i += DC_PREP) {
         const int t = i / (dv / 4), e = (i - t * (dv / 4)) * 4;
         copy16(Vs + t * dv + e, A.qkv + (size_t)(t0 + t) * A.stride + A.v_off + h * dv + e, t < n);
     }
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A)
     __syncthreads();
     if (h == hq * rep) {                                 // the parts of K and Q, once for the heads that share them
         unsigned char* to = A.K + ((size_t)blockIdx.x * A.nqk + hq) * 2 * dc_parts(DP);
-        for (int i = tid; i < 2 * DC_C * DP / 4; i += 256) {
+        for (int i = tid; i < 2 * DC_C * DP / 4; i += DC_PREP) {
             const bool isq = i >= DC_C * DP / 4;
             const int j = isq ? i - DC_C * DP / 4 : i, t = j / (DP / 4), e = (j % (DP / 4)) * 4;
             const float4 x = *reinterpret_cast<const float4*>((isq ? Qs : Ks) + t * LD + e);
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A)
             for (int c = 0; c < 3; ++c) *reinterpret_cast<uint2*>(to + (isq ? dc_parts(DP) : 0) + (c * DC_C + t) * ROW + e * 2) = p[c];
         }
     }
-    {                                                    // k_t . k_s and q_t . k_s: tokens ty, ty + 16 against tx, tx + 16
+    if (wid < 8) {                                       // k_t . k_s and q_t . k_s: tokens ty, ty + 16 against tx, tx + 16
         const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
         float kk[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qk[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll 4
@@ -163,7 +164,7 @@ __global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A)
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int i = tid; i < DC_C * DC_C / 2; i += 256) {
+    for (int i = tid; i < DC_C * DC_C / 2; i += DC_PREP) {
         const int t = i / (DC_C / 2), x = (i % (DC_C / 2)) * 2;
         const float2 v = *reinterpret_cast<const float2*>(&Ps[t][x]);
         uint32_t p[3];
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(256) dc_prepare_kernel(const DeltaChunkArgs A)
         for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(A.P + at * DC_PB + (c * DC_C + t) * DC_PROW + x * 2) = p[c];
     }
     const int wide = (dv + 15) & ~15;                    // columns behind the last are zeros, like rows behind d
-    for (int c = tid; c < wide + DP; c += 256) {
+    for (int c = tid; c < wide + DP; c += DC_PREP) {
         float u[DC_C];
         const bool isw = c >= wide;
         const int e = c - wide;
@@ -420,7 +421,7 @@ static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int n_chunks, int
     A.M = A.P + ch * DC_PB;
     A.U = A.M + ch * DC_MB;
     A.K = A.U + ch * A.nz * DC_UB;
-    dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), 256, prep_smem, stream>>>(A);
+    dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), DC_PREP, prep_smem, stream>>>(A);
     const int e = tl_launch_status();
     if (e) return e;
     dc_walk_kernel<DP><<<dim3(requests, A.H, A.nz), 128, Sh::BYTES, stream>>>(A);
