@@ -33,6 +33,20 @@ struct ChannelScanArgs {
     int H, d, dv, nz;
 };
 
+// pairs of floats: a + b, a b + c, each rounded as alone
+__device__ __forceinline__ float2 cs_add2(const float2 a, const float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 cs_fma2(const float2 a, float b, const float2 c) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmov.b64 z, {%5, %6};\n\tfma.rn.f32x2 x, x, y, z;\n\t"
+        "mov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b), "f"(c.x), "f"(c.y));
+    return r;
+}
 __device__ __forceinline__ float cs_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // x_q -> silu(x_q), x_f -> f in place; grid (column groups, rows)
@@ -83,13 +97,14 @@ __global__ void __launch_bounds__(256, 2) channel_chunk_kernel(const ChannelScan
         return ((size_t)(col / CS_COLS) * R + row % R) * NT + (col % CS_COLS) * IS + row / R;
     };
     const bool owns = col0 + cg * 4 < A.nz * CS_COLS;
-    float S[8][4], F[8];
+    float2 S[8][2];                                      // pairs of columns: the architecture's pairs of float operations
+    float F[8];
     const float* from = nc == 1 ? slot : mine;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         F[r] = 1.0f;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) S[r][cc] = OUT && owns ? from[at(r, cc)] : 0.f;
+        for (int cc = 0; cc < 2; ++cc) S[r][cc] = OUT && owns ? make_float2(from[at(r, 2 * cc)], from[at(r, 2 * cc + 1)]) : make_float2(0.f, 0.f);
     }
     // a stage's rows on their way into buffer `buf`: f, q, v; rows that do not exist and tokens behind the chunk change nothing
     const bool four = ((A.stride | A.q_off | A.f_off | A.v_off | A.d | A.dv) & 3) == 0 && ((uintptr_t)A.proj & 15) == 0;
@@ -141,15 +156,16 @@ __global__ void __launch_bounds__(256, 2) channel_chunk_kernel(const ChannelScan
                     *reinterpret_cast<float4*>(q) = *reinterpret_cast<const float4*>(q_s + t * RG * RS);
                     *reinterpret_cast<float4*>(q + 4) = *reinterpret_cast<const float4*>(q_s + t * RG * RS + 4);
                 }
-                float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+                float2 o0 = make_float2(0.f, 0.f), o1 = o0;
+                const float2 v0 = make_float2(v.x, v.y), v1 = make_float2(v.z, v.w), n0 = make_float2(-v.x, -v.y), n1 = make_float2(-v.z, -v.w);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) {
-                    S[r][0] = fmaf(f[r], S[r][0] - v.x, v.x); S[r][1] = fmaf(f[r], S[r][1] - v.y, v.y);
-                    S[r][2] = fmaf(f[r], S[r][2] - v.z, v.z); S[r][3] = fmaf(f[r], S[r][3] - v.w, v.w);
-                    if (OUT) { o0 = fmaf(S[r][0], q[r], o0); o1 = fmaf(S[r][1], q[r], o1); o2 = fmaf(S[r][2], q[r], o2); o3 = fmaf(S[r][3], q[r], o3); }
+                    S[r][0] = cs_fma2(cs_add2(S[r][0], n0), f[r], v0);
+                    S[r][1] = cs_fma2(cs_add2(S[r][1], n1), f[r], v1);
+                    if (OUT) { o0 = cs_fma2(S[r][0], q[r], o0); o1 = cs_fma2(S[r][1], q[r], o1); }
                     else F[r] *= f[r];
                 }
-                po[k * 4] = o0; po[k * 4 + 1] = o1; po[k * 4 + 2] = o2; po[k * 4 + 3] = o3;
+                po[k * 4] = o0.x; po[k * 4 + 1] = o0.y; po[k * 4 + 2] = o1.x; po[k * 4 + 3] = o1.y;
             }
             if (OUT) {
                 // halve what a lane holds while the lanes of a row group's set add up: lane bit i picks the upper half at step i
@@ -184,13 +200,13 @@ __global__ void __launch_bounds__(256, 2) channel_chunk_kernel(const ChannelScan
 #pragma unroll
             for (int r = 0; r < 8; ++r)
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) slot[at(r, cc)] = S[r][cc];
+                for (int cc = 0; cc < 4; ++cc) slot[at(r, cc)] = cc & 1 ? S[r][cc / 2].y : S[r][cc / 2].x;
     } else {
         if (owns)
 #pragma unroll
             for (int r = 0; r < 8; ++r)
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) mine[at(r, cc)] = S[r][cc];
+                for (int cc = 0; cc < 4; ++cc) mine[at(r, cc)] = cc & 1 ? S[r][cc / 2].y : S[r][cc / 2].x;
         if (cg == 0 && blockIdx.z == 0)
 #pragma unroll
             for (int r = 0; r < 8; ++r) A.decay[((size_t)(ck.w + c) * A.H + h) * DP + rg * 8 + r] = F[r];
