@@ -22,6 +22,7 @@
 // accumulators, which are the next product's first operand as they lie; W, K, Q and P come as bfloat16 parts, cut once
 // by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 36.
 #include "common.cuh"
+#include "parts_mma.cuh"
 
 constexpr int DC_C = 32;                 // tokens a chunk
 constexpr int DC_COLS = 16;              // columns a block of the walk and a slice of the state's layout
@@ -48,18 +49,6 @@ struct DeltaChunkArgs {
 };
 
 __device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
-// The three bfloat16 parts of two floats, packed (the first in the low half).
-__device__ __forceinline__ void dc_cut(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-    auto pack = [](float x, float y) {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-        return *reinterpret_cast<const uint32_t*>(&v);
-    };
-    hi = pack(a, b);
-    a -= __uint_as_float(hi << 16); b -= __uint_as_float(hi & 0xffff0000u);
-    mid = pack(a, b);
-    a -= __uint_as_float(mid << 16); b -= __uint_as_float(mid & 0xffff0000u);
-    lo = pack(a, b);
-}
 
 // ------------------------------------------------------------------ prepare
 // grid (chunks, H); shared memory K, Q [32][DP + 4], V [32][dv].  384 threads: the columns of a head of 128 x 256 at once
@@ -124,8 +113,8 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
             const int j = isq ? i - DC_C * DP / 4 : i, t = j / (DP / 4), e = (j % (DP / 4)) * 4;
             const float4 x = *reinterpret_cast<const float4*>((isq ? Qs : Ks) + t * LD + e);
             uint2 p[3];
-            dc_cut(x.x, x.y, p[0].x, p[1].x, p[2].x);
-            dc_cut(x.z, x.w, p[0].y, p[1].y, p[2].y);
+            parts_cut(x.x, x.y, p[0].x, p[1].x, p[2].x);
+            parts_cut(x.z, x.w, p[0].y, p[1].y, p[2].y);
 #pragma unroll
             for (int c = 0; c < 3; ++c) *reinterpret_cast<uint2*>(to + (isq ? dc_parts(DP) : 0) + (c * DC_C + t) * ROW + e * 2) = p[c];
         }
@@ -168,7 +157,7 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
         const int t = i / (DC_C / 2), x = (i % (DC_C / 2)) * 2;
         const float2 v = *reinterpret_cast<const float2*>(&Ps[t][x]);
         uint32_t p[3];
-        dc_cut(v.x, v.y, p[0], p[1], p[2]);
+        parts_cut(v.x, v.y, p[0], p[1], p[2]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(A.P + at * DC_PB + (c * DC_C + t) * DC_PROW + x * 2) = p[c];
     }
@@ -216,26 +205,6 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
 }
 
 // ------------------------------------------------------------------ walk
-__device__ __forceinline__ void dc_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void dc_load4(uint32_t (&r)[4], uint32_t at) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
-}
-__device__ __forceinline__ void dc_load4_trans(uint32_t (&r)[4], uint32_t at) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
-}
-// c (leading parts) and s (the rest) += A B over the parts a[3], b of the fragment pair starting at b[.][i]
-__device__ __forceinline__ void dc_mma6(float (&c)[4], float (&s)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int i) {
-    dc_mma(s, a[2], b[0][i], b[0][i + 1]);
-    dc_mma(c, a[0], b[0][i], b[0][i + 1]);
-    dc_mma(s, a[0], b[2][i], b[2][i + 1]);
-    dc_mma(s, a[1], b[1][i], b[1][i + 1]);
-    dc_mma(s, a[1], b[0][i], b[0][i + 1]);
-    dc_mma(s, a[0], b[1][i], b[1][i + 1]);
-}
-
 template <int DP> struct WalkShape {
     static constexpr int PARTS = dc_parts(DP);
     static constexpr int W = 0, K = PARTS, Q = 2 * PARTS, P = 3 * PARTS, U = P + DC_PB, M = U + DC_UB, BUF = M + DC_MB;      // bytes of a buffer
@@ -302,7 +271,7 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
                 const float (&v)[4] = S[2 * k + (x >> 1)];
-                dc_cut(v[(x & 1) * 2], v[(x & 1) * 2 + 1], sa[k][0][x], sa[k][1][x], sa[k][2][x]);
+                parts_cut(v[(x & 1) * 2], v[(x & 1) * 2 + 1], sa[k][0][x], sa[k][1][x], sa[k][2][x]);
             }
         // (W S)^T and (Q S)^T over this warp's rows: [16 columns][32 tokens]
 #pragma unroll
@@ -318,9 +287,9 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
                 for (int j = 0; j < 4; j += 2) {
                     uint32_t b[3][4];
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) dc_load4(b[p], at + (which ? Sh::Q : Sh::W) + (p * DC_C + j * 8) * ROW + x_at + k * 32);
-                    dc_mma6(big[j], rest[j], sa[k], b, 0);
-                    dc_mma6(big[j + 1], rest[j + 1], sa[k], b, 2);
+                    for (int p = 0; p < 3; ++p) parts_load4(b[p], at + (which ? Sh::Q : Sh::W) + (p * DC_C + j * 8) * ROW + x_at + k * 32);
+                    parts_mma6(big[j], rest[j], sa[k], b, 0);
+                    parts_mma6(big[j + 1], rest[j + 1], sa[k], b, 2);
                 }
             float* to = (which ? sums_q : sums_w) + (wid * DC_COLS + g) * LP + q2;
 #pragma unroll
@@ -344,8 +313,8 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
                     s.x += v.x; s.y += v.y;
                 }
                 const float a = u0[t * 20 + col] - s.x, b = u0[(t + 1) * 20 + col] - s.y;
-                dc_cut(a, b, ua[k][0][x], ua[k][1][x], ua[k][2][x]);
-                dc_cut(a * mk[DC_C + t], b * mk[DC_C + t + 1], wa[k][0][x], wa[k][1][x], wa[k][2][x]);
+                parts_cut(a, b, ua[k][0][x], ua[k][1][x], ua[k][2][x]);
+                parts_cut(a * mk[DC_C + t], b * mk[DC_C + t + 1], wa[k][0][x], wa[k][1][x], wa[k][2][x]);
             }
         // the new state
         {
@@ -357,9 +326,9 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
                 for (int k = 0; k < 2; ++k) {
                     uint32_t b[3][4];
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) dc_load4_trans(b[p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at + i * 16);
-                    dc_mma6(big[0], rest[0], wa[k], b, 0);
-                    dc_mma6(big[1], rest[1], wa[k], b, 2);
+                    for (int p = 0; p < 3; ++p) parts_load4_trans(b[p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at + i * 16);
+                    parts_mma6(big[0], rest[0], wa[k], b, 0);
+                    parts_mma6(big[1], rest[1], wa[k], b, 2);
                 }
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
@@ -372,9 +341,9 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
             float big[4] = {}, rest[4] = {};
             uint32_t b[3][4];
 #pragma unroll
-            for (int p = 0; p < 3; ++p) dc_load4(b[p], at + Sh::P + p * DC_C * DC_PROW + p_at);
-            dc_mma6(big, rest, ua[0], b, 0);
-            dc_mma6(big, rest, ua[1], b, 2);
+            for (int p = 0; p < 3; ++p) parts_load4(b[p], at + Sh::P + p * DC_C * DC_PROW + p_at);
+            parts_mma6(big, rest, ua[0], b, 0);
+            parts_mma6(big, rest, ua[1], b, 2);
             const int t = 8 * wid + q2;
             const float2 e = *reinterpret_cast<const float2*>(mk + t);
 #pragma unroll

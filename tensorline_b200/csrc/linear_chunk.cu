@@ -15,12 +15,13 @@
 // kernel, so the two may take turns on one request.  A position's sums depend on where its step began, to rounding.
 //
 // What the scan kernel is bound by is the chain over the tokens at one block a head and 16 columns (128 blocks, 0.36 us a token);
-// here 12 multiply-adds of matrix products a state element and chunk token pair up in tiles of 4 x 8 and 8 x 8 a thread.
-// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; local 36 (45 with K and V fetched behind the weights), carry 25, outputs 81 us
-// (93 as tiles of 8 x 8 in half the threads: fewer floats from shared memory, too few warps to hide them).
+// here the end states are tiles of 8 x 8 a thread, the outputs products of bfloat16 parts on the tensor cores.
+// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; now gates 4.6, local 33.5, carry 24, outputs 64 us
+// (81 as float multiply-adds).  Fixed decay, 1,650 tokens in 3 requests: local 26, carry 18.5, outputs 70 as multiply-adds.
 // 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
 // L2 once each way, weigh half as much again at 32.
 #include "common.cuh"
+#include "parts_mma.cuh"
 
 constexpr int LC_C = 64;                 // tokens a chunk
 constexpr int LC_COLS = 16;              // columns a slice of the state's layout (the scan kernel's)
@@ -37,6 +38,7 @@ struct LinearChunkArgs {
     const int* firsts;                   // the requests' first chunks
     float* ends;                         // [chunks][H][d dv (+ d)]: end states from zero, then start states
     double* marks;                       // [chunks][H][3]: the chunk's F, its maximum, the running maximum in front of it
+    double* weights;                     // gated: [chunks][H][3][64], F, u and top of lc_weights
     float* out;
     int H, d, dv, nz; float den_eps;
 };
@@ -48,14 +50,9 @@ __device__ __forceinline__ void lc_fma2(float& d0, float& d1, float a, float b0,
         : "+f"(d0), "+f"(d1) : "f"(a), "f"(b0), "f"(b1));
 }
 
-// Warp 0: for the n tokens of a chunk that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the running
-// maximum top[t] of u (gated).
-template <bool GATED>
+// A warp, gated: for the n tokens of a chunk that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the running
+// maximum top[t] of u.
 __device__ __forceinline__ void lc_weights(const LinearChunkArgs& A, int t0, int n, int h, int lane, double* F, double* u, double* top) {
-    if constexpr (!GATED) {
-        const double la = log((double)A.decay[h]);
-        for (int t = lane; t < LC_C; t += 32) { F[t] = (t + 1) * la; u[t] = -F[t]; }
-    } else {
     double f[2], in[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -85,6 +82,21 @@ __device__ __forceinline__ void lc_weights(const LinearChunkArgs& A, int t0, int
     F[2 * lane] = F0; F[2 * lane + 1] = F1;
     u[2 * lane] = u0; u[2 * lane + 1] = u1;
     top[2 * lane] = fmax(before, u0); top[2 * lane + 1] = best;
+}
+
+// A warp a (chunk, head): the gated kinds' weights, once for all blocks that need them (worked out in each of them, warp 0 held the
+// others up: end states 36 us, now 33.5 and 4.6 here, and the outputs need them without a wait).
+__global__ void __launch_bounds__(32) lc_gates_kernel(const LinearChunkArgs A) {
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, lane = threadIdx.x, t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    const size_t at = (size_t)blockIdx.x * A.H + h;
+    double* w = A.weights + at * 3 * LC_C;
+    lc_weights(A, t0, n, h, lane, w, w + LC_C, w + 2 * LC_C);
+    __syncwarp();
+    if (lane == 0) {
+        const double end = w[n - 1];
+        A.marks[at * 3] = end;
+        A.marks[at * 3 + 1] = (double)(float)(end + w[2 * LC_C + n - 1]);
     }
 }
 
@@ -125,7 +137,6 @@ __global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) 
     extern __shared__ __align__(16) float sm[];
     float* Ks = sm;                                      // [64][RB], weighted
     float* Vs = Ks + LC_C * RB;                          // [64][CB]
-    __shared__ double F[LC_C], u[LC_C], top[LC_C];
     __shared__ float w[LC_C];
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, col_tiles = (A.dv + CB - 1) / CB, row0 = (blockIdx.z / col_tiles) * RB, col0 = (blockIdx.z % col_tiles) * CB;
@@ -144,15 +155,14 @@ __global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) 
         copy16(Vs + t * CB + c, A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c, t < n && col0 + c < A.dv);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    if (wid == 0) {
-        lc_weights<GATED>(A, t0, n, h, lane, F, u, top);
-        __syncwarp();
-        const double end = F[n - 1], m = GATED ? (double)(float)(end + top[n - 1]) : 0.0;
-        for (int t = lane; t < LC_C; t += 32) w[t] = t < n ? expf((float)(end + u[t] - m)) * A.k_scale : 0.f;
-        if (lane == 0 && blockIdx.z == 0) {
-            double* mk = A.marks + ((size_t)blockIdx.x * A.H + h) * 3;
-            mk[0] = end; mk[1] = m;
-        }
+    const size_t ch = (size_t)blockIdx.x * A.H + h;
+    if (GATED) {
+        const double* g = A.weights + ch * 3 * LC_C;
+        if (tid < LC_C) w[tid] = tid < n ? expf((float)(A.marks[ch * 3] + g[LC_C + tid] - A.marks[ch * 3 + 1])) * A.k_scale : 0.f;
+    } else if (tid < LC_C) {
+        const double la = log((double)A.decay[h]);
+        w[tid] = tid < n ? expf((float)((n - 1 - tid) * la)) * A.k_scale : 0.f;
+        if (tid == 0 && blockIdx.z == 0) { A.marks[ch * 3] = n * la; A.marks[ch * 3 + 1] = 0.0; }
     }
     __syncthreads();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -307,7 +317,7 @@ __global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
     float* Pt = Qs + LC_C * LQ;                          // [64 s][LC_AT]: P transposed; behind it ...
     float* Qt = Pt + LC_C * LC_AT;                       // ... K [64][LQ], later the weighted Q transposed [DP][LC_AT]
     float* Bs = Qt + Sh::QT;                             // [S][ROWS][CB]
-    __shared__ double F[LC_C], u[LC_C], top[LC_C];
+    __shared__ double u[LC_C], top[LC_C];
     __shared__ float coef[LC_C], den[LC_C];
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
@@ -344,19 +354,20 @@ __global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
         *reinterpret_cast<float4*>(Qs + t * LQ + e) = q;
         *reinterpret_cast<float4*>(Qt + t * LQ + e) = k;
     }
-    if (wid == 0) {
-        lc_weights<GATED>(A, t0, n, h, lane, F, u, top);
-        __syncwarp();
-        for (int t = lane; t < LC_C; t += 32) {          // top: the running maximum less F; F: what is added to u for a weight
-            if (GATED) {
-                const double mm = fmax(m0, top[t]);
-                coef[t] = expf((float)(m0 - mm));
-                den[t] = expf((float)(-(F[t] + mm)));
-                top[t] = -mm;
-            } else {
-                coef[t] = expf((float)F[t]);
-                top[t] = F[t];
-            }
+    if (tid < LC_C) {                                    // top: the running maximum less F; u: what is added to it for a weight
+        const int t = tid;
+        if (GATED) {
+            const double* w = A.weights + ((size_t)blockIdx.x * A.H + h) * 3 * LC_C;
+            const double f = w[t], mm = fmax(m0, w[2 * LC_C + t]);
+            u[t] = w[LC_C + t];
+            coef[t] = expf((float)(m0 - mm));
+            den[t] = expf((float)(-(f + mm)));
+            top[t] = -mm;
+        } else {
+            const double f = (t + 1) * log((double)A.decay[h]);
+            u[t] = -f;
+            top[t] = f;
+            coef[t] = expf((float)f);
         }
     }
     __syncthreads();
@@ -456,6 +467,240 @@ __global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
     }
 }
 
+// The same with the products on the tensor cores (parts_mma.cuh), for heads of up to 128.  256 threads; a block cuts its Q and K (32
+// tokens at a time) into parts once, P where it is made, and the rows of [S ; V] as they come, 16 at a time, the next ones on their way in
+// registers: little enough shared memory for two blocks an SM, one of which computes while the other waits for its rows (gated, 8 heads
+// of 128 x 256, 2,048 tokens: 64 us; with all of K and 32 rows at a time, one block an SM, 83; multiply-adds 81).  Heads
+// of 256 need 178 KB, so one block an SM: they stay with the multiply-adds.  Q S is taken first and weighted by token, P V added to it.
+template <int DP, int CB> struct OutPartsShape {
+    static constexpr int RQ = DP * 2 + 16, RB = CB * 2 + 16, RP = LC_C * 2 + 16;       // bytes of a row of a part of Q and K, of [S ; V], of P
+    static constexpr int Q = 3 * LC_C * RQ, STAGE = 3 * 16 * RB, KB = Q / 2 > 2 * STAGE ? Q / 2 : 2 * STAGE, P = 3 * LC_C * RP;
+    static constexpr int BYTES = Q + KB + P;             // K's parts lie where the stages of [S ; V] come later
+};
+
+template <int DP, int CB, bool GATED>
+__global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkArgs A) {
+    using Sh = OutPartsShape<DP, CB>;
+    constexpr int RQ = Sh::RQ, RB = Sh::RB, RP = Sh::RP, NJ = CB / 32, PER = 16 * CB / 4 / 256;      // n8 tiles a warp, 16-byte loads of a thread a step
+    extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem), kb = base + Sh::Q, pb = kb + Sh::KB;
+    __shared__ double u[LC_C], top[LC_C], nq[LC_C], rowsum[2][LC_C];
+    __shared__ float coef[LC_C], den[LC_C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+    const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
+    const float* start = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
+    const double m0 = GATED ? A.marks[((size_t)blockIdx.x * A.H + h) * 3 + 2] : 0.0;
+    const int s_steps = (d + 15) / 16, steps = s_steps + (n + 15) / 16;
+    float4 ahead[PER];
+    auto fetch = [&](int step) {                         // 16 rows of S, then of V; zeros where there are none
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int r = (tid + 256 * i) / (CB / 4), c = col0 + ((tid + 256 * i) % (CB / 4)) * 4;
+            ahead[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c >= A.dv) continue;
+            if (step < s_steps) {
+                if (step * 16 + r < d) ahead[i] = *reinterpret_cast<const float4*>(start + (size_t)(step * 16 + r) * A.dv + c);
+            } else if ((step - s_steps) * 16 + r < n)
+                ahead[i] = *reinterpret_cast<const float4*>(A.v + (size_t)(t0 + (step - s_steps) * 16 + r) * A.v_stride + h * A.dv + c);
+        }
+    };
+    auto put4 = [&](unsigned char* to, int part, const float4 x) {      // four values' parts, `part` bytes from one part to the next
+        uint2 p[3];
+        parts_cut(x.x, x.y, p[0].x, p[1].x, p[2].x);
+        parts_cut(x.z, x.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(to + e * part) = p[e];
+    };
+    auto put = [&](int step) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int r = (tid + 256 * i) / (CB / 4), c = ((tid + 256 * i) % (CB / 4)) * 4;
+            put4(smem + Sh::Q + (step & 1) * Sh::STAGE + r * RB + c * 2, 16 * RB, ahead[i]);
+        }
+    };
+#pragma unroll
+    for (int i = tid; i < LC_C * DP / 4; i += 256) {
+        const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        double r = 0.0;                                  // n . q of the chunk's start state
+        if (t < n && e < d) {
+            q = *reinterpret_cast<const float4*>(A.q + (size_t)(t0 + t) * A.qk_stride + h * d + e);
+            q.x *= A.q_scale; q.y *= A.q_scale; q.z *= A.q_scale; q.w *= A.q_scale;
+            if (GATED) {
+                const float4 x = *reinterpret_cast<const float4*>(start + (size_t)d * A.dv + e);
+                r = (double)q.x * x.x + (double)q.y * x.y + (double)q.z * x.z + (double)q.w * x.w;
+            }
+        }
+        put4(smem + t * RQ + e * 2, LC_C * RQ, q);
+        if (GATED) {                                     // DP / 4 neighbouring lanes share a token
+#pragma unroll
+            for (int o = 1; o < DP / 4; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            if ((lane & (DP / 4 - 1)) == 0) nq[t] = r;
+        }
+    }
+    constexpr int KPER = 32 * DP / 4 / 256;              // 16-byte loads of a thread for 32 tokens of K
+    float4 keys[KPER];
+    auto fetch_keys = [&](int half) {
+#pragma unroll
+        for (int i = 0; i < KPER; ++i) {
+            const int t = 32 * half + (tid + 256 * i) / (DP / 4), e = ((tid + 256 * i) % (DP / 4)) * 4;
+            keys[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (t < n && e < d) {
+                keys[i] = *reinterpret_cast<const float4*>(A.k + (size_t)(t0 + t) * A.qk_stride + h * d + e);
+                keys[i].x *= A.k_scale; keys[i].y *= A.k_scale; keys[i].z *= A.k_scale; keys[i].w *= A.k_scale;
+            }
+        }
+    };
+    auto put_keys = [&]() {
+#pragma unroll
+        for (int i = 0; i < KPER; ++i)
+            put4(smem + Sh::Q + (tid + 256 * i) / (DP / 4) * RQ + ((tid + 256 * i) % (DP / 4)) * 8, 32 * RQ, keys[i]);
+    };
+    fetch_keys(0);
+    if (tid < LC_C) {                                    // top: the running maximum less F; u: what is added to it for a weight
+        const int t = tid;
+        if (GATED) {
+            const double* w = A.weights + ((size_t)blockIdx.x * A.H + h) * 3 * LC_C;
+            const double f = w[t], mm = fmax(m0, w[2 * LC_C + t]);
+            u[t] = w[LC_C + t];
+            coef[t] = expf((float)(m0 - mm));
+            den[t] = expf((float)(-(f + mm)));
+            top[t] = -mm;
+        } else {
+            const double f = (t + 1) * log((double)A.decay[h]);
+            u[t] = -f;
+            top[t] = f;
+            coef[t] = expf((float)f);
+        }
+    }
+    put_keys();
+    fetch_keys(1);
+    __syncthreads();
+    const uint32_t a_at = (lane & 15), a_hi = (lane >> 4) * 16;                          // rows of a first operand's tile, its second eight k
+    const uint32_t b_at = (lane & 7) + (lane >> 4) * 8, b_hi = ((lane >> 3) & 1) * 16;   // rows (tokens) of two tiles of K
+    const uint32_t v_at = (lane & 7) + ((lane >> 3) & 1) * 8, v_hi = (lane >> 4) * 16;   // rows of [S ; V], transposed
+    double sum[2] = {0.0, 0.0};
+    for (int half = 0; half < 2; ++half) {               // P: 16 tokens of the first operand a pair of warps, 16 of the second's 32 a warp
+        const int mi = wid >> 1, s0 = 32 * half + 16 * (wid & 1);
+        float big[2][4] = {}, rest[2][4] = {};
+        if (s0 <= 16 * mi + 15) {
+#pragma unroll 2
+            for (int k = 0; k < DP / 16; ++k) {
+                uint32_t a[3][4], b[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    parts_load4(a[p], base + (p * LC_C + 16 * mi + a_at) * RQ + a_hi + k * 32);
+                    parts_load4(b[p], kb + (p * 32 + 16 * (wid & 1) + b_at) * RQ + b_hi + k * 32);
+                }
+                parts_mma6(big[0], rest[0], a, b, 0);
+                parts_mma6(big[1], rest[1], a, b, 2);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int s = s0 + 8 * j + q2;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const int t = 16 * mi + g + 8 * x;
+                float v[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    v[e] = s + e <= t && t < n ? (big[j][2 * x + e] + rest[j][2 * x + e]) * expf((float)(top[t] + u[s + e])) : 0.f;
+                    sum[x] += v[e];
+                }
+                uint32_t p[3];
+                parts_cut(v[0], v[1], p[0], p[1], p[2]);
+#pragma unroll
+                for (int e = 0; e < 3; ++e) *reinterpret_cast<uint32_t*>(smem + Sh::Q + Sh::KB + (e * LC_C + t) * RP + s * 2) = p[e];
+            }
+        }
+        if (half == 0) {
+            __syncthreads();                             // the first half of K is read
+            put_keys();
+            __syncthreads();
+        }
+    }
+    fetch(0);
+    if (GATED) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], 1);
+            sum[x] += __shfl_xor_sync(0xffffffffu, sum[x], 2);
+            if (q2 == 0) rowsum[wid & 1][16 * (wid >> 1) + g + 8 * x] = sum[x];
+        }
+    }
+    __syncthreads();                                     // K is read, P is written
+    if (GATED && tid < LC_C)
+        den[tid] = fmaxf(fabsf((float)(rowsum[0][tid] + rowsum[1][tid] + coef[tid] * nq[tid])), den[tid]) + A.den_eps;
+    const int wm = wid >> 2, wn = wid & 3;               // 32 tokens and CB / 4 columns a warp
+    float big[2][NJ][4], rest[2][NJ][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) big[i][j][x] = rest[i][j][x] = 0.f;
+    put(0);
+    for (int step = 0; step < steps; ++step) {
+        __syncthreads();                                 // the step's rows are there, the step's before last are read
+        if (step + 1 < steps) fetch(step + 1);
+        const bool values = step >= s_steps;
+        if (step == s_steps) {                           // all of Q S is there: each token's weight
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) {
+                        const float c = coef[32 * wm + 16 * i + g + (x >> 1) * 8];
+                        big[i][j][x] *= c; rest[i][j][x] *= c;
+                    }
+        }
+        const int r0 = values ? (step - s_steps) * 16 : step * 16;
+        if (!values || r0 <= 32 * wm + 31) {             // values of later tokens meet zeros only
+            const uint32_t st = kb + (step & 1) * Sh::STAGE;
+            uint32_t a[2][3][4];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    const uint32_t row = p * LC_C + 32 * wm + 16 * i + a_at;
+                    parts_load4(a[i][p], (values ? pb + row * RP : base + row * RQ) + a_hi + r0 * 2);
+                }
+#pragma unroll
+            for (int j = 0; j < NJ; j += 2) {
+                uint32_t b[3][4];
+#pragma unroll
+                for (int p = 0; p < 3; ++p) parts_load4_trans(b[p], st + (p * 16 + v_at) * RB + v_hi + (wn * (CB / 4) + 8 * j) * 2);
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    parts_mma6(big[i][j], rest[i][j], a[i], b, 0);
+                    parts_mma6(big[i][j + 1], rest[i][j + 1], a[i], b, 2);
+                }
+            }
+        }
+        if (step + 1 < steps) put(step + 1);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int t = 32 * wm + 16 * i + g + 8 * x;
+            if (t >= n) continue;
+            float* to = A.out + (size_t)(t0 + t) * A.H * A.dv + (size_t)h * A.dv;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const int col = col0 + wn * (CB / 4) + 8 * j + q2;
+                float2 o = make_float2(big[i][j][2 * x] + rest[i][j][2 * x], big[i][j][2 * x + 1] + rest[i][j][2 * x + 1]);
+                if (GATED) { o.x /= den[t]; o.y /= den[t]; }
+                if (col < A.dv) *reinterpret_cast<float2*>(to + col) = o;
+            }
+        }
+}
+
 template <typename F>
 static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
     const int dev = tl_device_index();
@@ -475,9 +720,15 @@ static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaS
     constexpr int local_smem = LC_C * (RB + CB) * 4, out_smem = OutShape<DP, CB>::FLOATS * 4;
     static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
     int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
-    if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
+    if constexpr (DP >= 64 && DP <= 128) {
+        if (!e) e = lc_raise(lc_out_parts_kernel<DP, CB, GATED>, r2, OutPartsShape<DP, CB>::BYTES);
+    } else if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
     if (e) return e;
     const int col_tiles = (A.dv + CB - 1) / CB, row_tiles = (A.d + RB - 1) / RB;
+    if (GATED) {
+        lc_gates_kernel<<<dim3(n_chunks, A.H), 32, 0, stream>>>(A);
+        if ((e = tl_launch_status())) return e;
+    }
     lc_local_kernel<RB, CB, GATED><<<dim3(n_chunks, A.H, row_tiles * col_tiles), 256, local_smem, stream>>>(A);
     if ((e = tl_launch_status())) return e;
     const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
@@ -487,7 +738,9 @@ static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaS
         lc_maximum_kernel<<<dim3(A.H, requests), 32, 0, stream>>>(A, PB, R * NT);
         if ((e = tl_launch_status())) return e;
     }
-    lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
+    if constexpr (DP >= 64 && DP <= 128)
+        lc_out_parts_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, OutPartsShape<DP, CB>::BYTES, stream>>>(A);
+    else lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
     return tl_launch_status();
 }
 
@@ -500,7 +753,7 @@ static int lc_pick(const LinearChunkArgs& A, int n_chunks, int requests, cudaStr
 TL_EXPORT int tl_linear_chunk() { return LC_C; }
 
 // `rows` (float [T, 2 H d], with a rotation): where q and k go.  ends: float [n_chunks, H, d dv (+ d with gates)], marks: double
-// [n_chunks, H, 3].  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
+// [n_chunks, H, 3], with gates then [n_chunks, H, 192].  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
 TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, int k_off, int v_off, const float* gates, float cap,
                                const float* decay, const float* inv_freq, int rot, int interleaved, const int* pos, float q_scale,
                                float k_scale, float* rows, float* state, long long slot_stride, const int* q_start, const int* slots,
@@ -511,7 +764,7 @@ TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, 
         (rot && !rows) || (gates != nullptr) == (decay != nullptr) ||
         ((((uintptr_t)proj) | ((uintptr_t)rows) | ((uintptr_t)ends) | ((uintptr_t)out)) & 15)) return 1;
     LinearChunkArgs A{proj + q_off, proj + k_off, stride, proj + v_off, stride, gates, cap, decay, q_scale, k_scale, state, slot_stride,
-                      q_start, slots, (const int4*)chunks, firsts, ends, marks, out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
+                      q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
     if (rot) {
         lc_rotate_kernel<<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
         const int e = tl_launch_status();

@@ -850,12 +850,12 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
     dev = proj.device
     turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
     ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
-    marks = torch.empty((n, H, 3), dtype=torch.float64, device=dev)
+    marks = torch.empty(n * H * (3 if gates is None else 195), dtype=torch.float64, device=dev)
     _check(core().tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, _ptr(gates), float(cap), _ptr(decay),
                                    _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale), float(k_scale),
                                    _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n,
                                    requests, _ptr(ends), _ptr(marks), _ptr(out), H, d, dv, float(den_eps), _stream()), "linear_chunks",
-           launches=3 + bool(rot) + (gates is not None))
+           launches=3 + bool(rot) + 2 * (gates is not None))
 
 
 def channel_chunks(h_q_start, chunk: int) -> tuple:
