@@ -101,31 +101,84 @@ __global__ void __launch_bounds__(32) lc_gates_kernel(const LinearChunkArgs A) {
 }
 
 // ------------------------------------------------------------------ rotation
-// rows [T][2 H d]: q rotated and scaled, k rotated and scaled; a block a token
+// rows [T][2 H d]: q rotated and scaled, k rotated and scaled; a block a token.  VEC: four floats at a time, the first ones on their way
+// before the angles are known (8 heads of 128, 1,650 tokens: 7.5 us, a float at a time 11); rotations that don't cut a head into
+// whole 16-byte pieces stay with the latter.
+template <bool VEC>
 __global__ void __launch_bounds__(256) lc_rotate_kernel(const float* __restrict__ proj, int stride, int q_off, int k_off, const float* __restrict__ inv_freq,
                                                         int rot, int interleaved, const int* __restrict__ pos, float q_scale, float k_scale,
                                                         float* __restrict__ rows, int H, int d) {
-    extern __shared__ float cs[];                        // cos [rot / 2], sin [rot / 2]
-    const int t = blockIdx.x, half = rot >> 1;
-    for (int i = threadIdx.x; i < half; i += 256) sincosf(__fmul_rn((float)pos[t], inv_freq[i]), &cs[half + i], &cs[i]);
-    __syncthreads();
+    extern __shared__ __align__(16) float cs[];          // cos [rot / 2], sin [rot / 2]
+    const int t = blockIdx.x, half = rot >> 1, tid = threadIdx.x, rest = d - rot;
     const float* row = proj + (size_t)t * stride;
     float* to = rows + (size_t)t * 2 * H * d;
-    const int pairs = H * half, rest = d - rot;
-    for (int i = threadIdx.x; i < 2 * pairs; i += 256) {
-        const bool isk = i >= pairs;
-        const int j = isk ? i - pairs : i, h = j / half, p = j - h * half;
-        const int e1 = h * d + (interleaved ? 2 * p : p), e2 = h * d + (interleaved ? 2 * p + 1 : p + half);
-        const float* x = row + (isk ? k_off : q_off);
-        float* y = to + (isk ? H * d : 0);
-        const float sc = isk ? k_scale : q_scale, x1 = x[e1], x2 = x[e2], c = cs[p], s = cs[half + p];
-        y[e1] = (__fmul_rn(x1, c) - __fmul_rn(x2, s)) * sc;
-        y[e2] = (__fmul_rn(x2, c) + __fmul_rn(x1, s)) * sc;
-    }
-    for (int i = threadIdx.x; i < 2 * H * rest; i += 256) {
-        const bool isk = i >= H * rest;
-        const int j = isk ? i - H * rest : i, e = (j / rest) * d + rot + j % rest;
-        to[(isk ? H * d : 0) + e] = row[(isk ? k_off : q_off) + e] * (isk ? k_scale : q_scale);
+    auto angles = [&]() {
+        for (int i = tid; i < half; i += 256) sincosf(__fmul_rn((float)pos[t], inv_freq[i]), &cs[half + i], &cs[i]);
+        __syncthreads();
+    };
+    if constexpr (VEC) {
+        const int per = interleaved ? rot / 4 : half / 4, units = 2 * H * per;      // a unit: four pairs, interleaved two
+        auto place = [&](int i, bool& isk, int& e) {     // the unit's first element, its place among the angles
+            isk = i >= H * per;
+            const int j = isk ? i - H * per : i, h = j / per, p = (j - h * per) * 4;
+            e = h * d + p;
+            return p;
+        };
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+        auto fetch = [&](int i) {
+            bool isk; int e;
+            if (i >= units) return;
+            place(i, isk, e);
+            const float* from = row + (isk ? k_off : q_off) + e;
+            x = *reinterpret_cast<const float4*>(from);
+            if (!interleaved) y = *reinterpret_cast<const float4*>(from + half);
+        };
+        fetch(tid);
+        angles();
+        for (int i = tid; i < units; i += 256) {
+            bool isk; int e;
+            const int p = place(i, isk, e);
+            const float4 a = x, b = y;
+            fetch(i + 256);
+            const float sc = isk ? k_scale : q_scale;
+            float* out = to + (isk ? H * d : 0) + e;
+            auto first = [&](float u, float v, float c, float s) { return (__fmul_rn(u, c) - __fmul_rn(v, s)) * sc; };
+            auto second = [&](float u, float v, float c, float s) { return (__fmul_rn(v, c) + __fmul_rn(u, s)) * sc; };
+            if (interleaved) {
+                const float c0 = cs[p / 2], c1 = cs[p / 2 + 1], s0 = cs[half + p / 2], s1 = cs[half + p / 2 + 1];
+                *reinterpret_cast<float4*>(out) = make_float4(first(a.x, a.y, c0, s0), second(a.x, a.y, c0, s0), first(a.z, a.w, c1, s1), second(a.z, a.w, c1, s1));
+            } else {
+                const float4 c = *reinterpret_cast<const float4*>(cs + p), s = *reinterpret_cast<const float4*>(cs + half + p);
+                *reinterpret_cast<float4*>(out) = make_float4(first(a.x, b.x, c.x, s.x), first(a.y, b.y, c.y, s.y), first(a.z, b.z, c.z, s.z), first(a.w, b.w, c.w, s.w));
+                *reinterpret_cast<float4*>(out + half) = make_float4(second(a.x, b.x, c.x, s.x), second(a.y, b.y, c.y, s.y), second(a.z, b.z, c.z, s.z), second(a.w, b.w, c.w, s.w));
+            }
+        }
+        for (int i = tid; i < 2 * H * rest / 4; i += 256) {
+            const bool isk = i >= H * rest / 4;
+            const int j = (isk ? i - H * rest / 4 : i) * 4, e = (j / rest) * d + rot + j % rest;
+            const float sc = isk ? k_scale : q_scale;
+            float4 v = *reinterpret_cast<const float4*>(row + (isk ? k_off : q_off) + e);
+            v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
+            *reinterpret_cast<float4*>(to + (isk ? H * d : 0) + e) = v;
+        }
+    } else {
+        angles();
+        const int pairs = H * half;
+        for (int i = tid; i < 2 * pairs; i += 256) {
+            const bool isk = i >= pairs;
+            const int j = isk ? i - pairs : i, h = j / half, p = j - h * half;
+            const int e1 = h * d + (interleaved ? 2 * p : p), e2 = h * d + (interleaved ? 2 * p + 1 : p + half);
+            const float* x = row + (isk ? k_off : q_off);
+            float* y = to + (isk ? H * d : 0);
+            const float sc = isk ? k_scale : q_scale, x1 = x[e1], x2 = x[e2], c = cs[p], s = cs[half + p];
+            y[e1] = (__fmul_rn(x1, c) - __fmul_rn(x2, s)) * sc;
+            y[e2] = (__fmul_rn(x2, c) + __fmul_rn(x1, s)) * sc;
+        }
+        for (int i = tid; i < 2 * H * rest; i += 256) {
+            const bool isk = i >= H * rest;
+            const int j = isk ? i - H * rest : i, e = (j / rest) * d + rot + j % rest;
+            to[(isk ? H * d : 0) + e] = row[(isk ? k_off : q_off) + e] * (isk ? k_scale : q_scale);
+        }
     }
 }
 
@@ -289,14 +342,16 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(const LinearChunkArgs A) 
         for (int z = 0; z < (norm ? A.nz : 1); ++z) { slot[at(0, z)] = S.x; slot[at(1, z)] = S.y; slot[at(2, z)] = S.z; slot[at(3, z)] = S.w; }
     }
 }
-// The running maximum into every slice of the slot, after all blocks of the carry have read it.
-__global__ void lc_maximum_kernel(const LinearChunkArgs A, int pb, int at) {
-    const int first = A.firsts[blockIdx.y], h = blockIdx.x;
-    const int4 ck = A.chunks[first];
-    const double* g = A.marks + ((size_t)(first + ck.z - 1) * A.H + h) * 3;
+// The running maximum into every slice of the slot, by the outputs' block of the request's last chunk: all blocks of the carry have read
+// the old one by then (a kernel of its own took 3 to 4 us).
+template <int DP>
+__device__ __forceinline__ void lc_maximum(const LinearChunkArgs& A, const int4 ck, int h) {
+    constexpr int R = DP == 32 ? 4 : 8, IS = DP / R, NT = (IS * (LC_COLS + 1) + 31) / 32 * 32, PB = R * NT + 4;
+    if (blockIdx.z || ck.y != ck.z - 1) return;
+    const double* g = A.marks + ((size_t)blockIdx.x * A.H + h) * 3;
     const float m = (float)fmax(g[0] + g[2], g[1]);
-    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + (size_t)h * A.nz * pb;
-    for (int z = threadIdx.x; z < A.nz; z += blockDim.x) slot[(size_t)z * pb + at] = m;
+    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + (size_t)h * A.nz * PB;
+    for (int z = threadIdx.x; z < A.nz; z += blockDim.x) slot[(size_t)z * PB + R * NT] = m;
 }
 
 // ------------------------------------------------------------------ outputs
@@ -323,6 +378,7 @@ __global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
     const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    if (GATED) lc_maximum<DP>(A, ck, h);
     const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
     const float* start = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
     const double m0 = GATED ? A.marks[((size_t)blockIdx.x * A.H + h) * 3 + 2] : 0.0;
@@ -490,6 +546,7 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
     const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
     const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    if (GATED) lc_maximum<DP>(A, ck, h);
     const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
     const float* start = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
     const double m0 = GATED ? A.marks[((size_t)blockIdx.x * A.H + h) * 3 + 2] : 0.0;
@@ -716,7 +773,6 @@ static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
 template <int DP, int CB, bool GATED>
 static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
     constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
-    constexpr int NT = (IS * (LC_COLS + (GATED ? 1 : 0)) + 31) / 32 * 32, PB = R * NT + (GATED ? 4 : 0);
     constexpr int local_smem = LC_C * (RB + CB) * 4, out_smem = OutShape<DP, CB>::FLOATS * 4;
     static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
     int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
@@ -734,10 +790,6 @@ static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaS
     const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
     lc_carry_kernel<R, IS, GATED><<<dim3((unsigned)((per / 4 + 255) / 256), A.H, requests), 256, 0, stream>>>(A);
     if ((e = tl_launch_status())) return e;
-    if (GATED) {
-        lc_maximum_kernel<<<dim3(A.H, requests), 32, 0, stream>>>(A, PB, R * NT);
-        if ((e = tl_launch_status())) return e;
-    }
     if constexpr (DP >= 64 && DP <= 128)
         lc_out_parts_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, OutPartsShape<DP, CB>::BYTES, stream>>>(A);
     else lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
@@ -766,7 +818,10 @@ TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, 
     LinearChunkArgs A{proj + q_off, proj + k_off, stride, proj + v_off, stride, gates, cap, decay, q_scale, k_scale, state, slot_stride,
                       q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
     if (rot) {
-        lc_rotate_kernel<<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
+        if (rot % (interleaved ? 4 : 8) == 0)
+            lc_rotate_kernel<true><<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
+        else
+            lc_rotate_kernel<false><<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
         const int e = tl_launch_status();
         if (e) return e;
         A.q = rows; A.k = rows + (size_t)H * d; A.qk_stride = 2 * H * d;

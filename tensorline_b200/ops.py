@@ -855,7 +855,7 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
                                    _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale), float(k_scale),
                                    _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n,
                                    requests, _ptr(ends), _ptr(marks), _ptr(out), H, d, dv, float(den_eps), _stream()), "linear_chunks",
-           launches=3 + bool(rot) + 2 * (gates is not None))
+           launches=3 + bool(rot) + (gates is not None))
 
 
 def channel_chunks(h_q_start, chunk: int) -> tuple:
