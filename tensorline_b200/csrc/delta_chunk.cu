@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
             const float* g = A.gates + (size_t)(t0 + lane) * A.gate_stride;
             b = 1.0f / (1.0f + expf(-g[h]));
             x = -expf(A.A_log[h]) * dc_softplus(g[A.H + h] + A.dt_bias[h]);
+            if (x < -1e4) x = -1e4;                      // a decay of zero all the same; the differences behind it stay exact, -inf gives none
         }
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {

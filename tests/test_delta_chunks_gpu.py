@@ -64,6 +64,27 @@ def test_delta_chunks_against_the_recurrence_in_float64(H, nqk, d, dv, lens, lik
     assert torch.equal(state[0].cpu(), first[0])
 
 
+def test_decays_of_zero_forget_as_token_by_token():
+    """Log decays that a float does not hold, or that would swallow their neighbours' in a sum, beside ordinary ones."""
+    from tensorline_b200 import ops
+    g = torch.Generator().manual_seed(9)
+    H, nqk, d, dv, T = 3, 3, 64, 64, 100
+    qkv = torch.randn(T, H * (2 * d + dv), generator=g) * d ** -0.5
+    gates = torch.randn(T, 2 * H, generator=g)
+    gates[::7, H:] = 3e37                                # heads 0 and 1: products of 1e38 and more; head 2: every token
+    A_log, dt_bias = torch.tensor([3.0, 1.0, 100.0]), torch.zeros(H)
+    args = [x.cuda() for x in (qkv, gates, A_log, dt_bias)]
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, False)
+    first = torch.randn(2, floats, generator=g).cuda()
+    qs, sl = torch.tensor([0, T], dtype=torch.int32).cuda(), torch.tensor([1], dtype=torch.int32).cuda()
+    got, want = (torch.empty(T, H * dv, device="cuda") for _ in range(2))
+    state, scan_state = first.clone(), first.clone()
+    ops.delta_chunks(*args, state, SimpleNamespace(h_q_start=[0, T], scratch={}, q_start=qs, slots=sl), got, H=H, nqk=nqk, d=d, dv=dv)
+    ops.delta_scan(*args, scan_state, qs, sl, want, B=1, H=H, nqk=nqk, d=d, dv=dv, max_q_len=T)
+    for a, b in ((got, want), (state, scan_state)):
+        assert bool(b.isfinite().all()) and float((a - b).norm()) <= 4e-6 * float(b.norm())      # 2e-6 for either kernel, as above
+
+
 def test_heads_that_run_token_by_token_are_refused():
     from tensorline_b200 import ops
     for d, dv in ((32, 64), (132, 64), (64, 30), (62, 64), (64, 1028)):
