@@ -118,13 +118,14 @@ class Retention(_MatrixState):
         if len(decay) != num_heads:
             raise ValueError(f"{len(decay)} decays for {num_heads} heads")
         self.decay = torch.tensor([float(x) for x in decay], dtype=torch.float32, device=rt.device)
+        self.positive = bool((self.decay > 0).all())     # chunks work with the decays' logarithms
 
     def _scan(self, h, proj, ctx, state, o):
         H, d, dv = self.H, self.d, self.dv
         rotary = self.position.rotary()
         if not isinstance(rotary, Rotary):
             rotary = Rotary(*rotary)
-        if self._in_chunks(h, proj, ctx):
+        if self.positive and self._in_chunks(h, proj, ctx):
             ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, o, decay=self.decay, inv_freq=rotary.inv_freq,
                               rot=rotary.rot, pairing=rotary.pairing, k_scale=d ** -0.5)
             return

@@ -119,3 +119,30 @@ def test_chunks_against_the_recurrence_in_float64_and_the_scan_kernel(gated, H, 
             assert err <= max(2e-6, 1.5 * base), (err, base)
             assert float((got.double().cpu() - x).abs().max()) <= max(2e-5 * float(x.abs().max()), 4 * float((scan.double().cpu() - x).abs().max()))
     assert torch.equal(state[0].cpu(), first[0])
+
+
+@pytest.mark.parametrize("decay", [[0.0, 0.9], [-0.5, 0.9], [1e-38, 0.9]])
+def test_retention_with_decays_that_have_no_logarithm(decay):
+    """They run token by token; a tiny positive one in chunks: each must give what the scan kernel gives, which is the same
+    floats for the former, and sums in another order for the latter (2e-6 a kernel)."""
+    from tensorline_b200 import ops
+    from tensorline_b200.parts import Runtime
+    from tensorline_b200.parts.recurrent import Retention
+    H, d, dv, T = 2, 64, 64, 200
+    part = Retention(Runtime(torch.device("cuda"), torch.bfloat16, 16), 64, H, d, dv, decay, 1e-5)
+    g = torch.Generator().manual_seed(3)
+    proj = torch.randn(T, 2 * H * d + 2 * H * dv, generator=g).cuda()
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, False)
+    first = torch.zeros(2, floats, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(h_q_start=[0, T], scratch={}, decode_only=False, max_q_len=T, B=1, pos=torch.arange(T, **i32), q_start=torch.tensor([0, T], **i32),
+                          slots=torch.tensor([1], **i32))
+    got, want = (torch.empty(T, H * dv, device="cuda") for _ in range(2))
+    state, scan_state = first.clone(), first.clone()
+    part._scan(torch.empty(T, 64, dtype=torch.bfloat16, device="cuda"), proj, ctx, state, got)
+    ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, scan_state, ctx.q_start, ctx.slots, ctx.pos, want, B=1, decay=torch.tensor(decay).cuda(),
+                    k_scale=d ** -0.5)
+    for a, b in ((got, want), (state, scan_state)):
+        if min(decay) <= 0.0:
+            assert torch.equal(a, b)
+        assert bool(b.isfinite().all()) and float((a - b).norm()) <= 4e-6 * float(b.norm())
