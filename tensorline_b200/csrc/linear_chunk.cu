@@ -11,13 +11,13 @@
 //   carry    per state element, chunk after chunk: the chunk's start state takes the place of its end state; the slot's new state
 //   outputs  every chunk: P = (Q K^T) * weights, then [P | w Q] [V ; S] in one product
 // F and the maxima are sums and maxima in double (64 tokens a chunk and head: a warp's work), every weight the float exponential
-// of one difference of doubles; the products are float multiply-adds.  The state in the slots has the layout of the scan
+// of one difference of doubles; the products have a float's accuracy.  The state in the slots has the layout of the scan
 // kernel, so the two may take turns on one request.  A position's sums depend on where its step began, to rounding.
 //
 // What the scan kernel is bound by is the chain over the tokens at one block a head and 16 columns (128 blocks, 0.36 us a token);
-// here the end states are tiles of 8 x 8 a thread, the outputs products of bfloat16 parts on the tensor cores.
-// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; now gates 4.6, local 33.5, carry 24, outputs 64 us
-// (81 as float multiply-adds).  Fixed decay, 1,650 tokens in 3 requests: local 26, carry 18.5, outputs 70 as multiply-adds.
+// here everything but the carry is products, of bfloat16 parts on the tensor cores (the outputs of heads of up to 32 or above 128: float multiply-adds).
+// Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; now gates 4.6, local 30, carry 24, outputs 64 us
+// (81 as float multiply-adds).  Fixed decay, 1,650 tokens in 3 requests: local 23, carry 18, outputs 44 us (70 as multiply-adds).
 // 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
 // L2 once each way, weigh half as much again at 32.
 #include "common.cuh"
@@ -85,7 +85,7 @@ __device__ __forceinline__ void lc_weights(const LinearChunkArgs& A, int t0, int
 }
 
 // A warp a (chunk, head): the gated kinds' weights, once for all blocks that need them (worked out in each of them, warp 0 held the
-// others up: end states 36 us, now 33.5 and 4.6 here, and the outputs need them without a wait).
+// others up: end states 36 us, 33.5 without and 4.6 here, and the outputs need them without a wait).
 __global__ void __launch_bounds__(32) lc_gates_kernel(const LinearChunkArgs A) {
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, lane = threadIdx.x, t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
@@ -183,31 +183,40 @@ __global__ void __launch_bounds__(256) lc_rotate_kernel(const float* __restrict_
 }
 
 // ------------------------------------------------------------------ end states from zero
-// grid (chunks, H, tiles of RB rows and CB columns); 256 threads, 8 along the columns and 4 along the rows a warp
+// grid (chunks, H, tiles of RB rows and CB columns); 256 threads: two warps along the rows, four along the columns.  The block's K (weighted)
+// and V are cut into parts once; a chunk's 64 tokens are four steps of the tensor cores, so the five small products go first and
+// the leading one on top of them in the same accumulator: as exact as one of its own, and half the registers, which leaves
+// two blocks an SM.  8 heads of 128 x 256, 2,048 tokens, gated: 30 us, as float multiply-adds (tiles of 8 x 8 a thread, bound by the
+// floats they take from shared memory) 33.5; fixed decay, 1,650 tokens: 23.3 against 25.9.
+template <int RB, int CB> struct LocalShape {
+    static constexpr int RK = RB * 2 + 16, RV = CB * 2 + 16;        // bytes of a row of a part of K, of V
+    static constexpr int K = 3 * LC_C * RK, BYTES = K + 3 * LC_C * RV;
+};
+
 template <int RB, int CB, bool GATED>
-__global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) {
-    constexpr int TR = RB / 16, TC = CB / 16;
-    extern __shared__ __align__(16) float sm[];
-    float* Ks = sm;                                      // [64][RB], weighted
-    float* Vs = Ks + LC_C * RB;                          // [64][CB]
+__global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs A) {
+    using Sh = LocalShape<RB, CB>;
+    constexpr int RK = Sh::RK, RV = Sh::RV, MT = RB / 32, NJ = CB / 32, KPER = LC_C * RB / 4 / 256, VPER = LC_C * CB / 4 / 256;
+    extern __shared__ __align__(16) unsigned char smem[];
     __shared__ float w[LC_C];
+    const uint32_t kb = (uint32_t)__cvta_generic_to_shared(smem), vb = kb + Sh::K;
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, col_tiles = (A.dv + CB - 1) / CB, row0 = (blockIdx.z / col_tiles) * RB, col0 = (blockIdx.z % col_tiles) * CB;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
-    auto copy16 = [&](float* dst, const float* src, bool ok) {       // zeros where !ok
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(ok ? src : A.v), "r"(ok ? 16 : 0)
-                     : "memory");
-    };
-    for (int i = tid; i < LC_C * RB / 4; i += 256) {
-        const int t = i / (RB / 4), e = (i % (RB / 4)) * 4;
-        copy16(Ks + t * RB + e, A.k + (size_t)(t0 + t) * A.qk_stride + h * A.d + row0 + e, t < n && row0 + e < A.d);
+    float4 x[KPER], y[VPER];
+#pragma unroll
+    for (int i = 0; i < KPER; ++i) {
+        const int t = (tid + 256 * i) / (RB / 4), e = ((tid + 256 * i) % (RB / 4)) * 4;
+        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n && row0 + e < A.d) x[i] = *reinterpret_cast<const float4*>(A.k + (size_t)(t0 + t) * A.qk_stride + h * A.d + row0 + e);
     }
-    for (int i = tid; i < LC_C * CB / 4; i += 256) {
-        const int t = i / (CB / 4), c = (i % (CB / 4)) * 4;
-        copy16(Vs + t * CB + c, A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c, t < n && col0 + c < A.dv);
+#pragma unroll
+    for (int i = 0; i < VPER; ++i) {
+        const int t = (tid + 256 * i) / (CB / 4), c = ((tid + 256 * i) % (CB / 4)) * 4;
+        y[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < n && col0 + c < A.dv) y[i] = *reinterpret_cast<const float4*>(A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
     const size_t ch = (size_t)blockIdx.x * A.H + h;
     if (GATED) {
         const double* g = A.weights + ch * 3 * LC_C;
@@ -217,53 +226,88 @@ __global__ void __launch_bounds__(256) lc_local_kernel(const LinearChunkArgs A) 
         w[tid] = tid < n ? expf((float)((n - 1 - tid) * la)) * A.k_scale : 0.f;
         if (tid == 0 && blockIdx.z == 0) { A.marks[ch * 3] = n * la; A.marks[ch * 3 + 1] = 0.0; }
     }
+    auto put4 = [&](unsigned char* to, int part, const float4 z) {      // four values' parts, `part` bytes from one part to the next
+        uint2 p[3];
+        parts_cut(z.x, z.y, p[0].x, p[1].x, p[2].x);
+        parts_cut(z.z, z.w, p[0].y, p[1].y, p[2].y);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) *reinterpret_cast<uint2*>(to + e * part) = p[e];
+    };
+#pragma unroll
+    for (int i = 0; i < VPER; ++i)
+        put4(smem + Sh::K + (tid + 256 * i) / (CB / 4) * RV + ((tid + 256 * i) % (CB / 4)) * 8, LC_C * RV, y[i]);
     __syncthreads();
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    for (int i = tid; i < LC_C * RB / 4; i += 256) {     // a thread weighs what it has fetched
-        float4* x = reinterpret_cast<float4*>(Ks + i * 4);
-        const float wt = w[i / (RB / 4)];
-        float4 v = *x;
-        v.x *= wt; v.y *= wt; v.z *= wt; v.w *= wt;
-        *x = v;
+#pragma unroll
+    for (int i = 0; i < KPER; ++i) {
+        const int t = (tid + 256 * i) / (RB / 4);
+        const float wt = w[t];
+        put4(smem + t * RK + ((tid + 256 * i) % (RB / 4)) * 8, LC_C * RK, make_float4(x[i].x * wt, x[i].y * wt, x[i].z * wt, x[i].w * wt));
     }
     __syncthreads();
-    const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
-    float acc[TR][TC];
+    const int wm = wid >> 2, wn = wid & 3, steps = (n + 15) / 16;       // RB / 2 rows and CB / 4 columns a warp
+    // K transposed: tokens (lane & 7) and 8 further from lane 16 on, rows 8 further in every other group; V as in the outputs
+    const uint32_t k_at = kb + ((lane & 7) + (lane >> 4) * 8) * RK + ((lane >> 3) & 1) * 16 + wm * RB;
+    const uint32_t v_at = vb + ((lane & 7) + ((lane >> 3) & 1) * 8) * RV + (lane >> 4) * 16 + wn * (CB / 2);
+    float acc[MT][NJ][4];
 #pragma unroll
-    for (int i = 0; i < TR; ++i)
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
-    const int kn = (n + 3) & ~3;
-#pragma unroll 4
-    for (int t = 0; t < kn; ++t) {
-        float a[TR], b[TC];
-        if constexpr (TR >= 4) {
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
-            for (int i = 0; i < TR / 4; ++i) *reinterpret_cast<float4*>(a + 4 * i) = *reinterpret_cast<const float4*>(Ks + t * RB + 64 * i + ty * 4);
-        } else *reinterpret_cast<float2*>(a) = *reinterpret_cast<const float2*>(Ks + t * RB + ty * 2);
+            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+    for (int s = 0; s < steps; ++s) {                    // the small products
+        uint32_t b[NJ / 2][3][4];
 #pragma unroll
-        for (int j = 0; j < TC / 4; ++j) *reinterpret_cast<float4*>(b + 4 * j) = *reinterpret_cast<const float4*>(Vs + t * CB + 64 * j + tx * 4);
+        for (int j = 0; j < NJ / 2; ++j)
 #pragma unroll
-        for (int i = 0; i < TR; ++i)
+            for (int p = 0; p < 3; ++p) parts_load4_trans(b[j][p], v_at + (p * LC_C + 16 * s) * RV + j * 32);
 #pragma unroll
-            for (int j = 0; j < TC; j += 2) lc_fma2(acc[i][j], acc[i][j + 1], a[i], b[j], b[j + 1]);
-    }
-    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
-    float* to = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
+        for (int i = 0; i < MT; ++i) {
+            uint32_t a[3][4];
 #pragma unroll
-    for (int i = 0; i < TR; ++i) {
-        const int row = row0 + (TR >= 4 ? 64 * (i / 4) + ty * 4 + i % 4 : ty * 2 + i);
-        if (row >= A.d) continue;
+            for (int p = 0; p < 3; ++p) parts_load4_trans(a[p], k_at + (p * LC_C + 16 * s) * RK + i * 32);
 #pragma unroll
-        for (int j = 0; j < TC; j += 4) {
-            const int col = col0 + 16 * j + tx * 4;
-            if (col < A.dv) *reinterpret_cast<float4*>(to + (size_t)row * A.dv + col) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+            for (int p = 0; p < 5; ++p) {                // (lo, hi), (hi, lo), (mid, mid), (mid, hi), (hi, mid)
+                const int pa = p == 0 ? 2 : p == 2 || p == 3 ? 1 : 0, pb = p == 1 ? 2 : p == 2 || p == 4 ? 1 : 0;
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) parts_mma(acc[i][j], a[pa], b[j / 2][pb][(j & 1) * 2], b[j / 2][pb][(j & 1) * 2 + 1]);
+            }
         }
     }
+    for (int s = 0; s < steps; ++s) {                    // the leading one
+        uint32_t b[NJ / 2][4];
+#pragma unroll
+        for (int j = 0; j < NJ / 2; ++j) parts_load4_trans(b[j], v_at + 16 * s * RV + j * 32);
+#pragma unroll
+        for (int i = 0; i < MT; ++i) {
+            uint32_t a[4];
+            parts_load4_trans(a, k_at + 16 * s * RK + i * 32);
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) parts_mma(acc[i][j], a, b[j / 2][(j & 1) * 2], b[j / 2][(j & 1) * 2 + 1]);
+        }
+    }
+    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
+    float* to = A.ends + ch * per;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int row = row0 + wm * (RB / 2) + 16 * i + 8 * e + (lane >> 2);
+            if (row >= A.d) continue;
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                const int col = col0 + wn * (CB / 4) + 8 * j + (lane & 3) * 2;
+                if (col < A.dv) *reinterpret_cast<float2*>(to + (size_t)row * A.dv + col) = make_float2(acc[i][j][2 * e], acc[i][j][2 * e + 1]);
+            }
+        }
     if (GATED && col0 == 0 && tid < RB && row0 + tid < A.d) {        // the normaliser: the same with v = 1
         float s = 0.f;
 #pragma unroll 8
-        for (int t = 0; t < LC_C; ++t) s += Ks[t * RB + tid];
+        for (int t = 0; t < LC_C; ++t) {
+            const unsigned char* k = smem + t * RK + tid * 2;
+            auto part = [&](int p) { return __bfloat162float(*reinterpret_cast<const bf16*>(k + p * LC_C * RK)); };
+            s += part(0) + (part(1) + part(2));
+        }
         to[(size_t)A.d * A.dv + row0 + tid] = s;
     }
 }
@@ -773,7 +817,7 @@ static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
 template <int DP, int CB, bool GATED>
 static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
     constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
-    constexpr int local_smem = LC_C * (RB + CB) * 4, out_smem = OutShape<DP, CB>::FLOATS * 4;
+    constexpr int local_smem = LocalShape<RB, CB>::BYTES, out_smem = OutShape<DP, CB>::FLOATS * 4;
     static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
     int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
     if constexpr (DP >= 64 && DP <= 128) {
