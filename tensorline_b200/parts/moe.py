@@ -145,26 +145,18 @@ class RoutedExperts(Part):
         else:
             ops.topk_softmax(z[:, :E], top, idx, wts, scoring=self.scoring)
         extra = extra_gate = None
-        stream = T <= STREAM_MAX_TOKENS or ctx.graph_max_ctx or self.rt.exact
-        if not stream:
-            offsets, place_of, pair_at = ops.moe_sort(idx, E)
-            host = torch.empty(E + 1, dtype=torch.int32, pin_memory=True)
-            host.copy_(offsets, non_blocking=True)
-            copied = torch.cuda.current_stream(h.device).record_event()
         if self.shared is not None:
             extra, extra_gate = resolve(self.shared.forward(h, ctx)), (z[:, E] if self.shared_gate else None)
         on_input = self.weight_on == "input"
         y = torch.empty((T, self.hidden), dtype=h.dtype, device=h.device)
-        if stream:
+        if T <= STREAM_MAX_TOKENS or ctx.graph_max_ctx or self.rt.exact:
             a = torch.empty((T * top, self.inner), dtype=h.dtype, device=h.device)
             ops.moe_up(h, self.w_up, idx, a, act=self.act, gated=self.gated, in_scale=wts if on_input else None)
             ops.moe_down(a, self.w_down, idx, None if on_input else wts, y, extra=extra, extra_gate=extra_gate,
                          same=h if self.E_real < E else None)
             return y
-        # The one read-back of the step: where every expert's run ends.  It waits for the sort only: the shared expert's products,
-        # launched behind it, run meanwhile.
-        copied.synchronize()
-        bounds = host.tolist()
+        offsets, place_of, pair_at = ops.moe_sort(idx, E)
+        bounds = offsets.tolist()                        # the one read-back of the step: where every expert's run ends
         longest = max(bounds[e + 1] - bounds[e] for e in range(E))
         cap = -(-longest // 64) * 64                     # rows every expert gets in the batched products
         rows = torch.empty((E * cap, self.hidden), dtype=h.dtype, device=h.device)
