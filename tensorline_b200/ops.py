@@ -796,15 +796,16 @@ def linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, 
            "linear_step" if single_tokens else "linear_scan")
 
 
-# From this many tokens of one request a bfloat16 step's matrix memories run as chunks side by side instead of token by token (8 heads of
-# 128 x 256, one request: gated 64 tokens 28 us token by token against 55 in chunks, most of it the host's five launches; 128
-# tokens 51 against 56, 256 tokens 95 against 57, 2,048 tokens 720 against 140).
-LINEAR_CHUNKS_MIN_TOKENS = 128
+# From this many tokens of one request a bfloat16 step's matrix memories run as chunks side by side instead of token by token.  8 heads of
+# 128 x 256, one request, microseconds in chunks / token by token (the former's 38 to 48 are the host's launches): gated 64 tokens
+# 49 / 28, 128 tokens 48 / 50, 256 tokens 47 / 95, 2,048 tokens 115 / 721; fixed decay 128 tokens 38 / 30, 192 tokens 41 / 42,
+# 256 tokens 38 / 54, 2,048 tokens 96 / 400.
+LINEAR_CHUNKS_MIN_TOKENS = {True: 128, False: 192}       # by whether the decays are gated
 
 
-def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int) -> bool:
+def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gated: bool) -> bool:
     """Whether `linear_chunks` takes these sizes (q, k, v one behind the other in a projection's row) and is the faster way."""
-    return proj.dtype == torch.float32 and max_q_len >= LINEAR_CHUNKS_MIN_TOKENS and d % 4 == 0 and dv % 4 == 0 and d <= 256 and \
+    return proj.dtype == torch.float32 and max_q_len >= LINEAR_CHUNKS_MIN_TOKENS[gated] and d % 4 == 0 and dv % 4 == 0 and d <= 256 and \
         proj.shape[1] % 4 == 0 and proj.data_ptr() % 16 == 0
 
 

@@ -10,7 +10,8 @@
 Between steps a request keeps, in its state slots, S (float32, in the scan kernel's own layout) and the convolution's
 last `taps - 1` inputs (float32); both start at zero.  Everything that enters the recurrence beside the projections is
 float32 in both engines; the stacked projection's float32 accumulators are kept as they are.  The mixer reads the step from
-device tensors only (single-token steps sit in CUDA graphs).
+device tensors only (single-token steps sit in CUDA graphs).  In the bfloat16 engine portions of a prompt run as chunks of tokens
+(`ops.delta_chunks`), to rounding the same.
 """
 from __future__ import annotations
 

@@ -3,7 +3,7 @@
     S_t = a_t S_(t-1) + b_t k_t v_t^T,    o_t = S_t^T q_t          S: [d, dv] per head, float32
 
 Three kinds, one pipeline (one stacked projection, one scan kernel, one kernel for the per-head norm and the
-gate, the output projection):
+gate, the output projection; in the bfloat16 engine portions of a prompt run as chunks of tokens side by side instead of the scan):
 
 * `retention`: a_t is a fixed decay per head, b_t = 1; q and k are rotated by position and k is scaled by
   d^-1/2 after the rotation; every head's o is divided by its root mean square (no weight), multiplied by
@@ -90,7 +90,7 @@ class _MatrixState(Part):
 
     def _in_chunks(self, h, proj, ctx) -> bool:
         """Chunks of a portion side by side; the 32-bit engine walks every step in order: the same floats however cut."""
-        return h.dtype == torch.bfloat16 and not ctx.decode_only and ops.takes_linear_chunks(proj, self.d, self.dv, ctx.max_q_len)
+        return h.dtype == torch.bfloat16 and not ctx.decode_only and ops.takes_linear_chunks(proj, self.d, self.dv, ctx.max_q_len, self.gated)
 
     def _head_weight(self):
         return None
