@@ -15,7 +15,7 @@
 // kernel, so the two may take turns on one request.  A position's sums depend on where its step began, to rounding.
 //
 // What the scan kernel is bound by is the chain over the tokens at one block a head and 16 columns (128 blocks, 0.36 us a token);
-// here everything but the carry is products, of bfloat16 parts on the tensor cores (the outputs of heads of up to 32 or above 128: float multiply-adds).
+// here everything but the carry is products of bfloat16 parts on the tensor cores.
 // Measured, 2,048 tokens, 8 heads of 128 x 256: gated 728 us token by token; now gates 4.6, local 30, carry 24, outputs 64 us
 // (81 as float multiply-adds).  Fixed decay, 1,650 tokens in 3 requests: local 23, carry 18, outputs 44 us (70 as multiply-adds).
 // 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
@@ -25,7 +25,6 @@
 
 constexpr int LC_C = 64;                 // tokens a chunk
 constexpr int LC_COLS = 16;              // columns a slice of the state's layout (the scan kernel's)
-constexpr int LC_AT = LC_C + 4;          // stride of the transposed operands: 16-byte reads, neighbouring rows on other banks
 
 struct LinearChunkArgs {
     const float* q; const float* k; int qk_stride;           // element (t, h, e) at t * stride + h * d + e
@@ -44,11 +43,6 @@ struct LinearChunkArgs {
 };
 
 __device__ __forceinline__ float lc_log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
-__device__ __forceinline__ void lc_fma2(float& d0, float& d1, float a, float b0, float b1) {       // (d0, d1) += a (b0, b1)
-    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %2};\n\tmov.b64 y, {%3, %4};\n\tmov.b64 z, {%0, %1};\n\t"
-        "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
-        : "+f"(d0), "+f"(d1) : "f"(a), "f"(b0), "f"(b1));
-}
 
 // A warp, gated: for the n tokens of a chunk that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the running
 // maximum top[t] of u.
@@ -220,10 +214,10 @@ __global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs 
     const size_t ch = (size_t)blockIdx.x * A.H + h;
     if (GATED) {
         const double* g = A.weights + ch * 3 * LC_C;
-        if (tid < LC_C) w[tid] = tid < n ? expf((float)(A.marks[ch * 3] + g[LC_C + tid] - A.marks[ch * 3 + 1])) * A.k_scale : 0.f;
+        if (tid < LC_C) w[tid] = tid < n ? (float)exp(A.marks[ch * 3] + g[LC_C + tid] - A.marks[ch * 3 + 1]) * A.k_scale : 0.f;
     } else if (tid < LC_C) {
         const double la = log((double)A.decay[h]);
-        w[tid] = tid < n ? expf((float)((n - 1 - tid) * la)) * A.k_scale : 0.f;
+        w[tid] = tid < n ? (float)exp((n - 1 - tid) * la) * A.k_scale : 0.f;
         if (tid == 0 && blockIdx.z == 0) { A.marks[ch * 3] = n * la; A.marks[ch * 3 + 1] = 0.0; }
     }
     auto put4 = [&](unsigned char* to, int part, const float4 z) {      // four values' parts, `part` bytes from one part to the next
@@ -283,7 +277,7 @@ __global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs 
             uint32_t a[4];
             parts_load4_trans(a, k_at + 16 * s * RK + i * 32);
 #pragma unroll
-            for (int j = 0; j < NJ; ++j) parts_mma(acc[i][j], a, b[j / 2][(j & 1) * 2], b[j / 2][(j & 1) * 2 + 1]);
+            for (int j = 0; j < NJ; ++j) parts_mma_add(acc[i][j], a, b[j / 2][(j & 1) * 2], b[j / 2][(j & 1) * 2 + 1]);
         }
     }
     const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
@@ -301,14 +295,14 @@ __global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs 
             }
         }
     if (GATED && col0 == 0 && tid < RB && row0 + tid < A.d) {        // the normaliser: the same with v = 1
-        float s = 0.f;
-#pragma unroll 8
+        float s[8] = {};                                 // eight chains of eight tokens
+#pragma unroll
         for (int t = 0; t < LC_C; ++t) {
             const unsigned char* k = smem + t * RK + tid * 2;
             auto part = [&](int p) { return __bfloat162float(*reinterpret_cast<const bf16*>(k + p * LC_C * RK)); };
-            s += part(0) + (part(1) + part(2));
+            s[t & 7] += part(0) + (part(1) + part(2));
         }
-        to[(size_t)A.d * A.dv + row0 + tid] = s;
+        to[(size_t)A.d * A.dv + row0 + tid] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
     }
 }
 
@@ -357,8 +351,8 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(const LinearChunkArgs A) 
         }
         __syncthreads();
         for (int c = tid; c < nc; c += 256) {
-            keep[c] = expf((float)(mk[c][0] + ms[c] - ms[c + 1]));
-            gain[c] = expf((float)(mk[c][1] - ms[c + 1]));
+            keep[c] = (float)exp(mk[c][0] + ms[c] - ms[c + 1]);
+            gain[c] = (float)exp(mk[c][1] - ms[c + 1]);
             if (blockIdx.x == 0) A.marks[((size_t)(first + c0 + c) * A.H + h) * 3 + 2] = ms[c];
         }
         __syncthreads();
@@ -399,192 +393,26 @@ __device__ __forceinline__ void lc_maximum(const LinearChunkArgs& A, const int4 
 }
 
 // ------------------------------------------------------------------ outputs
-// grid (chunks, H, slices of CB columns); DP: rows a head, padded
+// grid (chunks, H, slices of CB columns); DP: rows a head, padded.  256 threads; a block cuts its Q and K (32 tokens at a time) into
+// parts once, P where it is made, and the rows of [S ; V] as they come, 16 at a time, the next ones on their way in registers: little
+// enough shared memory for two blocks an SM, one of which computes while the other waits for its rows (gated, 8 heads
+// of 128 x 256, 2,048 tokens: 64 us; with all of K and 32 rows at a time, one block an SM, 83; multiply-adds 81).  Heads of 256
+// need 178 KB, one block an SM (4 heads of 256 x 256, 1,024 tokens: 34 us; as multiply-adds 43, and in single chains of 320 their outputs were
+// 4.9e-7 off the recurrence in 64 bits where the token-by-token kernel is 1.8e-7 off; now 1.4e-7).  Q S is taken first and weighted by token, P V added to it.
 template <int DP, int CB> struct OutShape {
-    static constexpr int LQ = DP + 4;
-    static constexpr int QT = DP * LC_AT > LC_C * LQ ? DP * LC_AT : LC_C * LQ;       // K first, then Q transposed
-    static constexpr int ROWS = 16, STAGES = 3;                                      // rows of [V ; S] a stage
-    static constexpr int FLOATS = LC_C * LQ + LC_C * LC_AT + QT + STAGES * ROWS * CB;
-};
-
-template <int DP, int CB, bool GATED>
-__global__ void __launch_bounds__(256) lc_out_kernel(const LinearChunkArgs A) {
-    using Sh = OutShape<DP, CB>;
-    constexpr int LQ = Sh::LQ, TC = CB / 16, ROWS = Sh::ROWS, S = Sh::STAGES;
-    extern __shared__ __align__(16) float sm[];
-    float* Qs = sm;                                      // [64][LQ]
-    float* Pt = Qs + LC_C * LQ;                          // [64 s][LC_AT]: P transposed; behind it ...
-    float* Qt = Pt + LC_C * LC_AT;                       // ... K [64][LQ], later the weighted Q transposed [DP][LC_AT]
-    float* Bs = Qt + Sh::QT;                             // [S][ROWS][CB]
-    __shared__ double u[LC_C], top[LC_C];
-    __shared__ float coef[LC_C], den[LC_C];
-    const int4 ck = A.chunks[blockIdx.x];
-    const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
-    if (GATED) lc_maximum<DP>(A, ck, h);
-    const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
-    const float* start = A.ends + ((size_t)blockIdx.x * A.H + h) * per;
-    const double m0 = GATED ? A.marks[((size_t)blockIdx.x * A.H + h) * 3 + 2] : 0.0;
-    const int vr = (n + ROWS - 1) / ROWS * ROWS, sr = (d + ROWS - 1) / ROWS * ROWS, steps = (vr + sr) / ROWS;    // rows of V, of S
-    auto fetch = [&](int step) {                         // rows of [V ; S]: zeros where there are none
-        float* st = Bs + (step % S) * ROWS * CB;
-#pragma unroll
-        for (int i = tid; i < ROWS * CB / 4; i += 256) {
-            const int r = step * ROWS + i / (CB / 4), c = (i % (CB / 4)) * 4, sr0 = r - vr;
-            const bool in = col0 + c < A.dv && (r < vr ? r < n : sr0 < d);
-            const float* src = !in ? A.v : r < vr ? A.v + (size_t)(t0 + r) * A.v_stride + h * A.dv + col0 + c : start + (size_t)sr0 * A.dv + col0 + c;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(st + i * 4)), "l"(src), "r"(in ? 16 : 0)
-                         : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch(0);
-    fetch(1);                                            // d >= 1: at least two steps
-    for (int i = tid; i < LC_C * DP / 4; i += 256) {
-        const int t = i / (DP / 4), e = (i % (DP / 4)) * 4;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-        if (t < n && e < d) {
-            const size_t at = (size_t)(t0 + t) * A.qk_stride + h * d + e;
-            q = *reinterpret_cast<const float4*>(A.q + at);
-            k = *reinterpret_cast<const float4*>(A.k + at);
-            q.x *= A.q_scale; q.y *= A.q_scale; q.z *= A.q_scale; q.w *= A.q_scale;
-            k.x *= A.k_scale; k.y *= A.k_scale; k.z *= A.k_scale; k.w *= A.k_scale;
-        }
-        *reinterpret_cast<float4*>(Qs + t * LQ + e) = q;
-        *reinterpret_cast<float4*>(Qt + t * LQ + e) = k;
-    }
-    if (tid < LC_C) {                                    // top: the running maximum less F; u: what is added to it for a weight
-        const int t = tid;
-        if (GATED) {
-            const double* w = A.weights + ((size_t)blockIdx.x * A.H + h) * 3 * LC_C;
-            const double f = w[t], mm = fmax(m0, w[2 * LC_C + t]);
-            u[t] = w[LC_C + t];
-            coef[t] = expf((float)(m0 - mm));
-            den[t] = expf((float)(-(f + mm)));
-            top[t] = -mm;
-        } else {
-            const double f = (t + 1) * log((double)A.decay[h]);
-            u[t] = -f;
-            top[t] = f;
-            coef[t] = expf((float)f);
-        }
-    }
-    __syncthreads();
-    const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
-    {                                                    // P: tokens ty + 16 i against tx + 16 j, j <= i
-        float s[4][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-        const float* qp = Qs + ty * LQ;
-        const float* kp = Qt + tx * LQ;
-#pragma unroll 2
-        for (int e = 0; e < DP; e += 4) {
-            float4 q4[4], k4[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + 16 * i * LQ + e);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(kp + 16 * j * LQ + e);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j <= i; ++j) {
-                    s[i][j] = fmaf(q4[i].x, k4[j].x, s[i][j]);
-                    s[i][j] = fmaf(q4[i].y, k4[j].y, s[i][j]);
-                    s[i][j] = fmaf(q4[i].z, k4[j].z, s[i][j]);
-                    s[i][j] = fmaf(q4[i].w, k4[j].w, s[i][j]);
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int t = ty + 16 * i, x = tx + 16 * j;
-                float p = 0.f;
-                if (j <= i && x <= t && t < n) p = s[i][j] * expf((float)(top[t] + u[x]));
-                Pt[x * LC_AT + t] = p;
-            }
-    }
-    __syncthreads();                                     // K is read, P is written
-    for (int i = tid; i < LC_C * DP / 4; i += 256) {     // Q transposed, weighted: neighbouring lanes take neighbouring tokens
-        const int t = i % LC_C, e = (i / LC_C) * 4;
-        const float4 q = *reinterpret_cast<const float4*>(Qs + t * LQ + e);
-        const float c = coef[t];
-        Qt[e * LC_AT + t] = q.x * c; Qt[(e + 1) * LC_AT + t] = q.y * c; Qt[(e + 2) * LC_AT + t] = q.z * c; Qt[(e + 3) * LC_AT + t] = q.w * c;
-    }
-    if (GATED) {                                         // n_t . q_t, four lanes a token
-        const int t = tid >> 2, part = tid & 3;
-        double s = 0.0, r = 0.0;                         // the sum may nearly cancel, and everything is divided by it
-#pragma unroll 4
-        for (int x = part; x < LC_C; x += 4) s += Pt[x * LC_AT + t];
-        for (int e = part; e < d; e += 4) r = fma((double)Qs[t * LQ + e], (double)start[(size_t)d * A.dv + e], r);
-        s = fma((double)coef[t], r, s);
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (part == 0) den[t] = fmaxf(fabsf((float)s), den[t]) + A.den_eps;
-    }
-    float acc[4][TC];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < TC; ++j) acc[i][j] = 0.f;
-    for (int step = 0; step < steps; ++step) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();                                 // the step's rows have landed, the step before is read; before the first: Qt, den
-        if (step + 2 < steps) fetch(step + 2);
-        else asm volatile("cp.async.commit_group;" ::: "memory");
-        const int r0 = step * ROWS;
-        const float* at = r0 < vr ? Pt + r0 * LC_AT : Qt + (r0 - vr) * LC_AT;
-        const float* b = Bs + (step % S) * ROWS * CB;
-#pragma unroll 4
-        for (int r = 0; r < ROWS; ++r) {
-            const float4 a4 = *reinterpret_cast<const float4*>(at + r * LC_AT + ty * 4);
-            const float a[4] = {a4.x, a4.y, a4.z, a4.w};
-            float bv[TC];
-#pragma unroll
-            for (int j = 0; j < TC / 4; ++j) *reinterpret_cast<float4*>(bv + 4 * j) = *reinterpret_cast<const float4*>(b + r * CB + 64 * j + tx * 4);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < TC; j += 2) lc_fma2(acc[i][j], acc[i][j + 1], a[i], bv[j], bv[j + 1]);
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = ty * 4 + i;
-        if (t >= n) continue;
-        float* to = A.out + (size_t)(t0 + t) * A.H * A.dv + (size_t)h * A.dv;
-#pragma unroll
-        for (int j = 0; j < TC; j += 4) {
-            const int col = col0 + 16 * j + tx * 4;
-            float4 o = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
-            if (GATED) { o.x /= den[t]; o.y /= den[t]; o.z /= den[t]; o.w /= den[t]; }
-            if (col < A.dv) *reinterpret_cast<float4*>(to + col) = o;
-        }
-    }
-}
-
-// The same with the products on the tensor cores (parts_mma.cuh), for heads of up to 128.  256 threads; a block cuts its Q and K (32
-// tokens at a time) into parts once, P where it is made, and the rows of [S ; V] as they come, 16 at a time, the next ones on their way in
-// registers: little enough shared memory for two blocks an SM, one of which computes while the other waits for its rows (gated, 8 heads
-// of 128 x 256, 2,048 tokens: 64 us; with all of K and 32 rows at a time, one block an SM, 83; multiply-adds 81).  Heads
-// of 256 need 178 KB, so one block an SM: they stay with the multiply-adds.  Q S is taken first and weighted by token, P V added to it.
-template <int DP, int CB> struct OutPartsShape {
     static constexpr int RQ = DP * 2 + 16, RB = CB * 2 + 16, RP = LC_C * 2 + 16;       // bytes of a row of a part of Q and K, of [S ; V], of P
     static constexpr int Q = 3 * LC_C * RQ, STAGE = 3 * 16 * RB, KB = Q / 2 > 2 * STAGE ? Q / 2 : 2 * STAGE, P = 3 * LC_C * RP;
     static constexpr int BYTES = Q + KB + P;             // K's parts lie where the stages of [S ; V] come later
 };
 
 template <int DP, int CB, bool GATED>
-__global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkArgs A) {
-    using Sh = OutPartsShape<DP, CB>;
+__global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) lc_out_kernel(const LinearChunkArgs A) {
+    using Sh = OutShape<DP, CB>;
     constexpr int RQ = Sh::RQ, RB = Sh::RB, RP = Sh::RP, NJ = CB / 32, PER = 16 * CB / 4 / 256;      // n8 tiles a warp, 16-byte loads of a thread a step
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem), kb = base + Sh::Q, pb = kb + Sh::KB;
-    __shared__ double u[LC_C], top[LC_C], nq[LC_C], rowsum[2][LC_C];
+    constexpr int LPT = DP / 4 < 32 ? DP / 4 : 32;       // lanes of a warp that share a token's q
+    __shared__ double u[LC_C], top[LC_C], nq[DP / 4 / LPT][LC_C], rowsum[2][LC_C];
     __shared__ float coef[LC_C], den[LC_C];
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
@@ -636,10 +464,10 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
             }
         }
         put4(smem + t * RQ + e * 2, LC_C * RQ, q);
-        if (GATED) {                                     // DP / 4 neighbouring lanes share a token
+        if (GATED) {
 #pragma unroll
-            for (int o = 1; o < DP / 4; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-            if ((lane & (DP / 4 - 1)) == 0) nq[t] = r;
+            for (int o = 1; o < LPT; o <<= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+            if ((lane & (LPT - 1)) == 0) nq[e / 4 / LPT][t] = r;
         }
     }
     constexpr int KPER = 32 * DP / 4 / 256;              // 16-byte loads of a thread for 32 tokens of K
@@ -667,14 +495,14 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
             const double* w = A.weights + ((size_t)blockIdx.x * A.H + h) * 3 * LC_C;
             const double f = w[t], mm = fmax(m0, w[2 * LC_C + t]);
             u[t] = w[LC_C + t];
-            coef[t] = expf((float)(m0 - mm));
+            coef[t] = (float)exp(m0 - mm);
             den[t] = expf((float)(-(f + mm)));
             top[t] = -mm;
         } else {
             const double f = (t + 1) * log((double)A.decay[h]);
             u[t] = -f;
             top[t] = f;
-            coef[t] = expf((float)f);
+            coef[t] = (float)exp(f);
         }
     }
     put_keys();
@@ -696,8 +524,8 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
                     parts_load4(a[p], base + (p * LC_C + 16 * mi + a_at) * RQ + a_hi + k * 32);
                     parts_load4(b[p], kb + (p * 32 + 16 * (wid & 1) + b_at) * RQ + b_hi + k * 32);
                 }
-                parts_mma6(big[0], rest[0], a, b, 0);
-                parts_mma6(big[1], rest[1], a, b, 2);
+                parts_mma6_round(big[0], rest[0], a, b, 0);
+                parts_mma6_round(big[1], rest[1], a, b, 2);
             }
         }
 #pragma unroll
@@ -734,8 +562,11 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
         }
     }
     __syncthreads();                                     // K is read, P is written
-    if (GATED && tid < LC_C)
-        den[tid] = fmaxf(fabsf((float)(rowsum[0][tid] + rowsum[1][tid] + coef[tid] * nq[tid])), den[tid]) + A.den_eps;
+    if (GATED && tid < LC_C) {
+        double r = nq[0][tid];
+        if (DP / 4 > LPT) r += nq[DP / 4 / LPT - 1][tid];
+        den[tid] = fmaxf(fabsf((float)(rowsum[0][tid] + rowsum[1][tid] + coef[tid] * r)), den[tid]) + A.den_eps;
+    }
     const int wm = wid >> 2, wn = wid & 3;               // 32 tokens and CB / 4 columns a warp
     float big[2][NJ][4], rest[2][NJ][4];
 #pragma unroll
@@ -778,8 +609,8 @@ __global__ void __launch_bounds__(256, 2) lc_out_parts_kernel(const LinearChunkA
                 for (int p = 0; p < 3; ++p) parts_load4_trans(b[p], st + (p * 16 + v_at) * RB + v_hi + (wn * (CB / 4) + 8 * j) * 2);
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    parts_mma6(big[i][j], rest[i][j], a[i], b, 0);
-                    parts_mma6(big[i][j + 1], rest[i][j + 1], a[i], b, 2);
+                    parts_mma6_round(big[i][j], rest[i][j], a[i], b, 0);
+                    parts_mma6_round(big[i][j + 1], rest[i][j + 1], a[i], b, 2);
                 }
             }
         }
@@ -817,12 +648,10 @@ static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
 template <int DP, int CB, bool GATED>
 static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
     constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
-    constexpr int local_smem = LocalShape<RB, CB>::BYTES, out_smem = OutShape<DP, CB>::FLOATS * 4;
+    constexpr int local_smem = LocalShape<RB, CB>::BYTES, out_smem = OutShape<DP, CB>::BYTES;
     static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
     int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
-    if constexpr (DP >= 64 && DP <= 128) {
-        if (!e) e = lc_raise(lc_out_parts_kernel<DP, CB, GATED>, r2, OutPartsShape<DP, CB>::BYTES);
-    } else if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
+    if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
     if (e) return e;
     const int col_tiles = (A.dv + CB - 1) / CB, row_tiles = (A.d + RB - 1) / RB;
     if (GATED) {
@@ -834,9 +663,7 @@ static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaS
     const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
     lc_carry_kernel<R, IS, GATED><<<dim3((unsigned)((per / 4 + 255) / 256), A.H, requests), 256, 0, stream>>>(A);
     if ((e = tl_launch_status())) return e;
-    if constexpr (DP >= 64 && DP <= 128)
-        lc_out_parts_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, OutPartsShape<DP, CB>::BYTES, stream>>>(A);
-    else lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
+    lc_out_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, col_tiles), 256, out_smem, stream>>>(A);
     return tl_launch_status();
 }
 

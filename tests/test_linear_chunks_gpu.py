@@ -1,6 +1,6 @@
 """Matrix memories in chunks (`ops.linear_chunks`): against the recurrence in float64 over the forms it accepts, and against the
 token-by-token kernel, whose state it shares.  Bounds: sums of up to a few hundred float products of order one, 2e-5 of the largest, and
-in the norm no further off than the token-by-token kernel.  A gated output is divided by n . q, which may nearly cancel: what both
+in the norm no further off than the token-by-token kernel, give or take one rounding (2^-24; of the running maximum, whose rounding scales a gated state).  A gated output is divided by n . q, which may nearly cancel: what both
 kernels can be off by is the roundings of its terms over it, 32 of them (2e-6) times sum |terms| / |n . q| of the output and
 of the values it weighs (the norm then says little more than how one token's roundings fell)."""
 from types import SimpleNamespace
@@ -116,9 +116,39 @@ def test_chunks_against_the_recurrence_in_float64_and_the_scan_kernel(gated, H, 
                 assert float(far.max()) <= 0.0, float(far.max())
                 continue
             err, base = (float((y.double().cpu() - x).norm()) / float(x.norm()) for y in (got, scan))
-            assert err <= max(2e-6, 1.5 * base), (err, base)
+            rounding = 2.0 ** -24 * (max(1.0, float(m.abs().max())) if gated else 1.0)
+            assert err <= 1.05 * base + rounding, (err, base)
             assert float((got.double().cpu() - x).abs().max()) <= max(2e-5 * float(x.abs().max()), 4 * float((scan.double().cpu() - x).abs().max()))
     assert torch.equal(state[0].cpu(), first[0])
+
+
+@pytest.mark.parametrize("seed", [0, 1])
+@pytest.mark.parametrize("gated,H,d,dv,T", [(True, 4, 256, 256, 300), (True, 4, 32, 64, 500), (True, 8, 128, 256, 300), (True, 16, 64, 128, 200),
+                                            (False, 4, 128, 128, 130), (False, 4, 256, 128, 200), (False, 8, 96, 64, 300)])
+def test_errors_are_no_larger_than_token_by_token(gated, H, d, dv, T, seed):
+    """Sizes and distributions as the decoders have them, from a state of zero: the error against 64 bits of outputs and states (a
+    gated state with its maximum) is no larger than the token-by-token kernel's; 1.02: what is left of draws of this size."""
+    from tensorline_b200 import ops
+    g = torch.Generator().manual_seed(seed + T)
+    proj = torch.randn(T, 2 * H * d + H * dv, generator=g) * 0.9
+    gates = torch.cat([torch.randn(T, H, generator=g) * 1.3 - 2, torch.randn(T, H, generator=g) * 1.3 + 3], dim=1) if gated else None
+    decay = None if gated else torch.tensor([1.0 - 2.0 ** (-5 - 5 * i / (H - 1)) for i in range(H)])
+    rot, inv = (0, None) if gated else (d, (1e6 ** (-torch.arange(0, d, 2, dtype=torch.float64) / d)).float())
+    scales = dict(q_scale=d ** -0.5, k_scale=1.0) if gated else dict(q_scale=1.0, k_scale=d ** -0.5)
+    kw = dict(gates=gates.cuda(), cap=15.0, den_eps=1e-6, **scales) if gated else dict(decay=decay.cuda(), inv_freq=inv.cuda(), rot=rot, **scales)
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, gated)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(h_q_start=[0, T], scratch={}, pos=torch.arange(T, **i32), q_start=torch.tensor([0, T], **i32), slots=torch.zeros(1, **i32))
+    outs, states = [torch.empty(T, H * dv, device="cuda") for _ in range(2)], [torch.zeros(1, floats, device="cuda") for _ in range(2)]
+    x = proj.cuda()
+    ops.linear_chunks(x, 0, H * d, 2 * H * d, H, d, dv, states[0], ctx, outs[0], **kw)
+    ops.linear_scan(x, 0, H * d, 2 * H * d, H, d, dv, states[1], ctx.q_start, ctx.slots, ctx.pos, outs[1], B=1, **kw)
+    zero = torch.zeros(H, d, dv, dtype=torch.float64)
+    o, S, n, m, _ = recurrence(proj.double(), gates.double() if gated else None, decay, H, d, dv, zero, zero[:, :, 0] if gated else None,
+                               zero[:, 0, 0] if gated else None, torch.arange(T), inv, rot, False, 15.0, scales["q_scale"], scales["k_scale"], 1e-6)
+    for got, want in ((outs, o), ([s[0] for s in states], slot_rows(S, n, m))):
+        err, base = (float((y.double().cpu() - want).norm()) / float(want.norm()) for y in got)
+        assert err <= 1.02 * base + (2.0 ** -24 * float(m.abs().max()) if gated and want is not o else 0.0), (err, base)
 
 
 @pytest.mark.parametrize("decay", [[0.0, 0.9], [-0.5, 0.9], [1e-38, 0.9]])
