@@ -20,7 +20,7 @@
 // is bound by shared memory: a warp gets 32 floats of it a cycle and needs one for two multiply-adds with 16 columns a
 // block (measured 286 us for 2,048 tokens, 8 heads of 128 x 256; token by token 642).  On mma.sync a warp holds 32 rows of the transposed state [16 columns x 128 rows] as
 // accumulators, which are the next product's first operand as they lie; W, K, Q and P come as bfloat16 parts, cut once
-// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 36.
+// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 34.
 #include "common.cuh"
 #include "parts_mma.cuh"
 
@@ -51,7 +51,9 @@ struct DeltaChunkArgs {
 __device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
 // ------------------------------------------------------------------ prepare
-// grid (chunks, H); shared memory K, Q [32][DP + 4], V [32][dv].  384 threads: the columns of a head of 128 x 256 at once
+// grid (chunks, H); shared memory K, Q [32][DP + 4], V [32][dv].  384 threads: the columns of a head of 128 x 256 at once.  The dot
+// products of a chunk's keys and queries are taken on parts as well: as single chains of multiply-adds over 128 rows they were what
+// the outputs lost most by (130 tokens: 2.1e-7 off the recurrence in 64 bits, now 1.1e-7; the token-by-token kernel 1.5e-7).
 constexpr int DC_PREP = 384;
 template <int DP>
 __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArgs A) {
@@ -120,36 +122,34 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
             for (int c = 0; c < 3; ++c) *reinterpret_cast<uint2*>(to + (isq ? dc_parts(DP) : 0) + (c * DC_C + t) * ROW + e * 2) = p[c];
         }
     }
-    if (wid < 8) {                                       // k_t . k_s and q_t . k_s: tokens ty, ty + 16 against tx, tx + 16
-        const int tx = (wid & 1) * 8 + (lane & 7), ty = (wid >> 1) * 4 + (lane >> 3);
-        float kk[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, qk[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll 4
-        for (int e = 0; e < DP; e += 4) {
-            float4 a[2], q[2], b[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                a[i] = *reinterpret_cast<const float4*>(Ks + (ty + 16 * i) * LD + e);
-                q[i] = *reinterpret_cast<const float4*>(Qs + (ty + 16 * i) * LD + e);
-                b[i] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * i) * LD + e);
+    if (wid < 8) {                                       // k_t . k_s (even warps) and q_t . k_s: a warp 16 tokens t and 16 tokens s
+        const int g = lane >> 2, q2 = (lane & 3) * 2, t0w = ((wid >> 1) & 1) * 16, s0w = (wid >> 2) * 16;
+        const bool qk = wid & 1;
+        float big[2][4] = {}, rest[2][4] = {};
+        if (s0w <= t0w) {
+            const float* at = (qk ? Qs : Ks) + (t0w + g) * LD + q2;
+            const float* bt = Ks + (s0w + g) * LD + q2;
+            auto cut = [&](const float* x, uint32_t (&p)[3][4], int i) {
+                const float2 v = *reinterpret_cast<const float2*>(x);
+                parts_cut(v.x, v.y, p[0][i], p[1][i], p[2][i]);
+            };
+#pragma unroll 2
+            for (int e = 0; e < DP; e += 16) {
+                uint32_t a[3][4], b[3][4];
+                cut(at + e, a, 0); cut(at + 8 * LD + e, a, 1); cut(at + e + 8, a, 2); cut(at + 8 * LD + e + 8, a, 3);
+                cut(bt + e, b, 0); cut(bt + e + 8, b, 1); cut(bt + 8 * LD + e, b, 2); cut(bt + 8 * LD + e + 8, b, 3);
+                parts_mma6_round(big[0], rest[0], a, b, 0);
+                parts_mma6_round(big[1], rest[1], a, b, 2);
             }
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j <= i; ++j) {
-                    kk[i][j] = fmaf(a[i].x, b[j].x, kk[i][j]); kk[i][j] = fmaf(a[i].y, b[j].y, kk[i][j]);
-                    kk[i][j] = fmaf(a[i].z, b[j].z, kk[i][j]); kk[i][j] = fmaf(a[i].w, b[j].w, kk[i][j]);
-                    qk[i][j] = fmaf(q[i].x, b[j].x, qk[i][j]); qk[i][j] = fmaf(q[i].y, b[j].y, qk[i][j]);
-                    qk[i][j] = fmaf(q[i].z, b[j].z, qk[i][j]); qk[i][j] = fmaf(q[i].w, b[j].w, qk[i][j]);
-                }
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int t = ty + 16 * i, s = tx + 16 * j;
-                const float w = s <= t && t < n ? expf((float)(F[t] - F[s])) : 0.f;
-                As[t][s] = s < t ? beta[t] * (w * kk[i][j]) : 0.f;
-                Ps[t][s] = w * qk[i][j];
+            for (int x = 0; x < 4; ++x) {
+                const int t = t0w + g + (x >> 1) * 8, s = s0w + 8 * j + q2 + (x & 1);
+                const float dot = big[j][x] + rest[j][x], w = s <= t && t < n ? expf((float)(F[t] - F[s])) : 0.f;
+                if (qk) Ps[t][s] = w * dot;
+                else As[t][s] = s < t ? beta[t] * (w * dot) : 0.f;
             }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
