@@ -165,6 +165,26 @@ __device__ __forceinline__ int tl_checked(int v, int limit, const TlLimits& L, i
 }
 TL_EXPORT int tl_check_build();
 
+// A step's requests as the scan kernels take them beside kernels that work chunks of a request's tokens (linear_chunk.cu, delta_chunk.cu):
+// a run is (request, its first chunk, its chunks).  Those kernels leave a mark per chunk, head and tile of operands that hold a
+// value whose products they cannot take as the recurrence does (not a number, an infinity, above TL_CHUNK_LARGE); a marked
+// (request, head) is left to the scan kernel, which otherwise passes over requests that ran as chunks.
+constexpr float TL_CHUNK_LARGE = 1099511627776.0f;    // 2^40: products of three such values, and sums of them, are floats
+struct TlRuns { const int4* runs; const int* marked; int tiles; };
+__device__ __forceinline__ bool tl_chunk_odd(float x) { return !(fabsf(x) <= TL_CHUNK_LARGE); }
+// all threads of a block: whether the head `h` (of H) of a request is marked
+__device__ __forceinline__ bool tl_chunk_marked(const int* marked, int tiles, int first, int chunks, int h, int H) {
+    int any = 0;
+    for (int i = threadIdx.x; i < chunks * tiles; i += blockDim.x) any |= marked[((size_t)(first + i / tiles) * H + h) * tiles + i % tiles];
+    return __syncthreads_or(any);
+}
+// the request that block column `b` of a scan kernel works on, -1: none
+__device__ __forceinline__ int tl_run(const TlRuns& R, int b, int h, int H) {
+    if (!R.runs) return b;
+    const int4 r = R.runs[b];
+    return r.z == 0 || tl_chunk_marked(R.marked, R.tiles, r.y, r.z, h, H) ? r.x : -1;
+}
+
 // The tracing build (-DTL_TRACE=1): the kernels that wait on the kernel in front of them (the few-token product, the TMA
 // decode attention) leave global-timer stamps, eight a block, in a buffer the host names: when the block started, when
 // its dependency wait returned, when its first and its last operand tile had landed, when it ended, and three places of

@@ -285,6 +285,7 @@ struct DeltaArgs {
     const int* q_start; const int* slots;
     float* out;                            // [T, H * dv]
     int H, nqk, d, dv;
+    TlRuns runs;                           // beside chunks; runs.runs null: every request
 };
 
 template <int R, int IS> struct DeltaShape {
@@ -317,11 +318,13 @@ __global__ void __launch_bounds__(DeltaShape<R, IS>::NT) delta_scan_kernel(const
     __shared__ float vs[CH * DELTA_JS];
     __shared__ float gg[CH], gb[CH], gl[COMP ? CH : 1];
     const int d = A.d;
-    const int b = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
+    const int h = blockIdx.y, z = blockIdx.z;
     const int hq = h / (A.H / A.nqk);                            // the q/k head this value head reads
     const int tid = threadIdx.x, islice = tid % IS, j = tid / IS;
     grid_dependency_wait();
     grid_dependency_trigger();
+    const int b = tl_run(A.runs, blockIdx.x, h, A.H);
+    if (b < 0) return;
     const int t0 = A.q_start[b], t1 = A.q_start[b + 1];
     if (t0 >= t1) return;
     float* st = A.state + (size_t)A.slots[b] * A.slot_stride + ((size_t)h * gridDim.z + z) * (COMP ? 2 * PB : PB);
@@ -497,11 +500,11 @@ TL_EXPORT int tl_delta_columns() { return DELTA_JS; }
 TL_EXPORT int tl_delta_scan(const float* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, int gate_stride,
                             const float* A_log, const float* dt_bias, float* state, long long slot_stride, const int* q_start,
                             const int* slots, float* out, int B, int H, int nqk, int d, int dv, int max_q_len, int compensated,
-                            cudaStream_t stream) {
+                            const int* runs, const int* marked, int tiles, cudaStream_t stream) {      // runs: B of them
     if (B <= 0 || H <= 0) return 0;
     if (H > 65535 || nqk < 1 || H % nqk) return 1;
     const DeltaArgs A{qkv, stride, q_off, k_off, v_off, gates, gate_stride, A_log, dt_bias, state, slot_stride, q_start, slots, out,
-                      H, nqk, d, dv};
+                      H, nqk, d, dv, TlRuns{(const int4*)runs, marked, tiles}};
     const dim3 grid(B, H, (dv + DELTA_JS - 1) / DELTA_JS);
 #define DSK(R_, IS_, AH, CO) launch_after_wait(delta_scan_kernel<R_, IS_, AH, CO>, grid, dim3(DeltaShape<R_, IS_>::NT), 0, stream, A)
 #define DS(R_, IS_) (compensated ? (max_q_len > DeltaShape<R_, IS_>::CH ? DSK(R_, IS_, true, true) : DSK(R_, IS_, false, true)) \

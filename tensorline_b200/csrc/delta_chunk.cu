@@ -44,6 +44,7 @@ struct DeltaChunkArgs {
     unsigned char* M;                    // [chunks][H] marks
     unsigned char* U;                    // [chunks][H][nz] slices of U0
     unsigned char* K;                    // [chunks][nqk] parts of K, then of Q
+    int* marked;                         // [chunks][H]: operands that the scan kernel has to take (common.cuh)
     float* out;
     int H, nqk, d, dv, nz;
 };
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
         for (int c = 0; c < 3; ++c) *reinterpret_cast<uint32_t*>(A.P + at * DC_PB + (c * DC_C + t) * DC_PROW + x * 2) = p[c];
     }
     const int wide = (dv + 15) & ~15;                    // columns behind the last are zeros, like rows behind d
+    bool odd = false;                                    // a decay or a beta that is no number shows in W's columns
     for (int c = tid; c < wide + DP; c += DC_PREP) {
         float u[DC_C];
         const bool isw = c >= wide;
@@ -171,6 +173,7 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
         for (int t = 0; t < DC_C; ++t) {
             if (isw) u[t] = beta[t] * (grow[t] * Ks[t * LD + e]);
             else u[t] = c < dv ? beta[t] * Vs[t * dv + c] : 0.f;
+            odd = odd || tl_chunk_odd(isw ? u[t] + Ks[t * LD + e] : c < dv ? Vs[t * dv + c] : 0.f);
         }
 #pragma unroll
         for (int t = 1; t < DC_C; ++t) {
@@ -203,6 +206,8 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
             for (int t = 0; t < DC_C; ++t) to[t * 20] = u[t];
         }
     }
+    odd = __syncthreads_or(odd);
+    if (tid == 0) A.marked[at] = odd;
 }
 
 // ------------------------------------------------------------------ walk
@@ -253,6 +258,10 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0);
+    if (tl_chunk_marked(A.marked, 1, first, ck.z, h, A.H)) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        return;                                          // the scan kernel's
+    }
     // this lane's addresses in fragments of two tiles: rows (tokens) of W, Q, P, and of K as it is transposed
     const uint32_t x_at = ((lane & 7) + (lane >> 4) * 8) * ROW + ((lane >> 3) & 1) * 16 + wid * RW * 2;
     const uint32_t k_at = ((lane & 7) + ((lane >> 3) & 1) * 8) * ROW + (lane >> 4) * 16 + wid * RW * 2;
@@ -373,7 +382,7 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
 }
 
 template <int DP>
-static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int n_chunks, int requests, cudaStream_t stream) {
+static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int* marked, int n_chunks, int requests, cudaStream_t stream) {
     using Sh = WalkShape<DP>;
     const int prep_smem = (2 * DC_C * (DP + 4) + DC_C * A.dv) * 4;
     static int raised[TL_MAX_DEVICES] = {};              // what prepare's shared memory was raised to
@@ -391,6 +400,7 @@ static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int n_chunks, int
     A.M = A.P + ch * DC_PB;
     A.U = A.M + ch * DC_MB;
     A.K = A.U + ch * A.nz * DC_UB;
+    A.marked = marked;
     dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), DC_PREP, prep_smem, stream>>>(A);
     const int e = tl_launch_status();
     if (e) return e;
@@ -409,16 +419,16 @@ TL_EXPORT int tl_delta_chunk_bytes(int H, int nqk, int d, int dv) {
     return H * (parts + DC_PB + DC_MB + (dv + DC_COLS - 1) / DC_COLS * DC_UB) + nqk * 2 * parts;
 }
 
-// scratch: `tl_delta_chunk_bytes` bytes a chunk.  The offsets and the stride are multiples of 4, the pointers 16-byte aligned.
+// scratch: `tl_delta_chunk_bytes` bytes a chunk; marked: int [n_chunks, H], for the scan kernel (tiles: 1).  The offsets and the stride are multiples of 4, the pointers 16-byte aligned.
 TL_EXPORT int tl_delta_chunks(const float* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, int gate_stride,
                               const float* A_log, const float* dt_bias, float* state, long long slot_stride, const int* q_start,
-                              const int* slots, const int* chunks, int n_chunks, const int* firsts, int requests, void* scratch, float* out,
+                              const int* slots, const int* chunks, int n_chunks, const int* firsts, int requests, void* scratch, int* marked, float* out,
                               int H, int nqk, int d, int dv, cudaStream_t stream) {
     if (n_chunks <= 0 || H <= 0) return 0;
     if (H > 65535 || nqk < 1 || H % nqk || !tl_delta_chunk_bytes(H, nqk, d, dv) || ((stride | q_off | k_off | v_off) & 3) ||
         ((((uintptr_t)qkv) | ((uintptr_t)scratch) | ((uintptr_t)out)) & 15)) return 1;
     const DeltaChunkArgs A{qkv, stride, q_off, k_off, v_off, gates, gate_stride, A_log, dt_bias, state, slot_stride, q_start, slots,
-                           (const int4*)chunks, firsts, nullptr, nullptr, nullptr, nullptr, nullptr, out, H, nqk, d, dv, (dv + DC_COLS - 1) / DC_COLS};
-    if (d <= 64) return dc_launch<64>(A, (unsigned char*)scratch, n_chunks, requests, stream);
-    return dc_launch<128>(A, (unsigned char*)scratch, n_chunks, requests, stream);
+                           (const int4*)chunks, firsts, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, out, H, nqk, d, dv, (dv + DC_COLS - 1) / DC_COLS};
+    if (d <= 64) return dc_launch<64>(A, (unsigned char*)scratch, marked, n_chunks, requests, stream);
+    return dc_launch<128>(A, (unsigned char*)scratch, marked, n_chunks, requests, stream);
 }

@@ -38,6 +38,7 @@ struct LinearChunkArgs {
     float* ends;                         // [chunks][H][d dv (+ d)]: end states from zero, then start states
     double* marks;                       // [chunks][H][3]: the chunk's F, its maximum, the running maximum in front of it
     double* weights;                     // gated: [chunks][H][3][64], F, u and top of lc_weights
+    int* marked; int tiles;              // [chunks][H][tiles]: operands that the scan kernel has to take (common.cuh)
     float* out;
     int H, d, dv, nz; float den_eps;
 };
@@ -220,6 +221,11 @@ __global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs 
         w[tid] = tid < n ? (float)exp((n - 1 - tid) * la) * A.k_scale : 0.f;
         if (tid == 0 && blockIdx.z == 0) { A.marks[ch * 3] = n * la; A.marks[ch * 3 + 1] = 0.0; }
     }
+    bool odd = tid < LC_C && w[tid] != w[tid];           // a gate that is no number
+#pragma unroll
+    for (int i = 0; i < KPER; ++i) odd = odd || tl_chunk_odd(x[i].x) || tl_chunk_odd(x[i].y) || tl_chunk_odd(x[i].z) || tl_chunk_odd(x[i].w);
+#pragma unroll
+    for (int i = 0; i < VPER; ++i) odd = odd || tl_chunk_odd(y[i].x) || tl_chunk_odd(y[i].y) || tl_chunk_odd(y[i].z) || tl_chunk_odd(y[i].w);
     auto put4 = [&](unsigned char* to, int part, const float4 z) {      // four values' parts, `part` bytes from one part to the next
         uint2 p[3];
         parts_cut(z.x, z.y, p[0].x, p[1].x, p[2].x);
@@ -230,7 +236,8 @@ __global__ void __launch_bounds__(256, 2) lc_local_kernel(const LinearChunkArgs 
 #pragma unroll
     for (int i = 0; i < VPER; ++i)
         put4(smem + Sh::K + (tid + 256 * i) / (CB / 4) * RV + ((tid + 256 * i) % (CB / 4)) * 8, LC_C * RV, y[i]);
-    __syncthreads();
+    odd = __syncthreads_or(odd);
+    if (tid == 0) A.marked[ch * A.tiles + blockIdx.z] = odd;
 #pragma unroll
     for (int i = 0; i < KPER; ++i) {
         const int t = (tid + 256 * i) / (RB / 4);
@@ -331,6 +338,7 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(const LinearChunkArgs A) 
     float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
     if (mine) S = make_float4(slot[at(0, 0)], slot[at(1, 0)], slot[at(2, 0)], slot[at(3, 0)]);
     double m = GATED ? (double)slot[R * NT] : 0.0;
+    if (tl_chunk_marked(A.marked, A.tiles, first, ck.z, h, A.H)) return;      // the scan kernel's, outputs as well
     float* e = A.ends + ((size_t)first * A.H + h) * per + i4;
     const size_t step = (size_t)A.H * per;
     for (int c0 = 0; c0 < ck.z; c0 += LC_CARRY) {
@@ -385,7 +393,7 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(const LinearChunkArgs A) 
 template <int DP>
 __device__ __forceinline__ void lc_maximum(const LinearChunkArgs& A, const int4 ck, int h) {
     constexpr int R = DP == 32 ? 4 : 8, IS = DP / R, NT = (IS * (LC_COLS + 1) + 31) / 32 * 32, PB = R * NT + 4;
-    if (blockIdx.z || ck.y != ck.z - 1) return;
+    if (blockIdx.z || ck.y != ck.z - 1 || tl_chunk_marked(A.marked, A.tiles, ck.w, ck.z, h, A.H)) return;
     const double* g = A.marks + ((size_t)blockIdx.x * A.H + h) * 3;
     const float m = (float)fmax(g[0] + g[2], g[1]);
     float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + (size_t)h * A.nz * PB;
@@ -673,21 +681,27 @@ static int lc_pick(const LinearChunkArgs& A, int n_chunks, int requests, cudaStr
     return A.dv <= 64 ? lc_launch<DP, 64, false>(A, n_chunks, requests, stream) : lc_launch<DP, 128, false>(A, n_chunks, requests, stream);
 }
 
+// Blocks of the end states a (chunk, head).
+static int lc_tiles(int d, int dv) {
+    const int cb = dv <= 64 ? 64 : 128, rb = d <= 32 ? 32 : d <= 64 ? 64 : 128;
+    return ((d + rb - 1) / rb) * ((dv + cb - 1) / cb);
+}
 TL_EXPORT int tl_linear_chunk() { return LC_C; }
+TL_EXPORT int tl_linear_chunk_tiles(int d, int dv) { return lc_tiles(d, dv); }
 
 // `rows` (float [T, 2 H d], with a rotation): where q and k go.  ends: float [n_chunks, H, d dv (+ d with gates)], marks: double
-// [n_chunks, H, 3], with gates then [n_chunks, H, 192].  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
+// [n_chunks, H, 3], with gates then [n_chunks, H, 192].  marked: int [n_chunks, H, tl_linear_chunk_tiles(d, dv)], for the scan kernel.  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
 TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, int k_off, int v_off, const float* gates, float cap,
                                const float* decay, const float* inv_freq, int rot, int interleaved, const int* pos, float q_scale,
                                float k_scale, float* rows, float* state, long long slot_stride, const int* q_start, const int* slots,
-                               const int* chunks, int n_chunks, const int* firsts, int requests, float* ends, double* marks, float* out,
+                               const int* chunks, int n_chunks, const int* firsts, int requests, float* ends, double* marks, int* marked, float* out,
                                int H, int d, int dv, float den_eps, cudaStream_t stream) {
     if (n_chunks <= 0 || H <= 0) return 0;
     if (H > 65535 || requests > 65535 || d < 4 || d > 256 || ((d | dv | stride | q_off | k_off | v_off) & 3) || (rot & 1) || rot > d ||
         (rot && !rows) || (gates != nullptr) == (decay != nullptr) ||
         ((((uintptr_t)proj) | ((uintptr_t)rows) | ((uintptr_t)ends) | ((uintptr_t)out)) & 15)) return 1;
     LinearChunkArgs A{proj + q_off, proj + k_off, stride, proj + v_off, stride, gates, cap, decay, q_scale, k_scale, state, slot_stride,
-                      q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
+                      q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, marked, lc_tiles(d, dv), out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
     if (rot) {
         if (rot % (interleaved ? 4 : 8) == 0)
             lc_rotate_kernel<true><<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);

@@ -45,6 +45,7 @@ struct ScanArgs {
     int H, d, dv;
     float den_eps;
     const float* lower; const float* bias;  // channel gates: [H, d] each; k_off is then where x_f lies
+    TlRuns runs;                           // the scan kernel beside chunks; runs.runs null: every request
 };
 
 // KIND of the templates below
@@ -80,7 +81,10 @@ __global__ void __launch_bounds__(ScanShape<R, IS, KIND>::NT) linear_scan_kernel
     float* gb = ga + SCAN_C;
     float* gm = gb + SCAN_C;
     float* nq = gm + SCAN_C;
-    const int b = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
+    grid_dependency_wait();                              // launched as a dependent: nothing of another kernel is touched before this
+    grid_dependency_trigger();
+    const int h = blockIdx.y, z = blockIdx.z, b = tl_run(A.runs, blockIdx.x, h, A.H);
+    if (b < 0) return;
     const int tid = threadIdx.x, islice = tid % IS, j = tid / IS;
     const int t0 = A.q_start[b], t1 = A.q_start[b + 1];
     float* st = A.state + (size_t)A.slots[b] * A.slot_stride + ((size_t)h * gridDim.z + z) * PB;
@@ -392,8 +396,7 @@ static int launch_scan_shape(const ScanArgs& A, int B, bool single, cudaStream_t
             raised[dev] = true;
         }
     }
-    linear_scan_kernel<TA, R, IS, KIND><<<dim3(B, A.H, nz), Sh::NT, smem, stream>>>(A);
-    return tl_launch_status();
+    return launch_after_wait(linear_scan_kernel<TA, R, IS, KIND>, dim3(B, A.H, nz), dim3(Sh::NT), smem, stream, A);
 }
 
 template <typename TA, int KIND>
@@ -412,12 +415,13 @@ TL_EXPORT int tl_linear_scan(const void* proj, int act_dtype, int stride, int q_
                              int interleaved, const int* pos, float q_scale, float k_scale, float* state,
                              long long slot_stride, const int* q_start, const int* slots, float* out, int B, int H,
                              int d, int dv, float den_eps, int single_tokens, const float* lower, const float* bias,
-                             cudaStream_t stream) {
-    // single_tokens: every request of the step brings exactly one token (the caller knows; the step kernel takes it)
+                             const int* runs, const int* marked, int tiles, cudaStream_t stream) {
+    // single_tokens: every request of the step brings exactly one token (the caller knows; the step kernel takes it).  runs: B of them.
     if (B <= 0 || H <= 0) return 0;
     if (H > 65535 || (rot & 1) || rot > d) return 1;
     const ScanArgs A{proj, stride, q_off, k_off, v_off, gates, cap, decay, inv_freq, rot, interleaved, pos, q_scale, k_scale,
-                     state, slot_stride, q_start, slots, out, H, d, dv, den_eps, lower, bias};
+                     state, slot_stride, q_start, slots, out, H, d, dv, den_eps, lower, bias, TlRuns{(const int4*)runs, marked, tiles}};
+    if (runs && single_tokens) return 1;
     const bool gated = gates != nullptr;
     if ((lower == nullptr) != (bias == nullptr) || (lower && (gated || decay || rot))) return 1;
     const bool single = single_tokens != 0;

@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import collections
 import ctypes
+from types import SimpleNamespace
 
 import numpy as np
 import torch
@@ -35,12 +36,13 @@ _SIGNATURES = {
     "tl_argmax": [_P, _I, _I, _I, _P, _P, _P],
     "tl_sample": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
     "tl_linear_scan": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, ctypes.c_longlong, _P, _P, _P, _I, _I,
-                       _I, _I, _F, _I, _P, _P, _P],
+                       _I, _I, _F, _I, _P, _P, _P, _P, _I, _P],
     "tl_channel_scan": [_P, _I, _I, _I, _I, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
     "tl_channel_chunk": [],
     "tl_linear_chunks": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P,
-                         _P, _I, _I, _I, _F, _P],
+                         _P, _P, _I, _I, _I, _F, _P],
     "tl_linear_chunk": [],
+    "tl_linear_chunk_tiles": [_I, _I],
     "tl_scan_state_floats": [_I, _I],
     "tl_scan_columns": [],
     "tl_head_norm_gate": [_P, _P, _I, _I, _P, _I, _P, _I, _I, _I, _I, _F, _I, _P],
@@ -60,8 +62,8 @@ _SIGNATURES = {
     "tl_gelu": [_P, _I, ctypes.c_longlong, _P],
     "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
     "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P],
-    "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P],
-    "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _I, _I, _I, _I, _P],
+    "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
+    "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "tl_delta_chunk": [],
     "tl_delta_chunk_bytes": [_I, _I, _I, _I],
     "tl_delta_state_floats": [_I, _I],
@@ -792,7 +794,7 @@ def linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, 
     _check(core().tl_linear_scan(_ptr(proj), dtype_code(proj.dtype), proj.shape[1], q_off, k_off, v_off, _ptr(gates), float(cap),
                                  _ptr(decay), _ptr(inv_freq) if rot else None, int(rot), int(pairing == "interleaved"), _ptr(pos),
                                  float(q_scale), float(k_scale), _ptr(state), per_slot, _ptr(q_start), _ptr(slots), _ptr(out),
-                                 int(B), H, d, dv, float(den_eps), int(single_tokens), _ptr(lower), _ptr(bias), _stream()),
+                                 int(B), H, d, dv, float(den_eps), int(single_tokens), _ptr(lower), _ptr(bias), None, None, 0, _stream()),
            "linear_step" if single_tokens else "linear_scan")
 
 
@@ -809,14 +811,17 @@ def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gat
         proj.shape[1] % 4 == 0 and proj.data_ptr() % 16 == 0
 
 
-def _chunk_list(ctx, key: str, chunk: int, device) -> tuple:
-    """The step's chunks of `chunk` tokens on the device (`channel_chunks`' rows, then every request's first row), how many there
-    are, and of how many requests: one description a step, for every layer."""
+def _chunk_list(ctx, key: str, chunk: int, device) -> SimpleNamespace:
+    """The step's chunks of `chunk` tokens on the device: `rows` (`channel_chunks`' rows, `n` of them), `runs` (request, first chunk,
+    chunks, 0) of the `requests` requests, and `firsts`, their first rows.  One description a step, for every layer."""
     if key not in ctx.scratch:
         rows, _ = channel_chunks(ctx.h_q_start, chunk)
         firsts = np.nonzero(rows[:, 1] == 0)[0].astype(np.int32)
-        both = torch.from_numpy(np.concatenate([rows.reshape(-1), firsts])).to(device, non_blocking=True)
-        ctx.scratch[key] = (both, len(rows), len(firsts))
+        runs = np.stack([rows[firsts, 0], firsts, rows[firsts, 2], np.zeros_like(firsts)], axis=1)
+        words = torch.from_numpy(np.concatenate([rows.reshape(-1), runs.reshape(-1), firsts])).to(device, non_blocking=True)
+        at = _ptr(words)
+        ctx.scratch[key] = SimpleNamespace(words=words, rows=at, n=len(rows), runs=at + 16 * len(rows), requests=len(firsts),
+                                           firsts=at + 16 * (len(rows) + len(firsts)))
     return ctx.scratch[key]
 
 
@@ -825,7 +830,8 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
                   rot: int = 0, pairing: str = "half", q_scale: float = 1.0, k_scale: float = 1.0, den_eps: float = 0.0) -> None:
     """`linear_scan` with one decay a head (`decay` or `gates`) for steps of several tokens a request: chunks of a request's tokens
     side by side, as matrix products of floats.  proj float32 with 16-byte rows; the state as `linear_scan` keeps it, so the two may
-    take turns.  A position's sums depend on where its step began, to rounding."""
+    take turns.  A position's sums depend on where its step began, to rounding.  A head of a request whose keys, values or gates hold
+    something that is no number, infinite or above 2^40 goes token by token: what such a value reaches is what it reaches there."""
     T = proj.shape[0]
     _contig(proj, "proj"); _contig(state, "state"); _contig(out, "out")
     if (decay is None) == (gates is None):
@@ -847,16 +853,21 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
     if rot and (inv_freq is None or inv_freq.dtype != torch.float32 or inv_freq.numel() != rot // 2):
         raise KernelError("linear_chunks: inv_freq must be float32 [rot/2]")
     interleaved = _pairing(pairing, "linear_chunks")
-    both, n, requests = _chunk_list(ctx, "linear_chunks", core().tl_linear_chunk(), proj.device)
-    dev = proj.device
+    lib, dev = core(), proj.device
+    step = _chunk_list(ctx, "linear_chunks", lib.tl_linear_chunk(), dev)
+    n, tiles, doubles = step.n, lib.tl_linear_chunk_tiles(d, dv), 3 if gates is None else 195
     turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
     ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
-    marks = torch.empty(n * H * (3 if gates is None else 195), dtype=torch.float64, device=dev)
-    _check(core().tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, _ptr(gates), float(cap), _ptr(decay),
-                                   _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale), float(k_scale),
-                                   _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n,
-                                   requests, _ptr(ends), _ptr(marks), _ptr(out), H, d, dv, float(den_eps), _stream()), "linear_chunks",
-           launches=3 + bool(rot) + (gates is not None))
+    marks = torch.empty(n * H * (2 * doubles + tiles), dtype=torch.int32, device=dev)        # doubles, then marks of operands
+    marked = _ptr(marks) + 8 * n * H * doubles
+    heads = (_ptr(gates), float(cap), _ptr(decay), _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale),
+             float(k_scale))
+    _check(lib.tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, *heads, _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start),
+                                _ptr(ctx.slots), step.rows, n, step.firsts, step.requests, _ptr(ends), _ptr(marks), marked, _ptr(out), H, d, dv,
+                                float(den_eps), _stream()), "linear_chunks", launches=3 + bool(rot) + (gates is not None))
+    _check(lib.tl_linear_scan(_ptr(proj), dtype_code(proj.dtype), proj.shape[1], q_off, k_off, v_off, *heads, _ptr(state), per_slot,
+                              _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(out), step.requests, H, d, dv, float(den_eps), 0, None, None, step.runs,
+                              marked, tiles, _stream()), "linear_scan")
 
 
 def channel_chunks(h_q_start, chunk: int) -> tuple:
@@ -1162,7 +1173,7 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt_b
         raise KernelError(f"delta_scan: a slot holds {state[0].numel()} floats, these sizes need {per_slot}")
     _check(core().tl_delta_scan(_ptr(qkv), C, 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias),
                                 _ptr(state), per_slot, _ptr(q_start), _ptr(slots), _ptr(out), int(B), H, nqk, d, dv,
-                                int(T if max_q_len is None else max_q_len), int(compensated), _stream()),
+                                int(T if max_q_len is None else max_q_len), int(compensated), None, None, 0, _stream()),
            "delta_scan")
 
 
@@ -1201,11 +1212,15 @@ def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt
     per_chunk = core().tl_delta_chunk_bytes(H, nqk, d, dv)
     if not per_chunk or qkv.shape[1] & 3 or qkv.data_ptr() & 15:
         raise KernelError("delta_chunks: q/k heads of 36 to 128, sizes in multiples of 4, 16-byte rows")
-    both, n, requests = _chunk_list(ctx, "delta_chunks", core().tl_delta_chunk(), qkv.device)
-    scratch = torch.empty(n * per_chunk, dtype=torch.uint8, device=qkv.device)
-    _check(core().tl_delta_chunks(_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias),
-                                  _ptr(state), per_slot, _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(both), n, _ptr(both) + 16 * n, requests,
-                                  _ptr(scratch), _ptr(out), H, nqk, d, dv, _stream()), "delta_chunks", launches=2)
+    lib = core()
+    step = _chunk_list(ctx, "delta_chunks", lib.tl_delta_chunk(), qkv.device)
+    scratch = torch.empty(step.n * (per_chunk + 4 * H), dtype=torch.uint8, device=qkv.device)      # the chunks' operands, then their marks
+    marked = _ptr(scratch) + step.n * per_chunk
+    args = (_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(state), per_slot,
+            _ptr(ctx.q_start), _ptr(ctx.slots))
+    _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.requests, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv, _stream()),
+           "delta_chunks", launches=2)
+    _check(lib.tl_delta_scan(*args, _ptr(out), step.requests, H, nqk, d, dv, 1, 0, step.runs, marked, 1, _stream()), "delta_scan")
 
 
 def latent_prep(down: torch.Tensor, qr: int, rank: int, dr: int, wq: torch.Tensor, wkv: torch.Tensor, eps: float,

@@ -116,6 +116,50 @@ def test_decays_of_zero_forget_as_token_by_token():
         assert bool(b.isfinite().all()) and float((a - b).norm()) <= 4e-6 * float(b.norm())      # 2e-6 for either kernel, as above
 
 
+@pytest.mark.parametrize("what,value", [("v", float("nan")), ("v", float("inf")), ("k", float("nan")), ("k", -float("inf")), ("v", 1e30), ("q", float("nan")),
+                                        ("beta", float("nan")), ("decay", float("nan"))])
+@pytest.mark.parametrize("d,dv", [(64, 68), (128, 128)])
+def test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, value, d, dv):
+    """One element of one token (number 37 of 200) of one of two requests: tokens before it, other heads and the other request are as
+    they are without it; with one in the keys, the values or the gates the heads that read it have the token-by-token kernel's floats."""
+    from tensorline_b200 import ops
+    H, nqk, T, lens = 4, 2, 380, [180, 200]
+    g = torch.Generator().manual_seed(d + dv)
+    clean = torch.randn(T, 2 * nqk * d + H * dv, generator=g) * d ** -0.5
+    gates = torch.randn(T, 2 * H, generator=g)
+    odd, odd_gates = clean.clone(), gates.clone()
+    at = lens[0] + 37
+    if what in ("beta", "decay"):
+        odd_gates[at, 2 + (H if what == "decay" else 0)] = value
+    else:
+        odd[at, {"q": d, "k": nqk * d + d, "v": 2 * nqk * d + 2 * dv}[what] + 3] = value
+    hit = [2, 3] if what in "qk" else [2]                # heads 2 and 3 share the second q/k head
+    others = [h for h in range(H) if h not in hit]
+    floats = H * -(-dv // ops.delta_columns()) * ops.delta_state_floats(d)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    start = torch.tensor([0, lens[0], T], **i32)
+    ctx = SimpleNamespace(h_q_start=start.tolist(), scratch={}, q_start=start, slots=torch.arange(2, **i32))
+    consts = (torch.randn(H, generator=g).cuda() - 2.0, torch.randn(H, generator=g).cuda() - 1.0)
+
+    def run(x, gt, chunks):
+        state, out = torch.zeros(2, floats, device="cuda"), torch.empty(T, H * dv, device="cuda")
+        if chunks:
+            ops.delta_chunks(x.cuda(), gt.cuda(), *consts, state, ctx, out, H=H, nqk=nqk, d=d, dv=dv)
+        else:
+            ops.delta_scan(x.cuda(), gt.cuda(), *consts, state, ctx.q_start, ctx.slots, out, B=2, H=H, nqk=nqk, d=d, dv=dv, max_q_len=200)
+        return out.view(T, H, dv), state.view(2, H, -1)
+    (out, state), (want, want_state), (fine, fine_state) = run(odd, odd_gates, True), run(odd, odd_gates, False), run(clean, gates, True)
+    assert torch.equal(out[:lens[0]], fine[:lens[0]]) and torch.equal(state[0], fine_state[0])
+    assert torch.equal(out[:, others], fine[:, others]) and torch.equal(state[1, others], fine_state[1, others])
+    if what == "q":
+        assert torch.equal(out[lens[0]:at], fine[lens[0]:at]) and torch.equal(out[at + 1:], fine[at + 1:]) and torch.equal(state, fine_state)
+        assert bool(out[at, hit].isnan().all())
+    else:
+        assert bool(want[:at].isfinite().all())
+        torch.testing.assert_close(out[lens[0]:, hit], want[lens[0]:, hit], rtol=0, atol=0, equal_nan=True)
+        torch.testing.assert_close(state[1, hit], want_state[1, hit], rtol=0, atol=0, equal_nan=True)
+
+
 def test_heads_that_run_token_by_token_are_refused():
     from tensorline_b200 import ops
     for d, dv in ((32, 64), (132, 64), (64, 30), (62, 64), (64, 1028)):

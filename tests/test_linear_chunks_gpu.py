@@ -176,3 +176,48 @@ def test_retention_with_decays_that_have_no_logarithm(decay):
         if min(decay) <= 0.0:
             assert torch.equal(a, b)
         assert bool(b.isfinite().all()) and float((a - b).norm()) <= 4e-6 * float(b.norm())
+
+
+@pytest.mark.parametrize("what,value", [("v", float("nan")), ("v", float("inf")), ("k", float("nan")), ("k", -float("inf")), ("k", 1e30), ("q", float("nan")),
+                                        ("i", float("nan")), ("f", float("nan"))])
+@pytest.mark.parametrize("gated,d,dv", [(True, 64, 64), (False, 128, 132), (True, 256, 64), (False, 20, 20)])
+def test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, value, gated, d, dv):
+    """One element of one token (number 37 of 200) of head 1 of one of two requests: tokens before it, other heads and the other request
+    are as they are without it; with one in the keys, the values or the gates the head has the token-by-token kernel's floats."""
+    from tensorline_b200 import ops
+    if what in "if" and not gated:
+        return
+    H, T, lens = 3, 380, [180, 200]
+    g = torch.Generator().manual_seed(d + dv)
+    clean = torch.randn(T, 2 * H * d + H * dv, generator=g)
+    gates = torch.randn(T, 2 * H, generator=g) + 1.0
+    odd, odd_gates = clean.clone(), gates.clone()
+    at, h = lens[0] + 37, 1
+    if what == "i" or what == "f":
+        odd_gates[at, h + (H if what == "f" else 0)] = value
+    else:
+        odd[at, {"q": 0, "k": H * d, "v": 2 * H * d}[what] + h * (dv if what == "v" else d) + 3] = value
+    kw = dict(q_scale=d ** -0.5, den_eps=1e-6, cap=15.0) if gated else dict(decay=torch.tensor([0.9, 0.97, 0.99]).cuda(), k_scale=d ** -0.5)
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, gated)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    start = torch.tensor([0, lens[0], T], **i32)
+    ctx = SimpleNamespace(h_q_start=start.tolist(), scratch={}, pos=torch.arange(T, **i32), q_start=start, slots=torch.arange(2, **i32))
+
+    def run(x, gt, chunks):
+        state, out, extra = torch.zeros(2, floats, device="cuda"), torch.empty(T, H * dv, device="cuda"), dict(gates=gt.cuda()) if gated else {}
+        if chunks:
+            ops.linear_chunks(x.cuda(), 0, H * d, 2 * H * d, H, d, dv, state, ctx, out, **kw, **extra)
+        else:
+            ops.linear_scan(x.cuda(), 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, out, B=2, **kw, **extra)
+        return out.view(T, H, dv), state.view(2, H, -1)
+    (out, state), (want, want_state), (fine, fine_state) = run(odd, odd_gates, True), run(odd, odd_gates, False), run(clean, gates, True)
+    others = [0, 2]
+    assert torch.equal(out[:lens[0]], fine[:lens[0]]) and torch.equal(state[0], fine_state[0])
+    assert torch.equal(out[:, others], fine[:, others]) and torch.equal(state[1, others], fine_state[1, others])
+    if what == "q":
+        assert torch.equal(out[lens[0]:at], fine[lens[0]:at]) and torch.equal(out[at + 1:], fine[at + 1:]) and torch.equal(state, fine_state)
+        assert bool(out[at, h].isnan().all())
+    else:
+        assert bool(want[:at].isfinite().all()) and torch.equal(out[:at, h][lens[0]:], want[:at, h][lens[0]:])
+        torch.testing.assert_close(out[lens[0]:, h], want[lens[0]:, h], rtol=0, atol=0, equal_nan=True)
+        torch.testing.assert_close(state[1, h], want_state[1, h], rtol=0, atol=0, equal_nan=True)
