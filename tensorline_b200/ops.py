@@ -805,31 +805,50 @@ def linear_scan(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, 
 LINEAR_CHUNKS_MIN_TOKENS = {True: 128, False: 192}       # by whether the decays are gated
 
 
+# In such a step the requests of this many tokens and more run as chunks, the others (decoding ones above all, whose result so does not
+# depend on a portion beside them) token by token.  Chunks / token by token for the short requests, same sizes, beside 600 tokens: 8
+# requests of 16 gated 141 us / 169, fixed decay 128 / 125, 1 request of 16 97 / 101; 4 requests of 8 125 / 133 and 112 / 105.
+LINEAR_CHUNKS_LEAST_TOKENS = 16
+
+
 def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gated: bool) -> bool:
     """Whether `linear_chunks` takes these sizes (q, k, v one behind the other in a projection's row) and is the faster way."""
     return proj.dtype == torch.float32 and max_q_len >= LINEAR_CHUNKS_MIN_TOKENS[gated] and d % 4 == 0 and dv % 4 == 0 and d <= 256 and \
         proj.shape[1] % 4 == 0 and proj.data_ptr() % 16 == 0
 
 
-def _chunk_list(ctx, key: str, chunk: int, device) -> SimpleNamespace:
-    """The step's chunks of `chunk` tokens on the device: `rows` (`channel_chunks`' rows, `n` of them), `runs` (request, first chunk,
-    chunks, 0) of the `requests` requests, and `firsts`, their first rows.  One description a step, for every layer."""
+def chunk_runs(h_q_start, chunk: int, least: int) -> tuple:
+    """A step's requests of `least` tokens and more in chunks of `chunk` tokens: (int32 rows [n, 4] (request, number, the request's chunks,
+    its first row), int32 runs [requests, 4] (request, first row, chunks or 0, 0) of all requests with a token, int32 first
+    rows, the longest of the requests without chunks), numpy."""
+    lens = np.diff(np.asarray(h_q_start, dtype=np.int64))
+    chunks = np.where(lens >= least, -(-lens // chunk), 0)
+    firsts = np.cumsum(chunks) - chunks
+    request = np.repeat(np.arange(len(lens)), chunks)
+    rows = np.stack([request, np.arange(len(request)) - firsts[request], chunks[request], firsts[request]], axis=1).astype(np.int32)
+    some = np.nonzero(lens)[0]
+    runs = np.stack([some, firsts[some] * (chunks[some] > 0), chunks[some], 0 * some], axis=1).astype(np.int32)
+    return rows, runs, firsts[chunks > 0].astype(np.int32), int(lens[chunks == 0].max(initial=0))
+
+
+def _chunk_list(ctx, key: str, chunk: int, least: int, device) -> SimpleNamespace:
+    """`chunk_runs` on the device (`rows`, `n` of them; `runs`, `requests` of them; `firsts`, `long` of them) and the `longest` of the
+    requests that go token by token.  One description a step, for every layer."""
+    key = (key, least)
     if key not in ctx.scratch:
-        rows, _ = channel_chunks(ctx.h_q_start, chunk)
-        firsts = np.nonzero(rows[:, 1] == 0)[0].astype(np.int32)
-        runs = np.stack([rows[firsts, 0], firsts, rows[firsts, 2], np.zeros_like(firsts)], axis=1)
+        rows, runs, firsts, longest = chunk_runs(ctx.h_q_start, chunk, least)
         words = torch.from_numpy(np.concatenate([rows.reshape(-1), runs.reshape(-1), firsts])).to(device, non_blocking=True)
         at = _ptr(words)
-        ctx.scratch[key] = SimpleNamespace(words=words, rows=at, n=len(rows), runs=at + 16 * len(rows), requests=len(firsts),
-                                           firsts=at + 16 * (len(rows) + len(firsts)))
+        ctx.scratch[key] = SimpleNamespace(words=words, rows=at, n=len(rows), runs=at + 16 * len(rows), requests=len(runs),
+                                           firsts=at + 16 * (len(rows) + len(runs)), long=len(firsts), longest=longest)
     return ctx.scratch[key]
 
 
 def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int, d: int, dv: int, state: torch.Tensor, ctx, out: torch.Tensor,
                   *, decay: torch.Tensor | None = None, gates: torch.Tensor | None = None, cap: float = 1.0, inv_freq: torch.Tensor | None = None,
-                  rot: int = 0, pairing: str = "half", q_scale: float = 1.0, k_scale: float = 1.0, den_eps: float = 0.0) -> None:
-    """`linear_scan` with one decay a head (`decay` or `gates`) for steps of several tokens a request: chunks of a request's tokens
-    side by side, as matrix products of floats.  proj float32 with 16-byte rows; the state as `linear_scan` keeps it, so the two may
+                  rot: int = 0, pairing: str = "half", q_scale: float = 1.0, k_scale: float = 1.0, den_eps: float = 0.0, least: int = 1) -> None:
+    """`linear_scan` with one decay a head (`decay` or `gates`) for steps that hold long portions: requests of `least` tokens and more
+    run as chunks of their tokens side by side, as matrix products of floats, the others token by token.  proj float32 with 16-byte rows; the state as `linear_scan` keeps it, so the two may
     take turns.  A position's sums depend on where its step began, to rounding.  A head of a request whose keys, values or gates hold
     something that is no number, infinite or above 2^40 goes token by token: what such a value reaches is what it reaches there."""
     T = proj.shape[0]
@@ -854,7 +873,7 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
         raise KernelError("linear_chunks: inv_freq must be float32 [rot/2]")
     interleaved = _pairing(pairing, "linear_chunks")
     lib, dev = core(), proj.device
-    step = _chunk_list(ctx, "linear_chunks", lib.tl_linear_chunk(), dev)
+    step = _chunk_list(ctx, "linear_chunks", lib.tl_linear_chunk(), least, dev)
     n, tiles, doubles = step.n, lib.tl_linear_chunk_tiles(d, dv), 3 if gates is None else 195
     turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
     ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
@@ -863,7 +882,7 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
     heads = (_ptr(gates), float(cap), _ptr(decay), _ptr(inv_freq) if rot else None, int(rot), int(interleaved), _ptr(ctx.pos), float(q_scale),
              float(k_scale))
     _check(lib.tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, *heads, _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start),
-                                _ptr(ctx.slots), step.rows, n, step.firsts, step.requests, _ptr(ends), _ptr(marks), marked, _ptr(out), H, d, dv,
+                                _ptr(ctx.slots), step.rows, n, step.firsts, step.long, _ptr(ends), _ptr(marks), marked, _ptr(out), H, d, dv,
                                 float(den_eps), _stream()), "linear_chunks", launches=3 + bool(rot) + (gates is not None))
     _check(lib.tl_linear_scan(_ptr(proj), dtype_code(proj.dtype), proj.shape[1], q_off, k_off, v_off, *heads, _ptr(state), per_slot,
                               _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(out), step.requests, H, d, dv, float(den_eps), 0, None, None, step.runs,
@@ -1184,6 +1203,9 @@ def delta_scan(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt_b
 # 256: 64 tokens 24 us token by token against 34, the host's two launches and their scratch; 128 tokens 43 against 33; 2,048 tokens
 # 632 against 171).
 DELTA_CHUNKS_MIN_TOKENS = 96
+# As LINEAR_CHUNKS_LEAST_TOKENS: beside 600 tokens 8 requests of 16 179 us in chunks / 150 token by token, of 32 182 / 184, of 60 207 / 235
+# (a chunk costs the walk of a head and 16 columns 2 us on an SM of its own, however few its tokens).
+DELTA_CHUNKS_LEAST_TOKENS = 32
 
 
 def takes_delta_chunks(qkv: torch.Tensor, H: int, nqk: int, d: int, dv: int, max_q_len: int) -> bool:
@@ -1193,10 +1215,11 @@ def takes_delta_chunks(qkv: torch.Tensor, H: int, nqk: int, d: int, dv: int, max
 
 
 def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, ctx,
-                 out: torch.Tensor, *, H: int, nqk: int, d: int, dv: int) -> None:
-    """`delta_scan` (not compensated) for steps of several tokens a request: chunks of 32 tokens, inside a chunk matrix products of
-    floats (on the tensor cores as products of their bfloat16 parts).  The state as `delta_scan` keeps it, so the two may take turns.  A position's sums depend on where its step began, to
-    rounding."""
+                 out: torch.Tensor, *, H: int, nqk: int, d: int, dv: int, least: int = 1) -> None:
+    """`delta_scan` (not compensated) for steps that hold long portions: requests of `least` tokens and more run as chunks of 32 tokens,
+    inside a chunk matrix products of floats (on the tensor cores as products of their bfloat16 parts), the others token by
+    token.  The state as `delta_scan` keeps it, so the two may take turns.  A position's sums depend on where its step began, to
+    rounding.  Odd values: as in `linear_chunks`."""
     T = qkv.shape[0]
     _contig(qkv, "qkv"); _contig(out, "out"); _contig(state, "state")
     if qkv.dtype != torch.float32 or qkv.shape[1] != 2 * nqk * d + H * dv or out.dtype != torch.float32 or out.shape != (T, H * dv):
@@ -1213,14 +1236,14 @@ def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt
     if not per_chunk or qkv.shape[1] & 3 or qkv.data_ptr() & 15:
         raise KernelError("delta_chunks: q/k heads of 36 to 128, sizes in multiples of 4, 16-byte rows")
     lib = core()
-    step = _chunk_list(ctx, "delta_chunks", lib.tl_delta_chunk(), qkv.device)
+    step = _chunk_list(ctx, "delta_chunks", lib.tl_delta_chunk(), least, qkv.device)
     scratch = torch.empty(step.n * (per_chunk + 4 * H), dtype=torch.uint8, device=qkv.device)      # the chunks' operands, then their marks
     marked = _ptr(scratch) + step.n * per_chunk
     args = (_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(state), per_slot,
             _ptr(ctx.q_start), _ptr(ctx.slots))
-    _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.requests, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv, _stream()),
+    _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.long, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv, _stream()),
            "delta_chunks", launches=2)
-    _check(lib.tl_delta_scan(*args, _ptr(out), step.requests, H, nqk, d, dv, 1, 0, step.runs, marked, 1, _stream()), "delta_scan")
+    _check(lib.tl_delta_scan(*args, _ptr(out), step.requests, H, nqk, d, dv, step.longest, 0, step.runs, marked, 1, _stream()), "delta_scan")
 
 
 def latent_prep(down: torch.Tensor, qr: int, rank: int, dr: int, wq: torch.Tensor, wkv: torch.Tensor, eps: float,

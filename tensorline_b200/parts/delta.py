@@ -10,8 +10,8 @@
 Between steps a request keeps, in its state slots, S (float32, in the scan kernel's own layout) and the convolution's
 last `taps - 1` inputs (float32); both start at zero.  Everything that enters the recurrence beside the projections is
 float32 in both engines; the stacked projection's float32 accumulators are kept as they are.  The mixer reads the step from
-device tensors only (single-token steps sit in CUDA graphs).  In the bfloat16 engine portions of a prompt run as chunks of tokens
-(`ops.delta_chunks`), to rounding the same.
+device tensors only (single-token steps sit in CUDA graphs).  In the bfloat16 engine long portions of a prompt run as chunks of
+tokens (`ops.delta_chunks`), to rounding the same; decoding requests beside them do not.
 """
 from __future__ import annotations
 
@@ -92,7 +92,8 @@ class GatedDelta(Part):
                       nv=H, dv=dv, unit_eps=self.unit_eps, q_scale=d ** -0.5)
         o = torch.empty((T, H * dv), dtype=torch.float32, device=h.device)
         if not self.compensated and not ctx.decode_only and ops.takes_delta_chunks(qkv, H, nqk, d, dv, ctx.max_q_len):
-            ops.delta_chunks(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx, o, H=H, nqk=nqk, d=d, dv=dv)
+            ops.delta_chunks(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx, o, H=H, nqk=nqk, d=d, dv=dv,
+                             least=ops.DELTA_CHUNKS_LEAST_TOKENS)
         else:
             ops.delta_scan(qkv, gates, self.A_log, self.dt_bias, cache["memory"].state, ctx.q_start, ctx.slots, o, B=ctx.B, H=H,
                            nqk=nqk, d=d, dv=dv, max_q_len=ctx.max_q_len, compensated=self.compensated)

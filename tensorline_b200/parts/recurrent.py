@@ -3,7 +3,7 @@
     S_t = a_t S_(t-1) + b_t k_t v_t^T,    o_t = S_t^T q_t          S: [d, dv] per head, float32
 
 Three kinds, one pipeline (one stacked projection, one scan kernel, one kernel for the per-head norm and the
-gate, the output projection; in the bfloat16 engine portions of a prompt run as chunks of tokens side by side instead of the scan):
+gate, the output projection; in the bfloat16 engine long portions of a prompt run as chunks of tokens side by side instead of the scan):
 
 * `retention`: a_t is a fixed decay per head, b_t = 1; q and k are rotated by position and k is scaled by
   d^-1/2 after the rotation; every head's o is divided by its root mean square (no weight), multiplied by
@@ -127,7 +127,7 @@ class Retention(_MatrixState):
             rotary = Rotary(*rotary)
         if self.positive and self._in_chunks(h, proj, ctx):
             ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, o, decay=self.decay, inv_freq=rotary.inv_freq,
-                              rot=rotary.rot, pairing=rotary.pairing, k_scale=d ** -0.5)
+                              rot=rotary.rot, pairing=rotary.pairing, k_scale=d ** -0.5, least=ops.LINEAR_CHUNKS_LEAST_TOKENS)
             return
         ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, o, B=ctx.B,
                         decay=self.decay, inv_freq=rotary.inv_freq, rot=rotary.rot, pairing=rotary.pairing,
@@ -172,7 +172,7 @@ class MLSTM(_MatrixState):
         ops.small_proj(h, self.w_gates, self.b_gates, gates)
         if self._in_chunks(h, proj, ctx):
             ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, o, gates=gates, cap=self.cap, q_scale=d ** -0.5,
-                              den_eps=self.den_eps)
+                              den_eps=self.den_eps, least=ops.LINEAR_CHUNKS_LEAST_TOKENS)
             return
         ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, o, B=ctx.B,
                         gates=gates, cap=self.cap, q_scale=d ** -0.5, den_eps=self.den_eps, single_tokens=ctx.decode_only)

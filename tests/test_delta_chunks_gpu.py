@@ -160,6 +160,32 @@ def test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, 
         torch.testing.assert_close(state[1, hit], want_state[1, hit], rtol=0, atol=0, equal_nan=True)
 
 
+def test_short_requests_beside_a_portion_have_the_token_by_token_kernels_floats():
+    """Decoding requests and short portions in a step that holds long ones: outputs and states as the scan kernel gives them, whatever
+    runs beside them; and the long ones' do not depend on the short ones."""
+    from tensorline_b200 import ops
+    H, nqk, d, dv, lens, least = 4, 2, 64, 68, [1, 1, 130, 32, 31, 0, 1, 300, 7], 32
+    T, B = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(d)
+    args = [torch.randn(*s, generator=g).cuda() * x for s, x in (((T, 2 * nqk * d + H * dv), d ** -0.5), ((T, 2 * H), 1.0), ((H,), 1.0), ((H,), 1.0))]
+    first = torch.randn(B, H * -(-dv // ops.delta_columns()) * ops.delta_state_floats(d), generator=g).cuda()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    ctx = SimpleNamespace(h_q_start=start.tolist(), scratch={}, q_start=start, slots=torch.arange(B, **i32).flip(0).contiguous())
+    got = []
+    for n in (least, 1, None):
+        state, out = first.clone(), torch.full((T, H * dv), 7.0, device="cuda")
+        if n is None:
+            ops.delta_scan(*args, state, start, ctx.slots, out, B=B, H=H, nqk=nqk, d=d, dv=dv, max_q_len=300)
+        else:
+            ops.delta_chunks(*args, state, ctx, out, H=H, nqk=nqk, d=d, dv=dv, least=n)
+        got.append((out, state))
+    for b, n in enumerate(lens):
+        rows, slot = slice(int(start[b]), int(start[b + 1])), int(ctx.slots[b])
+        want, want_state = got[1 if n >= least else 2]
+        assert torch.equal(got[0][0][rows], want[rows]) and torch.equal(got[0][1][slot], want_state[slot]), n
+
+
 def test_heads_that_run_token_by_token_are_refused():
     from tensorline_b200 import ops
     for d, dv in ((32, 64), (132, 64), (64, 30), (62, 64), (64, 1028)):

@@ -221,3 +221,32 @@ def test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, 
         assert bool(want[:at].isfinite().all()) and torch.equal(out[:at, h][lens[0]:], want[:at, h][lens[0]:])
         torch.testing.assert_close(out[lens[0]:, h], want[lens[0]:, h], rtol=0, atol=0, equal_nan=True)
         torch.testing.assert_close(state[1, h], want_state[1, h], rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("gated,d,dv", [(True, 64, 64), (False, 128, 256), (False, 32, 20)])
+def test_short_requests_beside_a_portion_have_the_token_by_token_kernels_floats(gated, d, dv):
+    """Decoding requests and short portions in a step that holds long ones: outputs and states as the scan kernel gives them, whatever
+    runs beside them; and the long ones' do not depend on the short ones."""
+    from tensorline_b200 import ops
+    H, lens, least = 2, [1, 1, 130, 16, 15, 0, 1, 300, 7], 16
+    T, B = sum(lens), len(lens)
+    g = torch.Generator().manual_seed(d)
+    proj, gates = torch.randn(T, 2 * H * d + H * dv, generator=g).cuda(), torch.randn(T, 2 * H, generator=g).cuda() + 1.0
+    kw = dict(gates=gates, q_scale=d ** -0.5, den_eps=1e-6, cap=15.0) if gated else dict(decay=torch.tensor([0.9, 0.99]).cuda(), k_scale=d ** -0.5)
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, gated)
+    first = torch.randn(B, floats, generator=g).cuda()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    start = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    ctx = SimpleNamespace(h_q_start=start.tolist(), scratch={}, pos=torch.arange(T, **i32), q_start=start, slots=torch.arange(B, **i32).flip(0).contiguous())
+    got = []
+    for n in (least, 1, None):
+        state, out = first.clone(), torch.full((T, H * dv), 7.0, device="cuda")
+        if n is None:
+            ops.linear_scan(proj, 0, H * d, 2 * H * d, H, d, dv, state, start, ctx.slots, ctx.pos, out, B=B, **kw)
+        else:
+            ops.linear_chunks(proj, 0, H * d, 2 * H * d, H, d, dv, state, ctx, out, least=n, **kw)
+        got.append((out, state))
+    for b, n in enumerate(lens):
+        rows, slot = slice(int(start[b]), int(start[b + 1])), int(ctx.slots[b])
+        want, want_state = got[1 if n >= least else 2]
+        assert torch.equal(got[0][0][rows], want[rows]) and torch.equal(got[0][1][slot], want_state[slot]), n
