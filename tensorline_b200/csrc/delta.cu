@@ -149,7 +149,13 @@ __global__ void __launch_bounds__(256) conv_prep_tile_kernel(const TA* __restric
 // through: a channel and token cost it one load and no index arithmetic.  What is left is the accurate exponential and division
 // of silu, about 35 instructions an output (134 with rows and weights in shared memory): 2,048 tokens, 3,072 channels 25 us against
 // 47.  The arithmetic of an output is conv_prep_kernel's, operation for operation, so all give the same bits.
+// A run is a chain of 16 tokens, 14 us however little there is; so it takes steps of CONV_RUN_WORK outputs (with the update of the
+// inputs, tile kernel / runs: 1,024 tokens of 3,072 channels 22.5 / 20.5 us, 2,048 of 1,280 20.3 / 20.0, 2,048 of 2,048 26.3 / 23.1; 512 of
+// 4,096 16.4 / 18.6, 512 of 3,072 14.7 / 16.4, 1,024 of 2,048 19.8 / 21.8, 2,048 of 512 11.4 / 16.2), and of CONV_RUN_SOME where most
+// blocks of the tile kernel's grid would find nothing (48 single tokens beside 464 of 3,072 channels 32.5 / 27.0 us, beside
+// 200 25.2 / 23.0; of 1,280 channels, 200 tokens 15.0 / 18.3).
 constexpr int CONV_RUN = 16;
+constexpr long long CONV_RUN_WORK = 2500000, CONV_RUN_SOME = 600000, CONV_RUN_GRID = 5000;
 template <typename TA, typename TW, int TAPS>
 __global__ void __launch_bounds__(128) conv_prep_run_kernel(const TA* __restrict__ proj, int stride, const TW* __restrict__ taps_w,
                                                             const float* __restrict__ conv_state, long long slot_stride,
@@ -229,7 +235,7 @@ __global__ void conv_keep_kernel(const TA* __restrict__ proj, int stride, int ta
 }
 
 TL_EXPORT int tl_conv_prep(const void* proj, int act_dtype, int stride, const void* taps_w, int w_dtype, int taps, float* conv_state,
-                           long long slot_stride, const int* q_start, const int* slots, float* out, int B, int max_q_len,
+                           long long slot_stride, const int* q_start, const int* slots, float* out, int T, int B, int max_q_len,
                            int nqk, int d, int nv, int dv, float unit_eps, float q_scale, cudaStream_t stream) {
     if (B <= 0 || max_q_len <= 0) return 0;
     if (taps < 1 || (taps > 1 && !conv_state)) return 1;
@@ -238,7 +244,9 @@ TL_EXPORT int tl_conv_prep(const void* proj, int act_dtype, int stride, const vo
     const int widest = d > dv ? d : dv;
     int tt = (int)(40 * 1024 / sizeof(float)) / widest - (taps - 1);
     tt = tt > 32 ? 32 : tt;
-    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && taps >= 2 && taps <= 4) {
+    const long long work = (long long)T * C, tiles = tt > 0 ? (long long)B * ((max_q_len + tt - 1) / tt) * (2 * nqk + nv) : 0;
+    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && taps >= 2 && taps <= 4 &&
+        (work >= CONV_RUN_WORK || (work >= CONV_RUN_SOME && tiles >= CONV_RUN_GRID))) {
         const dim3 grid(B, (max_q_len + CONV_RUN - 1) / CONV_RUN, (2 * nqk + nv + 3) / 4);
         if (grid.y > 65535 || grid.z > 65535) return 1;
 #define CR_N(TA, TW, N) launch_after_wait(conv_prep_run_kernel<TA, TW, N>, grid, dim3(128), 0, stream, (const TA*)proj, stride, (const TW*)taps_w, \

@@ -61,7 +61,7 @@ _SIGNATURES = {
     "tl_relu_square": [_P, _I, ctypes.c_longlong, _P],
     "tl_gelu": [_P, _I, ctypes.c_longlong, _P],
     "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
-    "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P],
+    "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
     "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
     "tl_delta_chunk": [],
@@ -1162,7 +1162,7 @@ def conv_prep(proj: torch.Tensor, taps_w: torch.Tensor, conv_state: torch.Tensor
             raise KernelError("conv_prep: conv_state must be float32 [slots, (taps - 1) * C]")
         slot_stride = conv_state[0].numel()
     _check(core().tl_conv_prep(_ptr(proj), dtype_code(proj.dtype), proj.stride(0), _ptr(taps_w), dtype_code(taps_w.dtype), taps,
-                               _ptr(conv_state) if taps > 1 else None, slot_stride, _ptr(q_start), _ptr(slots), _ptr(out), int(B),
+                               _ptr(conv_state) if taps > 1 else None, slot_stride, _ptr(q_start), _ptr(slots), _ptr(out), T, int(B),
                                int(max_q_len), nqk, d, nv, dv, float(unit_eps), float(q_scale), _stream()), "conv_prep",
            launches=2 if taps > 1 else 1)
 
