@@ -19,7 +19,7 @@ def test_pairs_are_sorted_by_expert_in_their_own_order(T, E, top):
     assert torch.equal(offsets.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.long), torch.bincount(flat, minlength=E).cumsum(0)]))
 
 
-@pytest.mark.parametrize("N", [8, 136, 2048, 2056, 30])
+@pytest.mark.parametrize("N", [8, 136, 256, 504, 512, 520, 1000, 2048, 2056, 30])
 @pytest.mark.parametrize("top,weighted,shared", [(1, False, False), (3, True, True), (4, True, False), (5, False, True), (8, True, True)])
 def test_a_tokens_rows_are_summed_in_the_order_chosen(N, top, weighted, shared):
     from tensorline_b200 import ops
