@@ -539,7 +539,8 @@ __global__ void __launch_bounds__(128) moe_up_rows_kernel(const TA* __restrict__
     }
 }
 
-// 8 tokens, 4 of 32 experts, 2,048 x 1,024: 24 us (27).
+// 8 tokens, 4 of 32 experts, 2,048 x 1,024: 24 us (27).  With float activations a lane's two loads of the vector take half of every line
+// twice, which short rows do not hide: F 512, 2 of 8 experts, 32 tokens 44 us (37), F 768, 4 of 16, 32 (32), F 256, 8 of 64, 58 (60).
 template <typename TA>
 __global__ void __launch_bounds__(128) moe_down_rows_kernel(const TA* __restrict__ a, const bf16* __restrict__ w_down, const int* __restrict__ idx,
                                                             const float* __restrict__ wts, TA* __restrict__ y, int F, int N, int top,
@@ -608,7 +609,7 @@ TL_EXPORT int tl_moe_down(const void* a, int act_dtype, const void* w_down, int 
     if (smem > 48 * 1024) return 1;
     const dim3 grid(T, (N + MOE_DOWN_ROWS - 1) / MOE_DOWN_ROWS);
     if (grid.y > 65535) return 1;
-    if (w_dtype != TL_F32 && F % 8 == 0 && top <= 32 && ((((uintptr_t)a) | ((uintptr_t)w_down)) & 15) == 0) {
+    if (w_dtype != TL_F32 && F % 8 == 0 && top <= 32 && (act_dtype != TL_F32 || F <= 256 || F >= 768) && ((((uintptr_t)a) | ((uintptr_t)w_down)) & 15) == 0) {
 #define MDR(TA) return launch_after_wait(moe_down_rows_kernel<TA>, grid, dim3(128), 0, stream, (const TA*)a, (const bf16*)w_down, idx, wts, (TA*)y, F, N, top, (const TA*)extra, extra_gate, ldg, n_real, (const TA*)same)
         if (act_dtype == TL_F32) MDR(float);
         MDR(bf16);

@@ -45,7 +45,7 @@ def test_a_tokens_rows_are_summed_in_the_order_chosen(N, top, weighted, shared):
 
 @pytest.mark.parametrize("adt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,top,K,F,gated", [(1, 1, 8, 3, True), (3, 2, 264, 17, True), (5, 4, 2048, 40, False), (8, 4, 1032, 1, False), (2, 8, 520, 10, True),
-                                             (2, 2, 45, 6, True)])
+                                             (2, 2, 45, 6, True), (3, 2, 64, 256, True), (4, 3, 64, 264, True), (4, 2, 72, 768, False)])
 def test_streamed_experts_against_float64_and_token_by_token(T, top, K, F, gated, adt):
     """K products of unit normals with weights of 0.05 in float32, rounded to the activation type (2^-8 for bfloat16)."""
     from tensorline_b200 import ops
