@@ -103,8 +103,6 @@ __global__ void __launch_bounds__(128) small_proj_kernel(const TA* __restrict__ 
     }
 }
 
-// The same for bfloat16 weights in 16-byte rows, every output the chain of warp_dot: a lane's multiply-adds over its groups of eight
-// k, then the warp's sum.
 // eight values of an activation row as floats
 __device__ __forceinline__ void row8(const bf16* p, float (&x)[8]) {
     const uint4 v = *reinterpret_cast<const uint4*>(p);
@@ -117,6 +115,8 @@ __device__ __forceinline__ void row8(const float* p, float (&x)[8]) {
     *reinterpret_cast<float4*>(x + 4) = *reinterpret_cast<const float4*>(p + 4);
 }
 
+// The same for bfloat16 weights in 16-byte rows, every output the chain of warp_dot: a lane's multiply-adds over its groups of eight
+// k, then the warp's sum.
 // Few tokens: a warp an output, nothing in shared memory.  What bounds it is latency: the loads of 2,048 k, the weights' and the
 // row's, go out together (one token, 16 outputs, K 2,048: 4.3 us from a cold cache, through shared memory 13.7).
 constexpr int SP_FLIGHT = 8;             // 16-byte loads of a lane in flight
@@ -220,12 +220,14 @@ __global__ void __launch_bounds__(128) small_proj_tile_kernel(const TA* __restri
     }
 }
 
-// Up to this many tokens an output has a warp of its own.
-constexpr int SP_FEW = 32;
+// Up to this many tokens, and this many outputs in all (float, bfloat16 activations), an output has a warp of its own (256 outputs, K 7,168,
+// float: 16 tokens 13 us against 14 in tiles, 32 tokens 24 against 14; a block a token, 16 outputs at a time, 19 and 21; bfloat16, 32
+// tokens: 160 outputs, K 6,144 10.7 against 13.1, 256, K 7,168 17.3 against 15.1).
+constexpr int SP_FEW = 32, SP_FEW_OUTPUTS = 4096, SP_FEW_OUTPUTS_BF16 = 6144;
 
 template <typename TA>
 static int launch_small_proj_bf16(const TA* h, int ldh, const bf16* w, const bf16* bias, float* out, int ldo, int T, int N, int K, cudaStream_t stream) {
-    if (T <= SP_FEW) return launch_after_wait(small_proj_few_kernel<TA>, dim3(T, (N + 3) / 4), dim3(128), 0, stream, h, ldh, w, bias, out, ldo, N, K);
+    if (T <= SP_FEW && T * N <= (sizeof(TA) == 4 ? SP_FEW_OUTPUTS : SP_FEW_OUTPUTS_BF16)) return launch_after_wait(small_proj_few_kernel<TA>, dim3(T, (N + 3) / 4), dim3(128), 0, stream, h, ldh, w, bias, out, ldo, N, K);
     const int smem = SP_TOKENS * K * (int)sizeof(float);
     static bool raised[TL_MAX_DEVICES] = {};
     const int dev = tl_device_index();

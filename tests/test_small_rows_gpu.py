@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("adt", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("T,N,K", [(1, 1, 8), (1, 16, 2048), (32, 33, 2056), (33, 5, 264), (70, 40, 4096), (513, 17, 72), (3, 7, 45), (2100, 33, 512)])
+@pytest.mark.parametrize("T,N,K", [(1, 1, 8), (1, 16, 2048), (32, 33, 2056), (33, 5, 264), (70, 40, 4096), (513, 17, 72), (3, 7, 45), (2100, 33, 512),
+                                   (16, 256, 520), (17, 256, 520), (24, 256, 264), (25, 257, 264)])
 def test_small_products_at_every_length_of_a_step(T, N, K, adt):
     from tensorline_b200 import ops
     g = torch.Generator().manual_seed(T + N + K)
