@@ -26,7 +26,8 @@ def test_small_products_at_every_length_of_a_step(T, N, K, adt):
 
 @pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16, None])
-@pytest.mark.parametrize("T,H,dv,act", [(1, 1, 4, "silu"), (5, 3, 256, "sigmoid"), (2, 5, 132, "silu"), (3, 2, 512, None), (4, 2, 30, "silu"), (2, 2, 520, "sigmoid")])
+@pytest.mark.parametrize("T,H,dv,act", [(1, 1, 4, "silu"), (5, 3, 256, "sigmoid"), (2, 5, 132, "silu"), (3, 2, 512, None), (4, 2, 30, "silu"), (2, 2, 520, "sigmoid"),
+                                        (3, 5, 60, "silu"), (3, 5, 64, "sigmoid")])
 def test_head_norms_against_float64(T, H, dv, act, wdt, gdt):
     from tensorline_b200 import ops
     g = torch.Generator().manual_seed(T * dv + H)
