@@ -422,18 +422,13 @@ TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float
     if (nq % nkv || (chunk > 0 && window > 0) || chunk < 0 || d < 4 || d % 4 || d > 256 ||
         ((((uintptr_t)k_pages) | ((uintptr_t)v_pages) | ((uintptr_t)out)) & 15)) return 1;
     const int g = nq / nkv;
-    static bool raised[TL_MAX_DEVICES] = {};
-    const int dev = tl_device_index();
-    if (dev < 0) return 1;
-    if (!raised[dev]) {
-        const int most = ((ROWS_MAX + 64) * (256 + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
-        cudaError_t e = cudaFuncSetAttribute(attn_rows_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_rows_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_rows_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHAIN_SMEM);
-        if (e != cudaSuccess) return (int)e;
-        raised[dev] = true;
-    }
+    static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {}, r4[TL_MAX_DEVICES] = {}, rc[TL_MAX_DEVICES] = {};
+    constexpr int most = ((ROWS_MAX + 64) * (256 + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
+    int e = tl_raise_smem(attn_rows_kernel<1>, r1, most);
+    if (!e) e = tl_raise_smem(attn_rows_kernel<2>, r2, most);
+    if (!e) e = tl_raise_smem(attn_rows_kernel<4>, r4, most);
+    if (!e) e = tl_raise_smem(attn_chain_kernel, rc, CHAIN_SMEM);
+    if (e) return e;
     RowsArgs A{q, q_stride, out, k_pages, v_pages, table, max_pages, page_size, pos, req_slot, T, nq, nkv, d, window, scale,
                sink, window > 0 ? keep_first : 0, gate, chunk, slopes, cap, scores, keys, 0, TlLimits{table_rows, total_pages, fault}};
     if (scores) {
@@ -441,8 +436,7 @@ TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float
         const size_t smem = (size_t)g * d * sizeof(float);
         if (smem > 48 * 1024 || nkv > 65535 || T > 65535 || nkv * groups > 65535) return 1;
         attn_dots_kernel<<<dim3((keys + DOTS_KEYS - 1) / DOTS_KEYS, nkv, T), DOTS_KEYS, smem, stream>>>(A);
-        const int e = tl_launch_status();
-        if (e) return e;
+        if ((e = tl_launch_status())) return e;
         attn_chain_kernel<<<dim3((d + 31) / 32, nkv * groups, T), 32 * (g < DOTS_HEADS ? g : DOTS_HEADS), CHAIN_SMEM, stream>>>(A);
         return tl_launch_status();
     }

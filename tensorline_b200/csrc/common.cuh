@@ -122,6 +122,19 @@ static inline int tl_device_index() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= TL_MAX_DEVICES) return -1;
     return dev;
 }
+// More dynamic shared memory than a kernel has by default, once per device: `bytes`, the most any call of the kernel needs (two host
+// threads may both come here first, so the size must not depend on the call).  `raised`: the caller's, one per kernel.
+template <typename F>
+static inline int tl_raise_smem(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
+    const int dev = tl_device_index();
+    if (dev < 0) return 1;
+    if (!raised[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return (int)e;
+        raised[dev] = true;
+    }
+    return 0;
+}
 // Streaming multiprocessors of the current device, asked once per device.
 static inline int tl_num_sms() {
     static int count[TL_MAX_DEVICES] = {};

@@ -381,19 +381,16 @@ __global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
     }
 }
 
+constexpr int DC_DV_MAX = 1024;          // V of a chunk lies in shared memory beside K and Q
+
 template <int DP>
 static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int* marked, int n_chunks, int requests, cudaStream_t stream) {
     using Sh = WalkShape<DP>;
-    const int prep_smem = (2 * DC_C * (DP + 4) + DC_C * A.dv) * 4;
-    static int raised[TL_MAX_DEVICES] = {};              // what prepare's shared memory was raised to
-    const int dev = tl_device_index();
-    if (dev < 0) return 1;
-    if (raised[dev] < prep_smem) {
-        cudaError_t e = cudaFuncSetAttribute(dc_prepare_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(dc_walk_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::BYTES);
-        if (e != cudaSuccess) return (int)e;
-        raised[dev] = prep_smem;
-    }
+    constexpr int row_bytes = 2 * DC_C * (DP + 4) * 4;
+    static bool prepare[TL_MAX_DEVICES] = {}, walk[TL_MAX_DEVICES] = {};
+    int e = tl_raise_smem(dc_prepare_kernel<DP>, prepare, row_bytes + DC_C * DC_DV_MAX * 4);
+    if (!e) e = tl_raise_smem(dc_walk_kernel<DP>, walk, Sh::BYTES);
+    if (e) return e;
     const size_t ch = (size_t)n_chunks * A.H;
     A.W = scratch;
     A.P = A.W + ch * Sh::PARTS;
@@ -401,14 +398,11 @@ static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int* marked, int 
     A.U = A.M + ch * DC_MB;
     A.K = A.U + ch * A.nz * DC_UB;
     A.marked = marked;
-    dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), DC_PREP, prep_smem, stream>>>(A);
-    const int e = tl_launch_status();
-    if (e) return e;
+    dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), DC_PREP, row_bytes + DC_C * A.dv * 4, stream>>>(A);
+    if ((e = tl_launch_status())) return e;
     dc_walk_kernel<DP><<<dim3(requests, A.H, A.nz), 128, Sh::BYTES, stream>>>(A);
     return tl_launch_status();
 }
-
-constexpr int DC_DV_MAX = 1024;          // V of a chunk lies in shared memory beside K and Q
 
 TL_EXPORT int tl_delta_chunk() { return DC_C; }
 // Bytes of scratch a chunk; 0: these sizes run token by token (heads of up to 32, whose state has another layout, and wide ones,

@@ -293,24 +293,12 @@ gemm_f32_kernel(const float* __restrict__ A, int lda, const TW* __restrict__ W, 
     }
 }
 
-template <typename F>
-static int raise_smem(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
-    const int dev = tl_device_index();
-    if (dev < 0) return 1;
-    if (!raised[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return (int)e;
-        raised[dev] = true;
-    }
-    return 0;
-}
-
 template <typename TW, int MT, int ROW, int S>
 static int launch_few(const float* A, int lda, const TW* W, int ldw, const TW* bias, float* C, int ldc, int M, int N, int K,
                       cudaStream_t stream) {
     constexpr int BK = ROW / (int)sizeof(TW), MOST = S * (GF_FEW_N * (ROW + 16) + 8 * MT * BK * 4);      // at most 8 warps
     static bool raised[TL_MAX_DEVICES] = {};
-    const int e = raise_smem(gemm_f32_few_kernel<TW, MT, ROW, S>, raised, MOST);
+    const int e = tl_raise_smem(gemm_f32_few_kernel<TW, MT, ROW, S>, raised, MOST);
     if (e) return e;
     const int m = M < GF_FEW_MAX ? M : GF_FEW_MAX, warps = m > MT ? (m + MT - 1) / MT : 2;      // one warp alone would fetch too slowly
     const int smem = S * (GF_FEW_N * (ROW + 16) + warps * MT * BK * 4);
@@ -325,7 +313,7 @@ static int launch_tile(const float* A, int lda, const TW* W, int ldw, const TW* 
     using Sh = TileShape<TW, TM, TN>;
     constexpr int SMEM = Sh::STAGES * Sh::STAGE;
     static bool raised[TL_MAX_DEVICES] = {};
-    const int e = raise_smem(gemm_f32_tile_kernel<TW, TM, TN>, raised, SMEM);
+    const int e = tl_raise_smem(gemm_f32_tile_kernel<TW, TM, TN>, raised, SMEM);
     if (e) return e;
     const dim3 grid((M + Sh::BM - 1) / Sh::BM, (N + Sh::BN - 1) / Sh::BN);
     if (grid.y > 65535) return 1;

@@ -641,25 +641,13 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) lc_out_kernel(const Li
         }
 }
 
-template <typename F>
-static int lc_raise(F kernel, bool (&raised)[TL_MAX_DEVICES], int bytes) {
-    const int dev = tl_device_index();
-    if (dev < 0) return 1;
-    if (!raised[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e != cudaSuccess) return (int)e;
-        raised[dev] = true;
-    }
-    return 0;
-}
-
 template <int DP, int CB, bool GATED>
 static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
     constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
     constexpr int local_smem = LocalShape<RB, CB>::BYTES, out_smem = OutShape<DP, CB>::BYTES;
     static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
-    int e = lc_raise(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
-    if (!e) e = lc_raise(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
+    int e = tl_raise_smem(lc_local_kernel<RB, CB, GATED>, r1, local_smem);
+    if (!e) e = tl_raise_smem(lc_out_kernel<DP, CB, GATED>, r2, out_smem);
     if (e) return e;
     const int col_tiles = (A.dv + CB - 1) / CB, row_tiles = (A.d + RB - 1) / RB;
     if (GATED) {

@@ -230,13 +230,8 @@ static int launch_small_proj_bf16(const TA* h, int ldh, const bf16* w, const bf1
     if (T <= SP_FEW && T * N <= (sizeof(TA) == 4 ? SP_FEW_OUTPUTS : SP_FEW_OUTPUTS_BF16)) return launch_after_wait(small_proj_few_kernel<TA>, dim3(T, (N + 3) / 4), dim3(128), 0, stream, h, ldh, w, bias, out, ldo, N, K);
     const int smem = SP_TOKENS * K * (int)sizeof(float);
     static bool raised[TL_MAX_DEVICES] = {};
-    const int dev = tl_device_index();
-    if (dev < 0) return 1;
-    if (!raised[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(small_proj_tile_kernel<TA>, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_TOKENS * 48 * 1024);
-        if (e != cudaSuccess) return (int)e;
-        raised[dev] = true;
-    }
+    const int e = tl_raise_smem(small_proj_tile_kernel<TA>, raised, SP_TOKENS * 48 * 1024);
+    if (e) return e;
     const int tiles = (T + SP_TOKENS - 1) / SP_TOKENS;
     // outputs are dealt out to several blocks where the tokens alone leave SMs idle
     int split = 2 * tl_num_sms() / tiles;

@@ -386,15 +386,11 @@ static int launch_scan_shape(const ScanArgs& A, int B, bool single, cudaStream_t
         return launch_after_wait(linear_step_kernel<TA, R, IS, KIND>, dim3(B, A.H, nz), dim3(Sh::NT), 0, stream, A);
     }
     const size_t smem = (size_t)(2 * SCAN_C * Sh::TS + SCAN_C * SCAN_JS + 4 * SCAN_C + A.rot / 2) * sizeof(float);
-    if (smem > 48 * 1024) {                              // the widest heads: more dynamic shared memory than a kernel has by default
+    constexpr size_t most = (size_t)(2 * SCAN_C * Sh::TS + SCAN_C * SCAN_JS + 4 * SCAN_C + R * IS / 2) * sizeof(float);      // rot <= d <= R IS
+    if constexpr (most > 48 * 1024) {                    // the widest heads
         static bool raised[TL_MAX_DEVICES] = {};
-        const int dev = tl_device_index();
-        if (dev < 0) return 1;
-        if (!raised[dev]) {
-            const cudaError_t e = cudaFuncSetAttribute(linear_scan_kernel<TA, R, IS, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            raised[dev] = true;
-        }
+        const int e = tl_raise_smem(linear_scan_kernel<TA, R, IS, KIND>, raised, (int)most);
+        if (e) return e;
     }
     return launch_after_wait(linear_scan_kernel<TA, R, IS, KIND>, dim3(B, A.H, nz), dim3(Sh::NT), smem, stream, A);
 }
