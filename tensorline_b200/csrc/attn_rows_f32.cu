@@ -51,6 +51,12 @@ __device__ __forceinline__ const float* rows_at(const RowsArgs& A, const float* 
     const int page = tl_checked(tab[tl_checked(j / A.page_size, A.max_pages, A.L, TL_K_TOKENWISE)], A.L.total_pages, A.L, TL_K_TOKENWISE);
     return pages + (((size_t)page * A.nkv + kh) * A.page_size + (j % A.page_size)) * A.d;
 }
+// The position of a token whose scores lie in `scores`: one beyond the table is recorded by the checking build, and cut in every build, so
+// that nothing outside the scratch is touched.
+__device__ __forceinline__ int rows_position(const RowsArgs& A, int t) {
+    const int p = A.pos[t];
+    return p < 0 ? p : min(tl_checked(p, A.keys, A.L, TL_K_TOKENWISE), A.keys - 1);
+}
 __device__ __forceinline__ float rows_score(const RowsArgs& A, float dot, float slope, int p, int j) {
     float s = __fmul_rn(dot, A.scale);                   // spelt out: the same roundings in every kernel
     if (A.cap > 0.f) s = __fmul_rn(A.cap, tanhf(s / A.cap));
@@ -272,7 +278,7 @@ constexpr int DOTS_KEYS = 128, DOTS_HEADS = 8;
 __global__ void __launch_bounds__(DOTS_KEYS) attn_dots_kernel(const RowsArgs A) {
     extern __shared__ __align__(16) float qs[];          // [heads of the group][d]
     const int t = blockIdx.z, kh = blockIdx.y, g = A.nq / A.nkv, d = A.d;
-    const int p = min(A.pos[t], A.keys - 1), lo = rows_low(A, p), kept = min(A.keep_first, lo);
+    const int p = rows_position(A, t), lo = rows_low(A, p), kept = min(A.keep_first, lo);
     const int c0 = blockIdx.x * DOTS_KEYS;
     if (c0 > p || (c0 >= kept && c0 + DOTS_KEYS <= lo)) return;
     for (int i = threadIdx.x; i < g * d; i += DOTS_KEYS) qs[i] = A.q[(size_t)t * A.q_stride + (size_t)kh * g * d + i];
@@ -317,7 +323,7 @@ __global__ void __launch_bounds__(32 * DOTS_HEADS) attn_chain_kernel(const RowsA
     const int t = blockIdx.z, g = A.nq / A.nkv, d = A.d, groups = (g + DOTS_HEADS - 1) / DOTS_HEADS;
     const int kh = blockIdx.y / groups, h0 = (blockIdx.y % groups) * DOTS_HEADS;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, wid = tid >> 5;
-    const int p = min(A.pos[t], A.keys - 1), lo = rows_low(A, p), kept = min(A.keep_first, lo);
+    const int p = rows_position(A, t), lo = rows_low(A, p), kept = min(A.keep_first, lo);
     const int e0 = blockIdx.x * 32, e = e0 + lane;
     const bool live = h0 + wid < g;
     const int head = kh * g + min(h0 + wid, g - 1);
@@ -413,7 +419,7 @@ __global__ void __launch_bounds__(32 * DOTS_HEADS) attn_chain_kernel(const RowsA
 }
 
 // `scores` (float [T, nq, keys], keys >= every position of the step + 1, or null): scratch of the two kernels of few tokens.
-// Returns 1 where these kernels do not take the shape (the caller then runs the token-wise kernel).
+// Returns 1 for shapes that these kernels do not take; the caller gives those to the token-wise kernel beforehand.
 TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int* table,
                            int max_pages, int page_size, const int* pos, const int* req_slot, int T, int nq, int nkv, int d, int window,
                            float scale, const float* sink, int keep_first, const float* gate, int chunk, const float* slopes, float cap,

@@ -89,5 +89,39 @@ def main() -> int:
     return 0
 
 
+def float_cases() -> int:
+    """The float32 attention kernels: steps of few tokens (dot products, then chains), and of more than 64 (rows that share their keys)."""
+    from tensorline_b200 import ops
+    from tensorline_b200.csrc.build import CHECK_BUILD
+    from tensorline_b200.ops import KernelError
+    assert CHECK_BUILD and ops.core().tl_check_build() == 1, "not the checking build"
+    dev = torch.device("cuda")
+    POOL, REAL, ps, nq, nkv, d = 6, 16, 8, 4, 2, 64
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=dev)
+    real_k, real_v = torch.full((REAL, nkv, ps, d), 3.0, device=dev), torch.full((REAL, nkv, ps, d), -3.0, device=dev)
+    k, v = real_k[:POOL + 1], real_v[:POOL + 1]
+    good, bad_page = i32([[0, 1, 2, 3], [4, 5, POOL, POOL]]), i32([[0, 9, 2, 3], [4, 5, POOL, POOL]])
+    for T in (3, 70):
+        q, out = torch.randn(T, nq * d, device=dev), torch.zeros(T, nq * d, device=dev)
+        pos, slot = [20, 21] + [3] * (T - 2), [0, 0] + [1] * (T - 2)
+
+        def run(table, pos, slot):
+            ops.attn_tokenwise(q, nq * d, out, k, v, table, ps, i32(pos), i32(slot), nq, nkv, d, None, 0.125)
+            ops.check_device_status()
+        run(good, pos, slot)                                 # a clean call reports nothing
+        for what, args in (("page number beyond the pool", (bad_page, pos, slot)), ("slot beyond the table", (good, pos, [5] * T)),
+                           ("position beyond the table's width", (good, [40] + pos[1:], slot))):
+            try:
+                run(*args)
+            except KernelError as e:
+                assert "bounds check" in str(e) and "exact-order" in str(e), str(e)
+                print(f"caught: {what}, {T} tokens: {e}")
+                continue
+            raise AssertionError(f"{what}, {T} tokens: the checking build reported nothing")
+    assert bool((real_k == 3.0).all()) and bool((real_v == -3.0).all())
+    print("ok")
+    return 0
+
+
 if __name__ == "__main__":
-    sys.exit(main())
+    sys.exit(float_cases() if sys.argv[1:] == ["float32"] else main())

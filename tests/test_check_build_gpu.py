@@ -26,6 +26,13 @@ def test_checker_catches_entries_outside_its_bounds_and_redirects_them():
     assert lines[-1] == "ok" and sum(l.startswith("caught:") for l in lines) == 10, proc.stdout
 
 
+def test_checker_catches_entries_outside_its_bounds_in_the_float32_attention():
+    proc = run(["tests/check_build_cases.py", "float32"])
+    assert proc.returncode == 0, proc.stdout[-3000:] + proc.stderr[-3000:]
+    lines = proc.stdout.splitlines()
+    assert lines[-1] == "ok" and sum(l.startswith("caught:") for l in lines) == 6, proc.stdout
+
+
 def test_replay_schedules_and_kernel_tests_report_nothing_under_the_checking_build():
     proc = run(["-m", "pytest", "-x", "-q", "-m", "gpu", "-p", "no:cacheprovider",
                 "tests/test_replay_gpu.py", "tests/test_kernels_gpu.py", "tests/test_parts_gpu.py"])
