@@ -68,7 +68,8 @@ def recurrence(x, gates, decay, H, d, dv, S, n, m, pos, inv_freq, rot, interleav
 @pytest.mark.parametrize("H,d,dv,lens,rot,interleaved", [
     (3, 128, 256, [64, 65, 1], 64, False), (2, 64, 64, [200], 64, True), (1, 32, 128, [127, 63, 128], 0, False), (2, 256, 128, [130], 256, False),
     (2, 20, 36, [70, 3], 8, True), (1, 96, 20, [300, 64], 96, False), (2, 200, 132, [100], 0, False), (1, 4, 4, [193], 0, False),
-    (2, 52, 132, [77, 128], 0, False), (3, 20, 20, [70], 12, False), (3, 20, 20, [70], 6, True), (3, 20, 20, [70], 12, True)])
+    (2, 52, 132, [77, 128], 0, False), (3, 20, 20, [70], 12, False), (3, 20, 20, [70], 6, True), (3, 20, 20, [70], 12, True),
+    (2, 20, 20, [5, 4161], 8, False)])                   # more chunks than the carry holds factors of at a time
 def test_chunks_against_the_recurrence_in_float64_and_the_scan_kernel(gated, H, d, dv, lens, rot, interleaved):
     from tensorline_b200 import ops
     g = torch.Generator().manual_seed(d * dv + sum(lens))
