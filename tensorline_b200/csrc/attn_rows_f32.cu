@@ -15,8 +15,8 @@
 //                   128 keys at a time and then their chain.
 // Measured with 28 query heads of 128 on 4 KV heads: 333 tokens on 700 cached 350 us (the token-wise kernel 5,076), 2,048 tokens
 // 1.32 ms (33.4); single tokens at position 1,800: 4 of them 56 us (1,842; attn_rows 478), 64 of them 265 us (3,577; 611).
-// Masks, sinks, gates, caps and slopes: as described in attn_tokenwise.cu.  A sink's term joins the sum with a rounding of its own,
-// the same in both kernels here.
+// Masks, sinks, gates, caps and slopes: as described in attn_tokenwise.cu.  The roundings are spelt out here
+// and there: which kernel a row is given to does not show in its floats.
 #include "common.cuh"
 
 struct RowsArgs {
@@ -63,13 +63,6 @@ __device__ __forceinline__ float rows_score(const RowsArgs& A, float dot, float 
     if (A.slopes) s = fmaf(-slope, (float)(p - j), s);
     return s;
 }
-// The sink joins a finished row: (its sum with the sink, what the row's values are multiplied by).  One copy for both kernels.
-__device__ __noinline__ float2 rows_sink(float m, float l, float sink) {
-    const float m_new = fmaxf(m, sink);
-    const float alpha = expf(m - m_new);
-    return make_float2(l * alpha + expf(sink - m_new), alpha);
-}
-
 constexpr int ROWS_MAX = 64, ROWS_PS = ROWS_MAX + 4;     // rows a block, and the stride of a key's scores in shared memory
 
 // NC: groups of 64 output columns (d <= 64 NC)
@@ -246,7 +239,7 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
     {
         float alpha = 1.0f;
         if (A.sink && live) {
-            const float2 r = rows_sink(m, l, A.sink[head]);
+            const float2 r = tl_attn_sink(m, l, A.sink[head]);
             l = r.x; alpha = r.y;
         }
         float inv = 1.0f / l;
@@ -409,7 +402,7 @@ __global__ void __launch_bounds__(32 * DOTS_HEADS) attn_chain_kernel(const RowsA
     }
     ROWS_WAIT(0);
     if (A.sink) {
-        const float2 r = rows_sink(m, l, A.sink[head]);
+        const float2 r = tl_attn_sink(m, l, A.sink[head]);
         l = r.x;
         acc *= r.y;
     }

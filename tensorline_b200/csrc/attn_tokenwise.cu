@@ -60,14 +60,14 @@ __global__ void attn_tokenwise_kernel(const TA* __restrict__ q, int q_stride, TA
             const TA* kr = k_pages + row;
             float dot = 0.f;
             for (int e = 0; e < d; ++e) dot = fmaf(qs[e], to_f<TA>(kr[e]), dot);
-            s = dot * scale;
-            if (cap > 0.f) s = cap * tanhf(s / cap);
-            if (slopes) s -= slope * (float)(p - j);
+            s = __fmul_rn(dot, scale);                  // spelt out, as everywhere below: the roundings of attn_rows_f32.cu
+            if (cap > 0.f) s = __fmul_rn(cap, tanhf(s / cap));
+            if (slopes) s = fmaf(-slope, (float)(p - j), s);
         }
         const float m_new = fmaxf(m, warp_max(s));
         const float alpha = expf(m - m_new);            // 0 on the first tile (m = -inf)
         const float pj = valid ? expf(s - m_new) : 0.f;
-        l = l * alpha + warp_sum(pj);
+        l = fmaf(l, alpha, warp_sum(pj));
 #pragma unroll
         for (int c = 0; c < MAXC; ++c) acc[c] *= alpha;
         const int n_here = min(32, p - j0 + 1);
@@ -86,11 +86,10 @@ __global__ void attn_tokenwise_kernel(const TA* __restrict__ q, int q_stride, TA
         m = m_new;
     }
     if (sink) {                                          // one more term of the denominator: no key, no value
-        const float m_new = fmaxf(m, sink[h]);
-        const float alpha = expf(m - m_new);
-        l = l * alpha + expf(sink[h] - m_new);
+        const float2 r = tl_attn_sink(m, l, sink[h]);
+        l = r.x;
 #pragma unroll
-        for (int c = 0; c < MAXC; ++c) acc[c] *= alpha;
+        for (int c = 0; c < MAXC; ++c) acc[c] *= r.y;
     }
     TA* orow = out + ((size_t)t * nq + h) * d;
     float inv = 1.0f / l;

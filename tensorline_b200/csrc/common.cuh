@@ -178,6 +178,14 @@ __device__ __forceinline__ int tl_checked(int v, int limit, const TlLimits& L, i
 }
 TL_EXPORT int tl_check_build();
 
+// Exact-order attention's sink joins a finished row: (its sum with the sink, what the row's values are multiplied by).  The roundings are
+// spelt out, so that every kernel that may be given the row has the same floats.
+__device__ __forceinline__ float2 tl_attn_sink(float m, float l, float sink) {
+    const float m_new = fmaxf(m, sink);
+    const float alpha = expf(m - m_new);
+    return make_float2(__fadd_rn(__fmul_rn(l, alpha), expf(sink - m_new)), alpha);
+}
+
 // A step's requests as the scan kernels take them beside kernels that work chunks of a request's tokens (linear_chunk.cu, delta_chunk.cu):
 // a run is (request, its first chunk, its chunks).  Those kernels leave a mark per chunk, head and tile of operands that hold a
 // value whose products they cannot take as the recurrence does (not a number, an infinity, above TL_CHUNK_LARGE); a marked

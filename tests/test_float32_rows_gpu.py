@@ -40,7 +40,7 @@ def test_a_row_of_the_product_has_the_same_floats_in_every_step(ops, M, N, K, wd
 @pytest.mark.parametrize("d,g,ps", [(64, 1, 4), (128, 7, 16), (20, 4, 3), (96, 9, 8), (256, 2, 16), (160, 16, 16), (18, 2, 4)])
 @pytest.mark.parametrize("option", ["plain", "window", "sink", "chunk"])
 def test_attention_rows_have_the_same_floats_in_every_step(ops, d, g, ps, option):
-    """Portions and single tokens in one step of more than 64 tokens, the same tokens in short steps, and float64."""
+    """Portions and single tokens in one step of more than 64 tokens, the same tokens in short steps, the token-wise kernel, and float64."""
     nkv, scale = 2, d ** -0.5
     nq = nkv * g
     reqs = [(1, 130), (33, 31), (1, 0), (40, 64), (2, 300)]
@@ -72,6 +72,13 @@ def test_attention_rows_have_the_same_floats_in_every_step(ops, d, g, ps, option
     whole = run(0, T)
     cuts = [0, 1, 30, 61, T]
     assert torch.equal(whole, torch.cat([run(a, b) for a, b in zip(cuts, cuts[1:])]))
+    qd, kd, vd, td, pd, sd = dev
+    tokenwise = torch.empty_like(whole)
+    ops._check(ops.core().tl_attn_tokenwise(
+        ops._ptr(qd), nq * d, ops._ptr(tokenwise), ops.dtype_code(qd.dtype), ops._ptr(kd), ops._ptr(vd), ops._ptr(td), mp, ps, ops._ptr(pd), ops._ptr(sd),
+        T, nq, nkv, d, window or 0, scale, ops._ptr(kw.get("sink")), kw.get("keep_first", 0), ops._ptr(kw.get("gate")), kw.get("chunk", 0),
+        ops._ptr(kw.get("slopes")), kw.get("cap", 0.0), td.shape[0], kd.shape[0], ops.fault_words(qd.device), ops._stream()), "attn_tokenwise")
+    assert torch.equal(whole, tokenwise)
     for t in (0, 1, 33, 34, 74, T - 1):
         p, tab = int(pos[t]), table[int(slot[t])]
         j = torch.arange(p + 1)
