@@ -615,19 +615,27 @@ def rope_kv_write(qkv: torch.Tensor, bias: torch.Tensor | None, pos: torch.Tenso
 # 700 cached tokens: 64 tokens 124 us against 222, 128 tokens 242 against 239).
 FEW_ROWS_MAX_TOKENS = 64
 FEW_ROWS_MAX_SCORES = 1 << 24
+# Up to this many positions (the caller knows the step's largest; by whether a KV head has several query heads) the token-wise kernel is done
+# first, one launch: 28 heads on 4, 50 tokens up to position 9 18.6 us against 22.2, 2 tokens at position 5 13.3 against 15.4, 16 tokens at
+# position 10 18.6 against 16.5; 8 heads of 64 on 8, 64 tokens at position 14 14.8 against 20.6, 100 at position 20 20.6 against 24.8.
+SHORT_ROWS_MAX_CTX = {True: 10, False: 24}
+# More than FEW_ROWS_MAX_TOKENS single tokens from this many positions on (28 heads on 4, 65 of them: position 60 24.7 us against 32.9, 1,800
+# 278 against 610; 100 at position 20 28.8 against 24.7).
+MANY_SINGLES_MIN_CTX = 48
 
 
 def attn_tokenwise(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                    table: torch.Tensor, page_size: int, pos: torch.Tensor, req_slot: torch.Tensor,
                    nq: int, nkv: int, d: int, window: int | None, scale: float, sink: torch.Tensor | None = None,
                    keep_first: int = 0, gate: torch.Tensor | None = None, chunk: int | None = None,
-                   slopes: torch.Tensor | None = None, cap: float | None = None) -> None:
+                   slopes: torch.Tensor | None = None, cap: float | None = None, max_ctx: int = 0, singles: bool = False) -> None:
     """Exact-order paged attention; q rows `q_stride` elements apart, out [T, nq*d].  `sink` (float32 [nq]): one more
     term exp(sink[h]) in every softmax denominator of head h.  `keep_first` (with a window): the keys at positions below
     it stay visible beside the window.  `gate` (float32 [T, nq]): the row of (t, h) is multiplied by sigmoid(gate[t, h]).
     `chunk` (instead of a window): a query reads the keys of its own chunk of that many positions, counted from position 0.
     `slopes` (float32 [nq]): the score of key j seen from position p loses slopes[h] * (p - j).  `cap`: a score is
-    cap * tanh(score / cap) before a slope comes off it."""
+    cap * tanh(score / cap) before a slope comes off it.  `max_ctx`: no position of the step is as large (0: as the table is wide);
+    `singles`: every token is a request's only one.  Which kernel they choose does not show in the floats."""
     T = out.shape[0]
     if out.shape[1] != nq * d or out.dtype != q.dtype or k_pages.dtype != q.dtype:
         raise KernelError("attn_tokenwise: out must be [T, nq*d] and all tensors of one type")
@@ -643,10 +651,11 @@ def attn_tokenwise(q: torch.Tensor, q_stride: int, out: torch.Tensor, k_pages: t
     if chunk and window:
         raise KernelError("attn_tokenwise: a window or chunks, not both")
     _sink(slopes, nq, "attn_tokenwise (slopes)")
-    if q.dtype == torch.float32 and T and d % 4 == 0 and d <= 256 and nq // nkv <= 64 and nq // nkv * d <= 12288 and \
+    max_ctx = max_ctx or table.shape[1] * page_size
+    if q.dtype == torch.float32 and T and max_ctx > SHORT_ROWS_MAX_CTX[nq > nkv] and d % 4 == 0 and d <= 256 and nq // nkv <= 64 and nq // nkv * d <= 12288 and \
             not (out.data_ptr() | k_pages.data_ptr() | v_pages.data_ptr()) & 15:
-        keys = table.shape[1] * page_size
-        few = T <= FEW_ROWS_MAX_TOKENS and T * nq * keys <= FEW_ROWS_MAX_SCORES
+        keys = min(table.shape[1] * page_size, -(-max_ctx // 128) * 128)
+        few = (T <= FEW_ROWS_MAX_TOKENS or (singles and max_ctx >= MANY_SINGLES_MIN_CTX)) and T * nq * keys <= FEW_ROWS_MAX_SCORES
         scores = torch.empty(T * nq * keys, dtype=torch.float32, device=out.device) if few else None
         _check(core().tl_attn_rows(_ptr(q), q_stride, _ptr(out), _ptr(k_pages), _ptr(v_pages), _ptr(table), table.shape[1], page_size,
                                    _ptr(pos), _ptr(req_slot), T, nq, nkv, d, int(window or 0), float(scale), _ptr(sink), int(keep_first),

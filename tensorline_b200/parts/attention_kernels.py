@@ -34,7 +34,7 @@ def attend(mixer, qkv, o, ctx, cache, table, rope=None, gate=None) -> None:
             ((chunk or slopes is not None) and not ops_attention.TAKES_CHUNKS):   # heads wider than the tensor-core kernels take
         ops.attn_tokenwise(qkv, qkv.shape[1], o, cache.k, cache.v, table, ctx.page_size, ctx.pos, ctx.req_slot,
                            nq, nkv, d, mixer.window, mixer.scale, sink=sink, keep_first=keep_first, gate=gate, chunk=chunk,
-                           slopes=slopes, cap=cap)
+                           slopes=slopes, cap=cap, max_ctx=ctx.graph_max_ctx or ctx.max_ctx, singles=ctx.decode_only)
         return
     ops_attention.attend_bf16(qkv, o, ctx, cache.k, cache.v, table, nq, nkv, d, mixer.window, mixer.scale, rope=rope, sink=sink,
                               keep_first=keep_first, chunk=chunk, slopes=slopes, cap=cap)

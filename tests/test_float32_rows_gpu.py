@@ -62,16 +62,19 @@ def test_attention_rows_have_the_same_floats_in_every_step(ops, d, g, ps, option
         kw["chunk"], kw["slopes"] = 50, torch.rand(nq, generator=gen).cuda()
     dev = [t.cuda() for t in (q, k, v, table, pos, slot)]
 
-    def run(lo, hi):
+    def run(lo, hi, **hints):
         out = torch.full((hi - lo, nq * d), 7.0, device="cuda")
         part = {n: (x[lo:hi].contiguous() if n == "gate" else x) for n, x in kw.items()}
         qd, kd, vd, td, pd, sd = dev
         ops.attn_tokenwise(qd[lo:hi].contiguous(), nq * d, out, kd, vd, td, ps, pd[lo:hi].contiguous(), sd[lo:hi].contiguous(), nq, nkv, d,
-                           window, scale, **part)
+                           window, scale, **part, **hints)
         return out
     whole = run(0, T)
     cuts = [0, 1, 30, 61, T]
     assert torch.equal(whole, torch.cat([run(a, b) for a, b in zip(cuts, cuts[1:])]))
+    for hints in (dict(max_ctx=int(pos.max()) + 1), dict(singles=True), dict(max_ctx=int(pos.max()) + 1, singles=True)):
+        assert torch.equal(whole, run(0, T, **hints))
+    assert torch.equal(whole[34:35], run(34, 35, max_ctx=1))      # position 0
     qd, kd, vd, td, pd, sd = dev
     tokenwise = torch.empty_like(whole)
     ops._check(ops.core().tl_attn_tokenwise(
@@ -101,3 +104,24 @@ def test_attention_rows_have_the_same_floats_in_every_step(ops, d, g, ps, option
                 w = torch.softmax(s, 0)
             want = w @ vv[:, h // g]
             assert float((whole[t, h * d:(h + 1) * d].double().cpu() - want).abs().max()) <= 2e-5
+
+
+@pytest.mark.parametrize("window", [None, 700])
+def test_dot_products_of_tables_longer_than_a_grid(ops, window):
+    """Few tokens whose table holds more groups of keys than blocks fill the GPU: the same floats as with the table cut to the contexts,
+    and as the token-wise kernel."""
+    nq, nkv, d, ps, mp = 2, 2, 64, 16, 330
+    gen = torch.Generator().manual_seed(1)
+    table = torch.randperm(2 * mp, generator=gen).to(torch.int32).view(2, mp).contiguous().cuda()
+    k, v = (torch.randn(2 * mp + 1, nkv, ps, d, generator=gen).cuda() for _ in range(2))
+    pos = torch.cat([torch.arange(5000, 5060), torch.arange(3, 7)]).to(torch.int32).cuda()
+    slot = torch.tensor([0] * 60 + [1] * 4, dtype=torch.int32).cuda()
+    q, outs = torch.randn(64, nq * d, generator=gen).cuda(), []
+    for hints in ({}, dict(max_ctx=5060), dict(max_ctx=5060, singles=True)):
+        outs.append(torch.full((64, nq * d), 7.0, device="cuda"))
+        ops.attn_tokenwise(q, nq * d, outs[-1], k, v, table, ps, pos, slot, nq, nkv, d, window, 0.125, **hints)
+    outs.append(torch.empty_like(q))
+    ops._check(ops.core().tl_attn_tokenwise(
+        ops._ptr(q), nq * d, ops._ptr(outs[-1]), ops.dtype_code(q.dtype), ops._ptr(k), ops._ptr(v), ops._ptr(table), mp, ps, ops._ptr(pos), ops._ptr(slot),
+        64, nq, nkv, d, window or 0, 0.125, None, 0, None, 0, None, 0.0, 2, k.shape[0], ops.fault_words(q.device), ops._stream()), "attn_tokenwise")
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
