@@ -6,6 +6,7 @@ stand-in: a CPU tensor or a missing library raises.
 """
 from __future__ import annotations
 
+import array
 import collections
 import ctypes
 from types import SimpleNamespace
@@ -827,17 +828,22 @@ def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gat
 
 
 def chunk_runs(h_q_start, chunk: int, least: int) -> tuple:
-    """A step's requests of `least` tokens and more in chunks of `chunk` tokens: (int32 rows [n, 4] (request, number, the request's chunks,
-    its first row), int32 runs [requests, 4] (request, first row, chunks or 0, 0) of all requests with a token, int32 first
-    rows, the longest of the requests without chunks), numpy."""
-    lens = np.diff(np.asarray(h_q_start, dtype=np.int64))
-    chunks = np.where(lens >= least, -(-lens // chunk), 0)
-    firsts = np.cumsum(chunks) - chunks
-    request = np.repeat(np.arange(len(lens)), chunks)
-    rows = np.stack([request, np.arange(len(request)) - firsts[request], chunks[request], firsts[request]], axis=1).astype(np.int32)
-    some = np.nonzero(lens)[0]
-    runs = np.stack([some, firsts[some] * (chunks[some] > 0), chunks[some], 0 * some], axis=1).astype(np.int32)
-    return rows, runs, firsts[chunks > 0].astype(np.int32), int(lens[chunks == 0].max(initial=0))
+    """A step's requests of `least` tokens and more in chunks of `chunk` tokens, as int32 words: rows (request, number, the request's
+    chunks, its first row), then runs (request, first row, chunks or 0, 0) of all requests with a token, then first rows; with how
+    many there are of each, and the longest of the requests without chunks."""
+    rows, runs, firsts, longest = [], [], [], 0
+    for b in range(len(h_q_start) - 1):
+        n = h_q_start[b + 1] - h_q_start[b]
+        if n >= least and n:
+            count, first = -(-n // chunk), len(rows) // 4
+            firsts.append(first)
+            runs += (b, first, count, 0)
+            for c in range(count):
+                rows += (b, c, count, first)
+        elif n:
+            runs += (b, 0, 0, 0)
+            longest = max(longest, n)
+    return array.array("i", rows + runs + firsts), len(rows) // 4, len(runs) // 4, len(firsts), longest
 
 
 def _chunk_list(ctx, key: str, chunk: int, least: int, device) -> SimpleNamespace:
@@ -845,11 +851,11 @@ def _chunk_list(ctx, key: str, chunk: int, least: int, device) -> SimpleNamespac
     requests that go token by token.  One description a step, for every layer."""
     key = (key, least)
     if key not in ctx.scratch:
-        rows, runs, firsts, longest = chunk_runs(ctx.h_q_start, chunk, least)
-        words = torch.from_numpy(np.concatenate([rows.reshape(-1), runs.reshape(-1), firsts])).to(device, non_blocking=True)
+        words, n, requests, long, longest = chunk_runs(ctx.h_q_start, chunk, least)
+        words = torch.frombuffer(words, dtype=torch.int32).to(device, non_blocking=True)
         at = _ptr(words)
-        ctx.scratch[key] = SimpleNamespace(words=words, rows=at, n=len(rows), runs=at + 16 * len(rows), requests=len(runs),
-                                           firsts=at + 16 * (len(rows) + len(runs)), long=len(firsts), longest=longest)
+        ctx.scratch[key] = SimpleNamespace(words=words, rows=at, n=n, runs=at + 16 * n, requests=requests, firsts=at + 16 * (n + requests),
+                                           long=long, longest=longest)
     return ctx.scratch[key]
 
 

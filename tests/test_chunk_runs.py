@@ -12,7 +12,7 @@ def test_runs_of_random_steps(seed):
     lens = [r.choice([0, 1, 1, r.randint(2, 40), r.randint(40, 700)]) for _ in range(r.randint(1, 12))]
     chunk, least = r.choice([32, 64]), r.choice([1, 16, 32, 96])
     start = [sum(lens[:i]) for i in range(len(lens) + 1)]
-    rows, runs, firsts, longest = chunk_runs(start, chunk, least)
+    words, n_rows, n_runs, n_firsts, longest = chunk_runs(start, chunk, least)
     want_rows, want_runs, want_firsts = [], [], []
     for b, n in enumerate(lens):
         if n == 0:
@@ -24,7 +24,8 @@ def test_runs_of_random_steps(seed):
         want_firsts.append(first)
         want_runs.append([b, first, count, 0])
         want_rows += [[b, c, count, first] for c in range(count)]
-    assert rows.tolist() == want_rows and runs.tolist() == want_runs and firsts.tolist() == want_firsts
+    assert (n_rows, n_runs, n_firsts) == (len(want_rows), len(want_runs), len(want_firsts))
+    assert words.tolist() == [x for r in want_rows + want_runs for x in r] + want_firsts
     assert longest == max([n for n in lens if n < least], default=0)
     if least == 1:
-        assert rows.tolist() == channel_chunks(start, chunk)[0].tolist()
+        assert want_rows == channel_chunks(start, chunk)[0].tolist()
