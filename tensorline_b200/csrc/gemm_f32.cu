@@ -3,8 +3,8 @@
 //
 // Every output element is one chain of fmaf over k = 0..K-1 in ascending order, whatever M is
 // and wherever the element falls in a tile; a row's result therefore does not depend on which
-// other rows share the launch.  This is the matrix product of the 32-bit engine; the bfloat16
-// engine's products use tensor cores.
+// other rows share the launch.  This is the matrix product of the 32-bit engine for float weights, for small matrices and for
+// rows that are not 16-byte aligned; large matrices of bfloat16 weights go to gemm_f32_parts.cu.
 //
 // Three kernels, the same floats: tiles (many rows), few rows, and a plain one for strides and sizes without 16-byte rows.
 #include "common.cuh"

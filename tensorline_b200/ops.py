@@ -18,7 +18,7 @@ from .csrc.build import CHECK_BUILD, load_library
 
 CORE_SOURCES = ["elementwise.cu", "rope_kv.cu", "attn_tokenwise.cu", "gemm_f32.cu", "sampling.cu", "recurrent.cu", "moe.cu",
                 "delta.cu", "latent.cu", "rglru.cu", "streams.cu", "stream_norm.cu", "attn_mixed_tokenwise.cu",
-                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu", "delta_chunk.cu"]
+                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu", "delta_chunk.cu", "gemm_f32_parts.cu"]
 
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -34,6 +34,8 @@ _SIGNATURES = {
     "tl_attn_tokenwise": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _P, _F, _I, _I, _P, _P],
     "tl_attn_rows": [_P, _I, _P, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _P, _F, _P, _I, _I, _I, _P, _P],
     "tl_gemm_f32": [_P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _P],
+    "tl_gemm_f32_parts_scratch": [_P, _I, _P, _I, _I, _I],
+    "tl_gemm_f32_parts": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P],
     "tl_argmax": [_P, _I, _I, _I, _P, _P, _P],
     "tl_sample": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
     "tl_linear_scan": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, ctypes.c_longlong, _P, _P, _P, _I, _I,
@@ -163,6 +165,8 @@ STATUS_ROLES = {1: "tcgen05 product: the copy thread waited for a free stage", 2
                 3: "tcgen05 product: the epilogue waited for the accumulator",
                 31: "two-block product: a copy thread waited for a free stage", 32: "two-block product: the MMA thread waited for a free accumulator",
                 33: "two-block product: the MMA thread waited for a stage's copies", 34: "two-block product: the epilogue waited for the accumulator",
+                41: "32-bit product: a copy thread waited for a free stage", 42: "32-bit product: the MMA thread waited for a free accumulator",
+                43: "32-bit product: the MMA thread waited for a stage's copies", 44: "32-bit product: the sums waited for an accumulator",
                 20: "decode attention: a wait for a stage of keys and values"}
 
 
@@ -700,7 +704,9 @@ def _sink(sink, nq: int, who: str) -> None:
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None) -> None:
-    """out[M, N] = a[M, K] w[N, K]^T (+ bias), float32 FFMA; w float32 or bfloat16 (widened)."""
+    """out[M, N] = a[M, K] w[N, K]^T (+ bias) in float32; w float32 or bfloat16 (widened).  A row's result does not depend on the other
+    rows.  Large matrices of bfloat16 weights: the tensor cores on the three bfloat16 parts of a's values (`gemm_f32_parts.cu`); the
+    rest float multiply-adds."""
     M, K = a.shape
     N = w.shape[0]
     if a.dtype != torch.float32 or out.dtype != torch.float32 or w.shape[1] != K or out.shape != (M, N):
@@ -710,6 +716,16 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Te
     _contig(w, "w")
     if bias is not None and bias.dtype != w.dtype:
         raise KernelError("gemm_f32: bias must have w's type")
+    if w.dtype == torch.bfloat16:
+        blocks = core().tl_gemm_f32_parts_scratch(_ptr(a), a.stride(0), _ptr(w), M, N, K)
+        if blocks:
+            scratch = torch.empty(blocks * 256, dtype=torch.uint8, device=a.device)
+            slabs = -(-M // 2048)
+            split = blocks * 256 >= 6 * min(M, 2048) * K + 256 + 4 * min(M, 2048) * N      # sums along K of their own
+            _check(core().tl_gemm_f32_parts(_ptr(a), a.stride(0), _ptr(w), _ptr(bias), _ptr(out), out.stride(0), M, N, K,
+                                            scratch.data_ptr(), _ptr(device_status(a.device)), _stream()),
+                   "gemm_f32_parts", launches=slabs * (3 if split else 2))
+            return
     _check(core().tl_gemm_f32(_ptr(a), a.stride(0), _ptr(w), K, dtype_code(w.dtype), _ptr(bias), _ptr(out),
                               out.stride(0), M, N, K, _stream()), "gemm_f32")
 

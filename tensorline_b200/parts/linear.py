@@ -1,6 +1,6 @@
 """Matrix products of the parts: y = x W^T, weights [out, in] (tensorline/quant.py:3).
 
-The 32-bit engine uses the exact-order FFMA kernel of this package.  The bfloat16 engine has two
+The 32-bit engine uses the float products of this package (`ops.gemm_f32`), whose order of additions is fixed.  The bfloat16 engine has two
 routes, both with float32 accumulation:
   * the hand-written tcgen05 / TMA kernel (`csrc/gemm_tc.cu`) for steps of few tokens against large
     matrices, where it streams the weights faster than the library and chains with the kernels around

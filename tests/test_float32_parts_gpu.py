@@ -1,0 +1,62 @@
+"""The 32-bit engine's product on the tensor cores (bfloat16 weights, large matrices) at the edges of its tiles, segments and groups: a
+row's floats do not depend on the rows beside it, and the formula in float64.  Bound of an output's error: its sums round at most once
+a chunk of 64 k, a segment and a group, and a chunk is cut off at most at each of its twelve instructions, each time by less than
+2^-22 of the sum of absolute products."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tensorline_b200 import ops
+    return ops
+
+
+def product(ops, a, w, bias=None):
+    out = torch.full((a.shape[0], w.shape[0]), 7.0, device="cuda")
+    ops.gemm_f32(a, w, out, bias)
+    return out
+
+
+@pytest.mark.parametrize("N,K", [(2048, 1024), (257, 4104), (1029, 1088), (300, 8200), (4608, 3584), (200, 18944)])
+def test_rows_of_every_tile_width_have_the_same_floats(ops, N, K):
+    g = torch.Generator().manual_seed(N + K)
+    top = 2100
+    a = torch.randn(top, K, generator=g).cuda()
+    w = torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    bias = torch.randn(N, generator=g).to(torch.bfloat16).cuda()
+    assert ops.core().tl_gemm_f32_parts_scratch(a.data_ptr(), K, w.data_ptr(), 1, N, K) > 0
+    whole = product(ops, a, w, bias)                     # more rows than are taken at a time
+    want, size = a.double() @ w.double().T + bias.double(), a.double().abs() @ w.double().abs().T + 1.0
+    chunks = -(-K // 64)
+    assert float(((whole.double() - want).abs() / size).max()) <= (chunks + chunks // 16 + 60) * 2.0 ** -24
+    for n in (1, 2, 31, 33, 64, 65, 97, 128, 129, 177, 336, 353, 700):
+        lo = (n * 37) % (top - n)
+        assert torch.equal(product(ops, a[lo:lo + n], w, bias), whole[lo:lo + n]), n
+    ops.check_device_status()
+
+
+def test_rows_apart_and_odd_values(ops):
+    g = torch.Generator().manual_seed(3)
+    N, K = 700, 1600
+    wide = torch.randn(40, K + 12, generator=g).cuda()
+    a = wide[:, 4:4 + K]                                 # 16 bytes into its rows
+    w = torch.randn(N, K, generator=g).clamp_(-0.9, 0.9).to(torch.bfloat16).cuda()
+    assert torch.equal(product(ops, a, w), product(ops, a.contiguous(), w))
+    odd = a.contiguous().clone()
+    odd[1, 3] = 3.4028e38                                # would round up to an infinity in bfloat16
+    odd[2] *= 2.0 ** -140                                # below the smallest normal number
+    odd[3, 5] = float("inf")
+    odd[4, 7] = float("nan")
+    odd[5, 9] = torch.tensor(0x7f800001, dtype=torch.int32).view(torch.float32)      # a not-a-number whose high half is an infinity's
+    got = product(ops, odd, w)
+    keep = [0] + list(range(6, 40))
+    assert torch.equal(got[keep], product(ops, a, w)[keep])
+    want = odd.double() @ w.double().T
+    assert torch.equal(torch.isinf(got[3]), torch.isinf(want[3])) and torch.equal(got[3].sign(), want[3].sign().float())
+    assert bool(torch.isnan(got[4]).all()) and bool(torch.isnan(got[5]).all())
+    assert float((got[2].double() - want[2]).abs().max()) <= K * 2.0 ** -132
+    assert float(((got[1].double() - want[1]).abs() / want[1].abs().clamp_min(1.0)).max()) <= 2.0 ** -20
+    ops.check_device_status()
