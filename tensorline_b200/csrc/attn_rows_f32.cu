@@ -5,16 +5,17 @@
 // the rows (token, head) that read the same keys share them through shared memory, and a step of few tokens has its dot products
 // taken by as many blocks as there are tiles.
 //
-//   attn_rows       a block has up to 64 rows: neighbouring tokens of one request times the query heads of one KV head.  128
-//                   threads; a warp owns 16 rows from the dot products (4 x 4 outputs a lane) over the softmax (half a row a
-//                   lane) to the values (8 rows x 4 NC columns a lane), so between tiles only the tiles themselves are waited
-//                   for: K of the next tile arrives while the values are summed, V of it while the dot products are taken.
-//                   A tile costs 2 x 64 x 32 x d multiply-adds; FMA-bound.
+//   attn_rows       a block has up to 64 (or 32) rows: neighbouring tokens of one request times the query heads of one KV head.
+//                   Four warps; a warp owns 16 (or 8) rows from the dot products over the softmax to the values, so between tiles only the
+//                   tiles themselves are waited for: K of the next tile arrives while the values are summed, V of it while
+//                   the dot products are taken; where a tile's keys lie is looked up a tile ahead.  Operands come from shared memory
+//                   a step ahead of the multiply-adds.  A tile costs 2 x 64 x 32 x d multiply-adds; what bounds it is the latency of a
+//                   warp's instructions (one in 3.6 cycles) as long as few warps share an SM, then their issue.
 //   attn_dots, attn_chain   steps of few tokens: the chains over the keys are all that is left in order.  attn_dots: a thread
 //                   a key, all tiles at once, scores to memory; attn_chain: a warp a head and 32 output columns, the softmax of
 //                   128 keys at a time and then their chain.
-// Measured with 28 query heads of 128 on 4 KV heads: 333 tokens on 700 cached 350 us (the token-wise kernel 5,076), 2,048 tokens
-// 1.32 ms (33.4); single tokens at position 1,800: 4 of them 56 us (1,842; attn_rows 478), 64 of them 265 us (3,577; 611).
+// Measured with 28 query heads of 128 on 4 KV heads: 333 tokens on 700 cached 254 us (the token-wise kernel 5,076; blocks of 64 rows
+// without the look-ahead 350), 2,048 tokens 1.29 ms (33.4; 1.31); single tokens at position 1,800: 4 of them 56 us (1,842; attn_rows 478), 64 of them 265 us (3,577; 611).
 // Masks, sinks, gates, caps and slopes: as described in attn_tokenwise.cu.  The roundings are spelt out here
 // and there: which kernel a row is given to does not show in its floats.
 #include "common.cuh"
@@ -47,9 +48,12 @@ __device__ __forceinline__ void rows_fma2(float& d0, float& d1, float a, float b
 __device__ __forceinline__ int rows_low(const RowsArgs& A, int p) {
     return A.chunk > 0 ? (p / A.chunk) * A.chunk : (A.window > 0 && p - A.window + 1 > 0) ? p - A.window + 1 : 0;
 }
-__device__ __forceinline__ const float* rows_at(const RowsArgs& A, const float* pages, const int* tab, int j, int kh) {
+__device__ __forceinline__ size_t rows_offset(const RowsArgs& A, const int* tab, int j, int kh) {
     const int page = tl_checked(tab[tl_checked(j / A.page_size, A.max_pages, A.L, TL_K_TOKENWISE)], A.L.total_pages, A.L, TL_K_TOKENWISE);
-    return pages + (((size_t)page * A.nkv + kh) * A.page_size + (j % A.page_size)) * A.d;
+    return (((size_t)page * A.nkv + kh) * A.page_size + (j % A.page_size)) * A.d;
+}
+__device__ __forceinline__ const float* rows_at(const RowsArgs& A, const float* pages, const int* tab, int j, int kh) {
+    return pages + rows_offset(A, tab, j, kh);
 }
 // The position of a token whose scores lie in `scores`: one beyond the table is recorded by the checking build, and cut in every build, so
 // that nothing outside the scratch is touched.
@@ -63,15 +67,17 @@ __device__ __forceinline__ float rows_score(const RowsArgs& A, float dot, float 
     if (A.slopes) s = fmaf(-slope, (float)(p - j), s);
     return s;
 }
-constexpr int ROWS_MAX = 64, ROWS_PS = ROWS_MAX + 4;     // rows a block, and the stride of a key's scores in shared memory
+constexpr int ROWS_MAX = 64;
 
-// NC: groups of 64 output columns (d <= 64 NC)
-template <int NC>
-__global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
+// NC: groups of 64 output columns (d <= 64 NC); ROWS: rows a block, RW: a warp
+template <int NC, int ROWS, int RW>
+__global__ void __launch_bounds__(ROWS / RW * 32) attn_rows_kernel(const RowsArgs A) {
+    constexpr int NT = ROWS / RW * 32, TK = NT / 32, ROWS_PS = ROWS + 4;                      // threads, and those that fetch a key
+    constexpr int LC = RW == 16 || NC == 1 ? 16 : 32, VR = RW * LC / 32, VC = 16 * NC / LC;      // values: lanes over columns, rows and column groups a lane
     extern __shared__ __align__(16) float sm[];
     const int d = A.d, g = A.nq / A.nkv, ld = d + 4;
     float* Qs = sm;                                      // [64][ld], rows beyond the block's last are zeros
-    float* Ks = Qs + ROWS_MAX * ld;                      // [32][ld]
+    float* Ks = Qs + ROWS * ld;                      // [32][ld]
     float* Vs = Ks + 32 * ld;                            // [32][ld]
     float* Ps = Vs + 32 * ld;                            // [32 keys][ROWS_PS rows]: dot products, then weights
     float* al = Ps + 32 * ROWS_PS;                       // [64]
@@ -89,12 +95,13 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
     starts &= starts - 1;
     const int n = (starts ? __ffs(starts) - 1 : te - tb) - first, t0 = tb + first, rows = n * g;
     const int* tab = A.table + (size_t)tl_checked(A.req_slot[t0], A.L.table_rows, A.L, TL_K_TOKENWISE) * A.max_pages;
-    for (int i = tid; i < ROWS_MAX * d; i += 128) {
+    for (int i = tid; i < ROWS * d; i += NT) {
         const int r = i / d, e = i - r * d;
         Qs[r * ld + e] = r < rows ? A.q[(size_t)(t0 + r / g) * A.q_stride + (size_t)(kh * g + r % g) * d + e] : 0.f;
     }
-    // the softmax's row of this lane: 16 rows a warp, a lane and its neighbour 16 further on share a row, 16 keys each
-    const int row = wid * 16 + (lane & 15), kb = lane & 16;
+    // the softmax's row of this lane: the G lanes RW apart share a row, every G-th key each
+    constexpr int G = 32 / RW;
+    const int row = wid * RW + lane % RW, kb = lane / RW;
     const bool live = row < rows;
     const int p = live ? A.pos[t0 + row / g] : -1, head = kh * g + row % g;
     const int lo = live ? rows_low(A, p) : 0, kept = min(A.keep_first, lo);
@@ -106,93 +113,116 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
         last = max(last, pi); low = min(low, li); keep = max(keep, min(A.keep_first, li));
     }
     auto next = [&](int j0) { return (j0 >= keep && j0 + 32 <= low) ? (low / 32) * 32 : j0; };
-    auto fetch = [&](float* dst, const float* pages, int j0) {       // four threads a key; keys that no row sees are not read
-        const int j = j0 + (tid >> 2);
-        if (j <= last && (j >= low || j < keep)) {
-            const float* src = rows_at(A, pages, tab, j, kh);
-            for (int e = (tid & 3) * 4; e < d; e += 16) rows_copy16(dst + (tid >> 2) * ld + e, src + e);
-        }
+    // TK threads a key; keys that no row sees are not read.  Where a tile's keys lie is looked up a tile ahead, once for K and V.
+    constexpr size_t NOWHERE = ~(size_t)0;
+    auto where = [&](int j0) {
+        const int j = j0 + tid / TK;
+        return j <= last && (j >= low || j < keep) ? rows_offset(A, tab, j, kh) : NOWHERE;
+    };
+    auto fetch = [&](float* dst, const float* pages, size_t at) {
+        if (at != NOWHERE)
+            for (int e = tid % TK * 4; e < d; e += TK * 4) rows_copy16(dst + tid / TK * ld + e, pages + at + e);
         ROWS_COMMIT();
     };
-    float acc[8][4 * NC];
+    float acc[VR][4 * VC];
 #pragma unroll
-    for (int r = 0; r < 8; ++r)
+    for (int r = 0; r < VR; ++r)
 #pragma unroll
-        for (int c = 0; c < 4 * NC; ++c) acc[r][c] = 0.f;
-    const int kl = lane & 7, rl = lane >> 3;             // dot products: keys kl + 8 j, rows 16 wid + 4 i + rl
-    const int dg = (lane & 15) * 4, rg = wid * 16 + (lane >> 4) * 8;      // values: columns dg + 64 c, rows rg ..
+        for (int c = 0; c < 4 * VC; ++c) acc[r][c] = 0.f;
+    const int kl = lane & 7, rl = lane >> 3;             // dot products: keys kl + 8 j, rows RW wid + 4 i + rl
+    const int dg = lane % LC * 4, rg = wid * RW + lane / LC * VR;      // values: columns dg + 4 LC c, rows rg ..
     int j0 = next(0);
-    fetch(Ks, A.k_pages, j0);
-    fetch(Vs, A.v_pages, j0);
+    {
+        const size_t at = where(j0);
+        fetch(Ks, A.k_pages, at);
+        fetch(Vs, A.v_pages, at);
+    }
     while (j0 <= last) {
         const int j1 = next(j0 + 32);
+        const size_t at = where(j1);
         ROWS_WAIT(1);
         __syncthreads();
         {
-            float s[4][4];
+            float s[RW / 4][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RW / 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-            const float* qp = Qs + (wid * 16 + rl) * ld;
+            const float* qp = Qs + (wid * RW + rl) * ld;
             const float* kp = Ks + kl * ld;
-#pragma unroll 2
-            for (int e = 0; e < d; e += 4) {
-                float4 q4[4], k4[4];
+            // the next four dimensions are on their way from shared memory while these are multiplied
+            float4 q4[2][RW / 4], k4[2][4];
+            auto load = [&](int b, int e) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) q4[i] = *reinterpret_cast<const float4*>(qp + 4 * i * ld + e);
+                for (int i = 0; i < RW / 4; ++i) q4[b][i] = *reinterpret_cast<const float4*>(qp + 4 * i * ld + e);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) k4[j] = *reinterpret_cast<const float4*>(kp + 8 * j * ld + e);
+                for (int j = 0; j < 4; ++j) k4[b][j] = *reinterpret_cast<const float4*>(kp + 8 * j * ld + e);
+            };
+            auto dots = [&](int b) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+                for (int c = 0; c < 4; ++c)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        s[i][j] = fmaf(q4[i].x, k4[j].x, s[i][j]);
-                        s[i][j] = fmaf(q4[i].y, k4[j].y, s[i][j]);
-                        s[i][j] = fmaf(q4[i].z, k4[j].z, s[i][j]);
-                        s[i][j] = fmaf(q4[i].w, k4[j].w, s[i][j]);
+                    for (int i = 0; i < RW / 4; ++i) {
+                        const float x = c == 0 ? q4[b][i].x : c == 1 ? q4[b][i].y : c == 2 ? q4[b][i].z : q4[b][i].w;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            s[i][j] = fmaf(x, c == 0 ? k4[b][j].x : c == 1 ? k4[b][j].y : c == 2 ? k4[b][j].z : k4[b][j].w, s[i][j]);
                     }
+            };
+            load(0, 0);
+            int e = 0;
+            for (; e + 8 < d; e += 8) {
+                load(1, e + 4);
+                dots(0);
+                load(0, e + 8);
+                dots(1);
             }
+            if (e + 4 < d) { load(1, e + 4); dots(0); dots(1); } else dots(0);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RW / 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) Ps[(kl + 8 * j) * ROWS_PS + wid * 16 + 4 * i + rl] = s[i][j];
+                for (int j = 0; j < 4; ++j) Ps[(kl + 8 * j) * ROWS_PS + wid * RW + 4 * i + rl] = s[i][j];
         }
         __syncthreads();                                 // K is read; a warp's scores are its own
-        if (j1 <= last) fetch(Ks, A.k_pages, j1); else ROWS_COMMIT();
+        fetch(Ks, A.k_pages, at);
         bool full;
         {
-            float s[16];
+            float s[RW];
             float top = -INFINITY;
-            int valid = 0;
+            int any = 0;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int j = j0 + kb + i;
+            for (int i = 0; i < RW; ++i) {
+                const int j = j0 + kb + G * i;
                 s[i] = -INFINITY;
                 if ((j >= lo || j < kept) && j <= p) {
-                    s[i] = rows_score(A, Ps[(kb + i) * ROWS_PS + row], slope, p, j);
-                    ++valid;
+                    s[i] = rows_score(A, Ps[(kb + G * i) * ROWS_PS + row], slope, p, j);
+                    any = 1;
                 }
                 top = fmaxf(top, s[i]);
             }
-            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 16));
-            const int any = valid + __shfl_xor_sync(0xffffffffu, valid, 16);
+#pragma unroll
+            for (int o = 16; o >= RW; o >>= 1) {
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+                any |= __shfl_xor_sync(0xffffffffu, any, o);
+            }
             const float m_new = fmaxf(m, top);
             const float alpha = any ? expf(m - m_new) : 1.0f;        // a row without keys in this tile stays as it is
             bool nonzero = true;
-            float sum[16];
+            float sum[RW];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const int j = j0 + kb + i;
+            for (int i = 0; i < RW; ++i) {
+                const int j = j0 + kb + G * i;
                 const float pj = ((j >= lo || j < kept) && j <= p) ? expf(s[i] - m_new) : 0.f;
-                Ps[(kb + i) * ROWS_PS + row] = pj;
+                Ps[(kb + G * i) * ROWS_PS + row] = pj;
                 nonzero = nonzero && pj != 0.f;
-                sum[i] = pj + __shfl_xor_sync(0xffffffffu, pj, 16);  // the order of a warp's sum: keys 16 apart, then 8, 4, 2, 1
+                sum[i] = pj;
             }
 #pragma unroll
-            for (int o = 8; o > 0; o >>= 1)
+            for (int o = RW / 2; o > 0; o >>= 1)         // the order of a warp's sum: keys 16 apart, then 8, 4, 2, 1
 #pragma unroll
                 for (int i = 0; i < o; ++i) sum[i] += sum[i + o];
+#pragma unroll
+            for (int o = 16; o >= RW; o >>= 1) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
             if (any) { l = fmaf(l, alpha, sum[0]); m = m_new; }
             if (kb == 0) al[row] = alpha;
             full = __all_sync(0xffffffffu, nonzero || !live);        // no weight of the warp's rows is zero
@@ -200,39 +230,51 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
         ROWS_WAIT(1);
         __syncthreads();                                 // V has landed
         {
-            const float4 a0 = *reinterpret_cast<const float4*>(al + rg), a1 = *reinterpret_cast<const float4*>(al + rg + 4);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            float av[VR];
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
+            for (int r = 0; r < VR; r += 4) *reinterpret_cast<float4*>(av + r) = *reinterpret_cast<const float4*>(al + rg + r);
 #pragma unroll
-                for (int c = 0; c < 4 * NC; ++c) acc[r][c] *= av[r];
+            for (int r = 0; r < VR; ++r)
+#pragma unroll
+                for (int c = 0; c < 4 * VC; ++c) acc[r][c] *= av[r];
             const int keys = min(32, last - j0 + 1);
-            auto key = [&](int k, bool all) {
-                const float4 p0 = *reinterpret_cast<const float4*>(Ps + k * ROWS_PS + rg), p1 = *reinterpret_cast<const float4*>(Ps + k * ROWS_PS + rg + 4);
-                const float pv[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            auto load = [&](int k, float (&pv)[VR], float4 (&v)[VC]) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int e = dg + 64 * c;
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (e < d) v = *reinterpret_cast<const float4*>(Vs + k * ld + e);
+                for (int r = 0; r < VR; r += 4) *reinterpret_cast<float4*>(pv + r) = *reinterpret_cast<const float4*>(Ps + k * ROWS_PS + rg + r);
 #pragma unroll
-                    for (int r = 0; r < 8; ++r) {
-                        if (all || pv[r] != 0.f) {       // a weight of zero (no key, or one far below the maximum) adds nothing,
-                            rows_fma2(acc[r][4 * c], acc[r][4 * c + 1], pv[r], v.x, v.y);      // whatever its value holds
-                            rows_fma2(acc[r][4 * c + 2], acc[r][4 * c + 3], pv[r], v.z, v.w);
-                        }
-                    }
+                for (int c = 0; c < VC; ++c) {
+                    const int e = dg + 4 * LC * c;
+                    v[c] = e < d ? *reinterpret_cast<const float4*>(Vs + k * ld + e) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             };
+            auto key = [&](const float (&pv)[VR], const float4 (&v)[VC], bool all) {
+#pragma unroll
+                for (int c = 0; c < VC; ++c)
+#pragma unroll
+                    for (int r = 0; r < VR; ++r) {
+                        if (all || pv[r] != 0.f) {       // a weight of zero (no key, or one far below the maximum) adds nothing,
+                            rows_fma2(acc[r][4 * c], acc[r][4 * c + 1], pv[r], v[c].x, v[c].y);      // whatever its value holds
+                            rows_fma2(acc[r][4 * c + 2], acc[r][4 * c + 3], pv[r], v[c].z, v[c].w);
+                        }
+                    }
+            };
+            float pv[2][VR];
+            float4 v[2][VC];
             if (full && keys == 32) {
-#pragma unroll 2
-                for (int k = 0; k < 32; ++k) key(k, true);
+                load(0, pv[0], v[0]);
+#pragma unroll
+                for (int k = 0; k < 32; k += 2) {
+                    load(k + 1, pv[1], v[1]);
+                    key(pv[0], v[0], true);
+                    if (k + 2 < 32) load(k + 2, pv[0], v[0]);
+                    key(pv[1], v[1], true);
+                }
             } else {
-                for (int k = 0; k < keys; ++k) key(k, false);
+                for (int k = 0; k < keys; ++k) { load(k, pv[0], v[0]); key(pv[0], v[0], false); }
             }
         }
         __syncthreads();                                 // V and the weights are read
-        if (j1 <= last) fetch(Vs, A.v_pages, j1); else ROWS_COMMIT();
+        fetch(Vs, A.v_pages, at);
         j0 = j1;
     }
     ROWS_WAIT(0);
@@ -248,13 +290,13 @@ __global__ void __launch_bounds__(128) attn_rows_kernel(const RowsArgs A) {
     }
     __syncwarp();                                        // rows rg .. of this lane are its own warp's
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+    for (int r = 0; r < VR; ++r) {
         if (rg + r >= rows) continue;
         const float alpha = al[rg + r], inv = Ps[rg + r];
         float* o = A.out + ((size_t)(t0 + (rg + r) / g) * A.nq + kh * g + (rg + r) % g) * d;
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const int e = dg + 64 * c;
+        for (int c = 0; c < VC; ++c) {
+            const int e = dg + 4 * LC * c;
             if (e >= d) continue;
             float4 v = make_float4(acc[r][4 * c], acc[r][4 * c + 1], acc[r][4 * c + 2], acc[r][4 * c + 3]);
             if (A.sink) { v.x *= alpha; v.y *= alpha; v.z *= alpha; v.w *= alpha; }
@@ -418,6 +460,19 @@ __global__ void __launch_bounds__(32 * DOTS_HEADS) attn_chain_kernel(const RowsA
     if (live && e < d) A.out[((size_t)t * A.nq + head) * d + e] = acc * inv;
 }
 
+template <int NC, int ROWS, int RW>
+static int launch_rows(RowsArgs A, cudaStream_t stream) {
+    constexpr auto bytes = [](int d) { return ((ROWS + 64) * (d + 4) + 32 * (ROWS + 4) + ROWS) * (int)sizeof(float); };
+    static bool raised[TL_MAX_DEVICES] = {};
+    const int e = tl_raise_smem(attn_rows_kernel<NC, ROWS, RW>, raised, bytes(64 * NC));
+    if (e) return e;
+    const int g = A.nq / A.nkv;
+    A.tq = ROWS / g < 32 ? ROWS / g : 32;
+    const dim3 grid((A.T + A.tq - 1) / A.tq, A.nkv, A.tq < A.T ? A.tq : A.T);
+    attn_rows_kernel<NC, ROWS, RW><<<grid, ROWS / RW * 32, bytes(A.d), stream>>>(A);
+    return tl_launch_status();
+}
+
 // `scores` (float [T, nq, keys], keys >= every position of the step + 1, or null): scratch of the two kernels of few tokens.
 // Returns 1 for shapes that these kernels do not take; the caller gives those to the token-wise kernel beforehand.
 TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float* k_pages, const float* v_pages, const int* table,
@@ -428,12 +483,8 @@ TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float
     if (nq % nkv || (chunk > 0 && window > 0) || chunk < 0 || d < 4 || d % 4 || d > 256 ||
         ((((uintptr_t)k_pages) | ((uintptr_t)v_pages) | ((uintptr_t)out)) & 15)) return 1;
     const int g = nq / nkv;
-    static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {}, r4[TL_MAX_DEVICES] = {}, rc[TL_MAX_DEVICES] = {};
-    constexpr int most = ((ROWS_MAX + 64) * (256 + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
-    int e = tl_raise_smem(attn_rows_kernel<1>, r1, most);
-    if (!e) e = tl_raise_smem(attn_rows_kernel<2>, r2, most);
-    if (!e) e = tl_raise_smem(attn_rows_kernel<4>, r4, most);
-    if (!e) e = tl_raise_smem(attn_chain_kernel, rc, CHAIN_SMEM);
+    static bool rc[TL_MAX_DEVICES] = {};
+    int e = tl_raise_smem(attn_chain_kernel, rc, CHAIN_SMEM);
     if (e) return e;
     RowsArgs A{q, q_stride, out, k_pages, v_pages, table, max_pages, page_size, pos, req_slot, T, nq, nkv, d, window, scale,
                sink, window > 0 ? keep_first : 0, gate, chunk, slopes, cap, scores, keys, 0, TlLimits{table_rows, total_pages, fault}};
@@ -449,11 +500,12 @@ TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float
         return tl_launch_status();
     }
     if (g > ROWS_MAX || nkv > 65535) return 1;
-    A.tq = ROWS_MAX / g < 32 ? ROWS_MAX / g : 32;
-    const int smem = ((ROWS_MAX + 64) * (d + 4) + 32 * ROWS_PS + ROWS_MAX) * (int)sizeof(float);
-    const dim3 grid((T + A.tq - 1) / A.tq, nkv, A.tq < T ? A.tq : T);
-    if (d <= 64) attn_rows_kernel<1><<<grid, 128, smem, stream>>>(A);
-    else if (d <= 128) attn_rows_kernel<2><<<grid, 128, smem, stream>>>(A);
-    else attn_rows_kernel<4><<<grid, 128, smem, stream>>>(A);
-    return tl_launch_status();
+    // Blocks of 64 rows, 16 a warp, where they are three an SM or more (2,048 tokens, 28 heads: 1,294 us against 1,430); else of 32
+    // rows, 8 a warp: more of them, and a warp is done with a tile sooner (333 tokens on 700 cached: 254 us against 336; 100 on 300:
+    // 158 against 293; 700 tokens, 40 heads, three an SM: 300 both).
+    const int tokens = ROWS_MAX / g < 32 ? ROWS_MAX / g : 32;
+    const bool wide = g > ROWS_MAX / 2 || (long long)((T + tokens - 1) / tokens) * nkv >= 3LL * tl_num_sms();
+#define ROWS_GO(NC) (wide ? launch_rows<NC, ROWS_MAX, 16>(A, stream) : launch_rows<NC, ROWS_MAX / 2, 8>(A, stream))
+    return d <= 64 ? ROWS_GO(1) : d <= 128 ? ROWS_GO(2) : ROWS_GO(4);
+#undef ROWS_GO
 }
