@@ -115,19 +115,20 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------------------------------------------------------- TMA (both blocks)
+        const uint32_t one = pair_elect(), lead = rank == 0 ? one : 0u;
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
         auto load_w = [&](const Item& t, int c, int s) {
-            if (rank == 0) mbar_expect_tx(full_bar + s, 2 * Sh::STAGE);
+            pair_expect(full_bar + s, 2 * Sh::STAGE, lead);
             pair_load(smem_addr(tiles + s * Sh::STAGE), &map_w, pair_peer(smem_addr(full_bar + s), 0), c * GP_CHUNK,
-                    t.m * 2 * GP_ROWS + (int)rank * GP_ROWS);
+                      t.m * 2 * GP_ROWS + (int)rank * GP_ROWS, one);
         };
         auto load_x = [&](const Item& t, int c, int s) {
             const uint32_t bar = pair_peer(smem_addr(full_bar + s), 0), st = smem_addr(tiles + s * Sh::STAGE) + GP_W_BYTES;
 #pragma unroll
-            for (int p = 0; p < 3; ++p) pair_load(st + p * Sh::B_BYTES, &map_x, bar, c * GP_CHUNK, p * G.M + t.t * BN + (int)rank * (BN / 2));
+            for (int p = 0; p < 3; ++p) pair_load(st + p * Sh::B_BYTES, &map_x, bar, c * GP_CHUNK, p * G.M + t.t * BN + (int)rank * (BN / 2), one);
         };
         // W is nobody's output: its first tiles are asked for before the wait for the kernel that writes the tokens' parts
         const Item first = item_at(pair);

@@ -12,8 +12,8 @@
 // expert's rows (moe_up), and every token sums its experts' down products in the order they were chosen (moe_down):
 // one pass over the weights the step needs, no sorting, nothing on the host, so the step can sit in a CUDA graph.
 // Steps of many tokens: the pairs are sorted by expert on the device (moe_sort), the tokens' rows gathered in that
-// order (every expert's run in a buffer of `cap` rows of its own, so that one batched product serves all experts), two
-// dense products run on them, and moe_combine sums each token's rows by weight.
+// order, two products run over the experts' runs (moe_product.cu; where it does not take the sizes, batched products over runs of
+// `cap` rows each), and moe_combine sums each token's rows by weight.
 // Every output element is one fixed chain of additions, so a token's result does not depend on the step's other tokens.
 #include "common.cuh"
 
@@ -627,6 +627,8 @@ TL_EXPORT int tl_moe_down(const void* a, int act_dtype, const void* w_down, int 
 __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ idx, int P, int E, int* __restrict__ offsets,
                                                         int* __restrict__ place_of, int* __restrict__ pair_at) {
     extern __shared__ int cnt[];                         // [E][blockDim.x + 1] would be too much: counts per (expert, warp)
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int* base = cnt + E * nw;                            // [E + 1]
     for (int i = threadIdx.x; i < E * nw; i += blockDim.x) cnt[i] = 0;
@@ -682,8 +684,7 @@ TL_EXPORT int tl_moe_sort(const int* idx, int P, int E, int* offsets, int* place
     if (P <= 0) return 0;
     const size_t smem = ((size_t)E * 32 + E + 1) * sizeof(int);
     if (smem > 48 * 1024) return 1;
-    moe_sort_kernel<<<1, 1024, smem, stream>>>(idx, P, E, offsets, place_of, pair_at);
-    return tl_launch_status();
+    return launch_after_wait(moe_sort_kernel, dim3(1), dim3(1024), smem, stream, idx, P, E, offsets, place_of, pair_at);
 }
 
 // Where a sorted place lies in the experts' row buffer.  cap = 0: the runs lie one behind the other (row = place);
@@ -699,6 +700,8 @@ template <typename TA>
 __global__ void moe_gather_kernel(const TA* __restrict__ h, const int* __restrict__ pair_at, const int* __restrict__ offsets, int cap,
                                   TA* __restrict__ rows, int K, int top, const float* __restrict__ scale) {
     int place = blockIdx.x;
+    grid_dependency_wait();
+    grid_dependency_trigger();
     if (cap) {
         const int e = blockIdx.x / cap, r = blockIdx.x - e * cap;
         place = offsets[e] + r < offsets[e + 1] ? offsets[e] + r : -1;
@@ -726,9 +729,9 @@ TL_EXPORT int tl_moe_gather(const void* h, int act_dtype, const int* pair_at, co
     const long long blocks = cap ? (long long)E * cap : P;
     if (blocks <= 0) return 0;
     if (blocks > 2147483647LL) return 1;
-    if (act_dtype == TL_F32) moe_gather_kernel<float><<<(unsigned)blocks, 128, 0, stream>>>((const float*)h, pair_at, offsets, cap, (float*)rows, K, top, scale);
-    else moe_gather_kernel<bf16><<<(unsigned)blocks, 128, 0, stream>>>((const bf16*)h, pair_at, offsets, cap, (bf16*)rows, K, top, scale);
-    return tl_launch_status();
+    const dim3 grid((unsigned)blocks), block(128);
+    if (act_dtype == TL_F32) return launch_after_wait(moe_gather_kernel<float>, grid, block, 0, stream, (const float*)h, pair_at, offsets, cap, (float*)rows, K, top, scale);
+    return launch_after_wait(moe_gather_kernel<bf16>, grid, block, 0, stream, (const bf16*)h, pair_at, offsets, cap, (bf16*)rows, K, top, scale);
 }
 
 // u = relu(u)^2 in place
@@ -796,19 +799,22 @@ TL_EXPORT int tl_relu_square(void* u, int act_dtype, long long n, cudaStream_t s
     return tl_launch_status();
 }
 
-// y[t, :] = sum_j wts[t, j] * rows[row of place_of[t * top + j], :], j in the order chosen
+// y[t, :] = sum_j wts[t, j] * rows[row of place_of[t * top + j], :], j in the order chosen; an entry idx >= E_real has no row: it
+// counts with same[t, :]
 template <typename TA>
 __global__ void moe_combine_kernel(const TA* __restrict__ rows, const int* __restrict__ place_of, const int* __restrict__ idx,
                                    const int* __restrict__ offsets, int cap, const float* __restrict__ wts,
                                    TA* __restrict__ y, int N, int top, const TA* __restrict__ extra,
-                                   const float* __restrict__ extra_gate, int ldg) {
+                                   const float* __restrict__ extra_gate, int ldg, int E_real, const TA* __restrict__ same) {
     const int t = blockIdx.x;
+    grid_dependency_wait();
+    grid_dependency_trigger();
     const float gt = !extra ? 0.f : extra_gate ? 1.0f / (1.0f + expf(-extra_gate[(size_t)t * ldg])) : 1.0f;
     for (int n = threadIdx.x; n < N; n += blockDim.x) {
         float acc = 0.f;
         for (int j = 0; j < top; ++j) {
             const size_t pair = (size_t)t * top + j;
-            const float v = to_f<TA>(rows[moe_row(place_of[pair], idx[pair], offsets, cap) * N + n]);
+            const float v = to_f<TA>(idx[pair] >= E_real ? same[(size_t)t * N + n] : rows[moe_row(place_of[pair], idx[pair], offsets, cap) * N + n]);
             acc = wts ? fmaf(wts[pair], v, acc) : acc + v;
         }
         if (extra) acc = fmaf(gt, to_f<TA>(extra[(size_t)t * N + n]), acc);
@@ -824,13 +830,16 @@ constexpr int COMBINE_VEC = 512;
 __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* __restrict__ rows, const int* __restrict__ place_of, const int* __restrict__ idx,
                                                               const int* __restrict__ offsets, int cap, const float* __restrict__ wts,
                                                               bf16* __restrict__ y, int N, int top, const bf16* __restrict__ extra,
-                                                              const float* __restrict__ extra_gate, int ldg) {
-    __shared__ size_t at[32];
+                                                              const float* __restrict__ extra_gate, int ldg, int E_real,
+                                                              const bf16* __restrict__ same) {
+    __shared__ const bf16* at[32];
     __shared__ float ws[32];
     const int t = blockIdx.x;
+    grid_dependency_wait();
+    grid_dependency_trigger();
     if (threadIdx.x < top) {
         const size_t pair = (size_t)t * top + threadIdx.x;
-        at[threadIdx.x] = moe_row(place_of[pair], idx[pair], offsets, cap) * N;
+        at[threadIdx.x] = idx[pair] >= E_real ? same + (size_t)t * N : rows + moe_row(place_of[pair], idx[pair], offsets, cap) * N;
         ws[threadIdx.x] = wts ? wts[pair] : 1.0f;
     }
     const float gt = !extra ? 0.f : extra_gate ? 1.0f / (1.0f + expf(-extra_gate[(size_t)t * ldg])) : 1.0f;
@@ -842,7 +851,7 @@ __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* __rest
         for (int j0 = 0; j0 < top; j0 += 4) {
             uint4 v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) if (j0 + j < top) v[j] = *reinterpret_cast<const uint4*>(rows + at[j0 + j] + n);
+            for (int j = 0; j < 4; ++j) if (j0 + j < top) v[j] = *reinterpret_cast<const uint4*>(at[j0 + j] + n);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (j0 + j >= top) continue;
@@ -873,14 +882,17 @@ __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* __rest
 
 TL_EXPORT int tl_moe_combine(const void* rows, int act_dtype, const int* place_of, const int* idx, const int* offsets, int cap,
                              const float* wts, void* y, int T, int N, int top, const void* extra, const float* extra_gate, int ldg,
-                             cudaStream_t stream) {
+                             int E_real, const void* same, cudaStream_t stream) {
     if (T <= 0) return 0;
-    if (act_dtype != TL_F32 && N % 8 == 0 && N >= COMBINE_VEC && top <= 32 && ((((uintptr_t)rows) | ((uintptr_t)y) | ((uintptr_t)extra)) & 15) == 0) {
+    if (!same) E_real = 0x7fffffff;                      // every entry has a row
+    if (act_dtype != TL_F32 && N % 8 == 0 && N >= COMBINE_VEC && top <= 32 &&
+        ((((uintptr_t)rows) | ((uintptr_t)y) | ((uintptr_t)extra) | ((uintptr_t)same)) & 15) == 0) {
         const int pieces = (N / 8 + 31) / 32 * 32;
-        moe_combine_vec_kernel<<<T, pieces < 256 ? pieces : 256, 0, stream>>>((const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg);
-        return tl_launch_status();
+        return launch_after_wait(moe_combine_vec_kernel, dim3(T), dim3(pieces < 256 ? pieces : 256), 0, stream, (const bf16*)rows, place_of, idx, offsets,
+                                 cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg, E_real, (const bf16*)same);
     }
-    if (act_dtype == TL_F32) moe_combine_kernel<float><<<T, 256, 0, stream>>>((const float*)rows, place_of, idx, offsets, cap, wts, (float*)y, N, top, (const float*)extra, extra_gate, ldg);
-    else moe_combine_kernel<bf16><<<T, 256, 0, stream>>>((const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg);
-    return tl_launch_status();
+    if (act_dtype == TL_F32) return launch_after_wait(moe_combine_kernel<float>, dim3(T), dim3(256), 0, stream, (const float*)rows, place_of, idx, offsets, cap,
+                                                      wts, (float*)y, N, top, (const float*)extra, extra_gate, ldg, E_real, (const float*)same);
+    return launch_after_wait(moe_combine_kernel<bf16>, dim3(T), dim3(256), 0, stream, (const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top,
+                             (const bf16*)extra, extra_gate, ldg, E_real, (const bf16*)same);
 }

@@ -1,7 +1,7 @@
 // Device helpers of the kernels in which two thread blocks of a cluster work on one tile (tcgen05 cta_group::2).
 //
-// MMAs and commits are issued by a whole warp, the instruction itself predicated on one elected lane (`one`): their operands are then
-// uniform registers from the start.  Issued from a branch that only one thread takes, every MMA took that thread 61 cycles; so 27.
+// MMAs, commits and copies are issued by a whole warp, the instruction itself predicated on one elected lane (`one`): their operands are
+// then uniform registers from the start.  Issued from a branch that only one thread takes, every MMA took that thread 61 cycles; so 27.
 // Barriers are waited for and arrived at with the default order (this block's): a release at the cluster's scope waits for memory,
 // more than 1,000 cycles a time, and what the pair hands over (tensor memory, shared memory read by an MMA) is ordered by tcgen05's own fences and commits.
 #pragma once
@@ -25,9 +25,17 @@ __device__ __forceinline__ void pair_arrive(uint32_t cluster_address) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_address) : "memory");
 }
 // a box by TMA (no multicast) into this block's shared memory; its bytes count on `bar`, which may be the peer's barrier
-__device__ __forceinline__ void pair_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1) : "memory");
+__device__ __forceinline__ void pair_load(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, uint32_t one) {
+    asm volatile("{\n\t.reg .pred q;\n\t"
+                 "setp.ne.b32 q, %5, 0;\n\t"
+                 "@q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(one) : "memory");
+}
+__device__ __forceinline__ void pair_expect(uint64_t* bar, uint32_t bytes, uint32_t one) {
+    asm volatile("{\n\t.reg .pred q;\n\t"
+                 "setp.ne.b32 q, %2, 0;\n\t"
+                 "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}"
+                 ::"r"(smem_addr(bar)), "r"(bytes), "r"(one) : "memory");
 }
 __device__ __forceinline__ void pair_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t one) {
     asm volatile("{\n\t.reg .pred p, q;\n\t"

@@ -18,7 +18,7 @@ from .csrc.build import CHECK_BUILD, load_library
 
 CORE_SOURCES = ["elementwise.cu", "rope_kv.cu", "attn_tokenwise.cu", "gemm_f32.cu", "sampling.cu", "recurrent.cu", "moe.cu",
                 "delta.cu", "latent.cu", "rglru.cu", "streams.cu", "stream_norm.cu", "attn_mixed_tokenwise.cu",
-                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu", "delta_chunk.cu", "gemm_f32_parts.cu"]
+                "channel_scan.cu", "differential.cu", "attn_rows_f32.cu", "linear_chunk.cu", "delta_chunk.cu", "gemm_f32_parts.cu", "moe_product.cu"]
 
 _P, _I, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
 
@@ -63,7 +63,9 @@ _SIGNATURES = {
     "tl_moe_gather": [_P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _P],
     "tl_relu_square": [_P, _I, ctypes.c_longlong, _P],
     "tl_gelu": [_P, _I, ctypes.c_longlong, _P],
-    "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _P],
+    "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _I, _P, _P],
+    "tl_moe_product": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
+    "tl_moe_product_takes": [_I, _I, _I, _I],
     "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
     "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
@@ -167,6 +169,8 @@ STATUS_ROLES = {1: "tcgen05 product: the copy thread waited for a free stage", 2
                 33: "two-block product: the MMA thread waited for a stage's copies", 34: "two-block product: the epilogue waited for the accumulator",
                 41: "32-bit product: a copy thread waited for a free stage", 42: "32-bit product: the MMA thread waited for a free accumulator",
                 43: "32-bit product: the MMA thread waited for a stage's copies", 44: "32-bit product: the sums waited for an accumulator",
+                45: "experts' product: a copy thread waited for a free stage", 46: "experts' product: the MMA thread waited for a free accumulator",
+                47: "experts' product: the MMA thread waited for a stage's copies", 48: "experts' product: the epilogue waited for the accumulator",
                 20: "decode attention: a wait for a stage of keys and values"}
 
 
@@ -1129,6 +1133,38 @@ def moe_gather(h: torch.Tensor, pair_at: torch.Tensor, idx: torch.Tensor, offset
                                 int(top), _ptr(scale), _stream()), "moe_gather")
 
 
+def moe_product_takes(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, gated: bool) -> bool:
+    """Whether both products of these experts ([E, F or 2F, K] and [E, K, F]) run as `moe_product`."""
+    E, N, F = w_down.shape
+    takes = core().tl_moe_product_takes
+    return (h.dtype == w_up.dtype == w_down.dtype == torch.bfloat16 and bool(takes(E, w_up.shape[2], F, int(gated))) and bool(takes(E, F, N, 0))
+            and not (w_up.data_ptr() | w_down.data_ptr()) & 15)
+
+
+def moe_product(rows: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, act=None, gated: bool = False) -> None:
+    """out[p] = the rows p of expert e's run (offsets[e] .. offsets[e + 1] - 1, int32 on the device; e < E) times w[e] ([E, R, K])^T.
+    `gated`: w's rows are an expert's gate rows, then its up rows, and out = act(gate) * up, both rounded to bfloat16 first;
+    else `act` None or "relu_squared".  Rows of `out` in no run are left alone."""
+    E, R, K = w.shape
+    P = rows.shape[0]
+    cols = R // 2 if gated else R
+    if rows.shape != (P, K) or out.shape != (P, cols) or offsets.numel() < E + 1 or not (rows.dtype == w.dtype == out.dtype == torch.bfloat16):
+        raise KernelError("moe_product: rows [P, K], w [E, R, K], out [P, R] ([P, R / 2] gated), bfloat16; offsets [>= E + 1]")
+    _contig(rows, "rows"); _contig(w, "w"); _contig(out, "out"); _ints(offsets, "offsets")
+    kind, limit, alpha = 0, 0.0, 1.0
+    if gated:
+        code, limit, alpha = gate_act(act)
+        kind = {0: 1, 1: 2, 3: 3}.get(code, 0)
+        if not kind:
+            raise KernelError(f"moe_product: no gate {act!r}")
+    elif act == "relu_squared":
+        kind = 4
+    elif act is not None:
+        raise KernelError(f"moe_product: without a gate 'relu_squared' or nothing, not {act!r}")
+    _check(core().tl_moe_product(_ptr(rows), _ptr(w), _ptr(offsets), _ptr(out), out.stride(0), P, E, R, K, kind, limit, alpha,
+                                 _ptr(device_status(rows.device)), _stream()), "moe_product")
+
+
 def relu_square(u: torch.Tensor) -> None:
     """u = relu(u)^2 in place."""
     _contig(u, "u")
@@ -1142,9 +1178,10 @@ def gelu(u: torch.Tensor) -> None:
 
 
 def moe_combine(rows: torch.Tensor, place_of: torch.Tensor, idx: torch.Tensor, offsets: torch.Tensor, wts: torch.Tensor | None,
-                y: torch.Tensor, cap: int = 0, extra: torch.Tensor | None = None, extra_gate: torch.Tensor | None = None) -> None:
+                y: torch.Tensor, cap: int = 0, extra: torch.Tensor | None = None, extra_gate: torch.Tensor | None = None,
+                same: torch.Tensor | None = None, real: int = 0) -> None:
     """y[t] = sum_j wts[t, j] * rows[row of place_of[t * top + j]] (+ sigmoid(extra_gate[t]) * extra[t]); rows laid out as
-    `moe_gather` lays them out; wts None: an unweighted sum."""
+    `moe_gather` lays them out; wts None: an unweighted sum.  `same` ([T, N] of y's type): an entry idx >= `real` counts with same[t]."""
     T, top = idx.shape
     N = y.shape[1]
     E = offsets.numel() - 1
@@ -1153,8 +1190,10 @@ def moe_combine(rows: torch.Tensor, place_of: torch.Tensor, idx: torch.Tensor, o
         raise KernelError("moe_combine: rows [T top, N] (or [E cap, N]) of y's type, wts float32 [T, top]")
     _contig(rows, "rows"); _ints(place_of, "place_of"); _ints(idx, "idx"); _ints(offsets, "offsets"); _contig(y, "y")
     g_ptr, ldg = _extra(extra, extra_gate, y, "moe_combine")
+    if same is not None and (same.shape != y.shape or same.dtype != y.dtype or not same.is_contiguous()):
+        raise KernelError("moe_combine: the identity entries' rows must have y's shape and type")
     _check(core().tl_moe_combine(_ptr(rows), dtype_code(rows.dtype), _ptr(place_of), _ptr(idx), _ptr(offsets), int(cap), _ptr(wts),
-                                 _ptr(y), T, N, top, _ptr(extra), g_ptr, ldg, _stream()), "moe_combine")
+                                 _ptr(y), T, N, top, _ptr(extra), g_ptr, ldg, int(real), _ptr(same), _stream()), "moe_combine")
 
 
 # ---------------------------------------------------------------------------------------------

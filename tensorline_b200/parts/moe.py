@@ -24,9 +24,10 @@ that stand for no matrices: an identity entry's output is the token's input itse
 The experts' matrices are stacked ([E, F, K] and [E, K, F]) at load time.  Steps of few tokens stream, for every
 (token, chosen expert) pair, that expert's rows (`ops.moe_up`, `ops.moe_down`): nothing is sorted and nothing comes
 back to the host, so the step sits in a CUDA graph.  Steps of many tokens sort the pairs by expert on the device,
-gather the tokens' rows in that order, every expert's run into `cap` rows of its own (the longest run, rounded up), and
-run two batched dense products over all experts (the library's, as the engine's other long products are), which needs
-the runs' bounds on the host.  The 32-bit engine streams always: a token's result is then the
+gather the tokens' rows in that order and run two products over the experts' runs (`ops.moe_product`, which reads the runs'
+bounds on the device).  Rows that are no multiple of 16 bytes take two batched products of the library instead, every
+expert's run in `cap` rows of its own (the longest run, rounded up), which needs the bounds on the host.  The 32-bit
+engine streams always: a token's result is then the
 same chain of additions in every step, whatever else the step holds.
 """
 from __future__ import annotations
@@ -156,22 +157,31 @@ class RoutedExperts(Part):
                          same=h if self.E_real < E else None)
             return y
         offsets, place_of, pair_at = ops.moe_sort(idx, E)
+        if not self.gated and self.activation != "relu_squared":
+            raise NotImplementedError(f"long steps of experts without a gate run 'relu_squared', not {self.activation!r}")
+        R = self.E_real                                  # the entries behind it are identities: their rows pass as they are
+        if ops.moe_product_takes(h, self.w_up, self.w_down, self.gated):
+            rows = torch.empty((T * top, self.hidden), dtype=h.dtype, device=h.device)
+            ops.moe_gather(h, pair_at, idx, offsets, top, rows, scale=wts.view(-1) if on_input else None)
+            inner = torch.empty((T * top, self.inner), dtype=h.dtype, device=h.device)
+            ops.moe_product(rows, self.w_up, offsets, inner, act=self.act, gated=self.gated)
+            ops.moe_product(inner, self.w_down, offsets, rows)           # the gathered rows are read: their buffer takes the results
+            ops.moe_combine(rows, place_of, idx, offsets, None if on_input else wts, y, extra=extra, extra_gate=extra_gate,
+                            same=h if R < E else None, real=R)
+            return y
         bounds = offsets.tolist()                        # the one read-back of the step: where every expert's run ends
         longest = max(bounds[e + 1] - bounds[e] for e in range(E))
         cap = -(-longest // 64) * 64                     # rows every expert gets in the batched products
         rows = torch.empty((E * cap, self.hidden), dtype=h.dtype, device=h.device)
         ops.moe_gather(h, pair_at, idx, offsets, top, rows, cap=cap, scale=wts.view(-1) if on_input else None)
-        R = self.E_real                                  # the entries behind it are identities: their rows pass as they are
         inner = torch.bmm(rows.view(E, cap, self.hidden)[:R], self.w_up.transpose(1, 2))         # [R, cap, F] or [R, cap, 2F]
         ops.mark("library product")
         if self.gated:
             act = torch.empty((R * cap, self.inner), dtype=h.dtype, device=h.device)
             ops.silu_mul(inner.view(R * cap, 2 * self.inner), act, act=self.act)
             inner = act.view(R, cap, self.inner)
-        elif self.activation == "relu_squared":
-            ops.relu_square(inner)
         else:
-            raise NotImplementedError(f"long steps of experts without a gate run 'relu_squared', not {self.activation!r}")
+            ops.relu_square(inner)
         if R < E:
             outs = torch.empty((E, cap, self.hidden), dtype=h.dtype, device=h.device)
             torch.bmm(inner, self.w_down.transpose(1, 2), out=outs[:R])

@@ -1,0 +1,88 @@
+"""The experts' products of long steps at the edges of their tiles: empty runs, runs around a tile's width, matrices that end inside a
+tile, every epilogue; against float64 sums of the same bfloat16 values.  Bounds: a result is rounded once to bfloat16 (2^-9 of it),
+behind a gate both factors are rounded first (2^-9 each, and once more where a sum in another order falls on the other side); a
+float sum of K products is off by less than K 2^-23 times the sum of the absolute products."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tensorline_b200 import ops
+    return ops
+
+
+RUNS = [[5], [0, 1, 0, 17, 31, 33, 0], [256, 257, 3, 0, 512, 513, 64], [1] * 40, [300, 0, 40], [2, 0, 1031, 255]]
+
+
+@pytest.mark.parametrize("runs", RUNS)
+@pytest.mark.parametrize("K,F", [(64, 64), (200, 80), (1032, 336)])
+@pytest.mark.parametrize("kind", ["plain", "relu_squared", "silu", "gelu_tanh", "swish_clamped"])
+def test_runs_of_rows_times_their_own_matrices(ops, runs, K, F, kind):
+    g = torch.Generator().manual_seed(len(runs) * K + F)
+    E, P = len(runs), sum(runs) + 3                      # rows behind the last run (identity entries) are left alone
+    gated = kind not in ("plain", "relu_squared")
+    R = 2 * F if gated else F
+    x = torch.randn(P, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(E, R, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    offsets = torch.tensor([0] + torch.tensor(runs).cumsum(0).tolist() + [P], dtype=torch.int32).cuda()
+    out = torch.full((P, F), 7.0, dtype=torch.bfloat16, device="cuda")
+    act = ("swish_clamped", 1.5, 1.7) if kind == "swish_clamped" else None if kind == "plain" else kind
+    ops.moe_product(x, w, offsets, out, act=act, gated=gated)
+    ops.check_device_status()
+    assert bool((out[P - 3:] == 7.0).all())
+    at = 0
+    for e, n in enumerate(runs):
+        if n == 0:
+            continue
+        xe, we = x[at:at + n].double(), w[e].double()
+        z, size = xe @ we.T, xe.abs() @ we.abs().T * K * 2.0 ** -23
+        got = out[at:at + n].double()
+        if kind == "plain":
+            assert bool(((got - z).abs() <= z.abs() * 2.0 ** -8 + 2 * size).all())
+        elif kind == "relu_squared":
+            want = z.clamp_min(0) ** 2
+            assert bool(((got - want).abs() <= want * 4 * 2.0 ** -8 + 4 * z.abs() * size + size).all())
+        else:
+            a, b = z[:, :F], z[:, F:]
+            da, db = a.abs() * 2.0 ** -8 + 2 * size[:, :F], b.abs() * 2.0 ** -8 + 2 * size[:, F:]
+            if kind == "swish_clamped":
+                ga = a.clamp_max(1.5)
+                f, u = ga * torch.sigmoid(1.7 * ga), b.clamp(-1.5, 1.5) + 1.0
+            else:
+                f, u = a * torch.sigmoid(a) if kind == "silu" else torch.nn.functional.gelu(a, approximate="tanh"), b
+            want = f * u                                 # the gates' slopes are below 1.2
+            assert bool(((got - want).abs() <= 1.2 * da * u.abs() + f.abs() * db + 1.2 * da * db + want.abs() * 2.0 ** -8 + 1e-6).all())
+        at += n
+
+
+def test_columns_that_are_no_multiple_of_anything(ops):
+    g = torch.Generator().manual_seed(2)
+    x, w = torch.randn(70, 72, generator=g).to(torch.bfloat16).cuda(), torch.randn(2, 133, 72, generator=g).to(torch.bfloat16).cuda()
+    out = torch.empty(70, 133, dtype=torch.bfloat16, device="cuda")
+    ops.moe_product(x, w, torch.tensor([0, 37, 70], dtype=torch.int32).cuda(), out)
+    want = torch.cat([x[:37].double() @ w[0].double().T, x[37:].double() @ w[1].double().T])
+    assert bool(((out.double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-3).all())
+    assert not ops.core().tl_moe_product_takes(2, 72, 133, 1) and not ops.core().tl_moe_product_takes(2, 71, 133, 0)
+
+
+@pytest.mark.parametrize("gated,shared,on_input", [(True, True, False), (False, False, False), (True, False, True)])
+def test_long_steps_agree_with_streamed_experts(ops, gated, shared, on_input, monkeypatch):
+    """A step through the sorted runs and the same step token by token: roundings to bfloat16 in between are all that differs."""
+    from tensorline_b200.parts import FEED_FORWARDS, PartSpec, Runtime
+    from tensorline_b200.parts import moe
+    from types import SimpleNamespace
+    part = FEED_FORWARDS.build(PartSpec("routed_experts", dict(hidden=256, inner=192, experts=6, top=3, gated=gated, router_bias=False,
+                                                               activation="silu" if gated else "relu_squared", shared_inner=192 if shared else None,
+                                                               weight_on="input" if on_input else "output")), Runtime(torch.device("cuda", 0), torch.bfloat16, 16))
+    g = torch.Generator().manual_seed(1)
+    part.bind({n: (torch.randn(s.shape, generator=g) * 0.08).to(torch.bfloat16).cuda() for n, s in part.expected_tensors("l").items()}, "l")
+    h = torch.randn(77, 256, generator=g).to(torch.bfloat16).cuda()
+    ctx = SimpleNamespace(graph_max_ctx=0)
+    long = part.forward(h, ctx)
+    monkeypatch.setattr(moe, "STREAM_MAX_TOKENS", 100)
+    short = part.forward(h, ctx)
+    ops.check_device_status()
+    assert float((long.float() - short.float()).norm() / short.float().norm()) <= 2.0 ** -7      # three roundings of 2^-9 each way
