@@ -800,9 +800,9 @@ TL_EXPORT int tl_relu_square(void* u, int act_dtype, long long n, cudaStream_t s
 }
 
 // y[t, :] = sum_j wts[t, j] * rows[row of place_of[t * top + j], :], j in the order chosen; an entry idx >= E_real has no row: it
-// counts with same[t, :]
-template <typename TA>
-__global__ void moe_combine_kernel(const TA* __restrict__ rows, const int* __restrict__ place_of, const int* __restrict__ idx,
+// counts with same[t, :].  TR: the rows' type
+template <typename TR, typename TA>
+__global__ void moe_combine_kernel(const TR* __restrict__ rows, const int* __restrict__ place_of, const int* __restrict__ idx,
                                    const int* __restrict__ offsets, int cap, const float* __restrict__ wts,
                                    TA* __restrict__ y, int N, int top, const TA* __restrict__ extra,
                                    const float* __restrict__ extra_gate, int ldg, int E_real, const TA* __restrict__ same) {
@@ -814,7 +814,8 @@ __global__ void moe_combine_kernel(const TA* __restrict__ rows, const int* __res
         float acc = 0.f;
         for (int j = 0; j < top; ++j) {
             const size_t pair = (size_t)t * top + j;
-            const float v = to_f<TA>(idx[pair] >= E_real ? same[(size_t)t * N + n] : rows[moe_row(place_of[pair], idx[pair], offsets, cap) * N + n]);
+            const float v = idx[pair] >= E_real ? to_f<TA>(same[(size_t)t * N + n])
+                                                : to_f<TR>(rows[moe_row(place_of[pair], idx[pair], offsets, cap) * N + n]);
             acc = wts ? fmaf(wts[pair], v, acc) : acc + v;
         }
         if (extra) acc = fmaf(gt, to_f<TA>(extra[(size_t)t * N + n]), acc);
@@ -880,19 +881,22 @@ __global__ void __launch_bounds__(256) moe_combine_vec_kernel(const bf16* __rest
     }
 }
 
-TL_EXPORT int tl_moe_combine(const void* rows, int act_dtype, const int* place_of, const int* idx, const int* offsets, int cap,
+TL_EXPORT int tl_moe_combine(const void* rows, int rows_dtype, int act_dtype, const int* place_of, const int* idx, const int* offsets, int cap,
                              const float* wts, void* y, int T, int N, int top, const void* extra, const float* extra_gate, int ldg,
                              int E_real, const void* same, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (!same) E_real = 0x7fffffff;                      // every entry has a row
-    if (act_dtype != TL_F32 && N % 8 == 0 && N >= COMBINE_VEC && top <= 32 &&
+    if (rows_dtype != act_dtype && rows_dtype != TL_F32) return 1;
+    if (act_dtype != TL_F32 && rows_dtype != TL_F32 && N % 8 == 0 && N >= COMBINE_VEC && top <= 32 &&
         ((((uintptr_t)rows) | ((uintptr_t)y) | ((uintptr_t)extra) | ((uintptr_t)same)) & 15) == 0) {
         const int pieces = (N / 8 + 31) / 32 * 32;
         return launch_after_wait(moe_combine_vec_kernel, dim3(T), dim3(pieces < 256 ? pieces : 256), 0, stream, (const bf16*)rows, place_of, idx, offsets,
                                  cap, wts, (bf16*)y, N, top, (const bf16*)extra, extra_gate, ldg, E_real, (const bf16*)same);
     }
-    if (act_dtype == TL_F32) return launch_after_wait(moe_combine_kernel<float>, dim3(T), dim3(256), 0, stream, (const float*)rows, place_of, idx, offsets, cap,
-                                                      wts, (float*)y, N, top, (const float*)extra, extra_gate, ldg, E_real, (const float*)same);
-    return launch_after_wait(moe_combine_kernel<bf16>, dim3(T), dim3(256), 0, stream, (const bf16*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, top,
-                             (const bf16*)extra, extra_gate, ldg, E_real, (const bf16*)same);
+    if (act_dtype == TL_F32) return launch_after_wait(moe_combine_kernel<float, float>, dim3(T), dim3(256), 0, stream, (const float*)rows, place_of, idx, offsets,
+                                                      cap, wts, (float*)y, N, top, (const float*)extra, extra_gate, ldg, E_real, (const float*)same);
+#define COMBINE(TR) launch_after_wait(moe_combine_kernel<TR, bf16>, dim3(T), dim3(256), 0, stream, (const TR*)rows, place_of, idx, offsets, cap, wts, (bf16*)y, N, \
+                                      top, (const bf16*)extra, extra_gate, ldg, E_real, (const bf16*)same)
+    return rows_dtype == TL_F32 ? COMBINE(float) : COMBINE(bf16);
+#undef COMBINE
 }

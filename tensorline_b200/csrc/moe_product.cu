@@ -29,7 +29,7 @@ constexpr int MP_MAX_E = 1024;
 constexpr int MP_SMEM = MP_STAGES * MP_STAGE + 2 * (MP_MAX_E + 1) * 4 + 1024 + 256;
 
 struct MoeProductArgs {
-    bf16* out; int ldo;                                  // [P, ldo]
+    void* out; int ldo;                                  // [P, ldo] bfloat16 (KIND 8: float)
     const int* offsets; int E;                           // [E + 1]: expert e's run of rows
     int R, K;                                            // rows of an expert's matrix in memory, and their length
     int cols;                                            // columns of out: R, gated R / 2
@@ -66,8 +66,10 @@ __device__ __forceinline__ void moe_load5(uint32_t dst, const CUtensorMap* map, 
                  ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(group), "r"(e), "r"(one), "r"(0) : "memory");
 }
 
-// KIND 0: as it is, 1..3: gates (tl_gate_mul), 4: relu(.)^2.  A parameter of the kernel: with the choice inside the loop over a
-// thread's elements their chains did not overlap.
+// KIND 0: as it is, 1..3: gates (tl_gate_mul), 4: relu(.)^2, each of values rounded to bfloat16 first, as a stored product would have been.
+// Eight more: of the accumulators themselves, and 8 as floats (what streamed experts compute).  A parameter of the kernel: with
+// the choice inside the loop over a thread's elements their chains did not overlap.
+__device__ __forceinline__ float moe_rounded(float v, bool raw) { return raw ? v : __bfloat162float(__float2bfloat16_rn(v)); }
 template <int KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MP_THREADS, 1)
 moe_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_tall,
@@ -86,7 +88,7 @@ moe_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const uint32_t rank = pair_rank();
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, chunks = (G.K + MP_CHUNK - 1) / MP_CHUNK;
-    constexpr bool gated = KIND >= 1 && KIND <= 3;
+    constexpr bool raw = KIND >= 8, gated = KIND % 8 >= 1 && KIND % 8 <= 3;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < MP_STAGES; ++s) { mbar_init(full_bar + s, 1); mbar_init(empty_bar + s, 1); }
@@ -194,21 +196,29 @@ moe_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const float give = up ? r[j] : r[8 + j], keep = up ? r[8 + j] : r[j];
-                        const float a = __bfloat162float(__float2bfloat16_rn(keep));
-                        const float b = __bfloat162float(__float2bfloat16_rn(__shfl_xor_sync(0xffffffffu, give, 16)));
-                        y[j] = tl_gate_mul(up ? b : a, up ? a : b, KIND, G.limit, G.alpha);
+                        const float a = moe_rounded(keep, raw), b = moe_rounded(__shfl_xor_sync(0xffffffffu, give, 16), raw);
+                        y[j] = tl_gate_mul(up ? b : a, up ? a : b, KIND % 8, G.limit, G.alpha);
                     }
                     if (col < G.cols) {
-                        bf16* dst = G.out + (size_t)(t.row + c0 + (up ? 8 : 0)) * G.ldo + col;
+                        bf16* dst = (bf16*)G.out + (size_t)(t.row + c0 + (up ? 8 : 0)) * G.ldo + col;
 #pragma unroll
                         for (int j = 0; j < 8; ++j, dst += G.ldo) if (j < left) *dst = __float2bfloat16_rn(y[j]);
                     }
                 } else if (col < G.cols) {
                     const int left = t.rows - c0;
-                    bf16* dst = G.out + (size_t)(t.row + c0) * G.ldo + col;
+                    const size_t at = (size_t)(t.row + c0) * G.ldo + col;
+                    if (KIND == 8) {
+                        float* dst = (float*)G.out + at;
 #pragma unroll
-                    for (int j = 0; j < 16; ++j, dst += G.ldo)
-                        if (j < left) *dst = __float2bfloat16_rn(KIND == 4 ? tl_relu_squared_rounded(r[j]) : r[j]);
+                        for (int j = 0; j < 16; ++j, dst += G.ldo) if (j < left) *dst = r[j];
+                    } else {
+                        bf16* dst = (bf16*)G.out + at;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j, dst += G.ldo) {
+                            const float v = KIND == 12 ? fmaxf(r[j], 0.f) * fmaxf(r[j], 0.f) : KIND == 4 ? tl_relu_squared_rounded(r[j]) : r[j];
+                            if (j < left) *dst = __float2bfloat16_rn(v);
+                        }
+                    }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -259,13 +269,13 @@ TL_EXPORT int tl_moe_product_takes(int E, int K, int cols, int gated) {
 }
 
 // out[p, :] = rows p = offsets[e] .. offsets[e + 1] - 1 of x [P, K] times w[e] [R, K]^T, e = 0 .. E - 1, through `kind` (see the
-// kernel).  x, w and out bfloat16, x and w 16-byte aligned; out [P, cols], rows ldo elements apart.
+// kernel).  x, w and out (kind 8: float) bfloat16, x and w 16-byte aligned; out [P, cols], rows ldo elements apart.
 TL_EXPORT int tl_moe_product(const void* x, const void* w, const int* offsets, void* out, int ldo, int P, int E, int R, int K, int kind,
                              float limit, float alpha, int* status, cudaStream_t stream) {
     if (P <= 0) return 0;
-    const bool gated = kind >= 1 && kind <= 3;
+    const bool gated = kind % 8 >= 1 && kind % 8 <= 3;
     const int cols = gated ? R / 2 : R;
-    if (kind < 0 || kind > 4 || (gated && R % 2) || !tl_moe_product_takes(E, K, cols, gated) || (long long)E * R > 2147483647LL ||
+    if (kind < 0 || kind > 12 || kind % 8 > 4 || (gated && R % 2) || !tl_moe_product_takes(E, K, cols, gated) || (long long)E * R > 2147483647LL ||
         ((((uintptr_t)x) | ((uintptr_t)w)) & 15) || status == nullptr) return 1;
     int e = load_encode();
     if (e) return e;
@@ -273,12 +283,17 @@ TL_EXPORT int tl_moe_product(const void* x, const void* w, const int* offsets, v
     if ((e = gated ? gated_map(&mw, w, E, cols, K) : pair_map(&mw, w, (long long)E * R, K, MP_ROWS))) return e;
     if ((e = pair_map(&mx, x, P, K, MP_BOX))) return e;
     if ((e = pair_map(&mt, x, P, K, MP_TALL))) return e;
-    const MoeProductArgs G{(bf16*)out, ldo, offsets, E, R, K, cols, gated ? (cols + 127) / 128 : (cols + 255) / 256, limit, alpha, status};
+    const MoeProductArgs G{out, ldo, offsets, E, R, K, cols, gated ? (cols + 127) / 128 : (cols + 255) / 256, limit, alpha, status};
     switch (kind) {
         case 0: return launch_product<0>(mw, mx, mt, G, P, stream);
         case 1: return launch_product<1>(mw, mx, mt, G, P, stream);
         case 2: return launch_product<2>(mw, mx, mt, G, P, stream);
         case 3: return launch_product<3>(mw, mx, mt, G, P, stream);
-        default: return launch_product<4>(mw, mx, mt, G, P, stream);
+        case 4: return launch_product<4>(mw, mx, mt, G, P, stream);
+        case 8: return launch_product<8>(mw, mx, mt, G, P, stream);
+        case 9: return launch_product<9>(mw, mx, mt, G, P, stream);
+        case 10: return launch_product<10>(mw, mx, mt, G, P, stream);
+        case 11: return launch_product<11>(mw, mx, mt, G, P, stream);
+        default: return launch_product<12>(mw, mx, mt, G, P, stream);
     }
 }

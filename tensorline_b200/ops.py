@@ -63,7 +63,7 @@ _SIGNATURES = {
     "tl_moe_gather": [_P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _P],
     "tl_relu_square": [_P, _I, ctypes.c_longlong, _P],
     "tl_gelu": [_P, _I, ctypes.c_longlong, _P],
-    "tl_moe_combine": [_P, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _I, _P, _P],
+    "tl_moe_combine": [_P, _I, _I, _P, _P, _P, _I, _P, _P, _I, _I, _I, _P, _P, _I, _I, _P, _P],
     "tl_moe_product": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P, _P],
     "tl_moe_product_takes": [_I, _I, _I, _I],
     "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
@@ -1141,14 +1141,18 @@ def moe_product_takes(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor,
             and not (w_up.data_ptr() | w_down.data_ptr()) & 15)
 
 
-def moe_product(rows: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, act=None, gated: bool = False) -> None:
+def moe_product(rows: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor, act=None, gated: bool = False,
+                raw: bool = False) -> None:
     """out[p] = the rows p of expert e's run (offsets[e] .. offsets[e + 1] - 1, int32 on the device; e < E) times w[e] ([E, R, K])^T.
     `gated`: w's rows are an expert's gate rows, then its up rows, and out = act(gate) * up, both rounded to bfloat16 first;
-    else `act` None or "relu_squared".  Rows of `out` in no run are left alone."""
+    else `act` None or "relu_squared".  Rows of `out` in no run are left alone.  `raw`: the activation takes the float sums as they are,
+    and without one `out` is float32."""
     E, R, K = w.shape
     P = rows.shape[0]
     cols = R // 2 if gated else R
-    if rows.shape != (P, K) or out.shape != (P, cols) or offsets.numel() < E + 1 or not (rows.dtype == w.dtype == out.dtype == torch.bfloat16):
+    floats = raw and not gated and act is None
+    if rows.shape != (P, K) or out.shape != (P, cols) or offsets.numel() < E + 1 or not (rows.dtype == w.dtype == torch.bfloat16) or \
+            out.dtype != (torch.float32 if floats else torch.bfloat16):
         raise KernelError("moe_product: rows [P, K], w [E, R, K], out [P, R] ([P, R / 2] gated), bfloat16; offsets [>= E + 1]")
     _contig(rows, "rows"); _contig(w, "w"); _contig(out, "out"); _ints(offsets, "offsets")
     kind, limit, alpha = 0, 0.0, 1.0
@@ -1161,7 +1165,7 @@ def moe_product(rows: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, out:
         kind = 4
     elif act is not None:
         raise KernelError(f"moe_product: without a gate 'relu_squared' or nothing, not {act!r}")
-    _check(core().tl_moe_product(_ptr(rows), _ptr(w), _ptr(offsets), _ptr(out), out.stride(0), P, E, R, K, kind, limit, alpha,
+    _check(core().tl_moe_product(_ptr(rows), _ptr(w), _ptr(offsets), _ptr(out), out.stride(0), P, E, R, K, kind + 8 * raw, limit, alpha,
                                  _ptr(device_status(rows.device)), _stream()), "moe_product")
 
 
@@ -1185,14 +1189,14 @@ def moe_combine(rows: torch.Tensor, place_of: torch.Tensor, idx: torch.Tensor, o
     T, top = idx.shape
     N = y.shape[1]
     E = offsets.numel() - 1
-    if rows.shape != ((E * cap if cap else T * top), N) or rows.dtype != y.dtype or y.shape[0] != T or \
+    if rows.shape != ((E * cap if cap else T * top), N) or rows.dtype not in (y.dtype, torch.float32) or y.shape[0] != T or \
             (wts is not None and (wts.dtype != torch.float32 or wts.shape != idx.shape or not wts.is_contiguous())):
-        raise KernelError("moe_combine: rows [T top, N] (or [E cap, N]) of y's type, wts float32 [T, top]")
+        raise KernelError("moe_combine: rows [T top, N] (or [E cap, N]) of y's type or float32, wts float32 [T, top]")
     _contig(rows, "rows"); _ints(place_of, "place_of"); _ints(idx, "idx"); _ints(offsets, "offsets"); _contig(y, "y")
     g_ptr, ldg = _extra(extra, extra_gate, y, "moe_combine")
     if same is not None and (same.shape != y.shape or same.dtype != y.dtype or not same.is_contiguous()):
         raise KernelError("moe_combine: the identity entries' rows must have y's shape and type")
-    _check(core().tl_moe_combine(_ptr(rows), dtype_code(rows.dtype), _ptr(place_of), _ptr(idx), _ptr(offsets), int(cap), _ptr(wts),
+    _check(core().tl_moe_combine(_ptr(rows), dtype_code(rows.dtype), dtype_code(y.dtype), _ptr(place_of), _ptr(idx), _ptr(offsets), int(cap), _ptr(wts),
                                  _ptr(y), T, N, top, _ptr(extra), g_ptr, ldg, int(real), _ptr(same), _stream()), "moe_combine")
 
 

@@ -22,11 +22,12 @@ with s = softmax(z) over all entries of the router.  `identity`: the router has 
 that stand for no matrices: an identity entry's output is the token's input itself (times its weight).
 
 The experts' matrices are stacked ([E, F, K] and [E, K, F]) at load time.  Steps of few tokens stream, for every
-(token, chosen expert) pair, that expert's rows (`ops.moe_up`, `ops.moe_down`): nothing is sorted and nothing comes
-back to the host, so the step sits in a CUDA graph.  Steps of many tokens sort the pairs by expert on the device,
+(token, chosen expert) pair, that expert's rows (`ops.moe_up`, `ops.moe_down`): nothing is sorted.  Steps of many tokens (or of
+so many pairs that the same matrices would be streamed again and again, `sort_pays`) sort the pairs by expert on the device,
 gather the tokens' rows in that order and run two products over the experts' runs (`ops.moe_product`, which reads the runs'
-bounds on the device).  Rows that are no multiple of 16 bytes take two batched products of the library instead, every
-expert's run in `cap` rows of its own (the longest run, rounded up), which needs the bounds on the host.  The 32-bit
+bounds on the device).  Neither asks the host for anything, so both sit in a CUDA graph.  Rows that are no multiple of 16 bytes
+take two batched products of the library instead, every expert's run in `cap` rows of its own (the longest run, rounded up),
+which needs the bounds on the host; captured steps stream then.  The 32-bit
 engine streams always: a token's result is then the
 same chain of additions in every step, whatever else the step holds.
 """
@@ -40,13 +41,24 @@ from .. import ops
 from .base import Part, Runtime, TensorSpec, register_feed_forward
 from .linear import resolve
 
-# up to this many tokens a step the experts are streamed pair by pair
+# up to this many tokens a step the experts are streamed pair by pair ...
 STREAM_MAX_TOKENS = int(os.environ.get("TENSORLINE_B200_MOE_STREAM_MAX_TOKENS", 32))
+# ... as long as the pairs are not many more than the experts they chose: every pair brings its expert's matrices anew (from L2 at
+# about 10 TB/s), the products over sorted runs once, at 4.5 TB/s against 5.5, with 14 us of launches.  Experts of
+# 2,048 x 1,024, gated, 4 of 32 a token, streamed / sorted: 12 tokens 101 / 104 us, 16 115 / 115, 32 182 / 117; 2 of 8: 8 tokens
+# 43 / 45, 12 55 / 45, 32 111 / 47; 1,024 x 512, 4 of 32: 16 tokens 41 / 47, 24 53 / 47, 32 61 / 47.
+SORT_MIN_BYTES, SORT_SHARE = 140e6, 0.4
+
+
+def sort_pays(tokens: int, top: int, experts: int, expert_bytes: int) -> bool:
+    """Whether a step of few tokens moves enough bytes more than once to be sorted."""
+    chosen = experts * (1.0 - (1.0 - top / experts) ** tokens)               # experts that some token chose, on average
+    return (tokens * top - chosen) * expert_bytes >= SORT_MIN_BYTES + SORT_SHARE * chosen * expert_bytes
 
 
 @register_feed_forward("routed_experts")
 class RoutedExperts(Part):
-    graph_capturable = True              # a captured step streams the experts whatever its size (see forward)
+    graph_capturable = True              # a captured step never asks the host for the runs' bounds (see forward)
 
     def __init__(self, rt: Runtime, hidden: int, inner: int, experts: int, top: int, activation: str = "relu_squared",
                  router_bias: bool = True, names: dict | None = None, gated: bool = False, scoring: str = "softmax_chosen",
@@ -150,7 +162,13 @@ class RoutedExperts(Part):
             extra, extra_gate = resolve(self.shared.forward(h, ctx)), (z[:, E] if self.shared_gate else None)
         on_input = self.weight_on == "input"
         y = torch.empty((T, self.hidden), dtype=h.dtype, device=h.device)
-        if T <= STREAM_MAX_TOKENS or ctx.graph_max_ctx or self.rt.exact:
+        takes = (self.gated or self.activation == "relu_squared") and ops.moe_product_takes(h, self.w_up, self.w_down, self.gated)
+        few = T <= STREAM_MAX_TOKENS or bool(ctx.graph_max_ctx)
+        if takes and few and on_input:                   # the gathered rows round the weighted inputs, which streamed experts do not
+            takes = False
+        elif takes and T <= STREAM_MAX_TOKENS:
+            takes = sort_pays(T, top, E, 2 * (self.w_up[0].numel() + self.w_down[0].numel()))
+        if self.rt.exact or (few and not takes):
             a = torch.empty((T * top, self.inner), dtype=h.dtype, device=h.device)
             ops.moe_up(h, self.w_up, idx, a, act=self.act, gated=self.gated, in_scale=wts if on_input else None)
             ops.moe_down(a, self.w_down, idx, None if on_input else wts, y, extra=extra, extra_gate=extra_gate,
@@ -160,12 +178,15 @@ class RoutedExperts(Part):
         if not self.gated and self.activation != "relu_squared":
             raise NotImplementedError(f"long steps of experts without a gate run 'relu_squared', not {self.activation!r}")
         R = self.E_real                                  # the entries behind it are identities: their rows pass as they are
-        if ops.moe_product_takes(h, self.w_up, self.w_down, self.gated):
+        if takes:
             rows = torch.empty((T * top, self.hidden), dtype=h.dtype, device=h.device)
             ops.moe_gather(h, pair_at, idx, offsets, top, rows, scale=wts.view(-1) if on_input else None)
             inner = torch.empty((T * top, self.inner), dtype=h.dtype, device=h.device)
-            ops.moe_product(rows, self.w_up, offsets, inner, act=self.act, gated=self.gated)
-            ops.moe_product(inner, self.w_down, offsets, rows)           # the gathered rows are read: their buffer takes the results
+            # steps that could be streamed round nothing that streamed experts would not
+            ops.moe_product(rows, self.w_up, offsets, inner, act=self.act, gated=self.gated, raw=few)
+            if few:
+                rows = torch.empty((T * top, self.hidden), dtype=torch.float32, device=h.device)
+            ops.moe_product(inner, self.w_down, offsets, rows, raw=few)  # (else the gathered rows' buffer takes the results: they are read)
             ops.moe_combine(rows, place_of, idx, offsets, None if on_input else wts, y, extra=extra, extra_gate=extra_gate,
                             same=h if R < E else None, real=R)
             return y
