@@ -20,8 +20,10 @@
 // is bound by shared memory: a warp gets 32 floats of it a cycle and needs one for two multiply-adds with 16 columns a
 // block (measured 286 us for 2,048 tokens, 8 heads of 128 x 256; token by token 642).  On mma.sync a warp holds 32 rows of the transposed state [16 columns x 128 rows] as
 // accumulators, which are the next product's first operand as they lie; W, K, Q and P come as bfloat16 parts, cut once
-// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies: walk 134 us, prepare 34.
-#include "common.cuh"
+// by prepare, in rows padded for ldmatrix, so that a chunk's operands are linear copies.  With four warps that do everything and copy by
+// 16-byte cp.async the walk took 132 us; four more warps for the outputs 130, bulk copies 123, W a chunk and a half ahead 113 (the chain
+// alone, without outputs, 93).  Prepare 33.
+#include "umma.cuh"
 #include "parts_mma.cuh"
 
 constexpr int DC_C = 32;                 // tokens a chunk
@@ -47,6 +49,7 @@ struct DeltaChunkArgs {
     int* marked;                         // [chunks][H]: operands that the scan kernel has to take (common.cuh)
     float* out;
     int H, nqk, d, dv, nz;
+    int* status;
 };
 
 __device__ __forceinline__ float dc_softplus(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
@@ -212,172 +215,262 @@ __global__ void __launch_bounds__(DC_PREP) dc_prepare_kernel(const DeltaChunkArg
 
 // ------------------------------------------------------------------ walk
 template <int DP> struct WalkShape {
-    static constexpr int PARTS = dc_parts(DP);
-    static constexpr int W = 0, K = PARTS, Q = 2 * PARTS, P = 3 * PARTS, U = P + DC_PB, M = U + DC_UB, BUF = M + DC_MB;      // bytes of a buffer
+    static constexpr int PARTS = dc_parts(DP), KT = DP / 4 / 16;
+    static constexpr int W = 0, K = PARTS, Q = 2 * PARTS, P = 3 * PARTS, U = P + DC_PB, M = U + DC_UB, E = M + DC_MB,
+                         BUF = E + DC_C * 4;             // bytes of a buffer; E: the outputs' own copy of e^F_t
     static constexpr int LP = 40;                        // stride of a column of the partial sums, in tokens: float pairs of 16 lanes meet no bank twice
     static constexpr int SUMS = 4 * DC_COLS * LP * 4;    // bytes: [warp][column][LP]
-    static constexpr int BYTES = 2 * BUF + 2 * SUMS;
+    static constexpr int SF = 4 * KT * 3 * 512, UF = 2 * 3 * 512;      // bytes of the state's and of u's parts, as fragments
+    static constexpr int BYTES = 2 * BUF + 2 * SUMS + 2 * (SF + UF) + 64;      // behind them six barriers and a flag
 };
+// c[j] and s[j] += the parts of A times those of B's four tiles of 8, each sum in the order of parts_mma6; a product of parts at a time for all
+// four, so that neighbouring instructions do not wait for one another
+__device__ __forceinline__ void dc_mma6x4(float (&c)[4][4], float (&s)[4][4], const uint32_t (&a)[3][4], const uint32_t (&b)[2][3][4]) {
+    constexpr int pa[6] = {0, 2, 0, 1, 1, 0}, pb[6] = {0, 0, 2, 1, 0, 1};
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) parts_mma(i ? s[j] : c[j], a[pa[i]], b[j >> 1][pb[i]][(j & 1) * 2], b[j >> 1][pb[i]][(j & 1) * 2 + 1]);
+}
+// named barriers of the walk: the four warps of the chain, the four of the outputs, and what they hand over (for either buffer)
+enum { DC_BAR_CHAIN = 1, DC_BAR_OUT = 2, DC_BAR_S = 3, DC_BAR_U = 5, DC_BAR_FREE = 7 };
+__device__ __forceinline__ void dc_sync(int bar, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory"); }
+__device__ __forceinline__ void dc_arrive(int bar) { asm volatile("bar.arrive %0, 256;" ::"r"(bar) : "memory"); }
 
-// grid (requests, H, slices of 16 columns), four warps, DP / 4 rows of the state each
+// grid (requests, H, slices of 16 columns), eight warps.  Four carry the chain from chunk to chunk, DP / 4 rows of the state each: W S, u, the
+// new state.  Four follow a chunk behind with what nothing waits for: Q S, P u and the outputs, from the parts of the state and of u
+// that the others leave in shared memory (two buffers).  The chain is what bounds the kernel (its latency: one warp a scheduler).
 template <int DP>
-__global__ void __launch_bounds__(128) dc_walk_kernel(const DeltaChunkArgs A) {
+__global__ void __launch_bounds__(256, 1) dc_walk_kernel(const DeltaChunkArgs A) {
     using Sh = WalkShape<DP>;
-    constexpr int ROW = dc_row(DP), RW = DP / 4, NT = RW / 8, KT = RW / 16, LP = Sh::LP;
+    constexpr int ROW = dc_row(DP), RW = DP / 4, NT = RW / 8, KT = Sh::KT, LP = Sh::LP;
     constexpr int R = 8, IS = DP / R, LAYOUT = IS * DC_COLS, PB = R * LAYOUT;      // the slot's layout
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
     float* sums_w = reinterpret_cast<float*>(smem + 2 * Sh::BUF);
     float* sums_q = sums_w + Sh::SUMS / 4;
+    unsigned char* frags = smem + 2 * Sh::BUF + 2 * Sh::SUMS;        // per buffer: the state's parts [warp][k][part][lane], u's [k][part][lane]
     const int first = A.firsts[blockIdx.x], h = blockIdx.y, hq = h / (A.H / A.nqk), z = blockIdx.z, dv = A.dv;
     const int4 ck = A.chunks[first];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+    const int tid = threadIdx.x & 127, lane = tid & 31, wid = tid >> 5, g = lane >> 2, q2 = (lane & 3) * 2;
+    const bool chain = threadIdx.x < 128;
     const int row0 = A.q_start[ck.x], T = A.q_start[ck.x + 1] - row0;
-    float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + ((size_t)h * A.nz + z) * PB;
-    auto place = [&](int row, int c) { return (row % R) * LAYOUT + c * IS + row / R; };
-    // S transposed: element (column g or g + 8, row wid RW + 8 i + q2 or + 1)
-    float S[NT][4];
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-        const int row = wid * RW + 8 * i + q2;
-        S[i][0] = slot[place(row, g)]; S[i][1] = slot[place(row + 1, g)];
-        S[i][2] = slot[place(row, g + 8)]; S[i][3] = slot[place(row + 1, g + 8)];
+    if (tl_chunk_marked(A.marked, 1, first, ck.z, h, A.H)) return;       // the scan kernel's
+    uint64_t* landed = reinterpret_cast<uint64_t*>(smem + Sh::BYTES - 64);       // [2] W, [2] the chain's other operands, [2] the outputs'
+    volatile int* gave_up = reinterpret_cast<volatile int*>(smem + Sh::BYTES - 16);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 6; ++i) mbar_init(landed + i, 1);
+        *gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    auto copy = [&](int to, const unsigned char* from, int bytes) {
-        for (int i = tid * 16; i < bytes; i += 128 * 16)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(base + to + i), "l"(from + i) : "memory");
-    };
-    auto fetch = [&](int c) {
-        const int b = (c & 1) * Sh::BUF;
+    __syncthreads();
+    // Operands are linear copies, which one thread of those that use them asks for.  W is what a chunk starts with, and is read
+    // first: the next but one is asked for as soon as it is (a chunk and a half ahead).
+    enum { OF_W = 0, OF_CHAIN = 2, OF_OUT = 4 };
+    auto fetch = [&](int which, int c) {
+        if (tid || c >= ck.z) return;
+        const uint32_t to = base + (c & 1) * Sh::BUF;
+        uint64_t* bar = landed + which + (c & 1);
+        auto copy = [&](int at, const unsigned char* from, int bytes) {
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(to + at), "l"(from), "r"(bytes), "r"(smem_addr(bar)) : "memory");
+        };
         const size_t at = (size_t)(first + c) * A.H + h;
-        copy(b + Sh::W, A.W + at * Sh::PARTS, Sh::PARTS);
-        copy(b + Sh::K, A.K + ((size_t)(first + c) * A.nqk + hq) * 2 * Sh::PARTS, 2 * Sh::PARTS);      // K, then Q
-        copy(b + Sh::P, A.P + at * DC_PB, DC_PB);
-        copy(b + Sh::U, A.U + (at * A.nz + z) * DC_UB, DC_UB);
-        copy(b + Sh::M, A.M + at * DC_MB, DC_MB);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        const unsigned char* k = A.K + ((size_t)(first + c) * A.nqk + hq) * 2 * Sh::PARTS;      // K, then Q
+        mbar_expect_tx(bar, which == OF_W ? Sh::PARTS : which == OF_CHAIN ? Sh::PARTS + DC_UB + DC_MB : Sh::PARTS + DC_PB + DC_C * 4);
+        if (which == OF_W) copy(Sh::W, A.W + at * Sh::PARTS, Sh::PARTS);
+        if (which == OF_CHAIN) {
+            copy(Sh::U, A.U + (at * A.nz + z) * DC_UB, DC_UB);
+            copy(Sh::M, A.M + at * DC_MB, DC_MB);
+            copy(Sh::K, k, Sh::PARTS);
+        }
+        if (which == OF_OUT) {
+            copy(Sh::Q, k + Sh::PARTS, Sh::PARTS);
+            copy(Sh::P, A.P + at * DC_PB, DC_PB);
+            copy(Sh::E, A.M + at * DC_MB, DC_C * 4);
+        }
     };
-    fetch(0);
-    if (tl_chunk_marked(A.marked, 1, first, ck.z, h, A.H)) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        return;                                          // the scan kernel's
-    }
+    // a wait that runs out is recorded; the walk goes on with what there is (its result is not valid), so that no other warp waits for this one
+    auto wait = [&](int which, int c) { mbar_wait(landed + which + (c & 1), (c >> 1) & 1, gave_up, A.status, 51 + which / 2); };
     // this lane's addresses in fragments of two tiles: rows (tokens) of W, Q, P, and of K as it is transposed
     const uint32_t x_at = ((lane & 7) + (lane >> 4) * 8) * ROW + ((lane >> 3) & 1) * 16 + wid * RW * 2;
     const uint32_t k_at = ((lane & 7) + ((lane >> 3) & 1) * 8) * ROW + (lane >> 4) * 16 + wid * RW * 2;
     const uint32_t p_at = (wid * 8 + (lane & 7)) * DC_PROW + (lane >> 3) * 16;
-    for (int c = 0; c < ck.z; ++c) {
-        const int n = min(DC_C, T - c * DC_C);
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                 // the chunk's operands have landed, the chunk before is read
-        if (c + 1 < ck.z) fetch(c + 1);
-        const unsigned char* buf = smem + (c & 1) * Sh::BUF;
-        const uint32_t at = base + (c & 1) * Sh::BUF;
-        const float* u0 = reinterpret_cast<const float*>(buf + Sh::U);
-        const float* mk = reinterpret_cast<const float*>(buf + Sh::M);
-        uint32_t sa[KT][3][4];                           // S transposed as a first operand: [columns][rows]
+    // (X S)^T over this warp's rows of the state, X the rows at `from`: [16 columns][32 tokens], to the partial sums
+    auto times_state = [&](uint32_t from, const uint32_t (&sa)[KT][3][4], float* sums) {
+        float big[4][4], rest[4][4];
 #pragma unroll
-        for (int k = 0; k < KT; ++k)
+        for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const float (&v)[4] = S[2 * k + (x >> 1)];
-                parts_cut(v[(x & 1) * 2], v[(x & 1) * 2 + 1], sa[k][0][x], sa[k][1][x], sa[k][2][x]);
-            }
-        // (W S)^T and (Q S)^T over this warp's rows: [16 columns][32 tokens]
+            for (int x = 0; x < 4; ++x) big[j][x] = rest[j][x] = 0.f;
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-            float big[4][4], rest[4][4];
+        for (int k = 0; k < KT; ++k) {
+            uint32_t b[2][3][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
-                for (int x = 0; x < 4; ++x) big[j][x] = rest[j][x] = 0.f;
+                for (int p = 0; p < 3; ++p) parts_load4(b[j][p], from + (p * DC_C + j * 16) * ROW + x_at + k * 32);
+            dc_mma6x4(big, rest, sa[k], b);
+        }
+        float* to = sums + (wid * DC_COLS + g) * LP + q2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            *reinterpret_cast<float2*>(to + 8 * j) = make_float2(big[j][0] + rest[j][0], big[j][1] + rest[j][1]);
+            *reinterpret_cast<float2*>(to + 8 * LP + 8 * j) = make_float2(big[j][2] + rest[j][2], big[j][3] + rest[j][3]);
+        }
+    };
+    if (chain) {
+        fetch(OF_W, 0);
+        fetch(OF_CHAIN, 0);
+        fetch(OF_W, 1);
+        float* slot = A.state + (size_t)A.slots[ck.x] * A.slot_stride + ((size_t)h * A.nz + z) * PB;
+        auto place = [&](int row, int c) { return (row % R) * LAYOUT + c * IS + row / R; };
+        // S transposed: element (column g or g + 8, row wid RW + 8 i + q2 or + 1)
+        float S[NT][4];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const int row = wid * RW + 8 * i + q2;
+            S[i][0] = slot[place(row, g)]; S[i][1] = slot[place(row + 1, g)];
+            S[i][2] = slot[place(row, g + 8)]; S[i][3] = slot[place(row + 1, g + 8)];
+        }
+        for (int c = 0; c < ck.z; ++c) {
+            const int n = min(DC_C, T - c * DC_C), half = c & 1;
+            dc_sync(DC_BAR_CHAIN, 128);                  // the chunk before is read
+            fetch(OF_CHAIN, c + 1);
+            wait(OF_W, c);
+            const uint32_t at = base + half * Sh::BUF;
+            const float* u0 = reinterpret_cast<const float*>(smem + half * Sh::BUF + Sh::U);
+            const float* mk = reinterpret_cast<const float*>(smem + half * Sh::BUF + Sh::M);
+            uint4* sf = reinterpret_cast<uint4*>(frags + half * (Sh::SF + Sh::UF)) + wid * KT * 3 * 32 + lane;
+            uint4* uf = reinterpret_cast<uint4*>(frags + half * (Sh::SF + Sh::UF) + Sh::SF) + lane;
+            uint32_t sa[KT][3][4];                       // S transposed as a first operand: [columns][rows]
 #pragma unroll
             for (int k = 0; k < KT; ++k)
 #pragma unroll
-                for (int j = 0; j < 4; j += 2) {
-                    uint32_t b[3][4];
-#pragma unroll
-                    for (int p = 0; p < 3; ++p) parts_load4(b[p], at + (which ? Sh::Q : Sh::W) + (p * DC_C + j * 8) * ROW + x_at + k * 32);
-                    parts_mma6(big[j], rest[j], sa[k], b, 0);
-                    parts_mma6(big[j + 1], rest[j + 1], sa[k], b, 2);
+                for (int x = 0; x < 4; ++x) {
+                    const float (&v)[4] = S[2 * k + (x >> 1)];
+                    parts_cut(v[(x & 1) * 2], v[(x & 1) * 2 + 1], sa[k][0][x], sa[k][1][x], sa[k][2][x]);
                 }
-            float* to = (which ? sums_q : sums_w) + (wid * DC_COLS + g) * LP + q2;
+            if (c >= 2) dc_sync(DC_BAR_FREE + half, 256);          // the outputs of chunk c - 2 have read this buffer
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                *reinterpret_cast<float2*>(to + 8 * j) = make_float2(big[j][0] + rest[j][0], big[j][1] + rest[j][1]);
-                *reinterpret_cast<float2*>(to + 8 * LP + 8 * j) = make_float2(big[j][2] + rest[j][2], big[j][3] + rest[j][3]);
-            }
-        }
-        __syncthreads();
-        // u transposed as a first operand [columns][tokens]: as it is, and weighted for the end state
-        uint32_t ua[2][3][4], wa[2][3][4];
+            for (int k = 0; k < KT; ++k)
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+                for (int p = 0; p < 3; ++p) sf[(k * 3 + p) * 32] = make_uint4(sa[k][p][0], sa[k][p][1], sa[k][p][2], sa[k][p][3]);
+            dc_arrive(DC_BAR_S + half);
+            times_state(at + Sh::W, sa, sums_w);
+            dc_sync(DC_BAR_CHAIN, 128);
+            fetch(OF_W, c + 2);
+            wait(OF_CHAIN, c);
+            // u transposed as a first operand [columns][tokens]: weighted for the end state, and as it is for the outputs
+            uint32_t wa[2][3][4];
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int col = g + (x & 1) * 8, t = 16 * k + (x >> 1) * 8 + q2;
-                float2 s = make_float2(0.f, 0.f);
+            for (int k = 0; k < 2; ++k) {
+                uint32_t ua[3][4];
 #pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const float2 v = *reinterpret_cast<const float2*>(sums_w + (w * DC_COLS + col) * LP + t);
-                    s.x += v.x; s.y += v.y;
+                for (int x = 0; x < 4; ++x) {
+                    const int col = g + (x & 1) * 8, t = 16 * k + (x >> 1) * 8 + q2;
+                    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        const float2 v = *reinterpret_cast<const float2*>(sums_w + (w * DC_COLS + col) * LP + t);
+                        s.x += v.x; s.y += v.y;
+                    }
+                    const float a = u0[t * 20 + col] - s.x, b = u0[(t + 1) * 20 + col] - s.y;
+                    if (wid == k) parts_cut(a, b, ua[0][x], ua[1][x], ua[2][x]);
+                    parts_cut(a * mk[DC_C + t], b * mk[DC_C + t + 1], wa[k][0][x], wa[k][1][x], wa[k][2][x]);
                 }
-                const float a = u0[t * 20 + col] - s.x, b = u0[(t + 1) * 20 + col] - s.y;
-                parts_cut(a, b, ua[k][0][x], ua[k][1][x], ua[k][2][x]);
-                parts_cut(a * mk[DC_C + t], b * mk[DC_C + t + 1], wa[k][0][x], wa[k][1][x], wa[k][2][x]);
+                if (wid == k)                            // every warp holds all of u: two of them hand it over, half each
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) uf[(k * 3 + p) * 32] = make_uint4(ua[p][0], ua[p][1], ua[p][2], ua[p][3]);
             }
-        // the new state
-        {
+            dc_arrive(DC_BAR_U + half);
+            // the new state
             const float end = mk[n - 1];
+            float big[NT][4] = {}, rest[NT][4] = {};
 #pragma unroll
-            for (int i = 0; i < NT; i += 2) {
-                float big[2][4] = {}, rest[2][4] = {};
+            for (int k = 0; k < 2; ++k) {
+                if constexpr (NT == 4) {
+                    uint32_t b[2][3][4];
 #pragma unroll
-                for (int k = 0; k < 2; ++k) {
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) parts_load4_trans(b[j][p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at + j * 32);
+                    dc_mma6x4(big, rest, wa[k], b);
+                } else {
                     uint32_t b[3][4];
 #pragma unroll
-                    for (int p = 0; p < 3; ++p) parts_load4_trans(b[p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at + i * 16);
+                    for (int p = 0; p < 3; ++p) parts_load4_trans(b[p], at + Sh::K + (p * DC_C + 16 * k) * ROW + k_at);
                     parts_mma6(big[0], rest[0], wa[k], b, 0);
                     parts_mma6(big[1], rest[1], wa[k], b, 2);
                 }
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int x = 0; x < 4; ++x) S[i + j][x] = fmaf(end, S[i + j][x], big[j][x] + rest[j][x]);
             }
+#pragma unroll
+            for (int i = 0; i < NT; ++i)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) S[i][x] = fmaf(end, S[i][x], big[i][x] + rest[i][x]);
         }
-        // outputs of tokens 8 wid ..
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const int row = wid * RW + 8 * i + q2;
+            slot[place(row, g)] = S[i][0]; slot[place(row + 1, g)] = S[i][1];
+            slot[place(row, g + 8)] = S[i][2]; slot[place(row + 1, g + 8)] = S[i][3];
+        }
+    } else {
+        fetch(OF_OUT, 0);
+    }
+    for (int c = 0; !chain && c < ck.z; ++c) {
+        const int n = min(DC_C, T - c * DC_C), half = c & 1;
+        dc_sync(DC_BAR_OUT, 128);                        // the chunk before is read
+        fetch(OF_OUT, c + 1);
+        wait(OF_OUT, c);
+        const uint32_t at = base + half * Sh::BUF;
+        const float* grown = reinterpret_cast<const float*>(smem + half * Sh::BUF + Sh::E);
+        const uint4* sf = reinterpret_cast<const uint4*>(frags + half * (Sh::SF + Sh::UF)) + wid * KT * 3 * 32 + lane;
+        const uint4* uf = reinterpret_cast<const uint4*>(frags + half * (Sh::SF + Sh::UF) + Sh::SF) + lane;
+        dc_sync(DC_BAR_S + half, 256);
         {
-            float big[4] = {}, rest[4] = {};
-            uint32_t b[3][4];
+            uint32_t sa[KT][3][4];
 #pragma unroll
-            for (int p = 0; p < 3; ++p) parts_load4(b[p], at + Sh::P + p * DC_C * DC_PROW + p_at);
-            parts_mma6(big, rest, ua[0], b, 0);
-            parts_mma6(big, rest, ua[1], b, 2);
-            const int t = 8 * wid + q2;
-            const float2 e = *reinterpret_cast<const float2*>(mk + t);
+            for (int k = 0; k < KT; ++k)
 #pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                float2 s = make_float2(0.f, 0.f);
+                for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(sa[k][p]) = sf[(k * 3 + p) * 32];
+            times_state(at + Sh::Q, sa, sums_q);
+        }
+        dc_sync(DC_BAR_OUT, 128);
+        dc_sync(DC_BAR_U + half, 256);
+        // outputs of tokens 8 wid ..
+        float big[4] = {}, rest[4] = {};
+        uint32_t b[3][4], ua[2][3][4];
 #pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    const float2 v = *reinterpret_cast<const float2*>(sums_q + (w * DC_COLS + g + 8 * x) * LP + t);
-                    s.x += v.x; s.y += v.y;
-                }
-                const int col = z * DC_COLS + g + 8 * x;
-                if (col < dv) {
-                    float* to = A.out + (size_t)(row0 + c * DC_C + t) * A.H * dv + (size_t)h * dv + col;
-                    if (t < n) to[0] = fmaf(e.x, s.x, big[2 * x] + rest[2 * x]);
-                    if (t + 1 < n) to[(size_t)A.H * dv] = fmaf(e.y, s.y, big[2 * x + 1] + rest[2 * x + 1]);
-                }
+        for (int p = 0; p < 3; ++p) parts_load4(b[p], at + Sh::P + p * DC_C * DC_PROW + p_at);
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<uint4*>(ua[k][p]) = uf[(k * 3 + p) * 32];
+        if (c + 2 < ck.z) dc_arrive(DC_BAR_FREE + half);
+        parts_mma6(big, rest, ua[0], b, 0);
+        parts_mma6(big, rest, ua[1], b, 2);
+        const int t = 8 * wid + q2;
+        const float2 e = *reinterpret_cast<const float2*>(grown + t);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                const float2 v = *reinterpret_cast<const float2*>(sums_q + (w * DC_COLS + g + 8 * x) * LP + t);
+                s.x += v.x; s.y += v.y;
+            }
+            const int col = z * DC_COLS + g + 8 * x;
+            if (col < dv) {
+                float* to = A.out + (size_t)(row0 + c * DC_C + t) * A.H * dv + (size_t)h * dv + col;
+                if (t < n) to[0] = fmaf(e.x, s.x, big[2 * x] + rest[2 * x]);
+                if (t + 1 < n) to[(size_t)A.H * dv] = fmaf(e.y, s.y, big[2 * x + 1] + rest[2 * x + 1]);
             }
         }
     }
-#pragma unroll
-    for (int i = 0; i < NT; ++i) {
-        const int row = wid * RW + 8 * i + q2;
-        slot[place(row, g)] = S[i][0]; slot[place(row + 1, g)] = S[i][1];
-        slot[place(row, g + 8)] = S[i][2]; slot[place(row + 1, g + 8)] = S[i][3];
+    if (*gave_up) {                                      // give copies in flight time to land before the shared memory is handed on
+        const long long start = clock64();
+        while (clock64() - start < 2000000LL) { }
     }
 }
 
@@ -400,7 +493,7 @@ static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int* marked, int 
     A.marked = marked;
     dc_prepare_kernel<DP><<<dim3(n_chunks, A.H), DC_PREP, row_bytes + DC_C * A.dv * 4, stream>>>(A);
     if ((e = tl_launch_status())) return e;
-    dc_walk_kernel<DP><<<dim3(requests, A.H, A.nz), 128, Sh::BYTES, stream>>>(A);
+    dc_walk_kernel<DP><<<dim3(requests, A.H, A.nz), 256, Sh::BYTES, stream>>>(A);
     return tl_launch_status();
 }
 
@@ -413,16 +506,17 @@ TL_EXPORT int tl_delta_chunk_bytes(int H, int nqk, int d, int dv) {
     return H * (parts + DC_PB + DC_MB + (dv + DC_COLS - 1) / DC_COLS * DC_UB) + nqk * 2 * parts;
 }
 
-// scratch: `tl_delta_chunk_bytes` bytes a chunk; marked: int [n_chunks, H], for the scan kernel (tiles: 1).  The offsets and the stride are multiples of 4, the pointers 16-byte aligned.
+// scratch: `tl_delta_chunk_bytes` bytes a chunk; marked: int [n_chunks, H], for the scan kernel (tiles: 1); status: device int.  The offsets and the stride are multiples of 4, the pointers 16-byte aligned.
 TL_EXPORT int tl_delta_chunks(const float* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, int gate_stride,
                               const float* A_log, const float* dt_bias, float* state, long long slot_stride, const int* q_start,
                               const int* slots, const int* chunks, int n_chunks, const int* firsts, int requests, void* scratch, int* marked, float* out,
-                              int H, int nqk, int d, int dv, cudaStream_t stream) {
+                              int H, int nqk, int d, int dv, int* status, cudaStream_t stream) {
     if (n_chunks <= 0 || H <= 0) return 0;
+    if (status == nullptr) return 1;
     if (H > 65535 || nqk < 1 || H % nqk || !tl_delta_chunk_bytes(H, nqk, d, dv) || ((stride | q_off | k_off | v_off) & 3) ||
         ((((uintptr_t)qkv) | ((uintptr_t)scratch) | ((uintptr_t)out)) & 15)) return 1;
     const DeltaChunkArgs A{qkv, stride, q_off, k_off, v_off, gates, gate_stride, A_log, dt_bias, state, slot_stride, q_start, slots,
-                           (const int4*)chunks, firsts, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, out, H, nqk, d, dv, (dv + DC_COLS - 1) / DC_COLS};
+                           (const int4*)chunks, firsts, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, out, H, nqk, d, dv, (dv + DC_COLS - 1) / DC_COLS, status};
     if (d <= 64) return dc_launch<64>(A, (unsigned char*)scratch, marked, n_chunks, requests, stream);
     return dc_launch<128>(A, (unsigned char*)scratch, marked, n_chunks, requests, stream);
 }

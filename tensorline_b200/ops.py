@@ -68,7 +68,7 @@ _SIGNATURES = {
     "tl_moe_product_takes": [_I, _I, _I, _I],
     "tl_conv_prep": [_P, _I, _I, _P, _I, _I, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _F, _P],
     "tl_delta_scan": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _P, _P, _I, _P],
-    "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P],
+    "tl_delta_chunks": [_P, _I, _I, _I, _I, _P, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P],
     "tl_delta_chunk": [],
     "tl_delta_chunk_bytes": [_I, _I, _I, _I],
     "tl_delta_state_floats": [_I, _I],
@@ -171,6 +171,8 @@ STATUS_ROLES = {1: "tcgen05 product: the copy thread waited for a free stage", 2
                 43: "32-bit product: the MMA thread waited for a stage's copies", 44: "32-bit product: the sums waited for an accumulator",
                 45: "experts' product: a copy thread waited for a free stage", 46: "experts' product: the MMA thread waited for a free accumulator",
                 47: "experts' product: the MMA thread waited for a stage's copies", 48: "experts' product: the epilogue waited for the accumulator",
+                51: "delta rule's chunks: the chain waited for W", 52: "delta rule's chunks: the chain waited for K and U",
+                53: "delta rule's chunks: the outputs waited for Q and P",
                 20: "decode attention: a wait for a stage of keys and values"}
 
 
@@ -1315,8 +1317,8 @@ def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt
     marked = _ptr(scratch) + step.n * per_chunk
     args = (_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(state), per_slot,
             _ptr(ctx.q_start), _ptr(ctx.slots))
-    _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.long, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv, _stream()),
-           "delta_chunks", launches=2)
+    _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.long, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv,
+                               _ptr(device_status(qkv.device)), _stream()), "delta_chunks", launches=2)
     _check(lib.tl_delta_scan(*args, _ptr(out), step.requests, H, nqk, d, dv, step.longest, 0, step.runs, marked, 1, _stream()), "delta_scan")
 
 
