@@ -20,10 +20,11 @@
 // (81 as float multiply-adds).  Fixed decay, 1,650 tokens in 3 requests: local 23, carry 18, outputs 44 us (70 as multiply-adds).
 // 64 tokens a chunk: P costs as much as the two products with the state at 128 tokens, and the start states, which pass through
 // L2 once each way, weigh half as much again at 32.
-#include "common.cuh"
+#include "umma.cuh"
 #include "parts_mma.cuh"
 
 constexpr int LC_C = 64;                 // tokens a chunk
+constexpr int LC_WIDE = 128;             // tokens a chunk where a head's 33 to 128 rows fill the 5th-generation tensor cores' tiles
 constexpr int LC_COLS = 16;              // columns a slice of the state's layout (the scan kernel's)
 
 struct LinearChunkArgs {
@@ -41,57 +42,71 @@ struct LinearChunkArgs {
     int* marked; int tiles;              // [chunks][H][tiles]: operands that the scan kernel has to take (common.cuh)
     float* out;
     int H, d, dv, nz; float den_eps;
+    int* status;
 };
 
 __device__ __forceinline__ float lc_log_sigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
-// A warp, gated: for the n tokens of a chunk that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the running
-// maximum top[t] of u.
+// A warp, gated: for the n tokens of a chunk of C that starts at row t0, F[t] (the log decays' sum up to t), u[t] = i_t - F[t] and the
+// running maximum top[t] of u.
+template <int C>
 __device__ __forceinline__ void lc_weights(const LinearChunkArgs& A, int t0, int n, int h, int lane, double* F, double* u, double* top) {
-    double f[2], in[2];
+    constexpr int N = C / 32;                            // tokens a lane
+    double f[N], w[N], best = -INFINITY, sum = 0.0;
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-        const int t = 2 * lane + e;
-        f[e] = 0.0; in[e] = -INFINITY;
+    for (int e = 0; e < N; ++e) {
+        const int t = N * lane + e;
+        f[e] = 0.0; w[e] = -INFINITY;
         if (t < n) {
             const float* g = A.gates + (size_t)(t0 + t) * 2 * A.H;
-            in[e] = A.cap * tanhf(g[h] / A.cap);
+            w[e] = A.cap * tanhf(g[h] / A.cap);
             f[e] = lc_log_sigmoid(A.cap * tanhf(g[A.H + h] / A.cap));
         }
+        sum += f[e];
     }
-    double sum = f[0] + f[1];
+    const double mine = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double x = __shfl_up_sync(0xffffffffu, sum, o);
         if (lane >= o) sum += x;
     }
-    const double F1 = sum, F0 = sum - f[1], u0 = in[0] - F0, u1 = in[1] - F1;
-    double best = fmax(u0, u1);
+    double at = sum - mine;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        at += f[e];
+        f[e] = at;
+        w[e] -= at;
+        best = fmax(best, w[e]);
+    }
+    double before = best;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double x = __shfl_up_sync(0xffffffffu, best, o);
-        if (lane >= o) best = fmax(best, x);
+        const double x = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before = fmax(before, x);
     }
-    double before = __shfl_up_sync(0xffffffffu, best, 1);
+    before = __shfl_up_sync(0xffffffffu, before, 1);
     if (lane == 0) before = -INFINITY;
-    F[2 * lane] = F0; F[2 * lane + 1] = F1;
-    u[2 * lane] = u0; u[2 * lane + 1] = u1;
-    top[2 * lane] = fmax(before, u0); top[2 * lane + 1] = best;
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        before = fmax(before, w[e]);
+        F[N * lane + e] = f[e]; u[N * lane + e] = w[e]; top[N * lane + e] = before;
+    }
 }
 
 // A warp a (chunk, head): the gated kinds' weights, once for all blocks that need them (worked out in each of them, warp 0 held the
 // others up: end states 36 us, 33.5 without and 4.6 here, and the outputs need them without a wait).
+template <int C>
 __global__ void __launch_bounds__(32) lc_gates_kernel(const LinearChunkArgs A) {
     const int4 ck = A.chunks[blockIdx.x];
-    const int h = blockIdx.y, lane = threadIdx.x, t0 = A.q_start[ck.x] + ck.y * LC_C, n = min(LC_C, A.q_start[ck.x + 1] - t0);
+    const int h = blockIdx.y, lane = threadIdx.x, t0 = A.q_start[ck.x] + ck.y * C, n = min(C, A.q_start[ck.x + 1] - t0);
     const size_t at = (size_t)blockIdx.x * A.H + h;
-    double* w = A.weights + at * 3 * LC_C;
-    lc_weights(A, t0, n, h, lane, w, w + LC_C, w + 2 * LC_C);
+    double* w = A.weights + at * 3 * C;
+    lc_weights<C>(A, t0, n, h, lane, w, w + C, w + 2 * C);
     __syncwarp();
     if (lane == 0) {
         const double end = w[n - 1];
         A.marks[at * 3] = end;
-        A.marks[at * 3 + 1] = (double)(float)(end + w[2 * LC_C + n - 1]);
+        A.marks[at * 3 + 1] = (double)(float)(end + w[2 * C + n - 1]);
     }
 }
 
@@ -641,6 +656,581 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) lc_out_kernel(const Li
         }
 }
 
+// ------------------------------------------------------------------ wide chunks on the 5th-generation tensor cores
+// Heads of 33 to 128 rows: chunks of 128 tokens, so that tokens (outputs) and rows (end states) fill the MMA's 128.  Everything is a sum
+// over k (rows, tokens) in steps of 32, each an accumulator of its own in tensor memory: twelve tcgen05 products of bfloat16
+// parts, the five small ones of the six first, and sixteen worker warps add the accumulators up with additions that round (the tensor
+// cores cut; see parts_mma.cuh).  A worker owns a lane of tensor memory (a token or a row) and a quarter of the columns.  One more warp
+// issues.  Operands are cut into parts on their way to shared memory, in the 128-byte swizzle: rows of 64 values, K-major for Q, K and P,
+// MN-major for what is summed over its rows (V, S, and K for the end states).  192 KB, one block an SM.
+//   outputs     Q K^T (four accumulators, added up into the first); Q S, 32 rows of S a stage through a ring of four in K's place
+//               and three accumulators; P takes Q's place, then P V likewise.
+// Loops stay rolled: a block runs once through its code, and what is not in the instruction cache comes at one instruction in
+// about 13 cycles (the weights unrolled over a worker's 64 keys took 18,000 cycles).
+//   end states  K^T V, 32 tokens a stage, nothing is used twice.
+// Measured beside the mma.sync kernels (chunks of 64), 8 heads of 128 x 256, 2,048 tokens: end states 19 us (28), start states 12 (18),
+// outputs 39 (65); all of a gated memory 85 (127), a fixed decay's 73 (103).  A block runs its phases one after the other, about 35 us whatever else
+// there is, so short steps stay with the chunks of 64 (ops.py).
+constexpr int LW_WORK = 512, LW_THREADS = LW_WORK + 32, LW_MMA = LW_WORK / 32, LW_REGION = 3 * LC_WIDE * LC_WIDE * 2;
+constexpr int LW_SMEM = 2 * LW_REGION + 1024;
+
+__device__ __forceinline__ uint32_t lw_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one;
+}
+// by a whole warp, the instruction itself by one lane: its operands are uniform registers then (umma_pair.cuh)
+__device__ __forceinline__ void lw_mma(uint32_t acc, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate, uint32_t one) {
+    asm volatile("{\n\t.reg .pred p, q;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "setp.ne.b32 q, %5, 0;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 ::"r"(acc), "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
+}
+__device__ __forceinline__ void lw_commit(uint64_t* bar, uint32_t one) {
+    asm volatile("{\n\t.reg .pred q;\n\t"
+                 "setp.ne.b32 q, %1, 0;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+                 ::"r"(smem_addr(bar)), "r"(one) : "memory");
+}
+// The six products of parts of 32 k into `acc`, the small ones first.  a(p, k), b(p, k): descriptors of part p, k in steps of 16.
+template <typename FA, typename FB>
+__device__ __forceinline__ void lw_parts(uint32_t acc, uint32_t idesc, uint32_t one, FA a, FB b) {
+    constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+    for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) lw_mma(acc, a(pa[i], k), b(pb[i], k), idesc, (i || k) ? 1u : 0u, one);
+}
+// eight values' parts into the 16 bytes at `at` of three tiles, `part` bytes apart
+__device__ __forceinline__ void lw_put8(unsigned char* at, int part, const float (&x)[8]) {
+    uint4 p[3];
+    uint32_t* w[3] = {reinterpret_cast<uint32_t*>(&p[0]), reinterpret_cast<uint32_t*>(&p[1]), reinterpret_cast<uint32_t*>(&p[2])};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) parts_cut(x[2 * e], x[2 * e + 1], w[0][e], w[1][e], w[2][e]);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) *reinterpret_cast<uint4*>(at + e * part) = p[e];
+}
+// eight floats of a row, zeros where !ok or behind `left` values (a multiple of 4)
+__device__ __forceinline__ void lw_get8(float (&x)[8], const float* from, bool ok, int left) {
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(x) = ok && left > 0 ? *reinterpret_cast<const float4*>(from) : z;
+    *reinterpret_cast<float4*>(x + 4) = ok && left > 4 ? *reinterpret_cast<const float4*>(from + 4) : z;
+}
+__device__ __forceinline__ void lw_ld16(uint32_t at, float (&r)[16]) {
+    uint32_t* u = reinterpret_cast<uint32_t*>(r);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]),
+                   "=r"(u[8]), "=r"(u[9]), "=r"(u[10]), "=r"(u[11]), "=r"(u[12]), "=r"(u[13]), "=r"(u[14]), "=r"(u[15]) : "r"(at));
+}
+__device__ __forceinline__ void lw_ld8(uint32_t at, float (&r)[8]) {
+    uint32_t* u = reinterpret_cast<uint32_t*>(r);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7]) : "r"(at));
+}
+__device__ __forceinline__ void lw_st16(uint32_t at, const float (&r)[16]) {
+    const uint32_t* u = reinterpret_cast<const uint32_t*>(r);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n\t"
+                 "tcgen05.wait::st.sync.aligned;"
+                 ::"r"(at), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]),
+                   "r"(u[8]), "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]) : "memory");
+}
+// this lane's quarter of the columns of an accumulator, added to `sum`
+template <int N> __device__ __forceinline__ void lw_add(float (&sum)[N], uint32_t at) {
+    if constexpr (N == 32) {
+        float r[32];
+        tmem_ld32(at, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 32; ++x) sum[x] += r[x];
+    } else {
+        static_assert(N == 16, "columns a worker");
+        float r[16];
+        lw_ld16(at, r);
+#pragma unroll
+        for (int x = 0; x < 16; ++x) sum[x] += r[x];
+    }
+}
+__device__ __forceinline__ void lw_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LW_WORK) : "memory"); }      // the workers
+// A tile of floats out of registers (a lane a row, a quarter of the columns) through shared memory into rows `ld` floats apart, in whole
+// rows; by the worker warps.  Lane by lane, 16 bytes of 32 rows at a time, the outputs took 15,000 cycles.  `by`: what a row is divided by, `over` one over it.
+template <int CB>
+__device__ __forceinline__ void lw_store(float* tile, const float (&sum)[CB / 4], float* to, size_t ld, int rows, int cols, const float* by, const float* over) {
+    constexpr int LD = CB + 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = (warp & 3) * 32 + lane;
+#pragma unroll
+    for (int c = 0; c < CB / 4; c += 4)
+        *reinterpret_cast<float4*>(tile + row * LD + (warp >> 2) * (CB / 4) + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+    lw_sync();
+    constexpr int STEP = LW_WORK / (CB / 4);             // rows from one piece of a thread to its next
+    const int c = tid % (CB / 4) * 4;
+    if (c >= cols) return;
+    int r = tid / (CB / 4);
+    const float* at = tile + r * LD + c;
+    to += (size_t)r * ld + c;
+#pragma unroll 4
+    for (; r < rows; r += STEP, at += STEP * LD, to += STEP * ld) {
+        float4 x = *reinterpret_cast<const float4*>(at);
+        if (by) {
+            const float b = by[r], o = over[r];
+            if (b > 1e-30f && b < 1e30f) {               // a quotient by the reciprocal, corrected once with its remainder (Markstein 1990)
+                auto quotient = [&](float z) { const float q = z * o; return fmaf(fmaf(-q, b, z), o, q); };
+                x.x = quotient(x.x); x.y = quotient(x.y); x.z = quotient(x.z); x.w = quotient(x.w);
+            } else { x.x /= b; x.y /= b; x.z /= b; x.w /= b; }
+        }
+        *reinterpret_cast<float4*>(to) = x;
+    }
+}
+// sums of floats with what their additions lose, as exact as sums in double and on the float pipe (in double the weights and sums of a
+// chunk took 16,000 cycles)
+struct LwSum {
+    float s = 0.f, lost = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = s + x, b = t - s;
+        lost += (s - (t - b)) + (x - b);
+        s = t;
+    }
+    __device__ __forceinline__ void add_product(float x, float y) {
+        const float p = x * y;
+        lost += fmaf(x, y, -p);
+        add(p);
+    }
+    __device__ __forceinline__ double value() const { return (double)s + (double)lost; }
+};
+struct LwBars { uint64_t qk, full[4], done[4]; uint32_t tmem; int gave_up; };
+__device__ __forceinline__ void lw_start(LwBars& B, int warp) {
+    if (threadIdx.x == 0) {
+        mbar_init(&B.qk, 1);
+        for (int i = 0; i < 4; ++i) { mbar_init(B.full + i, LW_MMA); mbar_init(B.done + i, 1); }
+        B.gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == LW_MMA) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&B.tmem)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+}
+__device__ __forceinline__ void lw_end(LwBars& B, int warp, uint32_t tmem) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == LW_MMA) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+// a worker warp's part of a stage is in shared memory
+__device__ __forceinline__ void lw_filled(uint64_t* bar, int lane) {
+    fence_async_proxy();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
+// grid (chunks, H, slices of CB columns)
+template <int DP, int CB, bool GATED>
+__global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChunkArgs A) {
+    constexpr int C = LC_WIDE, PK = C * DP * 2, PV = C * CB * 2, HC = CB / 4;        // bytes of a part of K, of V; columns a worker
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* ks = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* vs = ks + LW_REGION;
+    __shared__ LwBars B;
+    __shared__ float w[C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, col0 = blockIdx.z * CB, d = A.d;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int t0 = A.q_start[ck.x] + ck.y * C, n = min(C, A.q_start[ck.x + 1] - t0), stages = (n + 31) / 32;
+    const size_t ch = (size_t)blockIdx.x * A.H + h;
+    lw_start(B, warp);
+    if (GATED) {
+        const double* g = A.weights + ch * 3 * C;
+        if (tid < C) w[tid] = tid < n ? (float)exp(A.marks[ch * 3] + g[C + tid] - A.marks[ch * 3 + 1]) * A.k_scale : 0.f;
+    } else if (tid < C) {
+        const double la = log((double)A.decay[h]);
+        w[tid] = tid < n ? (float)exp((n - 1 - tid) * la) * A.k_scale : 0.f;
+        if (tid == 0 && blockIdx.z == 0) { A.marks[ch * 3] = n * la; A.marks[ch * 3 + 1] = 0.0; }
+    }
+    bool odd = tid < C && w[tid] != w[tid];              // a gate that is no number
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = B.tmem;
+    volatile int* gave_up = &B.gave_up;
+    if (warp == LW_MMA) {
+        // A: K^T, B: V, both MN-major; heads of up to 64 rows: the upper half of the tile is whatever lies behind, and nobody reads it
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(CB >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t one = lw_elect(), ka = smem_addr(ks), va = smem_addr(vs);
+        for (int i = 0; i < stages; ++i) {
+            if (!mbar_wait(B.full + i, 0, gave_up, A.status, 61)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            lw_parts(tmem + i * 128, idesc, one,
+                     [&](int p, int k) { return desc_mnmajor(ka + p * PK + (i * 2 + k) * 16 * 128, C * 128); },
+                     [&](int p, int k) { return desc_mnmajor(va + p * PV + (i * 2 + k) * 16 * 128, C * 128); });
+            lw_commit(B.done + i, one);
+        }
+    } else {
+        constexpr int KN = 32 * DP / 8, VN = 32 * CB / 8, KPER = (KN + LW_WORK - 1) / LW_WORK, VPER = (VN + LW_WORK - 1) / LW_WORK;      // pieces of eight a stage, a thread
+        float keys[2][KPER][8], values[2][VPER][8];      // two stages on their way
+        auto fetch = [&](float (&x)[KPER][8], float (&y)[VPER][8], int i) {
+#pragma unroll
+            for (int j = 0; j < KPER; ++j) {
+                if (KN % LW_WORK && tid >= KN) continue;
+                const int t = 32 * i + (tid + LW_WORK * j) / (DP / 8), e = (tid + LW_WORK * j) % (DP / 8) * 8;
+                lw_get8(x[j], A.k + (size_t)(t0 + t) * A.qk_stride + h * d + e, t < n, d - e);
+            }
+#pragma unroll
+            for (int j = 0; j < VPER; ++j) {
+                if (VN % LW_WORK && tid >= VN) continue;
+                const int t = 32 * i + (tid + LW_WORK * j) / (CB / 8), c = (tid + LW_WORK * j) % (CB / 8) * 8;
+                lw_get8(y[j], A.v + (size_t)(t0 + t) * A.v_stride + h * A.dv + col0 + c, t < n, A.dv - col0 - c);
+            }
+        };
+        auto fill = [&](float (&x)[KPER][8], float (&y)[VPER][8], int i) {
+#pragma unroll
+            for (int j = 0; j < KPER; ++j) {
+                if (KN % LW_WORK && tid >= KN) continue;
+                const int t = 32 * i + (tid + LW_WORK * j) / (DP / 8), c = (tid + LW_WORK * j) % (DP / 8);
+                const float wt = w[t];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { odd = odd || tl_chunk_odd(x[j][e]); x[j][e] *= wt; }
+                lw_put8(ks + swz(C, t, c), PK, x[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < VPER; ++j) {
+                if (VN % LW_WORK && tid >= VN) continue;
+                const int t = 32 * i + (tid + LW_WORK * j) / (CB / 8), c = (tid + LW_WORK * j) % (CB / 8);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) odd = odd || tl_chunk_odd(y[j][e]);
+                lw_put8(vs + swz(C, t, c), PV, y[j]);
+            }
+            lw_filled(B.full + i, lane);
+            if (i + 2 < stages) fetch(x, y, i + 2);
+        };
+        fetch(keys[0], values[0], 0);
+        fetch(keys[1], values[1], 1);
+#pragma unroll 1
+        for (int i = 0; i < stages; i += 2) {
+            fill(keys[0], values[0], i);
+            if (i + 1 < stages) fill(keys[1], values[1], i + 1);
+        }
+    }
+    odd = __syncthreads_or(odd);                         // (also: all of K is there for the normaliser)
+    if (tid == 0) A.marked[ch * A.tiles + blockIdx.z] = odd;
+    if (warp < LW_MMA) {
+        const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
+        float* to = A.ends + ch * per;
+        if (GATED && col0 == 0 && tid < DP && tid < d) { // the normaliser: the same with v = 1, sixteen chains of eight tokens
+            float s[16] = {};
+            for (int t = 0; t < 32 * stages; t += 16)
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    const unsigned char* k = ks + swz(C, t + r, tid >> 3) + (tid & 7) * 2;
+                    auto part = [&](int p) { return __bfloat162float(*reinterpret_cast<const bf16*>(k + p * PK)); };
+                    s[r] += part(0) + (part(1) + part(2));
+                }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+                for (int r = 0; r < o; ++r) s[r] += s[r + o];
+            to[(size_t)d * A.dv + tid] = s[0];
+        }
+        const int quarter = warp & 3, share = warp >> 2;
+        float sum[HC];
+#pragma unroll
+        for (int c = 0; c < HC; ++c) sum[c] = 0.f;
+        for (int i = 0; i < stages; ++i) {
+            mbar_wait(B.done + i, 0, gave_up, A.status, 62);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            lw_add(sum, tmem + ((uint32_t)(quarter * 32) << 16) + i * 128 + share * HC);
+        }
+        lw_store<CB>(reinterpret_cast<float*>(vs), sum, to + col0, A.dv, d, A.dv - col0, nullptr, nullptr);      // (V is read)
+    }
+    lw_end(B, warp, tmem);
+}
+
+// grid (chunks, H, slices of NT tiles of CB columns)
+template <int DP, int CB, int NT, bool GATED>
+__global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunkArgs A) {
+    constexpr int C = LC_WIDE, PQ = C * DP * 2, PP = C * C * 2, PS = 32 * CB * 2, HC = CB / 4, GROUPS = DP / 32;      // bytes of a part of Q and K, of P, of a stage
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* qs = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);            // Q, then P
+    unsigned char* ks = qs + LW_REGION;                                                                               // K, then the ring
+    __shared__ LwBars B;
+    __shared__ double rowsum[4][C], nq[C];
+    __shared__ float2 u[C];                              // a double as two floats
+    __shared__ float below[C];                           // e^(u less the largest of its 32 keys)
+    __shared__ double most[4];                           // that
+    __shared__ float coef[C], den[C], over[C];
+    const int4 ck = A.chunks[blockIdx.x];
+    const int h = blockIdx.y, col0 = blockIdx.z * NT * CB, d = A.d;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int t0 = A.q_start[ck.x] + ck.y * C, n = min(C, A.q_start[ck.x + 1] - t0), nv = (n + 31) / 32, stages = NT * (GROUPS + nv);      // stages: Q S of every tile, P V of every tile
+    if (GATED) lc_maximum<DP>(A, ck, h);
+    const size_t ch = (size_t)blockIdx.x * A.H + h, per = (size_t)d * A.dv + (GATED ? d : 0);
+    const float* start = A.ends + ch * per;
+    const double m0 = GATED ? A.marks[ch * 3 + 2] : 0.0;
+    lw_start(B, warp);
+    if (warp < LW_MMA) {
+        constexpr int PER = C * DP / 8 / LW_WORK, PR = DP / 8, N = 2;        // pieces of eight a thread, of a row; on their way together
+        float norm[8], x[2][N][8];
+        if (GATED) lw_get8(norm, start + (size_t)d * A.dv + tid % PR * 8, true, d - tid % PR * 8);
+        auto get = [&](float (&to)[N][8], int j0) {      // Q's pieces, then K's
+            const float* from = (j0 < PER ? A.q : A.k) + h * d + tid % PR * 8;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int t = (tid + LW_WORK * (j0 + j - (j0 < PER ? 0 : PER))) / PR;
+                lw_get8(to[j], from + (size_t)(t0 + t) * A.qk_stride, t < n && j0 < 2 * PER, d - tid % PR * 8);
+            }
+        };
+        auto put = [&](float (&v)[N][8], int j0) {
+            const bool isq = j0 < PER;
+            const float scale = isq ? A.q_scale : A.k_scale;
+#pragma unroll
+            for (int j = 0; j < N; ++j) {
+                const int t = (tid + LW_WORK * (j0 + j - (isq ? 0 : PER))) / PR;
+                float nr[2] = {0.f, 0.f};                // n . q of the chunk's start state
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    v[j][e] *= scale;
+                    if (GATED) nr[e & 1] = fmaf(v[j][e], norm[e], nr[e & 1]);
+                }
+                lw_put8((isq ? qs : ks) + swz(C, t, tid % PR), PQ, v[j]);
+                if (GATED && isq) {
+                    LwSum r;
+                    r.add(nr[0]);
+                    r.add(nr[1]);
+#pragma unroll
+                    for (int o = 1; o < PR; o <<= 1) {
+                        const float lost = __shfl_xor_sync(0xffffffffu, r.lost, o);
+                        r.add(__shfl_xor_sync(0xffffffffu, r.s, o));
+                        r.lost += lost;
+                    }
+                    if (lane % PR == 0) nq[t] = r.value();
+                }
+            }
+        };
+        get(x[0], 0);
+#pragma unroll 1
+        for (int j0 = 0; j0 < 2 * PER; j0 += 2 * N) {
+            get(x[1], j0 + N);
+            put(x[0], j0);
+            get(x[0], j0 + 2 * N);
+            put(x[1], j0 + N);
+        }
+        fence_async_proxy();
+    }
+    auto pair = [](double x) { const float hi = (float)x; return make_float2(hi, (float)(x - (double)hi)); };
+    float2 top = make_float2(0.f, 0.f);                  // a token's running maximum less F; u: what is added to it for a weight
+    if (warp < LW_MMA) {
+        const int t = tid & (C - 1);                     // the worker's token: all that share it need top
+        double uv;
+        if (GATED) {
+            const double* w = A.weights + ch * 3 * C;
+            const double f = w[t], mm = fmax(m0, w[2 * C + t]);
+            uv = w[C + t];
+            if (tid < C) { coef[t] = (float)exp(m0 - mm); den[t] = expf((float)(-(f + mm))); }
+            top = pair(-mm);
+        } else {
+            const double f = (t + 1) * log((double)A.decay[h]);
+            uv = -f;
+            if (tid < C) coef[t] = (float)exp(f);
+            top = pair(f);
+        }
+        if (warp < 4) {
+            u[t] = pair(uv);
+            double best = t < n ? uv : -INFINITY;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
+            below[t] = expf((float)(uv - best));
+            if (lane == 0) most[warp] = best;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = B.tmem;
+    volatile int* gave_up = &B.gave_up;
+    if (warp == LW_MMA) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 4) << 24);
+        const uint32_t one = lw_elect(), qa = smem_addr(qs), ka = smem_addr(ks);
+        auto kmajor = [&](uint32_t tile, int k) { return tile + (k >> 2) * C * 128 + (k & 3) * 32; };       // k in steps of 16
+#pragma unroll
+        for (int i = 0; i < GROUPS; ++i)
+            lw_parts(tmem + i * 128, idesc | ((uint32_t)(C >> 3) << 17), one, [&](int p, int k) { return desc_kmajor(kmajor(qa + p * PQ, 2 * i + k)); },
+                     [&](int p, int k) { return desc_kmajor(kmajor(ka + p * PQ, 2 * i + k)); });
+        lw_commit(&B.qk, one);
+        uint32_t slot = 0;
+        int group = 0;
+        for (int i = 0; i < stages; ++i) {
+            const bool values = i >= NT * GROUPS;
+            if (!mbar_wait(B.full + (i & 3), (i >> 2) & 1, gave_up, A.status, 63)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t st = ka + (i & 3) * 3 * PS, at = kmajor(qa, 2 * group), part = values ? PP : PQ;
+            lw_parts(tmem + 128 + slot * 128, idesc | (1u << 16) | ((uint32_t)(CB >> 3) << 17), one,
+                     [&](int p, int k) { return desc_kmajor(at + p * part + k * 32); },
+                     [&](int p, int k) { return desc_mnmajor(st + p * PS + k * 16 * 128, 32 * 128); });
+            lw_commit(B.done + (i & 3), one);
+            slot = slot == 2 ? 0 : slot + 1;
+            group = group + 1 == (values ? nv : GROUPS) ? 0 : group + 1;
+        }
+    } else {
+        constexpr int SN = 32 * CB / 8, SPER = (SN + LW_WORK - 1) / LW_WORK;     // pieces of eight a stage, a thread
+        static_assert(SPER == 1, "a piece a thread");
+        const int quarter = warp & 3, share = warp >> 2, t = quarter * 32 + lane;
+        const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
+        const int r = tid / (CB / 8), col = tid % (CB / 8) * 8;
+        float ahead[2][8];
+        // 32 rows of S, then of V, tile after tile; zeros where there are none.  A cursor over the stages: the next one's first row and tile.
+        const float* from_s = start + (size_t)r * A.dv + col0 + col;
+        const float* from_v = A.v + (size_t)(t0 + r) * A.v_stride + h * A.dv + col0 + col;
+        int next_row = r, next_col = col0 + col;
+        bool values = false;
+        auto fetch = [&](float (&y)[8]) {
+            const int z = next_col - col0 - col, rows = values ? n : d;
+            const float* from = values ? from_v + (size_t)(next_row - r) * A.v_stride + z : from_s + (size_t)(next_row - r) * A.dv + z;
+            if (SN % LW_WORK == 0 || tid < SN) lw_get8(y, from, next_row < rows, A.dv - next_col);
+            next_row += 32;
+            if (next_row - r >= (values ? 32 * nv : DP)) {
+                next_row = r;
+                next_col += CB;
+                if (next_col - col0 >= NT * CB) { next_col = col0 + col; values = true; }
+            }
+        };
+        fetch(ahead[0]);
+        fetch(ahead[1]);
+        mbar_wait(&B.qk, 0, gave_up, A.status, 64);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const bool sees = share <= quarter;              // keys behind all of the warp's tokens weigh nothing
+        if (sees) {                                      // Q K^T into the first accumulator, so that the others are free for the stages
+#pragma unroll 1
+            for (int c = 32 * share; c < 32 * share + 32; c += 16) {
+                float v[16], r[16];
+                lw_ld16(acc + c, v);
+#pragma unroll
+                for (int i = 1; i < GROUPS; ++i) {
+                    lw_ld16(acc + i * 128 + c, r);
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) v[x] += r[x];
+                }
+                lw_st16(acc + c, v);
+            }
+        }
+        float sum[NT][HC];
+#pragma unroll
+        for (int z = 0; z < NT; ++z)
+#pragma unroll
+            for (int c = 0; c < HC; ++c) sum[z][c] = 0.f;
+        int taken = 0, tile = 0, group = 0;
+        uint32_t from = acc + 128 + share * HC;
+        auto take = [&](int below) {                     // the accumulators of the stages below
+#pragma unroll 1
+            for (; taken < below; ++taken) {
+                mbar_wait(B.done + (taken & 3), (taken >> 2) & 1, gave_up, A.status, 65);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int z = 0; z < NT; ++z) if (tile == z) lw_add(sum[z], from);
+                from = from == acc + 384 + share * HC ? acc + 128 + share * HC : from + 128;
+                if (++group == (taken < NT * GROUPS ? GROUPS : nv)) { group = 0; tile = tile + 1 == NT ? 0 : tile + 1; }
+            }
+        };
+        auto weigh = [&]() {                             // all of Q S is there: the token's weight; P takes Q's place
+            take(NT * GROUPS);
+            const float weight = coef[t];
+#pragma unroll
+            for (int z = 0; z < NT; ++z)
+#pragma unroll
+                for (int c = 0; c < HC; ++c) sum[z][c] *= weight;
+            LwSum total;
+            const int last = t < n ? t : -1;
+            // 32 keys before all of the warp's tokens: their weights are this times `below`, neither above one
+            const float base = t < n ? expf((float)(((double)top.x + (double)top.y) + most[share])) : 0.f;
+#pragma unroll 1
+            for (int s = 32 * share; s < 32 * share + 32; s += 8) {
+                float P[8] = {};
+                if (sees) {
+                    lw_ld8(acc + s, P);
+                    if (share < quarter) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) P[e] *= base * below[s + e];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {    // no branch in here (a key behind the token weighs e^-inf): the chains overlap
+                            const float2 v = u[s + e];
+                            const float y = top.x + v.x, b = y - top.x;      // the sum of two doubles, rounded once
+                            const float x = y + (((top.x - (y - b)) + (v.x - b)) + (top.y + v.y));
+                            P[e] *= expf(s + e <= last ? x : -INFINITY);
+                        }
+                    }
+                    if (GATED) total.add(((P[0] + P[1]) + (P[2] + P[3])) + ((P[4] + P[5]) + (P[6] + P[7])));
+                }
+                lw_put8(qs + swz(C, t, s / 8), PP, P);
+            }
+            if (GATED) {
+                rowsum[share][t] = total.value();
+                lw_sync();
+                if (share == 0) {
+                    den[t] = fmaxf(fabsf((float)((rowsum[0][t] + rowsum[1][t]) + (rowsum[2][t] + rowsum[3][t]) + coef[t] * nq[t])), den[t]) + A.den_eps;
+                    over[t] = 1.0f / den[t];
+                }
+            }
+        };
+        auto fill = [&](float (&y)[8], int i) {
+            take(i - 2);                                 // three accumulators: the stage three before has been read
+            if (!(SN % LW_WORK) || tid < SN) lw_put8(ks + (i & 3) * 3 * PS + swz(32, r, tid % (CB / 8)), PS, y);
+            lw_filled(B.full + (i & 3), lane);
+            if (i + 2 < stages) fetch(y);
+        };
+        static_assert(GROUPS % 2 == 0, "two stages at a time");
+#pragma unroll 1
+        for (int i = 0; i < stages; i += 2) {
+            if (i == NT * GROUPS) weigh();
+            fill(ahead[0], i);
+            if (i + 1 < stages) fill(ahead[1], i + 1);
+        }
+        take(stages);
+        // (the ring is read: its last sums have been taken; the barrier in there stands between den and its readers)
+#pragma unroll
+        for (int z = 0; z < NT; ++z) {
+            if (z) lw_sync();
+            lw_store<CB>(reinterpret_cast<float*>(ks), sum[z], A.out + (size_t)t0 * A.H * A.dv + (size_t)h * A.dv + col0 + z * CB, (size_t)A.H * A.dv, n,
+                         A.dv - col0 - z * CB, GATED ? den : nullptr, over);
+        }
+    }
+    lw_end(B, warp, tmem);
+}
+
+template <int DP, int CB, bool GATED>
+static int lw_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
+    static bool r1[TL_MAX_DEVICES] = {}, r2[TL_MAX_DEVICES] = {};
+    static bool r3[TL_MAX_DEVICES] = {};
+    int e = tl_raise_smem(lw_local_kernel<DP, CB, GATED>, r1, LW_SMEM);
+    if (!e) e = tl_raise_smem(lw_out_kernel<DP, CB, 1, GATED>, r2, LW_SMEM);
+    if (!e) e = tl_raise_smem(lw_out_kernel<DP, CB, 2, GATED>, r3, LW_SMEM);
+    if (e) return e;
+    const int tiles = (A.dv + CB - 1) / CB;
+    if (GATED) {
+        lc_gates_kernel<LC_WIDE><<<dim3(n_chunks, A.H), 32, 0, stream>>>(A);
+        if ((e = tl_launch_status())) return e;
+    }
+    lw_local_kernel<DP, CB, GATED><<<dim3(n_chunks, A.H, tiles), LW_THREADS, LW_SMEM, stream>>>(A);
+    if ((e = tl_launch_status())) return e;
+    const size_t per = (size_t)A.d * A.dv + (GATED ? A.d : 0);
+    lc_carry_kernel<8, DP / 8, GATED><<<dim3((unsigned)((per / 4 + 255) / 256), A.H, requests), 256, 0, stream>>>(A);
+    if ((e = tl_launch_status())) return e;
+    // Two tiles a block share its Q K^T and weights; where single tiles fit the GPU at once, they are done sooner.
+    if ((long long)n_chunks * A.H * tiles > tl_num_sms() && tiles > 1)
+        lw_out_kernel<DP, CB, 2, GATED><<<dim3(n_chunks, A.H, (tiles + 1) / 2), LW_THREADS, LW_SMEM, stream>>>(A);
+    else
+        lw_out_kernel<DP, CB, 1, GATED><<<dim3(n_chunks, A.H, tiles), LW_THREADS, LW_SMEM, stream>>>(A);
+    return tl_launch_status();
+}
+
+template <int DP>
+static int lw_pick(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
+    if (A.gates) return A.dv <= 64 ? lw_launch<DP, 64, true>(A, n_chunks, requests, stream) : lw_launch<DP, 128, true>(A, n_chunks, requests, stream);
+    return A.dv <= 64 ? lw_launch<DP, 64, false>(A, n_chunks, requests, stream) : lw_launch<DP, 128, false>(A, n_chunks, requests, stream);
+}
+
 template <int DP, int CB, bool GATED>
 static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaStream_t stream) {
     constexpr int RB = DP < 128 ? DP : 128, R = DP == 32 ? 4 : 8, IS = DP / R;
@@ -651,7 +1241,7 @@ static int lc_launch(const LinearChunkArgs& A, int n_chunks, int requests, cudaS
     if (e) return e;
     const int col_tiles = (A.dv + CB - 1) / CB, row_tiles = (A.d + RB - 1) / RB;
     if (GATED) {
-        lc_gates_kernel<<<dim3(n_chunks, A.H), 32, 0, stream>>>(A);
+        lc_gates_kernel<LC_C><<<dim3(n_chunks, A.H), 32, 0, stream>>>(A);
         if ((e = tl_launch_status())) return e;
     }
     lc_local_kernel<RB, CB, GATED><<<dim3(n_chunks, A.H, row_tiles * col_tiles), 256, local_smem, stream>>>(A);
@@ -674,22 +1264,24 @@ static int lc_tiles(int d, int dv) {
     const int cb = dv <= 64 ? 64 : 128, rb = d <= 32 ? 32 : d <= 64 ? 64 : 128;
     return ((d + rb - 1) / rb) * ((dv + cb - 1) / cb);
 }
-TL_EXPORT int tl_linear_chunk() { return LC_C; }
+// Tokens a chunk; the wide ones where heads have the rows for them (else 0).
+TL_EXPORT int tl_linear_chunk(int d, int wide) { return !wide ? LC_C : d > 32 && d <= 128 ? LC_WIDE : 0; }
 TL_EXPORT int tl_linear_chunk_tiles(int d, int dv) { return lc_tiles(d, dv); }
 
 // `rows` (float [T, 2 H d], with a rotation): where q and k go.  ends: float [n_chunks, H, d dv (+ d with gates)], marks: double
-// [n_chunks, H, 3], with gates then [n_chunks, H, 192].  marked: int [n_chunks, H, tl_linear_chunk_tiles(d, dv)], for the scan kernel.  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
+// [n_chunks, H, 3], with gates then [n_chunks, H, 3 chunk].  chunk: what a chunk of `chunks` holds, one of tl_linear_chunk's.  marked: int [n_chunks, H, tl_linear_chunk_tiles(d, dv)], for the scan kernel.  d, dv, the offsets and the stride are multiples of 4 and the pointers 16-byte aligned.
 TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, int k_off, int v_off, const float* gates, float cap,
                                const float* decay, const float* inv_freq, int rot, int interleaved, const int* pos, float q_scale,
                                float k_scale, float* rows, float* state, long long slot_stride, const int* q_start, const int* slots,
                                const int* chunks, int n_chunks, const int* firsts, int requests, float* ends, double* marks, int* marked, float* out,
-                               int H, int d, int dv, float den_eps, cudaStream_t stream) {
+                               int H, int d, int dv, float den_eps, int chunk, int* status, cudaStream_t stream) {
     if (n_chunks <= 0 || H <= 0) return 0;
+    if (status == nullptr || (chunk != LC_C && chunk != tl_linear_chunk(d, 1))) return 1;
     if (H > 65535 || requests > 65535 || d < 4 || d > 256 || ((d | dv | stride | q_off | k_off | v_off) & 3) || (rot & 1) || rot > d ||
         (rot && !rows) || (gates != nullptr) == (decay != nullptr) ||
         ((((uintptr_t)proj) | ((uintptr_t)rows) | ((uintptr_t)ends) | ((uintptr_t)out)) & 15)) return 1;
     LinearChunkArgs A{proj + q_off, proj + k_off, stride, proj + v_off, stride, gates, cap, decay, q_scale, k_scale, state, slot_stride,
-                      q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, marked, lc_tiles(d, dv), out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps};
+                      q_start, slots, (const int4*)chunks, firsts, ends, marks, marks + (size_t)n_chunks * H * 3, marked, lc_tiles(d, dv), out, H, d, dv, (dv + LC_COLS - 1) / LC_COLS, den_eps, status};
     if (rot) {
         if (rot % (interleaved ? 4 : 8) == 0)
             lc_rotate_kernel<true><<<T, 256, rot * sizeof(float), stream>>>(proj, stride, q_off, k_off, inv_freq, rot, interleaved, pos, q_scale, k_scale, rows, H, d);
@@ -701,6 +1293,7 @@ TL_EXPORT int tl_linear_chunks(const float* proj, int T, int stride, int q_off, 
         A.q_scale = A.k_scale = 1.0f;
     }
     if (d <= 32) return lc_pick<32>(A, n_chunks, requests, stream);
+    if (chunk == LC_WIDE) return d <= 64 ? lw_pick<64>(A, n_chunks, requests, stream) : lw_pick<128>(A, n_chunks, requests, stream);
     if (d <= 64) return lc_pick<64>(A, n_chunks, requests, stream);
     if (d <= 128) return lc_pick<128>(A, n_chunks, requests, stream);
     return lc_pick<256>(A, n_chunks, requests, stream);

@@ -43,8 +43,8 @@ _SIGNATURES = {
     "tl_channel_scan": [_P, _I, _I, _I, _I, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
     "tl_channel_chunk": [],
     "tl_linear_chunks": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P,
-                         _P, _P, _I, _I, _I, _F, _P],
-    "tl_linear_chunk": [],
+                         _P, _P, _I, _I, _I, _F, _P, _P],
+    "tl_linear_chunk": [_I, _I],
     "tl_linear_chunk_tiles": [_I, _I],
     "tl_scan_state_floats": [_I, _I],
     "tl_scan_columns": [],
@@ -173,6 +173,9 @@ STATUS_ROLES = {1: "tcgen05 product: the copy thread waited for a free stage", 2
                 47: "experts' product: the MMA thread waited for a stage's copies", 48: "experts' product: the epilogue waited for the accumulator",
                 51: "delta rule's chunks: the chain waited for W", 52: "delta rule's chunks: the chain waited for K and U",
                 53: "delta rule's chunks: the outputs waited for Q and P",
+                61: "matrix memory's end states: the MMA warp waited for a stage", 62: "matrix memory's end states: the workers waited for a sum",
+                63: "matrix memory's outputs: the MMA warp waited for a stage", 64: "matrix memory's outputs: the workers waited for Q K",
+                65: "matrix memory's outputs: the workers waited for a sum",
                 20: "decode attention: a wait for a stage of keys and values"}
 
 
@@ -843,6 +846,28 @@ LINEAR_CHUNKS_MIN_TOKENS = {True: 128, False: 192}       # by whether the decays
 LINEAR_CHUNKS_LEAST_TOKENS = 16
 
 
+# Heads of 33 to 128 rows run in chunks of 128 tokens on the 5th-generation tensor cores where a step has this many blocks of 64 tokens, a head and
+# 128 columns, by the rows of its heads (above 64 or not), and its requests fill the longer chunks (at most WIDE_CHUNKS_SHARE of the shorter
+# ones).  Chunks of 64 / 128, us: gated 8 heads of 128 x 256, 256 tokens (64 blocks) 52 / 52, 400 (112) 56 / 52, 1,024 (256) 71 / 56, 2,048
+# (512) 127 / 85; 4 heads of 128 x 128, 512 tokens (32) 50 / 50, 1,024 (64) 54 / 52, 2,048 (128) 63 / 54; 8 of 64 x 256, 512 tokens (128)
+# 42 / 46, 1,024 (256) 54 / 48; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 103, of 64 x 256 66 / 77.
+WIDE_CHUNKS_BLOCKS = {False: 200, True: 96}
+WIDE_CHUNKS_SHARE = 0.65
+
+
+def _wide_chunks(ctx, least: int, H: int, d: int, dv: int) -> bool:
+    lib = core()
+    wide, narrow = lib.tl_linear_chunk(d, 1), lib.tl_linear_chunk(d, 0)
+    if not wide:
+        return False
+    key = ("chunk counts", least)
+    if key not in ctx.scratch:                           # once a step
+        long = [n for n in (b - a for a, b in zip(ctx.h_q_start, ctx.h_q_start[1:])) if n >= least]
+        ctx.scratch[key] = sum(-(-n // narrow) for n in long), sum(-(-n // wide) for n in long)
+    short, tall = ctx.scratch[key]
+    return short * H * -(-dv // 128) >= WIDE_CHUNKS_BLOCKS[d > 64] and tall <= WIDE_CHUNKS_SHARE * short
+
+
 def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gated: bool) -> bool:
     """Whether `linear_chunks` takes these sizes (q, k, v one behind the other in a projection's row) and is the faster way."""
     return proj.dtype == torch.float32 and max_q_len >= LINEAR_CHUNKS_MIN_TOKENS[gated] and d % 4 == 0 and dv % 4 == 0 and d <= 256 and \
@@ -910,8 +935,9 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
         raise KernelError("linear_chunks: inv_freq must be float32 [rot/2]")
     interleaved = _pairing(pairing, "linear_chunks")
     lib, dev = core(), proj.device
-    step = _chunk_list(ctx, "linear_chunks", lib.tl_linear_chunk(), least, dev)
-    n, tiles, doubles = step.n, lib.tl_linear_chunk_tiles(d, dv), 3 if gates is None else 195
+    chunk = lib.tl_linear_chunk(d, int(_wide_chunks(ctx, least, H, d, dv)))
+    step = _chunk_list(ctx, ("linear_chunks", chunk), chunk, least, dev)
+    n, tiles, doubles = step.n, lib.tl_linear_chunk_tiles(d, dv), 3 if gates is None else 3 + 3 * chunk
     turned = torch.empty((T, 2 * H * d), dtype=torch.float32, device=dev) if rot else None
     ends = torch.empty((n, H, d * dv + (d if gates is not None else 0)), dtype=torch.float32, device=dev)
     marks = torch.empty(n * H * (2 * doubles + tiles), dtype=torch.int32, device=dev)        # doubles, then marks of operands
@@ -920,7 +946,7 @@ def linear_chunks(proj: torch.Tensor, q_off: int, k_off: int, v_off: int, H: int
              float(k_scale))
     _check(lib.tl_linear_chunks(_ptr(proj), T, proj.shape[1], q_off, k_off, v_off, *heads, _ptr(turned), _ptr(state), per_slot, _ptr(ctx.q_start),
                                 _ptr(ctx.slots), step.rows, n, step.firsts, step.long, _ptr(ends), _ptr(marks), marked, _ptr(out), H, d, dv,
-                                float(den_eps), _stream()), "linear_chunks", launches=3 + bool(rot) + (gates is not None))
+                                float(den_eps), chunk, _ptr(device_status(dev)), _stream()), "linear_chunks", launches=3 + bool(rot) + (gates is not None))
     _check(lib.tl_linear_scan(_ptr(proj), dtype_code(proj.dtype), proj.shape[1], q_off, k_off, v_off, *heads, _ptr(state), per_slot,
                               _ptr(ctx.q_start), _ptr(ctx.slots), _ptr(out), step.requests, H, d, dv, float(den_eps), 0, None, None, step.runs,
                               marked, tiles, _stream()), "linear_scan")
