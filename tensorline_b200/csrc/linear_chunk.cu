@@ -667,9 +667,10 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) lc_out_kernel(const Li
 //               and three accumulators; P takes Q's place, then P V likewise.
 // Loops stay rolled: a block runs once through its code, and what is not in the instruction cache comes at one instruction in
 // about 13 cycles (the weights unrolled over a worker's 64 keys took 18,000 cycles).
-//   end states  K^T V, 32 tokens a stage, nothing is used twice.
-// Measured beside the mma.sync kernels (chunks of 64), 8 heads of 128 x 256, 2,048 tokens: end states 19 us (28), start states 12 (18),
-// outputs 39 (65); all of a gated memory 85 (127), a fixed decay's 73 (103).  A block runs its phases one after the other, about 35 us whatever else
+//   end states  K^T V, 32 tokens a stage; states pass their errors on, so the leading product of every 16 tokens has an accumulator of its
+//               own (in one with the small ones a state is 2e-8 nearer to zero), four in turn.
+// Measured beside the mma.sync kernels (chunks of 64), 8 heads of 128 x 256, 2,048 tokens: end states 23 us (28), start states 12 (18),
+// outputs 39 (65); all of a gated memory 89 (127), a fixed decay's 77 (103).  A block runs its phases one after the other, about 35 us whatever else
 // there is, so short steps stay with the chunks of 64 (ops.py).
 constexpr int LW_WORK = 512, LW_THREADS = LW_WORK + 32, LW_MMA = LW_WORK / 32, LW_REGION = 3 * LC_WIDE * LC_WIDE * 2;
 constexpr int LW_SMEM = 2 * LW_REGION + 1024;
@@ -693,12 +694,13 @@ __device__ __forceinline__ void lw_commit(uint64_t* bar, uint32_t one) {
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
                  ::"r"(smem_addr(bar)), "r"(one) : "memory");
 }
-// The six products of parts of 32 k into `acc`, the small ones first.  a(p, k), b(p, k): descriptors of part p, k in steps of 16.
-template <typename FA, typename FB>
+// The six products of parts (or the five small ones) of 32 k into `acc`, the small ones first.  a(p, k), b(p, k): descriptors of part p, k in
+// steps of 16.
+template <int PRODUCTS = 6, typename FA, typename FB>
 __device__ __forceinline__ void lw_parts(uint32_t acc, uint32_t idesc, uint32_t one, FA a, FB b) {
     constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
-    for (int i = 0; i < 6; ++i)
+    for (int i = 0; i < PRODUCTS; ++i)
 #pragma unroll
         for (int k = 0; k < 2; ++k) lw_mma(acc, a(pa[i], k), b(pb[i], k), idesc, (i || k) ? 1u : 0u, one);
 }
@@ -798,11 +800,11 @@ struct LwSum {
     }
     __device__ __forceinline__ double value() const { return (double)s + (double)lost; }
 };
-struct LwBars { uint64_t qk, full[4], done[4]; uint32_t tmem; int gave_up; };
+struct LwBars { uint64_t qk, full[4], done[4], free[4]; uint32_t tmem; int gave_up; };
 __device__ __forceinline__ void lw_start(LwBars& B, int warp) {
     if (threadIdx.x == 0) {
         mbar_init(&B.qk, 1);
-        for (int i = 0; i < 4; ++i) { mbar_init(B.full + i, LW_MMA); mbar_init(B.done + i, 1); }
+        for (int i = 0; i < 4; ++i) { mbar_init(B.full + i, LW_MMA); mbar_init(B.done + i, 1); mbar_init(B.free + i, LW_MMA); }
         B.gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -818,6 +820,12 @@ __device__ __forceinline__ void lw_end(LwBars& B, int warp, uint32_t tmem) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
+}
+// a barrier of the workers alone (the MMA warp may be waiting for them): does `x` hold for any?
+__device__ __forceinline__ bool lw_workers_or(bool x) {
+    int any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.s32 %0, 1, 0, q;\n}" : "=r"(any) : "r"((int)x), "n"(LW_WORK) : "memory");
+    return any != 0;
 }
 // a worker warp's part of a stage is in shared memory
 __device__ __forceinline__ void lw_filled(uint64_t* bar, int lane) {
@@ -860,13 +868,20 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChu
         // A: K^T, B: V, both MN-major; heads of up to 64 rows: the upper half of the tile is whatever lies behind, and nobody reads it
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(CB >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const uint32_t one = lw_elect(), ka = smem_addr(ks), va = smem_addr(vs);
+        int g = 0;
         for (int i = 0; i < stages; ++i) {
             if (!mbar_wait(B.full + i, 0, gave_up, A.status, 61)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            lw_parts(tmem + i * 128, idesc, one,
-                     [&](int p, int k) { return desc_mnmajor(ka + p * PK + (i * 2 + k) * 16 * 128, C * 128); },
-                     [&](int p, int k) { return desc_mnmajor(va + p * PV + (i * 2 + k) * 16 * 128, C * 128); });
-            lw_commit(B.done + i, one);
+            auto k_at = [&](int p, int k) { return desc_mnmajor(ka + p * PK + (i * 2 + k) * 16 * 128, C * 128); };
+            auto v_at = [&](int p, int k) { return desc_mnmajor(va + p * PV + (i * 2 + k) * 16 * 128, C * 128); };
+            for (int a = 0; a < 3; ++a, ++g) {           // the leading product of 16 tokens, of the next 16, the small ones of both
+                const uint32_t acc = tmem + (g & 3) * 128;
+                if (g >= 4 && !mbar_wait(B.free + (g & 3), ((g >> 2) - 1) & 1, gave_up, A.status, 66)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (a < 2) lw_mma(acc, k_at(0, a), v_at(0, a), idesc, 0u, one);
+                else lw_parts<5>(acc, idesc, one, k_at, v_at);
+                lw_commit(B.done + (g & 3), one);
+            }
         }
     } else {
         constexpr int KN = 32 * DP / 8, VN = 32 * CB / 8, KPER = (KN + LW_WORK - 1) / LW_WORK, VPER = (VN + LW_WORK - 1) / LW_WORK;      // pieces of eight a stage, a thread
@@ -914,9 +929,9 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChu
             if (i + 1 < stages) fill(keys[1], values[1], i + 1);
         }
     }
-    odd = __syncthreads_or(odd);                         // (also: all of K is there for the normaliser)
-    if (tid == 0) A.marked[ch * A.tiles + blockIdx.z] = odd;
     if (warp < LW_MMA) {
+        odd = lw_workers_or(odd);                        // (also: all of K is there for the normaliser)
+        if (tid == 0) A.marked[ch * A.tiles + blockIdx.z] = odd;
         const size_t per = (size_t)d * A.dv + (GATED ? d : 0);
         float* to = A.ends + ch * per;
         if (GATED && col0 == 0 && tid < DP && tid < d) { // the normaliser: the same with v = 1, sixteen chains of eight tokens
@@ -938,10 +953,14 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChu
         float sum[HC];
 #pragma unroll
         for (int c = 0; c < HC; ++c) sum[c] = 0.f;
-        for (int i = 0; i < stages; ++i) {
-            mbar_wait(B.done + i, 0, gave_up, A.status, 62);
+#pragma unroll 1
+        for (int g = 0; g < 3 * stages; ++g) {
+            mbar_wait(B.done + (g & 3), (g >> 2) & 1, gave_up, A.status, 62);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            lw_add(sum, tmem + ((uint32_t)(quarter * 32) << 16) + i * 128 + share * HC);
+            lw_add(sum, tmem + ((uint32_t)(quarter * 32) << 16) + (g & 3) * 128 + share * HC);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(B.free + (g & 3));
         }
         lw_store<CB>(reinterpret_cast<float*>(vs), sum, to + col0, A.dv, d, A.dv - col0, nullptr, nullptr);      // (V is read)
     }
