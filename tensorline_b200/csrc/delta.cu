@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(128) conv_prep_kernel(const TA* __restrict__ p
     }
 }
 
-// The same for steps of many tokens: a block a (request, chunk of `tt` tokens, head); the chunk's rows of the head, with the
+// The same for steps of many tokens and any taps: a block a (request, chunk of `tt` tokens, head); the chunk's rows of the head, with the
 // taps - 1 rows in front of them, and the head's weights are brought into shared memory once (all loads in flight), then a warp
 // a token.  The arithmetic of an output is conv_prep_kernel's, operation for operation, so both give the same bits.
 template <typename TA, typename TW>
@@ -144,29 +144,27 @@ __global__ void __launch_bounds__(256) conv_prep_tile_kernel(const TA* __restric
     }
 }
 
-// The same for steps of many tokens and 2 to 4 taps: a warp a (request, run of CONV_RUN tokens, head); a lane has channels lane + 32 m
-// of the head, their weights and the last taps - 1 inputs in registers, and the next token's inputs on their way while one is worked
-// through: a channel and token cost it one load and no index arithmetic.  What is left is the accurate exponential and division
-// of silu, about 35 instructions an output (134 with rows and weights in shared memory): 2,048 tokens, 3,072 channels 25 us against
-// 47.  The arithmetic of an output is conv_prep_kernel's, operation for operation, so all give the same bits.
-// A run is a chain of 16 tokens, 14 us however little there is; so it takes steps of CONV_RUN_WORK outputs (with the update of the
-// inputs, tile kernel / runs: 1,024 tokens of 3,072 channels 22.5 / 20.5 us, 2,048 of 1,280 20.3 / 20.0, 2,048 of 2,048 26.3 / 23.1; 512 of
-// 4,096 16.4 / 18.6, 512 of 3,072 14.7 / 16.4, 1,024 of 2,048 19.8 / 21.8, 2,048 of 512 11.4 / 16.2), and of CONV_RUN_SOME where most
-// blocks of the tile kernel's grid would find nothing (48 single tokens beside 464 of 3,072 channels 32.5 / 27.0 us, beside
-// 200 25.2 / 23.0; of 1,280 channels, 200 tokens 15.0 / 18.3).
-constexpr int CONV_RUN = 16;
-constexpr long long CONV_RUN_WORK = 2500000, CONV_RUN_SOME = 600000, CONV_RUN_GRID = 5000;
+// The same for 2 to 4 taps: a warp a (request, run of 4 or 8 tokens, head); a lane has channels lane + 32 m of the head, their weights and
+// the last taps - 1 inputs in registers, and the next token's inputs on their way while one is worked through: a channel and token cost it
+// one load and no index arithmetic.  What is left is the accurate exponential and division of silu, about 35 instructions an output (134 with
+// rows and weights in shared memory).  The arithmetic of an output is conv_prep_kernel's, operation for operation, so all give the same bits.
+// A run is a chain, 0.9 us a token however little there is, and a longer one reads fewer rows and weights twice: runs of 8, and of 4 where the
+// grid's warps (those that find nothing too) are no more than CONV_RUN_WARPS.  With the update of the inputs, us, runs of 16 or the tile kernel
+// (as was the rule) / runs of 8 / of 4: 3,072 channels in 16 heads, 128 tokens (256 warps) 23.6 / 17.4 / 13.3, 512 (1,024) 23.6 / 17.4 / 15.4,
+// 1,024 (2,048) 25.3 / 19.5 / 19.5, 2,048 27.6 / 27.6 / 27.6, 48 single tokens beside 464 (45,472) 31.7 / 29.7 / 35.8; 1,024 channels in 8 heads,
+// 2,048 tokens (2,048) 21.5 / 17.4 / 19.3.  The tile kernel is never the faster one.
+constexpr int CONV_RUN = 8, CONV_RUN_SHORT = 4, CONV_RUN_WARPS = 1600;
 template <typename TA, typename TW, int TAPS>
 __global__ void __launch_bounds__(128) conv_prep_run_kernel(const TA* __restrict__ proj, int stride, const TW* __restrict__ taps_w,
                                                             const float* __restrict__ conv_state, long long slot_stride,
                                                             const int* __restrict__ q_start, const int* __restrict__ slots,
                                                             float* __restrict__ out, int C, int nqk, int d, int nv, int dv,
-                                                            float unit_eps, float q_scale) {
+                                                            float unit_eps, float q_scale, int run) {
     const int b = blockIdx.x, lane = threadIdx.x & 31, u = blockIdx.z * 4 + (threadIdx.x >> 5);
     grid_dependency_wait();
     grid_dependency_trigger();
     const int t0 = q_start[b], t1 = q_start[b + 1];
-    const int c0 = t0 + blockIdx.y * CONV_RUN, c1 = min(t1, c0 + CONV_RUN);
+    const int c0 = t0 + blockIdx.y * run, c1 = min(t1, c0 + run);
     if (c0 >= t1 || u >= 2 * nqk + nv) return;
     const bool qk = u < 2 * nqk;
     const int width = qk ? d : dv, base = (qk ? u * d : 2 * nqk * d + (u - 2 * nqk) * dv) + lane;
@@ -240,24 +238,23 @@ TL_EXPORT int tl_conv_prep(const void* proj, int act_dtype, int stride, const vo
     if (B <= 0 || max_q_len <= 0) return 0;
     if (taps < 1 || (taps > 1 && !conv_state)) return 1;
     const int C = 2 * nqk * d + nv * dv;
-    // steps of many tokens with heads of up to 32 * CONV_KEEP: the tile kernel, as many tokens a block as 40 KB of rows hold
-    const int widest = d > dv ? d : dv;
-    int tt = (int)(40 * 1024 / sizeof(float)) / widest - (taps - 1);
+    const int widest = d > dv ? d : dv, heads = 2 * nqk + nv;
+    int tt = (int)(40 * 1024 / sizeof(float)) / widest - (taps - 1);     // tokens a block of the tile kernel: what 40 KB of rows hold
     tt = tt > 32 ? 32 : tt;
-    const long long work = (long long)T * C, tiles = tt > 0 ? (long long)B * ((max_q_len + tt - 1) / tt) * (2 * nqk + nv) : 0;
-    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && taps >= 2 && taps <= 4 &&
-        (work >= CONV_RUN_WORK || (work >= CONV_RUN_SOME && tiles >= CONV_RUN_GRID))) {
-        const dim3 grid(B, (max_q_len + CONV_RUN - 1) / CONV_RUN, (2 * nqk + nv + 3) / 4);
-        if (grid.y > 65535 || grid.z > 65535) return 1;
+    if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && taps >= 2 && taps <= 4) {
+        int run = (long long)B * ((max_q_len + CONV_RUN - 1) / CONV_RUN) * heads <= CONV_RUN_WARPS ? CONV_RUN_SHORT : CONV_RUN;
+        while ((max_q_len + run - 1) / run > 65535) run *= 2;
+        const dim3 grid(B, (max_q_len + run - 1) / run, (heads + 3) / 4);
+        if (grid.z > 65535) return 1;
 #define CR_N(TA, TW, N) launch_after_wait(conv_prep_run_kernel<TA, TW, N>, grid, dim3(128), 0, stream, (const TA*)proj, stride, (const TW*)taps_w, \
-        (const float*)conv_state, slot_stride, q_start, slots, out, C, nqk, d, nv, dv, unit_eps, q_scale)
+        (const float*)conv_state, slot_stride, q_start, slots, out, C, nqk, d, nv, dv, unit_eps, q_scale, run)
 #define CR(TA, TW) { if (taps == 2) CR_N(TA, TW, 2); else if (taps == 3) CR_N(TA, TW, 3); else CR_N(TA, TW, 4); }
         if (act_dtype == TL_F32) { if (w_dtype == TL_F32) CR(float, float) else CR(float, bf16) }
         else { if (w_dtype == TL_F32) CR(bf16, float) else CR(bf16, bf16) }
 #undef CR
 #undef CR_N
-    } else if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && tt >= 8 && 2 * nqk + nv <= 65535) {
-        const dim3 grid(B, (max_q_len + tt - 1) / tt, 2 * nqk + nv);
+    } else if (max_q_len >= 16 && widest <= 32 * CONV_KEEP && tt >= 8 && heads <= 65535) {
+        const dim3 grid(B, (max_q_len + tt - 1) / tt, heads);
         if (grid.y > 65535) return 1;
         const size_t smem = ((size_t)(tt + taps - 1) * widest + (size_t)widest * taps) * sizeof(float);
         if (smem > 48 * 1024) return 1;
