@@ -43,7 +43,7 @@ _SIGNATURES = {
     "tl_channel_scan": [_P, _I, _I, _I, _I, _I, _P, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _P],
     "tl_channel_chunk": [],
     "tl_linear_chunks": [_P, _I, _I, _I, _I, _I, _P, _F, _P, _P, _I, _I, _P, _F, _F, _P, _P, ctypes.c_longlong, _P, _P, _P, _I, _P, _I, _P, _P,
-                         _P, _P, _I, _I, _I, _F, _P, _P],
+                         _P, _P, _I, _I, _I, _F, _I, _P, _P],
     "tl_linear_chunk": [_I, _I],
     "tl_linear_chunk_tiles": [_I, _I],
     "tl_scan_state_floats": [_I, _I],
