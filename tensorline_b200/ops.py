@@ -851,9 +851,9 @@ LINEAR_CHUNKS_LEAST_TOKENS = 16
 
 # Heads of 33 to 128 rows run in chunks of 128 tokens on the 5th-generation tensor cores where a step has this many blocks of 64 tokens, a head and
 # 128 columns, by the rows of its heads (above 64 or not), and its requests fill the longer chunks (at most WIDE_CHUNKS_SHARE of the shorter
-# ones).  Chunks of 64 / 128, us: gated 8 heads of 128 x 256, 256 tokens (64 blocks) 52 / 52, 400 (112) 56 / 52, 1,024 (256) 71 / 56, 2,048
-# (512) 127 / 85; 4 heads of 128 x 128, 512 tokens (32) 50 / 50, 1,024 (64) 54 / 52, 2,048 (128) 63 / 54; 8 of 64 x 256, 512 tokens (128)
-# 42 / 46, 1,024 (256) 54 / 48; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 103, of 64 x 256 66 / 77.
+# ones).  Chunks of 64 / 128, us: gated 8 heads of 128 x 256, 256 tokens (64 blocks) 52 / 52, 400 (112) 56 / 54, 1,024 (256) 71 / 58, 2,048
+# (512) 127 / 89; 4 heads of 128 x 128, 512 tokens (32) 50 / 50, 1,024 (64) 54 / 54, 2,048 (128) 62 / 56; 8 of 64 x 256, 512 tokens (128)
+# 42 / 46, 1,024 (256) 54 / 50; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 105, of 64 x 256 66 / 79.
 WIDE_CHUNKS_BLOCKS = {False: 200, True: 96}
 WIDE_CHUNKS_SHARE = 0.65
 
