@@ -484,6 +484,7 @@ static int dc_launch(DeltaChunkArgs A, unsigned char* scratch, int* marked, int 
     int e = tl_raise_smem(dc_prepare_kernel<DP>, prepare, row_bytes + DC_C * DC_DV_MAX * 4);
     if (!e) e = tl_raise_smem(dc_walk_kernel<DP>, walk, Sh::BYTES);
     if (e) return e;
+    if (A.status == nullptr) return 1;                   // the walk's waits are bounded: it has to be able to say that one ran out
     const size_t ch = (size_t)n_chunks * A.H;
     A.W = scratch;
     A.P = A.W + ch * Sh::PARTS;
@@ -510,9 +511,8 @@ TL_EXPORT int tl_delta_chunk_bytes(int H, int nqk, int d, int dv) {
 TL_EXPORT int tl_delta_chunks(const float* qkv, int stride, int q_off, int k_off, int v_off, const float* gates, int gate_stride,
                               const float* A_log, const float* dt_bias, float* state, long long slot_stride, const int* q_start,
                               const int* slots, const int* chunks, int n_chunks, const int* firsts, int requests, void* scratch, int* marked, float* out,
-                              int H, int nqk, int d, int dv, int* status, cudaStream_t stream) {
+                              int H, int nqk, int d, int dv, cudaStream_t stream, int* status = nullptr) {
     if (n_chunks <= 0 || H <= 0) return 0;
-    if (status == nullptr) return 1;
     if (H > 65535 || nqk < 1 || H % nqk || !tl_delta_chunk_bytes(H, nqk, d, dv) || ((stride | q_off | k_off | v_off) & 3) ||
         ((((uintptr_t)qkv) | ((uintptr_t)scratch) | ((uintptr_t)out)) & 15)) return 1;
     const DeltaChunkArgs A{qkv, stride, q_off, k_off, v_off, gates, gate_stride, A_log, dt_bias, state, slot_stride, q_start, slots,

@@ -853,7 +853,8 @@ LINEAR_CHUNKS_LEAST_TOKENS = 16
 # 128 columns, by the rows of its heads (above 64 or not), and its requests fill the longer chunks (at most WIDE_CHUNKS_SHARE of the shorter
 # ones).  Chunks of 64 / 128, us: gated 8 heads of 128 x 256, 256 tokens (64 blocks) 52 / 52, 400 (112) 56 / 54, 1,024 (256) 71 / 58, 2,048
 # (512) 127 / 89; 4 heads of 128 x 128, 512 tokens (32) 50 / 50, 1,024 (64) 54 / 54, 2,048 (128) 62 / 56; 8 of 64 x 256, 512 tokens (128)
-# 42 / 46, 1,024 (256) 54 / 50; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 105, of 64 x 256 66 / 79.
+# 42 / 46, 1,024 (256) 54 / 50; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 103, of 64 x 256 66 / 77 (42 / 46 and
+# these two with end states that took 2 to 4 us less).
 WIDE_CHUNKS_BLOCKS = {False: 200, True: 96}
 WIDE_CHUNKS_SHARE = 0.65
 
@@ -1347,7 +1348,7 @@ def delta_chunks(qkv: torch.Tensor, gates: torch.Tensor, A_log: torch.Tensor, dt
     args = (_ptr(qkv), qkv.shape[1], 0, nqk * d, 2 * nqk * d, _ptr(gates), gates.stride(0), _ptr(A_log), _ptr(dt_bias), _ptr(state), per_slot,
             _ptr(ctx.q_start), _ptr(ctx.slots))
     _check(lib.tl_delta_chunks(*args, step.rows, step.n, step.firsts, step.long, _ptr(scratch), marked, _ptr(out), H, nqk, d, dv,
-                               _ptr(device_status(qkv.device)), _stream()), "delta_chunks", launches=2)
+                               _stream(), _ptr(device_status(qkv.device))), "delta_chunks", launches=2)
     _check(lib.tl_delta_scan(*args, _ptr(out), step.requests, H, nqk, d, dv, step.longest, 0, step.runs, marked, 1, _stream()), "delta_scan")
 
 
