@@ -1173,11 +1173,12 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
                         for (int e = 0; e < 8; ++e) P[e] *= base * below[s + e];
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {    // no branch in here (a key behind the token weighs e^-inf): the chains overlap
+                        for (int e = 0; e < 8; ++e) {    // no branch in here: the chains overlap.  A key behind the token is left out, not weighed
+                                                         // with zero: its product may be an infinity
                             const float2 v = u[s + e];
                             const float y = top.x + v.x, b = y - top.x;      // the sum of two doubles, rounded once
                             const float x = y + (((top.x - (y - b)) + (v.x - b)) + (top.y + v.y));
-                            P[e] *= expf(s + e <= last ? x : -INFINITY);
+                            P[e] = s + e <= last ? P[e] * expf(x) : 0.f;
                         }
                     }
                     if (GATED) total.add(((P[0] + P[1]) + (P[2] + P[3])) + ((P[4] + P[5]) + (P[6] + P[7])));

@@ -1,6 +1,9 @@
 """Matrix memories in chunks of 128 tokens (33 to 128 rows a head): what chunks of 64 are asked for, at the edges of the longer ones.  The bounds
 are those of the tests they are called from."""
+from types import SimpleNamespace
+
 import pytest
+import torch
 
 from tests import test_linear_chunks_gpu as chunks
 
@@ -35,3 +38,39 @@ def test_errors_are_no_larger_than_token_by_token(gated, H, d, dv, T, seed):
 @pytest.mark.parametrize("gated,d,dv", [(True, 64, 64), (False, 128, 132), (True, 128, 256)])
 def test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, value, gated, d, dv):
     chunks.test_a_value_that_is_no_number_reaches_what_it_reaches_token_by_token(what, value, gated, d, dv)
+
+
+def both(proj, H, d, dv, gates=None, decay=None, q_scale=1.0):
+    """Outputs and states in wide chunks and token by token, one request from a state of zero."""
+    from tensorline_b200 import ops
+    T, gated = proj.shape[0], gates is not None
+    kw = dict(gates=gates.cuda(), cap=15.0, den_eps=1e-6) if gated else dict(decay=decay.cuda())
+    floats = H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, gated)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(h_q_start=[0, T], scratch={}, pos=torch.arange(T, **i32), q_start=torch.tensor([0, T], **i32), slots=torch.zeros(1, **i32))
+    got = []
+    for chunks in (True, False):
+        out, state, x = torch.empty(T, H * dv, device="cuda"), torch.zeros(1, floats, device="cuda"), proj.cuda()
+        if chunks:
+            ops.linear_chunks(x, 0, H * d, 2 * H * d, H, d, dv, state, ctx, out, q_scale=q_scale, **kw)
+        else:
+            ops.linear_scan(x, 0, H * d, 2 * H * d, H, d, dv, state, ctx.q_start, ctx.slots, ctx.pos, out, B=1, q_scale=q_scale, **kw)
+        got.append((out.view(T, H, dv), state))
+    return got
+
+
+@pytest.mark.parametrize("later", [1, 20, 60])
+@pytest.mark.parametrize("gated,d,dv", [(True, 64, 64), (False, 64, 132), (True, 128, 256), (False, 128, 64)])
+def test_a_query_whose_product_with_a_later_key_overflows(gated, d, dv, later):
+    """A large query, not marked as an operand that chunks can't take; the key that overflows with it is `later` tokens behind, so
+    the output is finite.  Bound: float sums of d products and 41 tokens, of values whose sums don't cancel (all are positive)."""
+    H, T, at = 2, 200, 40
+    g = torch.Generator().manual_seed(later + d)
+    proj = torch.rand(T, 2 * H * d + H * dv, generator=g) + 0.5
+    proj[at, d:2 * d] = 1e30
+    proj[at + later, H * d + d:H * d + 2 * d] = 1e10
+    gates = torch.cat([torch.randn(T, H, generator=g), torch.randn(T, H, generator=g) + 3.0], dim=1) if gated else None
+    (out, _), (want, _) = both(proj, H, d, dv, gates, None if gated else torch.tensor([0.9, 0.99]))
+    assert bool(want[:at + later].isfinite().all())
+    assert bool(out[:at + later].isfinite().all())
+    assert float(((out - want)[:at + later].abs() / want[:at + later].abs()).max()) <= (d + 41) * 2.0 ** -23
