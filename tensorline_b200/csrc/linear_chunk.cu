@@ -776,7 +776,10 @@ __device__ __forceinline__ void lw_store(float* tile, const float (&sum)[CB / 4]
         float4 x = *reinterpret_cast<const float4*>(at);
         if (by) {
             const float b = by[r], o = over[r];
-            if (b > 1e-30f && b < 1e30f) {               // a quotient by the reciprocal, corrected once with its remainder (Markstein 1990)
+            // A quotient by the reciprocal, corrected once with its remainder (Markstein 1990); where a quotient or its remainder leaves a float's
+            // range (infinities, numerators below 2^-80) the division itself.
+            auto fits = [&](float z) { const float q = fabsf(z * o); return q > 1e-30f && q < 1e38f && fabsf(z) > 1e-24f; };
+            if (b > 1e-30f && b < 1e30f && fits(x.x) && fits(x.y) && fits(x.z) && fits(x.w)) {
                 auto quotient = [&](float z) { const float q = z * o; return fmaf(fmaf(-q, b, z), o, q); };
                 x.x = quotient(x.x); x.y = quotient(x.y); x.z = quotient(x.z); x.w = quotient(x.w);
             } else { x.x /= b; x.y /= b; x.z /= b; x.w /= b; }

@@ -74,3 +74,19 @@ def test_a_query_whose_product_with_a_later_key_overflows(gated, d, dv, later):
     assert bool(want[:at + later].isfinite().all())
     assert bool(out[:at + later].isfinite().all())
     assert float(((out - want)[:at + later].abs() / want[:at + later].abs()).max()) <= (d + 41) * 2.0 ** -23
+
+
+def test_a_numerator_beyond_a_float_stays_an_infinity():
+    """Two opposite keys with opposite values: the normaliser nearly cancels, the products don't, and overflow where the divisor is
+    small.  All factors are powers of two, so that a value is its first part."""
+    H, d, dv, T = 1, 64, 128, 150
+    proj = torch.zeros(T, 2 * H * d + H * dv)
+    proj[3, d], proj[3, 2 * d:] = 1.0, 2.0 ** 17
+    proj[4, d], proj[4, 2 * d:] = -1.0, -2.0 ** 17
+    proj[4, 2 * d + dv // 2:] = 2.0 ** 17                # (these columns cancel)
+    proj[10, 0] = 2.0 ** 117
+    gates = torch.cat([torch.zeros(T, H), torch.full((T, H), 40.0)], dim=1)
+    (out, _), (want, _) = both(proj, H, d, dv, gates)
+    assert bool(want[10, 0, :dv // 2].isinf().all()) and bool(want[:10].isfinite().all())
+    assert torch.equal(out.isinf(), want.isinf()) and not bool(out.isnan().any())
+    assert torch.equal(out.sign(), want.sign())
