@@ -48,7 +48,34 @@ struct PartsArgs {
     int M, N, K;
     int m_tiles, t_tiles, k_parts, part_chunks;          // tiles of W rows, of tokens; items along K and their chunks
     int* status;
+    const float* A; int lda; const bf16* W;              // the operands themselves, for gp_chains
 };
+
+// Sums of parts that are no number: an infinite weight times a part that is zero is none, the float itself times it may be an infinity.
+// Outputs `at`, `at` + ld .. (rows m .. m + rows - 1 of A, row n of W) that are none are taken again as gemm_f32.cu takes them, in one
+// chain of multiply-adds.
+__device__ __noinline__ void gp_chains(const PartsArgs& G, const bf16* bias, int m, int rows, int n, float* at, size_t ld) {
+    for (int x0 = 0; x0 < rows; x0 += 8) {
+        bool odd = false;
+        for (int x = x0; x < min(rows, x0 + 8); ++x) odd = odd || at[x * ld] != at[x * ld];
+        if (!odd) continue;
+        float sum[8] = {};
+        for (int k = 0; k < G.K; k += 4) {
+            const uint2 w = *reinterpret_cast<const uint2*>(G.W + (size_t)n * G.K + k);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) {
+                const float4 a = *reinterpret_cast<const float4*>(G.A + (size_t)(m + min(x0 + x, rows - 1)) * G.lda + k);
+                sum[x] = fmaf(a.x, __uint_as_float(w.x << 16), sum[x]);
+                sum[x] = fmaf(a.y, __uint_as_float(w.x & 0xffff0000u), sum[x]);
+                sum[x] = fmaf(a.z, __uint_as_float(w.y << 16), sum[x]);
+                sum[x] = fmaf(a.w, __uint_as_float(w.y & 0xffff0000u), sum[x]);
+            }
+        }
+#pragma unroll
+        for (int x = 0; x < 8; ++x)
+            if (x0 + x < rows && at[(x0 + x) * ld] != at[(x0 + x) * ld]) at[(x0 + x) * ld] = bias ? sum[x] + to_f<bf16>(bias[n]) : sum[x];
+    }
+}
 
 __device__ __forceinline__ void gp_ld8(uint32_t at, float* r) {
     uint32_t* u = reinterpret_cast<uint32_t*>(r);
@@ -245,9 +272,12 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 const size_t ld = G.partial ? G.N : G.ldo;
                 const float b = !G.partial && G.bias ? to_f<bf16>(G.bias[n]) : 0.f;
                 const bool add = !G.partial && G.bias;
+                float* at = dst;
+                bool odd = false;
 #pragma unroll
-                for (int x = 0; x < CW; ++x, dst += ld)
-                    if (t0 + x < G.M) *dst = add ? seg[x] + b : seg[x];
+                for (int x = 0; x < CW; ++x, at += ld)
+                    if (t0 + x < G.M) { *at = add ? seg[x] + b : seg[x]; odd = odd || seg[x] != seg[x]; }
+                if (odd && !G.partial) gp_chains(G, G.bias, t0, min(CW, G.M - t0), n, dst, ld);
             }
         }
     }
@@ -304,8 +334,9 @@ __global__ void __launch_bounds__(256) gemm_f32_cut_kernel(const float* __restri
 // ------------------------------------------------------------------ items' sums
 // out = the sums of `parts` items along K; `seg`: items are segments, and four of them a group
 template <int V>
-__global__ void __launch_bounds__(256) gemm_f32_sum_kernel(const float* __restrict__ partial, const bf16* __restrict__ bias, float* __restrict__ out,
-                                                           int ldo, int M, int N, int parts, int seg) {
+__global__ void __launch_bounds__(256) gemm_f32_sum_kernel(const PartsArgs G, const bf16* __restrict__ bias, float* out, int ldo, int parts, int seg) {
+    const float* __restrict__ partial = G.partial;
+    const int M = G.M, N = G.N;
     grid_dependency_wait();
     grid_dependency_trigger();
     const int nv = N / V;
@@ -341,6 +372,8 @@ __global__ void __launch_bounds__(256) gemm_f32_sum_kernel(const float* __restri
         for (int x = 0; x < V; ++x) if (bias) total[x] += to_f<bf16>(bias[n + x]);
         if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(total[0], total[1], total[2], total[3]);
         else dst[0] = total[0];
+#pragma unroll
+        for (int x = 0; x < V; ++x) if (total[x] != total[x]) gp_chains(G, bias, m, 1, n + x, dst + x, 0);
     }
 }
 
@@ -423,7 +456,7 @@ TL_EXPORT int tl_gemm_f32_parts(const float* A, int lda, const void* W, const vo
         float* out = C + (size_t)m0 * ldc;
         const long long cut = ((long long)m * (K / 8) + 255) / 256;
         if ((e = launch_after_wait(gemm_f32_cut_kernel, dim3((unsigned)(cut < cap ? cut : cap)), dim3(256), 0, stream, A + (size_t)m0 * lda, lda, P, m, K))) return e;
-        const PartsArgs G{out, ldc, partial, (const bf16*)bias, m, N, K, (N + 255) / 256, (m + plan.bn - 1) / plan.bn, plan.k_parts, plan.part_chunks, status};
+        const PartsArgs G{out, ldc, partial, (const bf16*)bias, m, N, K, (N + 255) / 256, (m + plan.bn - 1) / plan.bn, plan.k_parts, plan.part_chunks, status, A + (size_t)m0 * lda, lda, (const bf16*)W};
         switch (plan.bn) {
             case 32: e = parts_launch<32>(mw, P, G, stream); break;
             case 64: e = parts_launch<64>(mw, P, G, stream); break;
@@ -437,8 +470,8 @@ TL_EXPORT int tl_gemm_f32_parts(const float* A, int lda, const void* W, const vo
         const bool vec = N % 4 == 0 && ldc % 4 == 0 && ((uintptr_t)out & 15) == 0;
         const long long blocks = ((long long)m * N / (vec ? 4 : 1) + 255) / 256;
         const dim3 grid((unsigned)(blocks < cap ? blocks : cap));
-        e = vec ? launch_after_wait(gemm_f32_sum_kernel<4>, grid, dim3(256), 0, stream, (const float*)partial, (const bf16*)bias, out, ldc, m, N, plan.k_parts, seg)
-                : launch_after_wait(gemm_f32_sum_kernel<1>, grid, dim3(256), 0, stream, (const float*)partial, (const bf16*)bias, out, ldc, m, N, plan.k_parts, seg);
+        e = vec ? launch_after_wait(gemm_f32_sum_kernel<4>, grid, dim3(256), 0, stream, G, (const bf16*)bias, out, ldc, plan.k_parts, seg)
+                : launch_after_wait(gemm_f32_sum_kernel<1>, grid, dim3(256), 0, stream, G, (const bf16*)bias, out, ldc, plan.k_parts, seg);
         if (e) return e;
     }
     return 0;

@@ -60,3 +60,24 @@ def test_rows_apart_and_odd_values(ops):
     assert float((got[2].double() - want[2]).abs().max()) <= K * 2.0 ** -132
     assert float(((got[1].double() - want[1]).abs() / want[1].abs().clamp_min(1.0)).max()) <= 2.0 ** -20
     ops.check_device_status()
+
+
+def test_infinite_weights(ops):
+    """An infinite weight meets parts of a float that are zero: still what a chain of multiply-adds gives, an infinity, or none where
+    the value is zero or infinities of both signs meet.  With sums along K in one piece, in several, and in several kernels."""
+    for M, N, K in ((5, 1029, 1088), (200, 1029, 8200), (1, 300, 18944)):
+        g = torch.Generator().manual_seed(K)
+        a = torch.randn(M, K, generator=g).cuda()
+        a[:, 3], a[:, 7], a[0, 3] = 2.0, -0.37, 0.0      # in bfloat16 exactly, not so, zero
+        w = torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+        w[1, 3], w[130, 7], w[257, 3], w[257, 7] = float("inf"), float("inf"), -float("inf"), -float("inf")
+        assert ops.core().tl_gemm_f32_parts_scratch(a.data_ptr(), K, w.data_ptr(), M, N, K) > 0
+        bias = torch.randn(N, generator=g).to(torch.bfloat16).cuda()
+        got, want, clean = product(ops, a, w, bias), product(ops, a, w.float(), bias.float()), product(ops, a, w.nan_to_num(0.0, 0.0, 0.0), bias)
+        rows = [1, 130, 257]
+        assert int(want[1:, rows].isnan().sum()) == M - 1 and bool(want[1:, 1].isinf().all())
+        assert torch.equal(got[:, rows].isnan(), want[:, rows].isnan())
+        assert torch.equal(got[:, rows].nan_to_num(0.0), want[:, rows].nan_to_num(0.0))
+        rest = [n for n in range(N) if n not in rows]
+        assert torch.equal(got[:, rest], clean[:, rest])
+    ops.check_device_status()
