@@ -680,10 +680,14 @@ __global__ void __launch_bounds__(1024) moe_sort_kernel(const int* __restrict__ 
     }
 }
 
+static size_t moe_sort_bytes(int E) { return ((size_t)E * 32 + E + 1) * sizeof(int); }
+// Whether the sort has room for the counts of E entries.
+TL_EXPORT int tl_moe_sort_takes(int E) { return moe_sort_bytes(E) <= 48 * 1024; }
+
 TL_EXPORT int tl_moe_sort(const int* idx, int P, int E, int* offsets, int* place_of, int* pair_at, cudaStream_t stream) {
     if (P <= 0) return 0;
-    const size_t smem = ((size_t)E * 32 + E + 1) * sizeof(int);
-    if (smem > 48 * 1024) return 1;
+    const size_t smem = moe_sort_bytes(E);
+    if (!tl_moe_sort_takes(E)) return 1;
     return launch_after_wait(moe_sort_kernel, dim3(1), dim3(1024), smem, stream, idx, P, E, offsets, place_of, pair_at);
 }
 

@@ -59,6 +59,7 @@ _SIGNATURES = {
     "tl_split3": [_P, _P, _I, _I, _I, _P],
     "tl_rglru_chunk": [],
     "tl_moe_down": [_P, _I, _P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _P],
+    "tl_moe_sort_takes": [_I],
     "tl_moe_sort": [_P, _I, _I, _P, _P, _P, _P],
     "tl_moe_gather": [_P, _I, _P, _P, _P, _I, _P, _I, _I, _I, _I, _P, _P],
     "tl_relu_square": [_P, _I, ctypes.c_longlong, _P],
@@ -1147,6 +1148,11 @@ def moe_sort(idx: torch.Tensor, E: int):
     pair_at = torch.empty(P, dtype=torch.int32, device=idx.device)
     _check(core().tl_moe_sort(_ptr(idx), P, E, _ptr(offsets), _ptr(place_of), _ptr(pair_at), _stream()), "moe_sort")
     return offsets, place_of, pair_at
+
+
+def moe_sort_takes(E: int) -> bool:
+    """Whether `moe_sort` takes a router of E entries."""
+    return bool(core().tl_moe_sort_takes(E))
 
 
 def moe_gather(h: torch.Tensor, pair_at: torch.Tensor, idx: torch.Tensor, offsets: torch.Tensor, top: int, rows: torch.Tensor,

@@ -164,7 +164,9 @@ class RoutedExperts(Part):
         y = torch.empty((T, self.hidden), dtype=h.dtype, device=h.device)
         takes = (self.gated or self.activation == "relu_squared") and ops.moe_product_takes(h, self.w_up, self.w_down, self.gated)
         few = T <= STREAM_MAX_TOKENS or bool(ctx.graph_max_ctx)
-        if takes and few and on_input:                   # the gathered rows round the weighted inputs, which streamed experts do not
+        # streamed all the same: weights on the input (the gathered rows round the products, which streamed experts do not), more entries than
+        # the sort takes
+        if takes and few and (on_input or not ops.moe_sort_takes(E)):
             takes = False
         elif takes and T <= STREAM_MAX_TOKENS:
             takes = sort_pays(T, top, E, 2 * (self.w_up[0].numel() + self.w_down[0].numel()))

@@ -108,3 +108,42 @@ def test_long_steps_agree_with_streamed_experts(ops, gated, shared, on_input, fe
     short = part.forward(h, ctx)
     ops.check_device_status()
     assert float((long.float() - short.float()).norm() / short.float().norm()) <= (2.0 ** -9 if few else 2.0 ** -7)      # few: only roundings that fall on the other side; else three more of 2^-8 at most
+
+
+def routed(hidden, inner, experts, top, **more):
+    from tensorline_b200.parts import FEED_FORWARDS, PartSpec, Runtime
+    part = FEED_FORWARDS.build(PartSpec("routed_experts", dict(hidden=hidden, inner=inner, experts=experts, top=top, router_bias=False, **more)),
+                               Runtime(torch.device("cuda", 0), torch.bfloat16, 16))
+    g = torch.Generator().manual_seed(1)
+    part.bind({n: (torch.randn(s.shape, generator=g) * 0.08).to(torch.bfloat16).cuda() for n, s in part.expected_tensors("l").items()}, "l")
+    return part
+
+
+def captured(part, h):
+    from types import SimpleNamespace
+    ctx = SimpleNamespace(graph_max_ctx=4096)
+    part.forward(h, ctx)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = part.forward(h, ctx)
+    graph.replay()
+    torch.cuda.synchronize()
+    return y
+
+
+@pytest.mark.parametrize("tokens", [8, 40, 64])
+@pytest.mark.parametrize("more", [dict(experts=512, top=8), dict(experts=373, top=16), dict(experts=300, identity=212, top=8, scoring="softmax_share"),
+                                  dict(experts=256, identity=16, top=8, scoring="softmax_share"), dict(experts=8, top=2)])
+def test_captured_steps_take_every_router(ops, more, tokens, monkeypatch):
+    """Decode steps are captured at any number of tokens, whatever the router: more entries than the sort takes, identities among them.
+    Streamed and, as far as the sort goes, through sorted runs: nothing is rounded in one that is not in the other, but the other way now and then."""
+    from tensorline_b200.parts import moe
+    part = routed(256, 64, gated=True, activation="silu", **more)
+    h = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES", -1e12)
+    y = captured(part, h)
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES", 1e12)
+    streamed = captured(part, h)
+    ops.check_device_status()
+    assert float((y.float() - streamed.float()).norm() / streamed.float().norm()) <= 2.0 ** -9
