@@ -1171,8 +1171,11 @@ def moe_gather(h: torch.Tensor, pair_at: torch.Tensor, idx: torch.Tensor, offset
                                 int(top), _ptr(scale), _stream()), "moe_gather")
 
 
-def moe_product_takes(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, gated: bool) -> bool:
-    """Whether both products of these experts ([E, F or 2F, K] and [E, K, F]) run as `moe_product`."""
+def moe_product_takes(h: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, gated: bool, activation: str) -> bool:
+    """Whether both products of these experts ([E, F or 2F, K] and [E, K, F]) run as `moe_product`: the square of relu without a gate,
+    every other activation with one."""
+    if gated == (activation == "relu_squared"):
+        return False
     E, N, F = w_down.shape
     takes = core().tl_moe_product_takes
     return (h.dtype == w_up.dtype == w_down.dtype == torch.bfloat16 and bool(takes(E, w_up.shape[2], F, int(gated))) and bool(takes(E, F, N, 0))

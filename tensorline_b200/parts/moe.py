@@ -162,7 +162,7 @@ class RoutedExperts(Part):
             extra, extra_gate = resolve(self.shared.forward(h, ctx)), (z[:, E] if self.shared_gate else None)
         on_input = self.weight_on == "input"
         y = torch.empty((T, self.hidden), dtype=h.dtype, device=h.device)
-        takes = (self.gated or self.activation == "relu_squared") and ops.moe_product_takes(h, self.w_up, self.w_down, self.gated)
+        takes = ops.moe_product_takes(h, self.w_up, self.w_down, self.gated, self.activation)
         few = T <= STREAM_MAX_TOKENS or bool(ctx.graph_max_ctx)
         # streamed all the same: weights on the input (the gathered rows round the products, which streamed experts do not), more entries than
         # the sort takes

@@ -147,3 +147,24 @@ def test_captured_steps_take_every_router(ops, more, tokens, monkeypatch):
     streamed = captured(part, h)
     ops.check_device_status()
     assert float((y.float() - streamed.float()).norm() / streamed.float().norm()) <= 2.0 ** -9
+
+
+def test_gates_that_the_sorted_products_do_not_have(ops, monkeypatch):
+    """relu(gate)^2 * up: steps of few tokens and captured ones are streamed, whatever sorting would save; longer ones are refused."""
+    from types import SimpleNamespace
+    from tensorline_b200.parts import moe
+    part = routed(256, 64, experts=8, top=2, gated=True, activation="relu_squared")
+    h = torch.randn(77, 256, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16).cuda()
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES", -1e12)
+    z = h.float() @ part.w_router.float().T
+    wts, idx = z.topk(2, dim=1)
+    wts = wts.softmax(dim=1)
+    want = torch.zeros(77, 256, device="cuda")
+    for t in range(77):
+        for j in range(2):
+            gate, up = (part.w_up[idx[t, j]].float() @ h[t].float()).split(64)
+            want[t] += wts[t, j] * (part.w_down[idx[t, j]].float() @ (gate.clamp_min(0) ** 2 * up))
+    for y in (captured(part, h), torch.cat([part.forward(x, SimpleNamespace(graph_max_ctx=0)) for x in h.split(32)])):
+        assert float((y.float() - want).norm() / want.norm()) <= 2.0 ** -7      # two roundings to bfloat16, each 2^-9 or less, and few sums' order
+    with pytest.raises(ops.KernelError):
+        part.forward(h, SimpleNamespace(graph_max_ctx=0))
