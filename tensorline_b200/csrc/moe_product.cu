@@ -67,7 +67,8 @@ __device__ __forceinline__ void moe_load5(uint32_t dst, const CUtensorMap* map, 
 }
 
 // KIND 0: as it is, 1..3: gates (tl_gate_mul), 4: relu(.)^2, each of values rounded to bfloat16 first, as a stored product would have been.
-// Eight more: of the accumulators themselves, and 8 as floats (what streamed experts compute).  A parameter of the kernel: with
+// Eight more: of the accumulators themselves, and 8 as floats, the gates by exact divisions (tl_act_pair: what streamed experts compute).  A
+// parameter of the kernel: with
 // the choice inside the loop over a thread's elements their chains did not overlap.
 __device__ __forceinline__ float moe_rounded(float v, bool raw) { return raw ? v : __bfloat162float(__float2bfloat16_rn(v)); }
 template <int KIND>
@@ -197,7 +198,8 @@ moe_product_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     for (int j = 0; j < 8; ++j) {
                         const float give = up ? r[j] : r[8 + j], keep = up ? r[8 + j] : r[j];
                         const float a = moe_rounded(keep, raw), b = moe_rounded(__shfl_xor_sync(0xffffffffu, give, 16), raw);
-                        y[j] = tl_gate_mul(up ? b : a, up ? a : b, KIND % 8, G.limit, G.alpha);
+                        y[j] = raw ? tl_act_pair(up ? b : a, up ? a : b, KIND == 11 ? TL_ACT_SWISH_CLAMPED : KIND == 10 ? TL_ACT_GELU_TANH : TL_ACT_SILU, G.limit, G.alpha)
+                                   : tl_gate_mul(up ? b : a, up ? a : b, KIND % 8, G.limit, G.alpha);
                     }
                     if (col < G.cols) {
                         bf16* dst = (bf16*)G.out + (size_t)(t.row + c0 + (up ? 8 : 0)) * G.ldo + col;

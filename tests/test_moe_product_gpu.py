@@ -168,3 +168,20 @@ def test_gates_that_the_sorted_products_do_not_have(ops, monkeypatch):
         assert float((y.float() - want).norm() / want.norm()) <= 2.0 ** -7      # two roundings to bfloat16, each 2^-9 or less, and few sums' order
     with pytest.raises(ops.KernelError):
         part.forward(h, SimpleNamespace(graph_max_ctx=0))
+
+
+@pytest.mark.parametrize("act", ["silu", "swish_clamped"])
+def test_far_gates_of_few_tokens_are_divided_exactly(ops, act):
+    """x / (1 + e^-x) where the divisor is above 2^126: small but no zero, and an up value brings it back into sight.  Against the
+    formula in float64; three roundings of bfloat16 values and floats (2^-8 and less) beside the exponential's argument."""
+    x = torch.zeros(5, 64)
+    x[:, 0], x[:, 1] = torch.tensor([-80.0, -87.0, -87.5, -88.0, -88.5]), 2.0 ** 100
+    w = torch.zeros(1, 32, 64)
+    w[0, :16, 0], w[0, 16:, 1] = 1.0, 1.0
+    x, w = x.to(torch.bfloat16).cuda(), w.to(torch.bfloat16).cuda()
+    out = torch.empty(5, 16, dtype=torch.bfloat16, device="cuda")
+    clamped = act == "swish_clamped"
+    ops.moe_product(x, w, torch.tensor([0, 5], dtype=torch.int32).cuda(), out, act=("swish_clamped", 1e38, 1.0) if clamped else act, gated=True, raw=True)
+    z = x[:, 0].double()
+    want = (z / (1.0 + torch.exp(-z)) * (2.0 ** 100 + (1.0 if clamped else 0.0)))[:, None]
+    assert float(((out.double() - want).abs() / want.abs()).max()) <= 2.0 ** -7
