@@ -787,8 +787,8 @@ __device__ __forceinline__ void lw_store(float* tile, const float (&sum)[CB / 4]
         *reinterpret_cast<float4*>(to) = x;
     }
 }
-// sums of floats with what their additions lose, as exact as sums in double and on the float pipe (in double the weights and sums of a
-// chunk took 16,000 cycles)
+// Sums of floats, or of products of two, with what their additions and roundings lose, which is itself a float sum (about 2^-46 of the
+// largest partial sum) and on the float pipe (in double the weights and sums of a chunk took 16,000 cycles).
 struct LwSum {
     float s = 0.f, lost = 0.f;
     __device__ __forceinline__ void add(float x) {
@@ -801,7 +801,7 @@ struct LwSum {
         lost += fmaf(x, y, -p);
         add(p);
     }
-    __device__ __forceinline__ double value() const { return (double)s + (double)lost; }
+    __device__ __forceinline__ double value() const { return (double)s + (lost == lost ? (double)lost : 0.0); }      // (an infinity has lost nothing)
 };
 struct LwBars { uint64_t qk, full[4], done[4], free[4]; uint32_t tmem; int gave_up; };
 __device__ __forceinline__ void lw_start(LwBars& B, int warp) {
@@ -1010,17 +1010,13 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
 #pragma unroll
             for (int j = 0; j < N; ++j) {
                 const int t = (tid + LW_WORK * (j0 + j - (isq ? 0 : PER))) / PR;
-                float nr[2] = {0.f, 0.f};                // n . q of the chunk's start state
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    v[j][e] *= scale;
-                    if (GATED) nr[e & 1] = fmaf(v[j][e], norm[e], nr[e & 1]);
-                }
+                for (int e = 0; e < 8; ++e) v[j][e] *= scale;
                 lw_put8((isq ? qs : ks) + swz(C, t, tid % PR), PQ, v[j]);
                 if (GATED && isq) {
-                    LwSum r;
-                    r.add(nr[0]);
-                    r.add(nr[1]);
+                    LwSum r;                             // n . q of the chunk's start state
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) r.add_product(v[j][e], norm[e]);
 #pragma unroll
                     for (int o = 1; o < PR; o <<= 1) {
                         const float lost = __shfl_xor_sync(0xffffffffu, r.lost, o);
@@ -1184,7 +1180,10 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
                             P[e] = s + e <= last ? P[e] * expf(x) : 0.f;
                         }
                     }
-                    if (GATED) total.add(((P[0] + P[1]) + (P[2] + P[3])) + ((P[4] + P[5]) + (P[6] + P[7])));
+                    if (GATED) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) total.add(P[e]);
+                    }
                 }
                 lw_put8(qs + swz(C, t, s / 8), PP, P);
             }

@@ -90,3 +90,35 @@ def test_a_numerator_beyond_a_float_stays_an_infinity():
     assert bool(want[10, 0, :dv // 2].isinf().all()) and bool(want[:10].isfinite().all())
     assert torch.equal(out.isinf(), want.isinf()) and not bool(out.isnan().any())
     assert torch.equal(out.sign(), want.sign())
+
+
+@pytest.mark.parametrize("what", ["start state", "keys"])
+def test_the_normaliser_adds_up_without_loss(what):
+    """n . q from terms of about 1,000 that cancel to between 2 and 4, behind numerators that don't: products with the start state's n (a first
+    chunk from a state in the slot, no keys), and weighted products with keys (gates that weigh every key with one).  What is left is
+    one rounding of a float or two each in the sum, its quotient and the numerator: 2^-20, where float sums would be off by 2^-12."""
+    from tensorline_b200 import ops
+    H, d, dv, T = 1, 128, 64, 200
+    g = torch.Generator().manual_seed(5)
+    proj = torch.zeros(T, 2 * d + dv)
+    gates = torch.cat([torch.zeros(T, H), torch.full((T, H), 2000.0)], dim=1)      # no decay at all below a cap of 400
+    state = torch.zeros(1, H * -(-dv // ops.scan_columns()) * ops.scan_state_floats(d, True))
+    terms = (torch.randn(T, d - 1, generator=g) * 1000.0).float()
+    if what == "keys":                                   # token t from 100 on sees the keys 0 .. 99, whose products are c
+        c = (torch.randn(100, generator=g) * 1000.0).float()
+        c[99] = 3.0 - c[:99].double().sum()
+        proj[:100, d], proj[:, 0] = c, 1.0
+        proj[:100, 2 * d:] = c.sign()[:, None]
+        at, want = slice(100, 128), c.double().abs().sum() / (c.double().sum().abs() + 1e-6)
+    else:
+        S, n = torch.zeros(H, d, dv), torch.randn(H, d, generator=g)
+        S[0, 0], n[0, 0], n[0, d - 1] = 1.0, 0.0, 1.0
+        state = chunks.slot_rows(S, n, torch.zeros(H))[None].float()
+        proj[:, 0], proj[:, 1:d] = 1.0, terms
+        proj[:, d - 1] = 3.0 - (proj[:, :d - 1].double() @ n[0, :d - 1].double())
+        at, want = slice(0, 128), 1.0 / ((proj[:128, :d].double() @ n[0].double()).abs() + 1e-6)[:, None]
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ctx = SimpleNamespace(h_q_start=[0, T], scratch={}, pos=torch.arange(T, **i32), q_start=torch.tensor([0, T], **i32), slots=torch.zeros(1, **i32))
+    out = torch.empty(T, H * dv, device="cuda")
+    ops.linear_chunks(proj.cuda(), 0, d, 2 * d, H, d, dv, state.cuda(), ctx, out, gates=gates.cuda(), cap=400.0, den_eps=1e-6)
+    assert float(((out[at].double().cpu() - want).abs() / want).max()) <= 2.0 ** -20
