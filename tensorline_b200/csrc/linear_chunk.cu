@@ -980,8 +980,6 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
     __shared__ LwBars B;
     __shared__ double rowsum[4][C], nq[C];
     __shared__ float2 u[C];                              // a double as two floats
-    __shared__ float below[C];                           // e^(u less the largest of its 32 keys)
-    __shared__ double most[4];                           // that
     __shared__ float coef[C], den[C], over[C];
     const int4 ck = A.chunks[blockIdx.x];
     const int h = blockIdx.y, col0 = blockIdx.z * NT * CB, d = A.d;
@@ -1054,14 +1052,7 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
             if (tid < C) coef[t] = (float)exp(f);
             top = pair(f);
         }
-        if (warp < 4) {
-            u[t] = pair(uv);
-            double best = t < n ? uv : -INFINITY;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
-            below[t] = expf((float)(uv - best));
-            if (lane == 0) most[warp] = best;
-        }
+        if (warp < 4) u[t] = pair(uv);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -1160,25 +1151,18 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
                 for (int c = 0; c < HC; ++c) sum[z][c] *= weight;
             LwSum total;
             const int last = t < n ? t : -1;
-            // 32 keys before all of the warp's tokens: their weights are this times `below`, neither above one
-            const float base = t < n ? expf((float)(((double)top.x + (double)top.y) + most[share])) : 0.f;
 #pragma unroll 1
             for (int s = 32 * share; s < 32 * share + 32; s += 8) {
                 float P[8] = {};
                 if (sees) {
                     lw_ld8(acc + s, P);
-                    if (share < quarter) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) P[e] *= base * below[s + e];
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {    // no branch in here: the chains overlap.  A key behind the token is left out, not weighed
-                                                         // with zero: its product may be an infinity
-                            const float2 v = u[s + e];
-                            const float y = top.x + v.x, b = y - top.x;      // the sum of two doubles, rounded once
-                            const float x = y + (((top.x - (y - b)) + (v.x - b)) + (top.y + v.y));
-                            P[e] = s + e <= last ? P[e] * expf(x) : 0.f;
-                        }
+                    for (int e = 0; e < 8; ++e) {        // no branch in here: the chains overlap.  A key behind the token is left out, not weighed with
+                                                         // zero: its product may be an infinity
+                        const float2 v = u[s + e];
+                        const float y = top.x + v.x, b = y - top.x;      // the sum of two doubles, rounded once
+                        const float x = y + (((top.x - (y - b)) + (v.x - b)) + (top.y + v.y));
+                        P[e] = s + e <= last ? P[e] * expf(x) : 0.f;
                     }
                     if (GATED) {
 #pragma unroll

@@ -122,3 +122,20 @@ def test_the_normaliser_adds_up_without_loss(what):
     out = torch.empty(T, H * dv, device="cuda")
     ops.linear_chunks(proj.cuda(), 0, d, 2 * d, H, d, dv, state.cuda(), ctx, out, gates=gates.cuda(), cap=400.0, den_eps=1e-6)
     assert float(((out[at].double().cpu() - want).abs() / want).max()) <= 2.0 ** -20
+
+
+def test_a_weight_is_one_exponential(monkeypatch):
+    """One key in the first 32 tokens of a head, seen from the next 32: an output is its weight, and the same float as in chunks of 64 (whose
+    argument is rounded from doubles; here from pairs of floats, which may round the other way at a tie)."""
+    from tensorline_b200 import ops
+    H, d, dv, T = 16, 64, 64, 64
+    proj = torch.zeros(T, 2 * H * d + H * dv)
+    proj[:, :H * d:d] = 1.0
+    for h in range(H):
+        proj[2 * h, H * d + h * d] = 1.0
+        proj[2 * h, 2 * H * d + h * dv:2 * H * d + (h + 1) * dv] = 1.0
+    decay = 1.0 - 0.3 * torch.rand(H, generator=torch.Generator().manual_seed(1))
+    wide = both(proj, H, d, dv, None, decay)[0][0]
+    monkeypatch.setattr(ops, "WIDE_CHUNKS_BLOCKS", {False: 1 << 40, True: 1 << 40})
+    narrow = both(proj, H, d, dv, None, decay)[0][0]
+    assert float((wide[32:, :, 0] == narrow[32:, :, 0]).float().mean()) >= 0.99
