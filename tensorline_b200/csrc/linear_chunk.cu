@@ -658,20 +658,22 @@ __global__ void __launch_bounds__(256, DP <= 128 ? 2 : 1) lc_out_kernel(const Li
 
 // ------------------------------------------------------------------ wide chunks on the 5th-generation tensor cores
 // Heads of 33 to 128 rows: chunks of 128 tokens, so that tokens (outputs) and rows (end states) fill the MMA's 128.  Everything is a sum
-// over k (rows, tokens) in steps of 32, each an accumulator of its own in tensor memory: twelve tcgen05 products of bfloat16
-// parts, the five small ones of the six first, and sixteen worker warps add the accumulators up with additions that round (the tensor
-// cores cut; see parts_mma.cuh).  A worker owns a lane of tensor memory (a token or a row) and a quarter of the columns.  One more warp
-// issues.  Operands are cut into parts on their way to shared memory, in the 128-byte swizzle: rows of 64 values, K-major for Q, K and P,
-// MN-major for what is summed over its rows (V, S, and K for the end states).  192 KB, one block an SM.
-//   outputs     Q K^T (four accumulators, added up into the first); Q S, 32 rows of S a stage through a ring of four in K's place
-//               and three accumulators; P takes Q's place, then P V likewise.
+// over k (rows, tokens) of twelve tcgen05 products of bfloat16 parts for every 32 k: the five small products of the six have one
+// accumulator in tensor memory for a whole sum, the leading products of 16 k one each, and sixteen worker warps add these up with additions
+// that round (the tensor cores cut; see parts_mma.cuh), so that no sum is further from 64 bits than in chunks of 64.  A worker owns a
+// lane of tensor memory (a token or a row) and a quarter of the columns.  One more warp issues.  Operands are cut into parts on their
+// way to shared memory, in the 128-byte swizzle: rows of 64 values, K-major for Q, K and P, MN-major for what is summed over its rows
+// (V, S, and K for the end states).  192 KB, one block an SM.
+//   outputs     Q K^T, its sum back into the fourth accumulator; Q S, 32 rows of S a stage through a ring of four in K's place; P takes
+//               Q's place, then P V likewise.  A stage's leading products are read while the next one's small ones run.
 // Loops stay rolled: a block runs once through its code, and what is not in the instruction cache comes at one instruction in
 // about 13 cycles (the weights unrolled over a worker's 64 keys took 18,000 cycles).
-//   end states  K^T V, 32 tokens a stage; states pass their errors on, so the leading product of every 16 tokens has an accumulator of its
-//               own (in one with the small ones a state is 2e-8 nearer to zero), four in turn.
-// Measured beside the mma.sync kernels (chunks of 64), 8 heads of 128 x 256, 2,048 tokens: end states 23 us (28), start states 12 (18),
-// outputs 39 (65); all of a gated memory 89 (127), a fixed decay's 77 (103).  A block runs its phases one after the other, about 35 us whatever else
-// there is, so short steps stay with the chunks of 64 (ops.py).
+//   end states  K^T V, 32 tokens a stage; the small products of all tokens first, then the leading ones, three accumulators in turn.
+// Measured beside the mma.sync kernels (chunks of 64), 8 heads of 128 x 256, 2,048 tokens: end states 23 us (28), start states 16 (18),
+// outputs 48 (65); all of a gated memory 85 (124), a fixed decay's 70 (101).  Against 64 bits, gated / fixed decay: outputs (the median of tokens and
+// heads) 1.16e-7 / 1.10e-7 (chunks of 64 1.16 / 1.11), states 0.85e-7 / 1.00e-7 (0.85 / 1.76); with the leading products in the small ones'
+// accumulators 1.25 / 1.34 and 0.89 / 1.09.  With the code of a stage's sums in the outputs' loop four times instead of once they took 59 us.  A block runs
+// its phases one after the other, about 35 us whatever else there is, so short steps stay with the chunks of 64 (ops.py).
 constexpr int LW_WORK = 512, LW_THREADS = LW_WORK + 32, LW_MMA = LW_WORK / 32, LW_REGION = 3 * LC_WIDE * LC_WIDE * 2;
 constexpr int LW_SMEM = 2 * LW_REGION + 1024;
 
@@ -694,15 +696,20 @@ __device__ __forceinline__ void lw_commit(uint64_t* bar, uint32_t one) {
                  "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
                  ::"r"(smem_addr(bar)), "r"(one) : "memory");
 }
-// The six products of parts (or the five small ones) of 32 k into `acc`, the small ones first.  a(p, k), b(p, k): descriptors of part p, k in
-// steps of 16.
-template <int PRODUCTS = 6, typename FA, typename FB>
-__device__ __forceinline__ void lw_parts(uint32_t acc, uint32_t idesc, uint32_t one, FA a, FB b) {
-    constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+// The five small products of parts of 32 k, into `acc` (`more`: to what it holds).  a(p, k), b(p, k): descriptors of part p, k in steps of 16.
+template <typename FA, typename FB>
+__device__ __forceinline__ void lw_small(uint32_t acc, bool more, uint32_t idesc, uint32_t one, FA a, FB b) {
+    constexpr int pa[5] = {2, 0, 1, 1, 0}, pb[5] = {0, 2, 1, 0, 1};
 #pragma unroll
-    for (int i = 0; i < PRODUCTS; ++i)
+    for (int i = 0; i < 5; ++i)
 #pragma unroll
-        for (int k = 0; k < 2; ++k) lw_mma(acc, a(pa[i], k), b(pb[i], k), idesc, (i || k) ? 1u : 0u, one);
+        for (int k = 0; k < 2; ++k) lw_mma(acc, a(pa[i], k), b(pb[i], k), idesc, (i || k || more) ? 1u : 0u, one);
+}
+// the leading products of 16 k each
+template <typename FA, typename FB>
+__device__ __forceinline__ void lw_lead(uint32_t first, uint32_t second, uint32_t idesc, uint32_t one, FA a, FB b) {
+    lw_mma(first, a(0, 0), b(0, 0), idesc, 0u, one);
+    lw_mma(second, a(0, 1), b(0, 1), idesc, 0u, one);
 }
 // eight values' parts into the 16 bytes at `at` of three tiles, `part` bytes apart
 __device__ __forceinline__ void lw_put8(unsigned char* at, int part, const float (&x)[8]) {
@@ -738,20 +745,48 @@ __device__ __forceinline__ void lw_st16(uint32_t at, const float (&r)[16]) {
                  ::"r"(at), "r"(u[0]), "r"(u[1]), "r"(u[2]), "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7]),
                    "r"(u[8]), "r"(u[9]), "r"(u[10]), "r"(u[11]), "r"(u[12]), "r"(u[13]), "r"(u[14]), "r"(u[15]) : "memory");
 }
-// this lane's quarter of the columns of an accumulator, added to `sum`
-template <int N> __device__ __forceinline__ void lw_add(float (&sum)[N], uint32_t at) {
-    if constexpr (N == 32) {
-        float r[32];
-        tmem_ld32(at, r);
-        tmem_ld_wait();
+// N columns of two leading products added to `sum`, one after the other
+template <int N> __device__ __forceinline__ void lw_add(float (&sum)[N], uint32_t first, uint32_t second) {
 #pragma unroll
-        for (int x = 0; x < 32; ++x) sum[x] += r[x];
-    } else {
-        static_assert(N == 16, "columns a worker");
+    for (int c = 0; c < N; c += 8) {
+        uint32_t a[8], b[8];
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%16];\n\t"
+                     "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%17];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]), "=r"(a[4]), "=r"(a[5]), "=r"(a[6]), "=r"(a[7]),
+                       "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]), "=r"(b[4]), "=r"(b[5]), "=r"(b[6]), "=r"(b[7])
+                     : "r"(first + c), "r"(second + c));
+#pragma unroll
+        for (int x = 0; x < 8; ++x) sum[c + x] = (sum[c + x] + __uint_as_float(a[x])) + __uint_as_float(b[x]);
+    }
+}
+template <int N> __device__ __forceinline__ void lw_put(const float (&sum)[N], uint32_t at) {
+#pragma unroll
+    for (int c = 0; c < N; c += 16) {
         float r[16];
-        lw_ld16(at, r);
 #pragma unroll
-        for (int x = 0; x < 16; ++x) sum[x] += r[x];
+        for (int x = 0; x < 16; ++x) r[x] = sum[c + x];
+        lw_st16(at + c, r);
+    }
+}
+// one of them
+template <int N> __device__ __forceinline__ void lw_add_one(float (&sum)[N], uint32_t at) {
+#pragma unroll
+    for (int c = 0; c < N; c += 16) {
+        float r[16];
+        lw_ld16(at + c, r);
+#pragma unroll
+        for (int x = 0; x < 16; ++x) sum[c + x] += r[x];
+    }
+}
+// and the small products' accumulator at the end of a sum: sum = weight (sum + small)
+template <int N> __device__ __forceinline__ void lw_end_sum(float (&sum)[N], uint32_t small, float weight) {
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+        float r[8];
+        lw_ld8(small + c, r);
+#pragma unroll
+        for (int x = 0; x < 8; ++x) sum[c + x] = fmaf(weight, sum[c + x], weight * r[x]);
     }
 }
 __device__ __forceinline__ void lw_sync() { asm volatile("bar.sync 1, %0;" ::"n"(LW_WORK) : "memory"); }      // the workers
@@ -803,10 +838,9 @@ struct LwSum {
     }
     __device__ __forceinline__ double value() const { return (double)s + (lost == lost ? (double)lost : 0.0); }      // (an infinity has lost nothing)
 };
-struct LwBars { uint64_t qk, full[4], done[4], free[4]; uint32_t tmem; int gave_up; };
+struct LwBars { uint64_t full[4], done[4], free[4]; uint32_t tmem; int gave_up; };
 __device__ __forceinline__ void lw_start(LwBars& B, int warp) {
     if (threadIdx.x == 0) {
-        mbar_init(&B.qk, 1);
         for (int i = 0; i < 4; ++i) { mbar_init(B.full + i, LW_MMA); mbar_init(B.done + i, 1); mbar_init(B.free + i, LW_MMA); }
         B.gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -829,6 +863,12 @@ __device__ __forceinline__ bool lw_workers_or(bool x) {
     int any;
     asm volatile("{\n.reg .pred p, q;\nsetp.ne.s32 p, %1, 0;\nbar.red.or.pred q, 1, %2, p;\nselp.s32 %0, 1, 0, q;\n}" : "=r"(any) : "r"((int)x), "n"(LW_WORK) : "memory");
     return any != 0;
+}
+// a worker warp has read its part of the accumulators
+__device__ __forceinline__ void lw_taken(uint64_t* bar, int lane) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
 }
 // a worker warp's part of a stage is in shared memory
 __device__ __forceinline__ void lw_filled(uint64_t* bar, int lane) {
@@ -871,20 +911,22 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChu
         // A: K^T, B: V, both MN-major; heads of up to 64 rows: the upper half of the tile is whatever lies behind, and nobody reads it
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(CB >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
         const uint32_t one = lw_elect(), ka = smem_addr(ks), va = smem_addr(vs);
-        int g = 0;
-        for (int i = 0; i < stages; ++i) {
-            if (!mbar_wait(B.full + i, 0, gave_up, A.status, 61)) break;
+        auto k_at = [&](int i, int p, int k) { return desc_mnmajor(ka + p * PK + (i * 2 + k) * 16 * 128, C * 128); };
+        auto v_at = [&](int i, int p, int k) { return desc_mnmajor(va + p * PV + (i * 2 + k) * 16 * 128, C * 128); };
+        bool ok = true;
+        for (int i = 0; ok && i < stages; ++i) {
+            ok = mbar_wait(B.full + i, 0, gave_up, A.status, 61);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            auto k_at = [&](int p, int k) { return desc_mnmajor(ka + p * PK + (i * 2 + k) * 16 * 128, C * 128); };
-            auto v_at = [&](int p, int k) { return desc_mnmajor(va + p * PV + (i * 2 + k) * 16 * 128, C * 128); };
-            for (int a = 0; a < 3; ++a, ++g) {           // the leading product of 16 tokens, of the next 16, the small ones of both
-                const uint32_t acc = tmem + (g & 3) * 128;
-                if (g >= 4 && !mbar_wait(B.free + (g & 3), ((g >> 2) - 1) & 1, gave_up, A.status, 66)) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (a < 2) lw_mma(acc, k_at(0, a), v_at(0, a), idesc, 0u, one);
-                else lw_parts<5>(acc, idesc, one, k_at, v_at);
-                lw_commit(B.done + (g & 3), one);
-            }
+            lw_small(tmem, i > 0, idesc, one, [&](int p, int k) { return k_at(i, p, k); }, [&](int p, int k) { return v_at(i, p, k); });
+        }
+        lw_commit(B.done + 3, one);
+        int slot = 0, lap = 0;
+        for (int g = 0; ok && g < 2 * stages; ++g) {
+            if (lap && !mbar_wait(B.free + slot, (lap - 1) & 1, gave_up, A.status, 66)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            lw_mma(tmem + 128 + slot * 128, k_at(g >> 1, 0, g & 1), v_at(g >> 1, 0, g & 1), idesc, 0u, one);
+            lw_commit(B.done + slot, one);
+            if (++slot == 3) { slot = 0; ++lap; }
         }
     } else {
         constexpr int KN = 32 * DP / 8, VN = 32 * CB / 8, KPER = (KN + LW_WORK - 1) / LW_WORK, VPER = (VN + LW_WORK - 1) / LW_WORK;      // pieces of eight a stage, a thread
@@ -956,15 +998,25 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_local_kernel(const LinearChu
         float sum[HC];
 #pragma unroll
         for (int c = 0; c < HC; ++c) sum[c] = 0.f;
+        const uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + share * HC;
+        mbar_wait(B.done + 3, 0, gave_up, A.status, 62);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        lw_add_one(sum, at);
+        int slot = 0, lap = 0;
 #pragma unroll 1
-        for (int g = 0; g < 3 * stages; ++g) {
-            mbar_wait(B.done + (g & 3), (g >> 2) & 1, gave_up, A.status, 62);
+        for (int g = 0; g < 2 * stages; ++g) {
+            if (!GATED && g == 4) {                      // like terms: the first 64 tokens' sum waits in tensor memory for the others' (gated, the later
+                lw_put(sum, at);                         // terms are the large ones)
+#pragma unroll
+                for (int c = 0; c < HC; ++c) sum[c] = 0.f;
+            }
+            mbar_wait(B.done + slot, lap & 1, gave_up, A.status, 62);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            lw_add(sum, tmem + ((uint32_t)(quarter * 32) << 16) + (g & 3) * 128 + share * HC);
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(B.free + (g & 3));
+            lw_add_one(sum, at + 128 + slot * 128);
+            lw_taken(B.free + slot, lane);
+            if (++slot == 3) { slot = 0; ++lap; }
         }
+        if (!GATED && stages > 2) lw_add_one(sum, at);
         lw_store<CB>(reinterpret_cast<float*>(vs), sum, to + col0, A.dv, d, A.dv - col0, nullptr, nullptr);      // (V is read)
     }
     lw_end(B, warp, tmem);
@@ -1063,23 +1115,33 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 4) << 24);
         const uint32_t one = lw_elect(), qa = smem_addr(qs), ka = smem_addr(ks);
         auto kmajor = [&](uint32_t tile, int k) { return tile + (k >> 2) * C * 128 + (k & 3) * 32; };       // k in steps of 16
-#pragma unroll
-        for (int i = 0; i < GROUPS; ++i)
-            lw_parts(tmem + i * 128, idesc | ((uint32_t)(C >> 3) << 17), one, [&](int p, int k) { return desc_kmajor(kmajor(qa + p * PQ, 2 * i + k)); },
-                     [&](int p, int k) { return desc_kmajor(kmajor(ka + p * PQ, 2 * i + k)); });
-        lw_commit(&B.qk, one);
-        uint32_t slot = 0;
+        int turn = 0;
+        auto products = [&](bool more, uint32_t kind, auto a, auto b) {  // of 32 k; a new sum starts once the one before has been read
+            auto freed = [&]() { return !turn || mbar_wait(B.free, (turn - 1) & 1, gave_up, A.status, 67); };
+            if (!more && !freed()) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            lw_small(tmem + 128, more, kind, one, a, b);
+            if (more && !freed()) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            lw_lead(tmem + 256, tmem + 384, kind, one, a, b);
+            lw_commit(B.done, one);
+            ++turn;
+            return true;
+        };
+        bool ok = true;
+#pragma unroll 1
+        for (int i = 0; ok && i < GROUPS; ++i)
+            ok = products(i > 0, idesc | ((uint32_t)(C >> 3) << 17), [&](int p, int k) { return desc_kmajor(kmajor(qa + p * PQ, 2 * i + k)); },
+                          [&](int p, int k) { return desc_kmajor(kmajor(ka + p * PQ, 2 * i + k)); });
         int group = 0;
-        for (int i = 0; i < stages; ++i) {
+#pragma unroll 1
+        for (int i = 0; ok && i < stages; ++i) {
             const bool values = i >= NT * GROUPS;
             if (!mbar_wait(B.full + (i & 3), (i >> 2) & 1, gave_up, A.status, 63)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = ka + (i & 3) * 3 * PS, at = kmajor(qa, 2 * group), part = values ? PP : PQ;
-            lw_parts(tmem + 128 + slot * 128, idesc | (1u << 16) | ((uint32_t)(CB >> 3) << 17), one,
-                     [&](int p, int k) { return desc_kmajor(at + p * part + k * 32); },
-                     [&](int p, int k) { return desc_mnmajor(st + p * PS + k * 16 * 128, 32 * 128); });
-            lw_commit(B.done + (i & 3), one);
-            slot = slot == 2 ? 0 : slot + 1;
+            ok = products(group > 0, idesc | (1u << 16) | ((uint32_t)(CB >> 3) << 17), [&](int p, int k) { return desc_kmajor(at + p * part + k * 32); },
+                          [&](int p, int k) { return desc_mnmajor(st + p * PS + k * 16 * 128, 32 * 128); });
             group = group + 1 == (values ? nv : GROUPS) ? 0 : group + 1;
         }
     } else {
@@ -1088,16 +1150,16 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
         const int quarter = warp & 3, share = warp >> 2, t = quarter * 32 + lane;
         const uint32_t acc = tmem + ((uint32_t)(quarter * 32) << 16);
         const int r = tid / (CB / 8), col = tid % (CB / 8) * 8;
-        float ahead[2][8];
+        float ahead[8];
         // 32 rows of S, then of V, tile after tile; zeros where there are none.  A cursor over the stages: the next one's first row and tile.
         const float* from_s = start + (size_t)r * A.dv + col0 + col;
         const float* from_v = A.v + (size_t)(t0 + r) * A.v_stride + h * A.dv + col0 + col;
         int next_row = r, next_col = col0 + col;
         bool values = false;
-        auto fetch = [&](float (&y)[8]) {
+        auto fetch = [&]() {
             const int z = next_col - col0 - col, rows = values ? n : d;
             const float* from = values ? from_v + (size_t)(next_row - r) * A.v_stride + z : from_s + (size_t)(next_row - r) * A.dv + z;
-            if (SN % LW_WORK == 0 || tid < SN) lw_get8(y, from, next_row < rows, A.dv - next_col);
+            if (SN % LW_WORK == 0 || tid < SN) lw_get8(ahead, from, next_row < rows, A.dv - next_col);
             next_row += 32;
             if (next_row - r >= (values ? 32 * nv : DP)) {
                 next_row = r;
@@ -1105,24 +1167,21 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
                 if (next_col - col0 >= NT * CB) { next_col = col0 + col; values = true; }
             }
         };
-        fetch(ahead[0]);
-        fetch(ahead[1]);
-        mbar_wait(&B.qk, 0, gave_up, A.status, 64);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        fetch();
         const bool sees = share <= quarter;              // keys behind all of the warp's tokens weigh nothing
-        if (sees) {                                      // Q K^T into the first accumulator, so that the others are free for the stages
+        {                                                // Q K^T, into the fourth accumulator; all of it is there before the ring takes K's place
+            float qk[32] = {};
 #pragma unroll 1
-            for (int c = 32 * share; c < 32 * share + 32; c += 16) {
-                float v[16], r[16];
-                lw_ld16(acc + c, v);
-#pragma unroll
-                for (int i = 1; i < GROUPS; ++i) {
-                    lw_ld16(acc + i * 128 + c, r);
-#pragma unroll
-                    for (int x = 0; x < 16; ++x) v[x] += r[x];
+            for (int i = 0; i < GROUPS; ++i) {
+                mbar_wait(B.done, i & 1, gave_up, A.status, 64);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (sees) {
+                    lw_add(qk, acc + 256 + 32 * share, acc + 384 + 32 * share);
+                    if (i + 1 == GROUPS) lw_end_sum(qk, acc + 128 + 32 * share, 1.0f);
                 }
-                lw_st16(acc + c, v);
+                lw_taken(B.free, lane);
             }
+            if (sees) lw_put(qk, acc + 32 * share);
         }
         float sum[NT][HC];
 #pragma unroll
@@ -1130,25 +1189,26 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
 #pragma unroll
             for (int c = 0; c < HC; ++c) sum[z][c] = 0.f;
         int taken = 0, tile = 0, group = 0;
-        uint32_t from = acc + 128 + share * HC;
-        auto take = [&](int below) {                     // the accumulators of the stages below
+        const float weight = coef[t];                    // the token's, of the chunk's start state
+        auto take = [&](int below) {                     // the accumulators of the stages below (GROUPS is even: a stage's parity is its own)
+            static_assert(GROUPS % 2 == 0, "parity of the stages");
 #pragma unroll 1
             for (; taken < below; ++taken) {
-                mbar_wait(B.done + (taken & 3), (taken >> 2) & 1, gave_up, A.status, 65);
+                mbar_wait(B.done, taken & 1, gave_up, A.status, 65);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t at = acc + share * HC;
+                const bool states = taken < NT * GROUPS, last = ++group == (states ? GROUPS : nv);
 #pragma unroll
-                for (int z = 0; z < NT; ++z) if (tile == z) lw_add(sum[z], from);
-                from = from == acc + 384 + share * HC ? acc + 128 + share * HC : from + 128;
-                if (++group == (taken < NT * GROUPS ? GROUPS : nv)) { group = 0; tile = tile + 1 == NT ? 0 : tile + 1; }
+                for (int z = 0; z < NT; ++z) {
+                    if (tile != z) continue;
+                    lw_add(sum[z], at + 256, at + 384);
+                    if (last) lw_end_sum(sum[z], at + 128, states ? weight : 1.0f);
+                }
+                lw_taken(B.free, lane);
+                if (last) { group = 0; tile = tile + 1 == NT ? 0 : tile + 1; }
             }
         };
-        auto weigh = [&]() {                             // all of Q S is there: the token's weight; P takes Q's place
-            take(NT * GROUPS);
-            const float weight = coef[t];
-#pragma unroll
-            for (int z = 0; z < NT; ++z)
-#pragma unroll
-                for (int c = 0; c < HC; ++c) sum[z][c] *= weight;
+        auto weigh = [&]() {                             // all of Q S is there: P takes Q's place
             LwSum total;
             const int last = t < n ? t : -1;
 #pragma unroll 1
@@ -1180,20 +1240,16 @@ __global__ void __launch_bounds__(LW_THREADS, 1) lw_out_kernel(const LinearChunk
                 }
             }
         };
-        auto fill = [&](float (&y)[8], int i) {
-            take(i - 2);                                 // three accumulators: the stage three before has been read
-            if (!(SN % LW_WORK) || tid < SN) lw_put8(ks + (i & 3) * 3 * PS + swz(32, r, tid % (CB / 8)), PS, y);
-            lw_filled(B.full + (i & 3), lane);
-            if (i + 2 < stages) fetch(y);
-        };
-        static_assert(GROUPS % 2 == 0, "two stages at a time");
+        // Each part of this loop stands in it once (see above): a stage's accumulators are taken while the next stage's products run.
 #pragma unroll 1
-        for (int i = 0; i < stages; i += 2) {
+        for (int i = 0; i <= stages; ++i) {
+            take(i == NT * GROUPS || i == stages ? i : i - 1);
+            if (i == stages) break;
             if (i == NT * GROUPS) weigh();
-            fill(ahead[0], i);
-            if (i + 1 < stages) fill(ahead[1], i + 1);
+            if (!(SN % LW_WORK) || tid < SN) lw_put8(ks + (i & 3) * 3 * PS + swz(32, r, tid % (CB / 8)), PS, ahead);
+            lw_filled(B.full + (i & 3), lane);
+            if (i + 1 < stages) fetch();
         }
-        take(stages);
         // (the ring is read: its last sums have been taken; the barrier in there stands between den and its readers)
 #pragma unroll
         for (int z = 0; z < NT; ++z) {

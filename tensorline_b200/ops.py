@@ -852,12 +852,20 @@ LINEAR_CHUNKS_LEAST_TOKENS = 16
 
 # Heads of 33 to 128 rows run in chunks of 128 tokens on the 5th-generation tensor cores where a step has this many blocks of 64 tokens, a head and
 # 128 columns, by the rows of its heads (above 64 or not), and its requests fill the longer chunks (at most WIDE_CHUNKS_SHARE of the shorter
-# ones).  Chunks of 64 / 128, us: gated 8 heads of 128 x 256, 256 tokens (64 blocks) 52 / 52, 400 (112) 56 / 54, 1,024 (256) 71 / 58, 2,048
-# (512) 127 / 89; 4 heads of 128 x 128, 512 tokens (32) 50 / 50, 1,024 (64) 54 / 54, 2,048 (128) 62 / 56; 8 of 64 x 256, 512 tokens (128)
-# 42 / 46, 1,024 (256) 54 / 50; 8 requests of 20 beside 600 tokens, 8 heads of 128 x 256 101 / 103, of 64 x 256 66 / 77 (42 / 46 and
-# these two with end states that took 2 to 4 us less).
-WIDE_CHUNKS_BLOCKS = {False: 200, True: 96}
+# ones).  Chunks of 64 / 128, us: gated, 8 heads of 128 x 256, 300 tokens (80 blocks) 51 / 55, 640 (160) 66 / 54, 1,024 71 / 56, 2,048 124 / 85; of 128 x
+# 128, 1,024 tokens (128) 56 / 54, of 96 x 128 53 / 54, 1,280 (160) 65 / 55; fixed decay, 8 of 128 x 256, 2,048 101 / 70, of 128 x 128, 1,024 (128) 41 / 44; 8 requests
+# of 20 beside 600 tokens 98 / 103.  The longer chunks' blocks are one an SM, and those of up to 64 rows or up to 64 columns have half the work: not
+# where a second round of them has less than about a third (16 heads of 64 x 128, gated, 1,024 tokens, 128 of them, 53 / 50, 1,280 (160) 72 / 76, 1,536 (192) 74 /
+# 77, 2,048 (256) 89 / 81; 16 of 128 x 64, 1,280 76 / 78, 2,048 93 / 83), and with both never (16 of 64 x 64, 1,280 60 / 70, 2,048 71 / 72).
+WIDE_CHUNKS_BLOCKS = {False: 200, True: 160}
 WIDE_CHUNKS_SHARE = 0.65
+WIDE_CHUNKS_ROUND = 1.35
+
+
+def _wide_fills(H: int, d: int, dv: int, tall: int) -> bool:
+    if d <= 64 and dv <= 64:
+        return False
+    return (d > 64 and dv > 64) or not num_sms() < tall * H * -(-dv // 128) < WIDE_CHUNKS_ROUND * num_sms()
 
 
 def _wide_chunks(ctx, least: int, H: int, d: int, dv: int) -> bool:
@@ -870,7 +878,7 @@ def _wide_chunks(ctx, least: int, H: int, d: int, dv: int) -> bool:
         long = [n for n in (b - a for a, b in zip(ctx.h_q_start, ctx.h_q_start[1:])) if n >= least]
         ctx.scratch[key] = sum(-(-n // narrow) for n in long), sum(-(-n // wide) for n in long)
     short, tall = ctx.scratch[key]
-    return short * H * -(-dv // 128) >= WIDE_CHUNKS_BLOCKS[d > 64] and tall <= WIDE_CHUNKS_SHARE * short
+    return short * H * -(-dv // 128) >= WIDE_CHUNKS_BLOCKS[d > 64] and tall <= WIDE_CHUNKS_SHARE * short and _wide_fills(H, d, dv, tall)
 
 
 def takes_linear_chunks(proj: torch.Tensor, d: int, dv: int, max_q_len: int, gated: bool) -> bool:

@@ -15,6 +15,7 @@ def wide(monkeypatch):
     from tensorline_b200 import ops
     monkeypatch.setattr(ops, "WIDE_CHUNKS_BLOCKS", {False: 0, True: 0})
     monkeypatch.setattr(ops, "WIDE_CHUNKS_SHARE", 1.0)
+    monkeypatch.setattr(ops, "_wide_fills", lambda *a: True)
     yield
     ops.check_device_status()
 
@@ -139,3 +140,25 @@ def test_a_weight_is_one_exponential(monkeypatch):
     monkeypatch.setattr(ops, "WIDE_CHUNKS_BLOCKS", {False: 1 << 40, True: 1 << 40})
     narrow = both(proj, H, d, dv, None, decay)[0][0]
     assert float((wide[32:, :, 0] == narrow[32:, :, 0]).float().mean()) >= 0.99
+
+
+@pytest.mark.parametrize("gated,H,d,dv,T", [(True, 8, 128, 256, 256), (True, 8, 64, 128, 300), (False, 8, 128, 256, 300), (False, 16, 64, 64, 512)])
+def test_errors_are_no_larger_than_in_chunks_of_64(gated, H, d, dv, T, monkeypatch):
+    """Sizes and distributions as the decoders have them, from a state of zero, against 64 bits: outputs (a token's and a head's error, the
+    median of all) and states.  1.02: what is left of draws of this size."""
+    from tensorline_b200 import ops
+    g = torch.Generator().manual_seed(T)
+    proj = torch.randn(T, 2 * H * d + H * dv, generator=g) * 0.9
+    gates = torch.cat([torch.randn(T, H, generator=g) * 1.3 - 2, torch.randn(T, H, generator=g) * 1.3 + 3], dim=1) if gated else None
+    decay = None if gated else torch.tensor([1.0 - 2.0 ** (-5 - 5 * i / (H - 1)) for i in range(H)])
+    zero = torch.zeros(H, d, dv, dtype=torch.float64)
+    o, S, n, m, _ = chunks.recurrence(proj.double(), gates.double() if gated else None, decay, H, d, dv, zero, zero[:, :, 0] if gated else None,
+                                      zero[:, 0, 0] if gated else None, torch.arange(T), None, 0, False, 15.0, d ** -0.5, 1.0, 1e-6)
+    o, S = o.view(T, H, dv), chunks.slot_rows(S, n, m)
+    errors = []
+    for least in (0, 1 << 40):
+        monkeypatch.setattr(ops, "WIDE_CHUNKS_BLOCKS", {False: least, True: least})
+        out, state = both(proj, H, d, dv, gates, decay, d ** -0.5)[0]
+        errors.append((float(((out.double().cpu() - o).norm(dim=-1) / o.norm(dim=-1)).median()), float((state[0].double().cpu() - S).norm() / S.norm())))
+    for err, base in zip(*errors):
+        assert err <= 1.02 * base, errors
