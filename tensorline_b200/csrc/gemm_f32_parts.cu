@@ -28,7 +28,8 @@ constexpr int GP_CHUNK = 64;                             // k a chunk: 64 bfloat
 constexpr int GP_SEG = 16, GP_GROUP = 64;                // chunks a segment, a group
 constexpr int GP_THREADS = 320;                          // warp 0: TMA, warp 1: tensor memory + MMA, warps 2..9: sums
 constexpr int GP_W_BYTES = GP_ROWS * GP_CHUNK * 2;
-constexpr int GP_SLAB = 2048;                            // rows of A at a time: bounds the scratch
+constexpr int GP_SLAB = 2048;                            // rows of A at a time, at most: bounds the scratch for their parts
+constexpr long long GP_SUMS = 256LL << 20;               // bytes of the items' sums, at most: bounds the rows at a time as well (parts_rows)
 
 template <int BN> struct PartsShape {
     static constexpr int B_BYTES = (BN / 2) * GP_CHUNK * 2;              // a block's half of one part of the tokens
@@ -390,6 +391,7 @@ PartsPlan parts_plan(int M, int N, int K) {
     for (int bn : GP_WIDTHS)
         for (int len : {GP_SEG, GP_GROUP}) {
             const long long t_tiles = (M + bn - 1) / bn, k_parts = (chunks + len - 1) / len, items = t_tiles * m_tiles * k_parts;
+            if (len == GP_SEG && k_parts > 1 && 4 * k_parts * M * N > GP_SUMS) continue;
             const long long rounds = (items + pairs - 1) / pairs, most = chunks < len ? chunks : len;
             const double hbm = 700.0 * (items < pairs ? (double)items / pairs : 1.0) / t_tiles, mma = 6.0 * bn, smem = 512.0 + 3.0 * bn;
             double c = mma > smem ? mma : smem;
@@ -399,6 +401,15 @@ PartsPlan parts_plan(int M, int N, int K) {
             if (cycles < best.cycles) best = PartsPlan{bn, len, (int)k_parts, cycles};
         }
     return best;
+}
+// Rows of A at a time: the sums of items of a group fit in GP_SUMS (152,064 outputs of K 5,120: 176 rows; a product of 2,048 rows would need
+// 2.5 GB), whole tiles of the widest kind, or of the narrowest.  A row's floats do not depend on them.
+int parts_rows(int N, int K) {
+    const long long groups = (K + GP_CHUNK * GP_GROUP - 1) / (GP_CHUNK * GP_GROUP);
+    if (groups == 1) return GP_SLAB;
+    const long long rows = GP_SUMS / (4 * groups * N);
+    const int widest = GP_WIDTHS[4], narrowest = GP_WIDTHS[0];
+    return rows >= GP_SLAB ? GP_SLAB : rows >= widest ? (int)(rows / widest) * widest : rows >= narrowest ? (int)(rows / narrowest) * narrowest : narrowest;
 }
 bool parts_takes(const void* A, int lda, const void* W, int N, int K) {
     // Whether a product comes here depends on the weights' size and the rows' alignment alone, never on M: a row's floats do not change
@@ -429,13 +440,22 @@ int parts_launch(const CUtensorMap& mw, const bf16* P, const PartsArgs& G, cudaS
 TL_EXPORT int tl_gemm_f32_parts_scratch(const float* A, int lda, const void* W, int M, int N, int K) {
     if (M <= 0 || N <= 0 || !parts_takes(A, lda, W, N, K)) return 0;
     size_t most = 0;
-    for (int m : {M < GP_SLAB ? M : GP_SLAB, M % GP_SLAB}) {             // whole slabs and the last one
+    const int rows = parts_rows(N, K);
+    for (int m : {M < rows ? M : rows, M % rows}) {      // whole slabs and the last one
         if (m == 0) continue;
         const PartsPlan p = parts_plan(m, N, K);
         const size_t b = parts_bytes(K, m) + (p.k_parts > 1 ? (size_t)p.k_parts * m * N * sizeof(float) : 0);
         if (b > most) most = b;
     }
     return (int)((most + 255) / 256);
+}
+
+// How many kernels the function below launches.
+TL_EXPORT int tl_gemm_f32_parts_launches(int M, int N, int K) {
+    int n = 0;
+    const int rows = parts_rows(N, K);
+    for (int m0 = 0; m0 < M; m0 += rows) n += parts_plan(M - m0 < rows ? M - m0 : rows, N, K).k_parts > 1 ? 3 : 2;
+    return n;
 }
 
 // C = A W^T (+ bias), W and bias bfloat16.  `scratch`: as much as the function above says, 256-byte aligned; `status`: device int.
@@ -448,8 +468,9 @@ TL_EXPORT int tl_gemm_f32_parts(const float* A, int lda, const void* W, const vo
     CUtensorMap mw;
     if ((e = pair_map(&mw, W, N, K, GP_ROWS))) return e;
     const long long cap = (long long)tl_num_sms() * 8;
-    for (int m0 = 0; m0 < M; m0 += GP_SLAB) {
-        const int m = M - m0 < GP_SLAB ? M - m0 : GP_SLAB;
+    const int rows = parts_rows(N, K);
+    for (int m0 = 0; m0 < M; m0 += rows) {
+        const int m = M - m0 < rows ? M - m0 : rows;
         const PartsPlan plan = parts_plan(m, N, K);
         bf16* P = (bf16*)scratch;
         float* partial = plan.k_parts > 1 ? (float*)((unsigned char*)scratch + parts_bytes(K, m)) : nullptr;

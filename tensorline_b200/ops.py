@@ -9,6 +9,7 @@ from __future__ import annotations
 import array
 import collections
 import ctypes
+import functools
 from types import SimpleNamespace
 
 import numpy as np
@@ -35,6 +36,7 @@ _SIGNATURES = {
     "tl_attn_rows": [_P, _I, _P, _P, _P, _P, _I, _I, _P, _P, _I, _I, _I, _I, _I, _F, _P, _I, _P, _I, _P, _F, _P, _I, _I, _I, _P, _P],
     "tl_gemm_f32": [_P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _I, _P],
     "tl_gemm_f32_parts_scratch": [_P, _I, _P, _I, _I, _I],
+    "tl_gemm_f32_parts_launches": [_I, _I, _I],
     "tl_gemm_f32_parts": [_P, _I, _P, _P, _P, _I, _I, _I, _I, _P, _P, _P],
     "tl_argmax": [_P, _I, _I, _I, _P, _P, _P],
     "tl_sample": [_P, _I, _I, _I, _P, _P, _P, _P, _P],
@@ -716,6 +718,11 @@ def _sink(sink, nq: int, who: str) -> None:
         raise KernelError(f"{who}: sink must be float32 [query heads]")
 
 
+@functools.lru_cache(maxsize=4096)
+def _parts_launches(M: int, N: int, K: int) -> int:
+    return core().tl_gemm_f32_parts_launches(M, N, K)
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None) -> None:
     """out[M, N] = a[M, K] w[N, K]^T (+ bias) in float32; w float32 or bfloat16 (widened).  A row's result does not depend on the other
     rows.  Large matrices of bfloat16 weights: the tensor cores on the three bfloat16 parts of a's values (`gemm_f32_parts.cu`); the
@@ -733,11 +740,9 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Te
         blocks = core().tl_gemm_f32_parts_scratch(_ptr(a), a.stride(0), _ptr(w), M, N, K)
         if blocks:
             scratch = torch.empty(blocks * 256, dtype=torch.uint8, device=a.device)
-            slabs = -(-M // 2048)
-            split = blocks * 256 >= 6 * min(M, 2048) * K + 256 + 4 * min(M, 2048) * N      # sums along K of their own
             _check(core().tl_gemm_f32_parts(_ptr(a), a.stride(0), _ptr(w), _ptr(bias), _ptr(out), out.stride(0), M, N, K,
                                             scratch.data_ptr(), _ptr(device_status(a.device)), _stream()),
-                   "gemm_f32_parts", launches=slabs * (3 if split else 2))
+                   "gemm_f32_parts", launches=_parts_launches(M, N, K))
             return
     _check(core().tl_gemm_f32(_ptr(a), a.stride(0), _ptr(w), K, dtype_code(w.dtype), _ptr(bias), _ptr(out),
                               out.stride(0), M, N, K, _stream()), "gemm_f32")

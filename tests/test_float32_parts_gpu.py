@@ -81,3 +81,22 @@ def test_infinite_weights(ops):
         rest = [n for n in range(N) if n not in rows]
         assert torch.equal(got[:, rest], clean[:, rest])
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(2048, 152064, 5120), (2048, 37888, 18944), (700, 152064, 8192), (1, 152064, 18944), (2048, 3584, 18944)])
+def test_the_scratch_has_a_bound(ops, M, N, K):
+    """The parts of 2,048 rows, and sums along K in pieces only as far as they are small."""
+    a = torch.zeros(256, device="cuda")
+    blocks = ops.core().tl_gemm_f32_parts_scratch(a.data_ptr(), K, a.data_ptr(), M, N, K)
+    assert 0 < blocks * 256 <= 6 * 2048 * K + 256 + (256 << 20)
+
+
+@pytest.mark.parametrize("N,K", [(16640, 4104), (152064, 4104)])
+def test_rows_in_slabs_have_the_same_floats(ops, N, K):
+    """So many outputs that the sums along K of all rows would be more than the scratch may hold: 1,936 and 176 rows at a time."""
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(2048 if N < 20000 else 400, K, generator=g).cuda(), torch.randn(N, K, generator=g, dtype=torch.bfloat16).cuda()
+    whole = product(ops, a, w)
+    for lo, n in ((0, 33), (100, 128), (a.shape[0] - 148, 148)):
+        assert torch.equal(product(ops, a[lo:lo + n], w), whole[lo:lo + n]), n
+    ops.check_device_status()
