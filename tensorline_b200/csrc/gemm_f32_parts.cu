@@ -414,7 +414,7 @@ int parts_rows(int N, int K) {
 bool parts_takes(const void* A, int lda, const void* W, int N, int K) {
     // Whether a product comes here depends on the weights' size and the rows' alignment alone, never on M: a row's floats do not change
     // with the step it is in.  Smaller matrices (N 2,048, K 512: 4 rows 13 us against 8 as chains, 336 rows 15 against 37) are two or
-    // three launches instead of one for single tokens and are left to the chains.
+    // three launches instead of one for single tokens and are left to the chains (so are longer rows up to where the caller draws its line).
     return K % 8 == 0 && K >= 1024 && (long long)N * K >= (1 << 20) && lda % 4 == 0 && ((((uintptr_t)A) | ((uintptr_t)W)) & 15) == 0;
 }
 size_t parts_bytes(int K, int m) { return ((size_t)3 * m * K * sizeof(bf16) + 255) & ~(size_t)255; }

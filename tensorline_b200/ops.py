@@ -723,6 +723,12 @@ def _parts_launches(M: int, N: int, K: int) -> int:
     return core().tl_gemm_f32_parts_launches(M, N, K)
 
 
+# Rows of this many bfloat16 weights on go to the tensor cores.  Two or three launches there, one as chains, whose time grows with K: K 1,024,
+# 1,024 to 4,096 outputs, 4 rows 7.6 us as chains, 10.8 as parts, 64 rows 27 and 11; K 2,048, 2,048 outputs 13.4 and 12.6, 52 and 12.8.  A question of
+# the weights alone, so that a row's floats do not change with the step it is in.
+PARTS_LEAST_K = 2048
+
+
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Tensor | None = None) -> None:
     """out[M, N] = a[M, K] w[N, K]^T (+ bias) in float32; w float32 or bfloat16 (widened).  A row's result does not depend on the other
     rows.  Large matrices of bfloat16 weights: the tensor cores on the three bfloat16 parts of a's values (`gemm_f32_parts.cu`); the
@@ -736,7 +742,7 @@ def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: torch.Te
     _contig(w, "w")
     if bias is not None and bias.dtype != w.dtype:
         raise KernelError("gemm_f32: bias must have w's type")
-    if w.dtype == torch.bfloat16:
+    if w.dtype == torch.bfloat16 and K >= PARTS_LEAST_K:
         blocks = core().tl_gemm_f32_parts_scratch(_ptr(a), a.stride(0), _ptr(w), M, N, K)
         if blocks:
             scratch = torch.empty(blocks * 256, dtype=torch.uint8, device=a.device)

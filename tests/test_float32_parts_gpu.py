@@ -100,3 +100,12 @@ def test_rows_in_slabs_have_the_same_floats(ops, N, K):
     for lo, n in ((0, 33), (100, 128), (a.shape[0] - 148, 148)):
         assert torch.equal(product(ops, a[lo:lo + n], w), whole[lo:lo + n]), n
     ops.check_device_status()
+
+
+@pytest.mark.parametrize("N,K", [(2048, 1024), (1029, 2040)])
+def test_short_rows_of_weights_are_chains(ops, N, K):
+    """One launch there, two or three here: a few rows were slower.  The floats of the widened weights' chains."""
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(40, K, generator=g).cuda(), torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    for n in (1, 4, 40):
+        assert torch.equal(product(ops, a[:n], w), product(ops, a[:n], w.float()))
