@@ -48,12 +48,16 @@ STREAM_MAX_TOKENS = int(os.environ.get("TENSORLINE_B200_MOE_STREAM_MAX_TOKENS", 
 # 2,048 x 1,024, gated, 4 of 32 a token, streamed / sorted: 12 tokens 101 / 104 us, 16 115 / 115, 32 182 / 117; 2 of 8: 8 tokens
 # 43 / 45, 12 55 / 45, 32 111 / 47; 1,024 x 512, 4 of 32: 16 tokens 41 / 47, 24 53 / 47, 32 61 / 47.
 SORT_MIN_BYTES, SORT_SHARE = 140e6, 0.4
+# Captured steps of more tokens sort from fewer bytes on.  2 of 8 experts of 256 x 192, 33 tokens (17 MB more than once) 14 / 19, 64 (35) 18.3 / 19.3, 128 (73) 28.6 / 19.9;
+# of 512 x 512, 33 (91) 24 / 22; 1 of 64 of 1,024 x 512, 33 (22) 36 / 35, 64 (73) 60 / 47; 8 of 256 of 2,048 x 512, 33 (617) 205 / 206, 64 (1,890) 343 / 260.
+SORT_MIN_BYTES_LONG = 40e6
 
 
 def sort_pays(tokens: int, top: int, experts: int, expert_bytes: int) -> bool:
-    """Whether a step of few tokens moves enough bytes more than once to be sorted."""
+    """Whether a step that could be streamed moves enough bytes more than once to be sorted."""
     chosen = experts * (1.0 - (1.0 - top / experts) ** tokens)               # experts that some token chose, on average
-    return (tokens * top - chosen) * expert_bytes >= SORT_MIN_BYTES + SORT_SHARE * chosen * expert_bytes
+    again = (tokens * top - chosen) * expert_bytes
+    return again >= (SORT_MIN_BYTES + SORT_SHARE * chosen * expert_bytes if tokens <= STREAM_MAX_TOKENS else SORT_MIN_BYTES_LONG)
 
 
 @register_feed_forward("routed_experts")
@@ -168,7 +172,7 @@ class RoutedExperts(Part):
         # the sort takes
         if takes and few and (on_input or not ops.moe_sort_takes(E)):
             takes = False
-        elif takes and T <= STREAM_MAX_TOKENS:
+        elif takes and few:
             takes = sort_pays(T, top, E, 2 * (self.w_up[0].numel() + self.w_down[0].numel()))
         if self.rt.exact or (few and not takes):
             a = torch.empty((T * top, self.inner), dtype=h.dtype, device=h.device)

@@ -142,8 +142,10 @@ def test_captured_steps_take_every_router(ops, more, tokens, monkeypatch):
     part = routed(256, 64, gated=True, activation="silu", **more)
     h = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
     monkeypatch.setattr(moe, "SORT_MIN_BYTES", -1e12)
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES_LONG", -1e12)
     y = captured(part, h)
     monkeypatch.setattr(moe, "SORT_MIN_BYTES", 1e12)
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES_LONG", 1e12)
     streamed = captured(part, h)
     ops.check_device_status()
     assert float((y.float() - streamed.float()).norm() / streamed.float().norm()) <= 2.0 ** -9
@@ -156,6 +158,7 @@ def test_gates_that_the_sorted_products_do_not_have(ops, monkeypatch):
     part = routed(256, 64, experts=8, top=2, gated=True, activation="relu_squared")
     h = torch.randn(77, 256, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16).cuda()
     monkeypatch.setattr(moe, "SORT_MIN_BYTES", -1e12)
+    monkeypatch.setattr(moe, "SORT_MIN_BYTES_LONG", -1e12)
     z = h.float() @ part.w_router.float().T
     wts, idx = z.topk(2, dim=1)
     wts = wts.softmax(dim=1)
@@ -185,3 +188,14 @@ def test_far_gates_of_few_tokens_are_divided_exactly(ops, act):
     z = x[:, 0].double()
     want = (z / (1.0 + torch.exp(-z)) * (2.0 ** 100 + (1.0 if clamped else 0.0)))[:, None]
     assert float(((out.double() - want).abs() / want.abs()).max()) <= 2.0 ** -7
+
+
+@pytest.mark.parametrize("tokens,inner,sorts", [(40, 64, False), (64, 64, False), (64, 1024, True)])
+def test_captured_steps_over_small_experts_are_streamed(ops, tokens, inner, sorts, monkeypatch):
+    """Above STREAM_MAX_TOKENS too a captured step is sorted only where that is the faster way."""
+    part = routed(256, inner, experts=8, top=2, gated=True, activation="silu")
+    h = torch.randn(tokens, 256, generator=torch.Generator().manual_seed(tokens)).to(torch.bfloat16).cuda()
+    calls, sort = [], ops.moe_sort
+    monkeypatch.setattr(ops, "moe_sort", lambda *a: calls.append(a) or sort(*a))
+    captured(part, h)
+    assert bool(calls) == sorts
