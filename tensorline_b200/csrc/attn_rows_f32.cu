@@ -71,8 +71,11 @@ constexpr int ROWS_MAX = 64;
 
 // NC: groups of 64 output columns (d <= 64 NC); ROWS: rows a block, RW: a warp
 template <int NC, int ROWS, int RW>
-__global__ void __launch_bounds__(ROWS / RW * 32) attn_rows_kernel(const RowsArgs A) {
+__global__ void __launch_bounds__(ROWS / RW * 32, NC == 1 && RW == 16 ? 4 : 0) attn_rows_kernel(const RowsArgs A) {
     constexpr int NT = ROWS / RW * 32, TK = NT / 32, ROWS_PS = ROWS + 4;                      // threads, and those that fetch a key
+    // Operands a step ahead of the multiply-adds: not in blocks of 64 rows of short heads, where four blocks an SM hide the latency (40 heads of 64 on
+    // 1, 4,096 tokens 4.73 ms; ahead 4.98, and ahead with the registers that leave three blocks 5.39)
+    constexpr bool AHEAD = NC > 1 || RW == 8;
     constexpr int LC = RW == 16 || NC == 1 ? 16 : 32, VR = RW * LC / 32, VC = 16 * NC / LC;      // values: lanes over columns, rows and column groups a lane
     extern __shared__ __align__(16) float sm[];
     const int d = A.d, g = A.nq / A.nkv, ld = d + 4;
@@ -169,15 +172,20 @@ __global__ void __launch_bounds__(ROWS / RW * 32) attn_rows_kernel(const RowsArg
                             s[i][j] = fmaf(x, c == 0 ? k4[b][j].x : c == 1 ? k4[b][j].y : c == 2 ? k4[b][j].z : k4[b][j].w, s[i][j]);
                     }
             };
-            load(0, 0);
-            int e = 0;
-            for (; e + 8 < d; e += 8) {
-                load(1, e + 4);
-                dots(0);
-                load(0, e + 8);
-                dots(1);
+            if constexpr (AHEAD) {
+                load(0, 0);
+                int e = 0;
+                for (; e + 8 < d; e += 8) {
+                    load(1, e + 4);
+                    dots(0);
+                    load(0, e + 8);
+                    dots(1);
+                }
+                if (e + 4 < d) { load(1, e + 4); dots(0); dots(1); } else dots(0);
+            } else {
+#pragma unroll 2
+                for (int e = 0; e < d; e += 4) { load(0, e); dots(0); }
             }
-            if (e + 4 < d) { load(1, e + 4); dots(0); dots(1); } else dots(0);
 #pragma unroll
             for (int i = 0; i < RW / 4; ++i)
 #pragma unroll
@@ -260,7 +268,10 @@ __global__ void __launch_bounds__(ROWS / RW * 32) attn_rows_kernel(const RowsArg
             };
             float pv[2][VR];
             float4 v[2][VC];
-            if (full && keys == 32) {
+            if (!AHEAD && full && keys == 32) {
+#pragma unroll 2
+                for (int k = 0; k < 32; ++k) { load(k, pv[0], v[0]); key(pv[0], v[0], true); }
+            } else if (full && keys == 32) {
                 load(0, pv[0], v[0]);
 #pragma unroll
                 for (int k = 0; k < 32; k += 2) {
@@ -503,8 +514,10 @@ TL_EXPORT int tl_attn_rows(const float* q, int q_stride, float* out, const float
     // Blocks of 64 rows, 16 a warp, where they are three an SM or more (2,048 tokens, 28 heads: 1,294 us against 1,430); else of 32
     // rows, 8 a warp: more of them, and a warp is done with a tile sooner (333 tokens on 700 cached: 254 us against 336; 100 on 300:
     // 158 against 293; 700 tokens, 40 heads, three an SM: 300 both).
+    // A block has at most 32 tokens: with one query head a KV head 64 rows would be half empty (32 heads of 64, 2,048 tokens: 1,548 us in such blocks, 834 in
+    // those of 32; of 128 2,445 and 1,455).
     const int tokens = ROWS_MAX / g < 32 ? ROWS_MAX / g : 32;
-    const bool wide = g > ROWS_MAX / 2 || (long long)((T + tokens - 1) / tokens) * nkv >= 3LL * tl_num_sms();
+    const bool wide = g > ROWS_MAX / 2 || (g > 1 && (long long)((T + tokens - 1) / tokens) * nkv >= 3LL * tl_num_sms());
 #define ROWS_GO(NC) (wide ? launch_rows<NC, ROWS_MAX, 16>(A, stream) : launch_rows<NC, ROWS_MAX / 2, 8>(A, stream))
     return d <= 64 ? ROWS_GO(1) : d <= 128 ? ROWS_GO(2) : ROWS_GO(4);
 #undef ROWS_GO

@@ -125,3 +125,22 @@ def test_dot_products_of_tables_longer_than_a_grid(ops, window):
         ops._ptr(q), nq * d, ops._ptr(outs[-1]), ops.dtype_code(q.dtype), ops._ptr(k), ops._ptr(v), ops._ptr(table), mp, ps, ops._ptr(pos), ops._ptr(slot),
         64, nq, nkv, d, window or 0, 0.125, None, 0, None, 0, None, 0.0, 2, k.shape[0], ops.fault_words(q.device), ops._stream()), "attn_tokenwise")
     assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+@pytest.mark.parametrize("nq,nkv,d,T", [(16, 8, 64, 1900), (32, 16, 20, 950), (40, 1, 64, 600), (16, 8, 128, 1900), (16, 16, 64, 950), (16, 16, 128, 950)])
+def test_prompts_in_blocks_of_either_size_have_the_token_wise_kernels_floats(ops, nq, nkv, d, T):
+    """Three blocks of 64 rows an SM and more, several query heads a KV head and one; two requests, the second on cached tokens."""
+    gen = torch.Generator().manual_seed(d + T)
+    ps, lens, cached = 16, [T - 70, 70], [0, 50]
+    mp = -(-T // ps)
+    table = torch.randperm(2 * mp, generator=gen).to(torch.int32).view(2, mp).cuda()
+    k, v = (torch.randn(2 * mp, nkv, ps, d, generator=gen).cuda() for _ in range(2))
+    pos = torch.tensor([c + i for n, c in zip(lens, cached) for i in range(n)], dtype=torch.int32).cuda()
+    slot = torch.tensor([b for b, n in enumerate(lens) for _ in range(n)], dtype=torch.int32).cuda()
+    q, out = torch.randn(T, nq * d, generator=gen).cuda(), torch.full((T, nq * d), 7.0, device="cuda")
+    ops.attn_tokenwise(q, nq * d, out, k, v, table, ps, pos, slot, nq, nkv, d, None, d ** -0.5)
+    want = torch.empty_like(out)
+    ops._check(ops.core().tl_attn_tokenwise(
+        ops._ptr(q), nq * d, ops._ptr(want), ops.dtype_code(q.dtype), ops._ptr(k), ops._ptr(v), ops._ptr(table), mp, ps, ops._ptr(pos), ops._ptr(slot), T, nq, nkv, d,
+        0, d ** -0.5, None, 0, None, 0, None, 0.0, 2, 2 * mp, ops.fault_words(q.device), ops._stream()), "attn_tokenwise")
+    assert torch.equal(out, want)
