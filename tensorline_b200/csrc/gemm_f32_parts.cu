@@ -55,7 +55,7 @@ struct PartsArgs {
 // Sums of parts that are no number: an infinite weight times a part that is zero is none, the float itself times it may be an infinity.
 // Outputs `at`, `at` + ld .. (rows m .. m + rows - 1 of A, row n of W) that are none are taken again as gemm_f32.cu takes them, in one
 // chain of multiply-adds.
-__device__ __noinline__ void gp_chains(const PartsArgs& G, const bf16* bias, int m, int rows, int n, float* at, size_t ld) {
+__device__ __forceinline__ void gp_chains(const PartsArgs& G, const bf16* bias, int m, int rows, int n, float* at, size_t ld) {
     for (int x0 = 0; x0 < rows; x0 += 8) {
         bool odd = false;
         for (int x = x0; x < min(rows, x0 + 8); ++x) odd = odd || at[x * ld] != at[x * ld];
@@ -78,6 +78,12 @@ __device__ __noinline__ void gp_chains(const PartsArgs& G, const bf16* bias, int
     }
 }
 
+// the largest of N sums and `w`, no number if one of them is none: an instruction for two
+template <int N> __device__ __forceinline__ float gp_worst(const float (&x)[N], float w) {
+#pragma unroll
+    for (int i = 0; i < N; i += 2) asm("max.NaN.f32 %0, %0, %1, %2;" : "+f"(w) : "f"(x[i]), "f"(x[i + 1 < N ? i + 1 : i]));
+    return w;
+}
 __device__ __forceinline__ void gp_ld8(uint32_t at, float* r) {
     uint32_t* u = reinterpret_cast<uint32_t*>(r);
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
@@ -210,6 +216,7 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         const uint32_t leader_empty = pair_peer(smem_addr(acc_empty), 0);
         int it = 0;
         bool ok = true;
+        float worst = 0.f;                               // no number if an output is none
         grid_dependency_wait();
         for (int i = pair; i < items && ok; i += pairs) {
             const Item t = item_at(i);
@@ -273,14 +280,18 @@ gemm_f32_parts_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 const size_t ld = G.partial ? G.N : G.ldo;
                 const float b = !G.partial && G.bias ? to_f<bf16>(G.bias[n]) : 0.f;
                 const bool add = !G.partial && G.bias;
-                float* at = dst;
-                bool odd = false;
 #pragma unroll
-                for (int x = 0; x < CW; ++x, at += ld)
-                    if (t0 + x < G.M) { *at = add ? seg[x] + b : seg[x]; odd = odd || seg[x] != seg[x]; }
-                if (odd && !G.partial) gp_chains(G, G.bias, t0, min(CW, G.M - t0), n, dst, ld);
+                for (int x = 0; x < CW; ++x, dst += ld)
+                    if (t0 + x < G.M) *dst = add ? seg[x] + b : seg[x];
+                worst = gp_worst(seg, worst);
             }
         }
+        if (worst != worst && ok && !G.partial)         // behind the loop, and inline: a call took 0.8 us of every launch for its stack
+            for (int i = pair; i < items; i += pairs) {
+                const Item t = item_at(i);
+                const int n = t.m * 2 * GP_ROWS + (int)rank * GP_ROWS + quarter * 32 + lane, t0 = t.t * BN + half * CW;
+                if (n < G.N && t0 < G.M) gp_chains(G, G.bias, t0, min(CW, G.M - t0), n, G.out + (size_t)t0 * G.ldo + n, G.ldo);
+            }
     }
     // ---------------------------------------------------------------- teardown
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -342,6 +353,7 @@ __global__ void __launch_bounds__(256) gemm_f32_sum_kernel(const PartsArgs G, co
     grid_dependency_trigger();
     const int nv = N / V;
     const size_t stride = (size_t)M * N;
+    float worst = 0.f;                                   // no number if a sum is none
     for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < (long long)M * nv; i += (long long)gridDim.x * 256) {
         const int m = (int)(i / nv), n = (int)(i - (long long)m * nv) * V;
         const float* src = partial + (size_t)m * N + n;
@@ -373,9 +385,13 @@ __global__ void __launch_bounds__(256) gemm_f32_sum_kernel(const PartsArgs G, co
         for (int x = 0; x < V; ++x) if (bias) total[x] += to_f<bf16>(bias[n + x]);
         if constexpr (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(total[0], total[1], total[2], total[3]);
         else dst[0] = total[0];
-#pragma unroll
-        for (int x = 0; x < V; ++x) if (total[x] != total[x]) gp_chains(G, bias, m, 1, n + x, dst + x, 0);
+        worst = gp_worst(total, worst);
     }
+    if (worst != worst)
+        for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < (long long)M * nv; i += (long long)gridDim.x * 256) {
+            const int m = (int)(i / nv), n = (int)(i - (long long)m * nv) * V;
+            for (int x = 0; x < V; ++x) gp_chains(G, bias, m, 1, n + x, out + (size_t)m * ldo + n + x, 0);
+        }
 }
 
 // ------------------------------------------------------------------ the plan
