@@ -109,3 +109,16 @@ def test_short_rows_of_weights_are_chains(ops, N, K):
     a, w = torch.randn(40, K, generator=g).cuda(), torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
     for n in (1, 4, 40):
         assert torch.equal(product(ops, a[:n], w), product(ops, a[:n], w.float()))
+
+
+@pytest.mark.parametrize("N,K", [(2048, 2048), (257, 4104), (300, 8200), (4608, 3584), (200, 18944)])
+def test_errors_are_those_of_three_parts(ops, N, K):
+    """In the norm: a chunk's cuts and the additions behind it come to less than 4e-7 of a sum of random signs (two parts only: 1e-5), and to
+    no more than what chains of multiply-adds on the same values are off by.  For every width of the tiles."""
+    g = torch.Generator().manual_seed(K)
+    a, w = torch.randn(353, K, generator=g).cuda(), torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    for n in (1, 32, 64, 96, 128, 176, 353):
+        want = a[:n].double() @ w.double().T
+        err, chains = (float((x.double() - want).norm() / want.norm()) for x in (product(ops, a[:n], w), product(ops, a[:n], w.float())))
+        assert err <= 4e-7 and err <= chains, (n, err, chains)
+    ops.check_device_status()
