@@ -1,6 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias) of the 32-bit engine for weights stored as bfloat16, on the tensor cores without giving up a
-// bit of an operand: a float is the sum of three bfloat16 parts (24 bits, cut off one after the other, so that the parts are
-// exact and none overflows), a product of a part and a weight is exact in float, and the sums are float.
+// bit of an operand of 2^-110 or more: a float is the sum of three bfloat16 parts (24 bits, cut off one after the other, so that
+// the parts are exact and none overflows), a product of a part and a weight is exact in float, and the sums are float.  Of smaller
+// operands what lies below 2^-133, the smallest bfloat16, is lost.  Outputs that come out as no number (an infinite weight times
+// a part that is zero is none) are taken again as chains.
 //
 // What a row's result is does not depend on the rows beside it, nor on how many there are: every output is
 //     sum over groups of 4,096 k ( sum over segments of 1,024 k ( sum over chunks of 64 k ( the tensor cores' sum of the chunk's products )))
@@ -15,10 +17,13 @@
 // into registers and add it to the segment's sum while the next is made; a group's sum waits in tensor memory.
 // What bounds it: with few tokens the weights from memory (a chunk of W takes an SM about 700 cycles at HBM's rate; the three
 // passes over it from shared memory take 512 + 3 BN), with many the tensor cores (6 BN cycles a chunk: 1,056 measured at BN 176).
+// 176 tokens are the widest tile whose copies still have four stages in shared memory (a stage of 181 would be a quarter of it), and a
+// group's sums in tensor memory beside two accumulators but for nine columns a warp.
 // Measured beside chains of float multiply-adds (gemm_f32.cu), us and error against 64 bits, norm over norm:
-//     N 37,888  K 3,584     336 rows 185 (2,108)   64 rows 69 (406)   4 rows 67 (80)    1.2e-7 (1.1e-6)
-//     N  3,584  K 18,944    336 rows 122 (1,714)   64 rows 50 (475)   4 rows 44 (113)   1.3e-7 (2.5e-6)
-//     N  1,024  K 1,024     336 rows  17 (47)      64 rows 15 (33)    4 rows 15 (12)    1.1e-7 (5.7e-7)
+//     N 37,888  K 3,584     336 rows 186 (2,101)   64 rows 60 (396)   4 rows 51 (72)    1.2e-7 (1.1e-6)
+//     N  3,584  K 18,944    336 rows 111 (1,703)   64 rows 41 (470)   4 rows 35 (109)   1.3e-7 (2.5e-6)
+//     N  2,048  K 2,048     336 rows  21 (116)     64 rows 13 (53)    4 rows 13 (14)    1.1e-7 (8.1e-7)
+//     N  1,024  K 1,024     336 rows  12 (43)      64 rows 11 (28)    4 rows 11 (8)     1.1e-7 (5.7e-7), so left to the chains (ops.py)
 #include "umma_pair.cuh"
 
 namespace {

@@ -14,7 +14,8 @@
 // Steps of many tokens: the pairs are sorted by expert on the device (moe_sort), the tokens' rows gathered in that
 // order, two products run over the experts' runs (moe_product.cu; where it does not take the sizes, batched products over runs of
 // `cap` rows each), and moe_combine sums each token's rows by weight.
-// Every output element is one fixed chain of additions, so a token's result does not depend on the step's other tokens.
+// Every output element is one fixed chain of additions within a route, so a token's result does not depend on the step's other
+// tokens but for the route, which their number chooses (parts/moe.py; the 32-bit engine streams always).
 #include "common.cuh"
 
 // dot product of a weight row with a float vector in shared memory, lanes striding; every lane gets the sum

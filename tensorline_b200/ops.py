@@ -182,6 +182,7 @@ STATUS_ROLES = {1: "tcgen05 product: the copy thread waited for a free stage", 2
                 61: "matrix memory's end states: the MMA warp waited for a stage", 62: "matrix memory's end states: the workers waited for a sum",
                 63: "matrix memory's outputs: the MMA warp waited for a stage", 64: "matrix memory's outputs: the workers waited for Q K",
                 65: "matrix memory's outputs: the workers waited for a sum", 66: "matrix memory's end states: the MMA warp waited for a free accumulator",
+                67: "matrix memory's outputs: the MMA warp waited for free accumulators",
                 20: "decode attention: a wait for a stage of keys and values"}
 
 

@@ -27,9 +27,10 @@ so many pairs that the same matrices would be streamed again and again, `sort_pa
 gather the tokens' rows in that order and run two products over the experts' runs (`ops.moe_product`, which reads the runs'
 bounds on the device).  Neither asks the host for anything, so both sit in a CUDA graph.  Rows that are no multiple of 16 bytes
 take two batched products of the library instead, every expert's run in `cap` rows of its own (the longest run, rounded up),
-which needs the bounds on the host; captured steps stream then.  The 32-bit
-engine streams always: a token's result is then the
-same chain of additions in every step, whatever else the step holds.
+which needs the bounds on the host; captured steps stream then, and where the sort does not take the router or the products
+not the gate.  A bfloat16 token's sums so depend on the number of tokens in its step (when decoding, on the batch's bucket), by
+their order.  The 32-bit engine streams always: a token's result is then the same chain of additions in every step,
+whatever else the step holds.
 """
 from __future__ import annotations
 
@@ -41,7 +42,7 @@ from .. import ops
 from .base import Part, Runtime, TensorSpec, register_feed_forward
 from .linear import resolve
 
-# up to this many tokens a step the experts are streamed pair by pair ...
+# up to this many tokens a step the experts are streamed pair by pair (more are sorted, but in captured steps, where the bytes below decide) ...
 STREAM_MAX_TOKENS = int(os.environ.get("TENSORLINE_B200_MOE_STREAM_MAX_TOKENS", 32))
 # ... as long as the pairs are not many more than the experts they chose: every pair brings its expert's matrices anew (from L2 at
 # about 10 TB/s), the products over sorted runs once, at 4.5 TB/s against 5.5, with 14 us of launches.  Experts of
